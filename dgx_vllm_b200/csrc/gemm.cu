@@ -812,7 +812,7 @@ EncodeTiledFn encode_fn() {
 // Encoded maps are remembered by their arguments (a weight is encoded once, not once per call).
 struct MapKey {
   const void* base;
-  uint64_t rows, row_bytes;
+  uint64_t rows, row_bytes, row_stride;
   uint32_t box_rows;
   int box_bytes;
 };
@@ -825,38 +825,22 @@ struct MapCache {
 };
 MapCache g_map_cache;
 
-bool make_map_uncached(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, int box_bytes);
-
-// [rows, row_bytes] u8 row-major; box = box_bytes (128/64/32) x box_rows with the matching swizzle, zero fill out of bounds
-bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, int box_bytes) {
-  const MapKey k{base, rows, row_bytes, box_rows, box_bytes};
-  const size_t h = (reinterpret_cast<uintptr_t>(base) >> 8) * 0x9E3779B97F4A7C15ull + rows * 31 + box_rows;
-  const int slot = (int)(h % MapCache::kSlots);
-  std::lock_guard<std::mutex> lock(g_map_cache.mu);
-  if (g_map_cache.used[slot] && memcmp(&g_map_cache.key[slot], &k, sizeof(MapKey)) == 0) {
-    *map = g_map_cache.map[slot];
-    return true;
-  }
-  if (!make_map_uncached(map, base, rows, row_bytes, box_rows, box_bytes)) return false;
-  memset(&g_map_cache.key[slot], 0, sizeof(MapKey));
-  g_map_cache.key[slot] = k;
-  g_map_cache.map[slot] = *map;
-  g_map_cache.used[slot] = true;
-  return true;
-}
-
-bool make_map_uncached(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, int box_bytes) {
+bool encode_rows_map(CUtensorMap* map, const MapKey& k) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {row_bytes};
-  cuuint32_t box[2] = {(cuuint32_t)box_bytes, box_rows};
-  const CUtensorMapSwizzle sw = box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                                : (box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+  cuuint64_t dims[2] = {k.row_bytes, k.rows};
+  cuuint64_t strides[1] = {k.row_stride};
+  cuuint32_t box[2] = {(cuuint32_t)k.box_bytes, k.box_rows};
+  const CUtensorMapSwizzle sw = k.box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                : (k.box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
   cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(k.base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, int box_bytes) {
+  return make_rows_map(map, base, rows, row_bytes, row_bytes, box_rows, box_bytes);
 }
 
 // [rows, cols] 16-bit row-major output; box = 64 columns (128 bytes) x 32 rows, 128-byte swizzle
@@ -871,6 +855,28 @@ bool make_out_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t co
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+}  // namespace
+
+bool make_rows_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t row_stride, uint32_t box_rows,
+                   int box_bytes) {
+  const MapKey k{base, rows, row_bytes, row_stride, box_rows, box_bytes};
+  const size_t h = (reinterpret_cast<uintptr_t>(base) >> 8) * 0x9E3779B97F4A7C15ull + rows * 31 + box_rows;
+  const int slot = (int)(h % MapCache::kSlots);
+  std::lock_guard<std::mutex> lock(g_map_cache.mu);
+  if (g_map_cache.used[slot] && memcmp(&g_map_cache.key[slot], &k, sizeof(MapKey)) == 0) {
+    *map = g_map_cache.map[slot];
+    return true;
+  }
+  if (!encode_rows_map(map, k)) return false;
+  memset(&g_map_cache.key[slot], 0, sizeof(MapKey));
+  g_map_cache.key[slot] = k;
+  g_map_cache.map[slot] = *map;
+  g_map_cache.used[slot] = true;
+  return true;
+}
+
+namespace {
 
 template <int BN, int KB, bool kGrouped, bool kSiluQuant = false>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int max_m_tiles, cudaStream_t st,

@@ -4,144 +4,295 @@
 // divided by their sum -- sparse_fp4_kernel/bench_moe_layer_e2e.py:230-236); here it is two small kernels whose
 // outputs (topk_weights f32, topk_ids i32) are exactly the device tensors the fused MoE layer and the expert-parallel
 // dispatch take, so no host round trip sits between the router and the experts.
-//   router_logits_kernel   block = 64 experts x 8 tokens; the tokens' activations sit in shared memory, every warp
-//                          streams whole weight rows (16-byte loads) and keeps 8 fp32 dot products per row
-//   router_topk_kernel     one warp per token: k rounds of warp-wide arg-max (ties -> lower expert id), weights
-//                          exp(l - max) normalised over the selected experts (or over all of them)
-#include "common.cuh"
+//   router_mma_kernel      small batches: 16 experts x up to 64 tokens per block, mma.sync, operands straight from global
+//                          memory into fragments; bound by latency, so K is split over warps and blocks until every
+//                          warp has about one round of loads (M=32, H=2048, E=512: 31 us with one dot product per warp and
+//                          weight row on 32 blocks)
+//   router_gemm_kernel     larger batches: 128 tokens x 128 or 256 experts per CTA on tcgen05 (kind::f16, fp32 accumulators
+//                          in tensor memory), operands by TMA; bound by L2 -> shared-memory bandwidth
+//   router_topk_kernel     one warp per token: adds the K-slices of its logits in a fixed order, then k rounds of warp-wide
+//                          arg-max (ties -> lower expert id), weights exp(l - max) normalised over the selected experts
+//                          (or over all of them)
+#include "sm100_ptx.cuh"
 
 namespace b200fp4 {
 namespace {
 
-constexpr int kRtTokens = 8;
-constexpr int kRtExperts = 64;
+// ------------------------------------------------------------------------------------------ projection, small batches
+
 constexpr int kRtThreads = 256;
+constexpr int kRtWarps = kRtThreads / 32;
+constexpr int kRtMaxTokens = 64;       // per block
 
 template <typename T>
-__device__ __forceinline__ void unpack8(const uint4& raw, float* v);
+__device__ __forceinline__ void mma_m16n8k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1);
 template <>
-__device__ __forceinline__ void unpack8<__nv_bfloat16>(const uint4& raw, float* v) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[2 * i] = __uint_as_float(w[i] << 16);
-    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
+__device__ __forceinline__ void mma_m16n8k16<__nv_bfloat16>(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                            uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 template <>
-__device__ __forceinline__ void unpack8<__half>(const uint4& raw, float* v) {
-  const __half2* h = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __half22float2(h[i]);
-    v[2 * i] = f.x;
-    v[2 * i + 1] = f.y;
-  }
+__device__ __forceinline__ void mma_m16n8k16<__half>(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                     uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <typename T>
+// parts[z][m][e] = sum over the k of slice z of hidden[m][k] * gate_w[e][k].
+// Block = experts [16 x, +16) x tokens [8 NT y, +8 NT), slice z of K; its warps take 64-wide pieces of K in turn.  In a 32-wide
+// step lane (g, t) = (lane / 4, lane % 4) loads the 8 elements at k = 8t of rows g and g + 8 (experts) and g (tokens): the
+// order of k inside a product sum is free, so elements 0-3 of the 8 serve as the lane's k of one mma and 4-7 as those of
+// another, on both sides alike.
+template <typename T, int NT>
 __global__ void __launch_bounds__(kRtThreads)
-    router_logits_kernel(const T* __restrict__ hidden, int64_t ld_h, const T* __restrict__ gate_w, int M, int H, int E,
-                         float* __restrict__ logits) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  T* sx = reinterpret_cast<T*>(smem);                     // [kRtTokens][H]
-  const int m0 = blockIdx.y * kRtTokens, e0 = blockIdx.x * kRtExperts;
-  const int chunks = H >> 3;
-  for (int i = threadIdx.x; i < kRtTokens * chunks; i += kRtThreads) {
-    const int tk = i / chunks, c = i - tk * chunks;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (m0 + tk < M) v = *reinterpret_cast<const uint4*>(hidden + (int64_t)(m0 + tk) * ld_h + c * 8);
-    reinterpret_cast<uint4*>(sx)[i] = v;
+    router_mma_kernel(const T* __restrict__ hidden, int64_t ld_h, const T* __restrict__ gate_w, int M, int H, int E,
+                      int* __restrict__ status, float* __restrict__ parts) {
+  __shared__ float s_part[kRtWarps][16][8 * NT + 1];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int e0 = blockIdx.x * 16, m0 = blockIdx.y * 8 * NT;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *status = 0;
+  float acc[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  const T* wa = gate_w + (int64_t)min(e0 + g, E - 1) * H;            // rows past the end repeat the last: never stored
+  const T* wb = gate_w + (int64_t)min(e0 + g + 8, E - 1) * H;
+  const T* x[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) x[n] = hidden + (int64_t)min(m0 + 8 * n + g, M - 1) * ld_h;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int k0 = 64 * (blockIdx.z * kRtWarps + warp); k0 < H; k0 += 64 * kRtWarps * gridDim.z) {
+    uint4 a[2][2], b[2][NT];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int k = k0 + 32 * s + 8 * t;
+      const bool in = k < H;
+      a[s][0] = in ? ldg_stream_u4(wa + k) : zero;
+      a[s][1] = in ? ldg_stream_u4(wb + k) : zero;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) b[s][n] = in ? *reinterpret_cast<const uint4*>(x[n] + k) : zero;
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        mma_m16n8k16<T>(acc[n], a[s][0].x, a[s][1].x, a[s][0].y, a[s][1].y, b[s][n].x, b[s][n].y);
+        mma_m16n8k16<T>(acc[n], a[s][0].z, a[s][1].z, a[s][0].w, a[s][1].w, b[s][n].z, b[s][n].w);
+      }
+  }
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    s_part[warp][g][8 * n + 2 * t] = acc[n][0];
+    s_part[warp][g][8 * n + 2 * t + 1] = acc[n][1];
+    s_part[warp][g + 8][8 * n + 2 * t] = acc[n][2];
+    s_part[warp][g + 8][8 * n + 2 * t + 1] = acc[n][3];
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = warp; i < kRtExperts; i += kRtThreads / 32) {
-    const int e = e0 + i;
-    if (e >= E) break;
-    float acc[kRtTokens];
+  for (int i = threadIdx.x; i < 16 * 8 * NT; i += kRtThreads) {
+    const int r = i & 15, c = i >> 4;
+    float v = 0.f;
 #pragma unroll
-    for (int tk = 0; tk < kRtTokens; ++tk) acc[tk] = 0.f;
-    for (int c = lane; c < chunks; c += 32) {
-      float w[8];
-      unpack8<T>(ldg_stream_u4(gate_w + (int64_t)e * H + c * 8), w);
-#pragma unroll
-      for (int tk = 0; tk < kRtTokens; ++tk) {
-        float x[8];
-        unpack8<T>(reinterpret_cast<const uint4*>(sx)[tk * chunks + c], x);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[tk] = fmaf(w[k], x[k], acc[tk]);
-      }
-    }
-#pragma unroll
-    for (int tk = 0; tk < kRtTokens; ++tk) {
-      float v = acc[tk];
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-      if (lane == 0 && m0 + tk < M) logits[(int64_t)(m0 + tk) * E + e] = v;
-    }
+    for (int w = 0; w < kRtWarps; ++w) v += s_part[w][r][c];
+    if (e0 + r < E && m0 + c < M) parts[((int64_t)blockIdx.z * M + m0 + c) * E + e0 + r] = v;
   }
 }
 
-// One warp per token; E <= 32 * kRtPerLane.
+// ------------------------------------------------------------------------------------------ projection, larger batches
+
+constexpr int kRgThreads = 192;              // warp 0 TMA, warp 1 MMA and tensor memory, warps 2-5 epilogue
+constexpr int kRgStages = 4;
+constexpr int kRgK = 64;                     // elements per stage: 128-byte rows
+
+template <int BN>
+struct RouterGemm {
+  static constexpr int kStageA = 128 * 128, kStageB = BN * 128, kStage = kStageA + kStageB;
+  static constexpr size_t kSmem = (size_t)kRgStages * kStage + 1024 + 256;
+};
+
+__device__ __forceinline__ void tcgen05_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// parts[z][m][e] as above, for the tile of 128 tokens (blockIdx.y) x BN experts (blockIdx.x) and K-slice z.  Rows and columns
+// past the tensors are filled with zeros by the copies and not stored.
+template <int BN>
+__global__ void __launch_bounds__(kRgThreads, 1)
+    router_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int M, int H, int E,
+                       uint32_t idesc, int* __restrict__ status, float* __restrict__ parts) {
+  using C = RouterGemm<BN>;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kRgStages * C::kStage);
+  uint64_t* empty_bar = full_bar + kRgStages;
+  uint64_t* acc_full = empty_bar + kRgStages;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_full + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.y * 128, e0 = blockIdx.x * BN;
+  const int steps = (H + kRgK - 1) / kRgK;
+  const int first = (int)((int64_t)steps * blockIdx.z / gridDim.z), n_steps = (int)((int64_t)steps * (blockIdx.z + 1) / gridDim.z) - first;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRgStages; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(acc_full), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr_smem)), "r"((uint32_t)BN)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = *tmem_ptr_smem;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *status = 0;    // a wait writes it only after ~1 s
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int i = 0; i < n_steps; ++i) {
+        const uint32_t s = i % kRgStages, ph = (i / kRgStages) & 1;
+        if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, status, 31)) break;
+        unsigned char* st = smem + s * C::kStage;
+        const uint32_t bar = smem_u32(&full_bar[s]);
+        mbar_expect_tx(bar, C::kStage);
+        tma_load_2d(smem_u32(st), &map_x, (first + i) * 128, m0, bar);
+        tma_load_2d(smem_u32(st + C::kStageA), &map_w, (first + i) * 128, e0, bar);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      bool ok = true;
+      for (int i = 0; i < n_steps; ++i) {
+        const uint32_t s = i % kRgStages, ph = (i / kRgStages) & 1;
+        ok = mbar_wait(smem_u32(&full_bar[s]), ph, status, 32);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t a = smem_u32(smem + s * C::kStage), b = a + C::kStageA;
+#pragma unroll
+        for (int k = 0; k < kRgK / 16; ++k)       // 16 elements are 32 bytes further along the swizzled rows
+          tcgen05_mma_f16(tmem, desc_kmajor<128>(a + 32 * k), desc_kmajor<128>(b + 32 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
+        tcgen05_commit(smem_u32(&empty_bar[s]));
+      }
+      if (ok) tcgen05_commit(smem_u32(acc_full));
+    }
+  } else {
+    bool ok = mbar_wait(smem_u32(acc_full), 0, status, 33);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      tcgen05_fence_after();
+      const int quarter = warp & 3;               // tensor-memory lanes [32 quarter, +32) belong to this warp
+      const int m = m0 + quarter * 32 + lane;
+      float* dst = parts + ((int64_t)blockIdx.z * M + m) * E + e0;
+#pragma unroll 1
+      for (int c = 0; c < BN / 32; ++c) {
+        uint32_t r[32];
+        tcgen05_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + c * 32, r);
+        tcgen05_wait_ld();
+        const int left = E - e0 - c * 32;
+        if (m < M && left > 0) {
+          if (left >= 32 && (E & 3) == 0 && (reinterpret_cast<uintptr_t>(parts) & 15) == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              reinterpret_cast<uint4*>(dst + c * 32)[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < left) dst[c * 32 + i] = __uint_as_float(r[i]);
+          }
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------------------------------ top-k
+
+// unsigned keys in the order of the floats; 0 is below every float
+__device__ __forceinline__ uint32_t float_key(float v) {
+  const uint32_t u = __float_as_uint(v);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_float(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
+
+// One warp per token; E <= 32 * PER.  The warp-wide arg-max of a round is two warp reductions (largest key, then the lowest
+// expert id that holds it); shuffle trees of (value, id) pairs over 32 slots per lane took 5.8 us at M=32.
 constexpr int kRtPerLane = 32;
 
+template <int PER>
 __global__ void __launch_bounds__(128)
-    router_topk_kernel(const float* __restrict__ logits, int M, int E, int topk, int renormalize,
+    router_topk_kernel(const float* __restrict__ parts, int splits, int M, int E, int topk, int renormalize,
                        float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M) return;
-  float v[kRtPerLane];
-  float mx = -INFINITY;
+  uint32_t key[PER];
+  {
+    float v[PER];
 #pragma unroll
-  for (int i = 0; i < kRtPerLane; ++i) {
-    const int e = i * 32 + lane;                 // lane-interleaved: expert e lives in lane e % 32, slot e / 32
-    v[i] = e < E ? logits[(int64_t)m * E + e] : -INFINITY;
-    mx = fmaxf(mx, v[i]);
+    for (int i = 0; i < PER; ++i) v[i] = 0.f;
+    for (int z = 0; z < splits; ++z) {
+      const float* src = parts + ((int64_t)z * M + m) * E + lane;
+#pragma unroll
+      for (int i = 0; i < PER; ++i)                // lane-interleaved: expert e lives in lane e % 32, slot e / 32
+        if (i * 32 + lane < E) v[i] += src[i * 32];
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) key[i] = i * 32 + lane < E ? float_key(v[i]) : 0u;
   }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-  float total = 0.f;
-  if (!renormalize) {
-#pragma unroll
-    for (int i = 0; i < kRtPerLane; ++i) total += (i * 32 + lane < E) ? __expf(v[i] - mx) : 0.f;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
-  }
-  float sel_sum = 0.f, my_w = 0.f;
+  float mx = 0.f, total = 0.f, sel_sum = 0.f, my_w = 0.f;
   int my_id = 0;
   for (int r = 0; r < topk; ++r) {
-    // this lane's best remaining (lowest slot wins ties, which is the lowest expert id within the lane)
-    float best = -INFINITY;
-    int slot = 0;
+    uint32_t best = key[0];
 #pragma unroll
-    for (int i = 0; i < kRtPerLane; ++i)
-      if (v[i] > best) {
-        best = v[i];
-        slot = i;
-      }
-    int id = slot * 32 + lane;
-    float cand = best;
+    for (int i = 1; i < PER; ++i) best = max(best, key[i]);
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+    uint32_t id = 0xffffffffu;                     // the lane's lowest expert that holds the largest key
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, cand, d);
-      const int oid = __shfl_xor_sync(0xffffffffu, id, d);
-      if (ov > cand || (ov == cand && oid < id)) {
-        cand = ov;
-        id = oid;
+    for (int i = PER - 1; i >= 0; --i)
+      if (key[i] == top) id = i * 32 + lane;
+    id = __reduce_min_sync(0xffffffffu, id);
+#pragma unroll
+    for (int i = 0; i < PER; ++i)                  // compile-time indexed: keeps key[] in registers
+      if (id == (uint32_t)(i * 32 + lane)) key[i] = 0u;
+    const float value = key_float(top);
+    if (r == 0) {
+      mx = value;
+      if (!renormalize) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) total += key[i] != 0u ? __expf(key_float(key[i]) - mx) : 0.f;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+        total += 1.f;                              // the largest itself, already taken out
       }
     }
-    if ((id & 31) == lane) {
-#pragma unroll
-      for (int i = 0; i < kRtPerLane; ++i)
-        if (i == (id >> 5)) v[i] = -INFINITY;      // compile-time indexed: keeps v[] in registers
-    }
-    const float w = __expf(cand - mx);
+    const float w = __expf(value - mx);
     sel_sum += w;
     if (lane == r) {
       my_w = w;
-      my_id = id;
+      my_id = (int)id;
     }
   }
   const float denom = renormalize ? sel_sum : total;
@@ -151,14 +302,81 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// ------------------------------------------------------------------------------------------ host
+
+// K-slices of the projection: enough blocks to cover the SMs, at most eight (the top-k kernel reads them all).
+// Up to one block of tokens (64) the mma.sync kernel is the faster one (M=32: 3.4 us); it reads every weight row once per block
+// of tokens through L2, so from there on the tcgen05 tiles win (M=200: 12.7 us against about 6; M=1000: 7.9 us, M=8192: 22 us
+// where one dot product per warp and weight row took 832 us).
+constexpr int kRtMmaMaxTokens = kRtMaxTokens;
+constexpr int kRtMaxSplits = 8;
+
+struct RouterShape {
+  bool small;
+  int tokens, bn, splits;      // small: tokens per block; else the expert tile
+};
+
+RouterShape router_shape(int64_t M, int64_t E) {
+  RouterShape s = {};
+  s.small = M <= kRtMmaMaxTokens;
+  int64_t blocks;
+  if (s.small) {
+    s.tokens = M <= 8 ? 8 : (M <= 16 ? 16 : (M <= 32 ? 32 : kRtMaxTokens));
+    blocks = ((E + 15) / 16) * ((M + s.tokens - 1) / s.tokens);
+  } else {
+    const int64_t mt = (M + 127) / 128;
+    s.bn = mt * ((E + 127) / 128) <= sm_count() ? 128 : 256;
+    blocks = mt * ((E + s.bn - 1) / s.bn);
+  }
+  const int64_t z = sm_count() / (blocks > 0 ? blocks : 1);
+  s.splits = (int)(z < 1 ? 1 : (z > kRtMaxSplits ? kRtMaxSplits : z));
+  return s;
+}
+
+template <typename T>
+void launch_router_mma(const RouterShape& s, int splits, const void* hidden, int64_t ld_h, const void* gate_w, int M, int H, int E,
+                       int* status, float* parts, cudaStream_t st) {
+  const dim3 grid((unsigned)((E + 15) / 16), (unsigned)((M + s.tokens - 1) / s.tokens), (unsigned)splits);
+  auto go = [&](auto kernel) {
+    launch_pdl(kernel, grid, dim3(kRtThreads), 0, st, static_cast<const T*>(hidden), ld_h, static_cast<const T*>(gate_w), M, H, E,
+               status, parts);
+  };
+  if (s.tokens == 8) go(router_mma_kernel<T, 1>);
+  else if (s.tokens == 16) go(router_mma_kernel<T, 2>);
+  else if (s.tokens == 32) go(router_mma_kernel<T, 4>);
+  else go(router_mma_kernel<T, 8>);
+}
+
+template <int BN>
+int launch_router_gemm(const CUtensorMap& mx, const CUtensorMap& mw, int splits, bool bf16, int M, int H, int E, int* status,
+                       float* parts, cudaStream_t st) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return B200FP4_STATUS_NOT_SUPPORTED;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(router_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RouterGemm<BN>::kSmem) != cudaSuccess) {
+      cudaGetLastError();
+      return B200FP4_STATUS_EXECUTION_FAILED;
+    }
+    attr_set[dev] = true;
+  }
+  const uint32_t fmt = bf16 ? 1u : 0u;        // fp32 accumulators, f16 / bf16 operands, K-major both, N = BN, M = 128
+  const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
+  const dim3 grid((unsigned)((E + BN - 1) / BN), (unsigned)((M + 127) / 128), (unsigned)splits);
+  launch_pdl(router_gemm_kernel<BN>, grid, dim3(kRgThreads), RouterGemm<BN>::kSmem, st, mx, mw, M, H, E, idesc, status, parts);
+  return B200FP4_STATUS_SUCCESS;
+}
+
 }  // namespace
 }  // namespace b200fp4
 
 using namespace b200fp4;
 
+// workspace: 256 bytes (first int: status word of the tcgen05 kernel's bounded waits), then the K-slices of the logits
 extern "C" size_t b200fp4_moe_router_workspace_bytes(int64_t M, int64_t E) {
-  if (M < 0 || E < 0) return 0;
-  return (size_t)M * (size_t)E * sizeof(float);
+  if (M <= 0 || E <= 0) return 0;
+  return 256 + (size_t)router_shape(M, E).splits * (size_t)M * (size_t)E * sizeof(float);
 }
 
 extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, const void* gate_w, int64_t M, int64_t H,
@@ -166,51 +384,45 @@ extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, c
                                   void* workspace, size_t workspace_bytes, void* stream) {
   if (M < 0 || H <= 0 || E <= 0 || topk <= 0 || (H % 8) != 0 || ld_h < H || (ld_h % 8) != 0) return B200FP4_STATUS_INVALID_VALUE;
   if (dtype != B200FP4_DTYPE_BF16 && dtype != B200FP4_DTYPE_F16) return B200FP4_STATUS_NOT_SUPPORTED;
-  if (topk > 32 || topk > E || E > 32 * kRtPerLane || (size_t)kRtTokens * H * 2 > 200 * 1024) return B200FP4_STATUS_NOT_SUPPORTED;
+  if (topk > 32 || topk > E || E > 32 * kRtPerLane || H > 12800) return B200FP4_STATUS_NOT_SUPPORTED;
   if (M == 0) return B200FP4_STATUS_SUCCESS;
   if (!hidden || !gate_w || !topk_weights || !topk_ids || !aligned(hidden, 16) || !aligned(gate_w, 16))
     return B200FP4_STATUS_INVALID_VALUE;
   if (!workspace || workspace_bytes < b200fp4_moe_router_workspace_bytes(M, E) || !aligned(workspace, 4))
     return B200FP4_STATUS_ALLOC_FAILED;
+  if (M > (int64_t)65535 * 128) return B200FP4_STATUS_NOT_SUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
-  float* logits = static_cast<float*>(workspace);
-  const size_t smem = (size_t)kRtTokens * H * 2;
-  dim3 grid((unsigned)((E + kRtExperts - 1) / kRtExperts), (unsigned)((M + kRtTokens - 1) / kRtTokens));
-  if (dtype == B200FP4_DTYPE_BF16) {
-    static bool set[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !set[dev]) {
-      cudaFuncSetAttribute(router_logits_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      set[dev] = true;
-    }
-    router_logits_kernel<__nv_bfloat16><<<grid, kRtThreads, smem, st>>>(static_cast<const __nv_bfloat16*>(hidden), ld_h,
-                                                                        static_cast<const __nv_bfloat16*>(gate_w), (int)M,
-                                                                        (int)H, (int)E, logits);
+  int* status = static_cast<int*>(workspace);
+  float* parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
+  const RouterShape sh = router_shape(M, E);
+  const bool bf = dtype == B200FP4_DTYPE_BF16;
+  int splits = sh.splits;
+  if (sh.small) {
+    // no more slices than there are rounds of 64 per warp
+    const int most = (int)((H + 64 * kRtWarps - 1) / (64 * kRtWarps));
+    if (splits > most) splits = most;
+    if (bf) launch_router_mma<__nv_bfloat16>(sh, splits, hidden, ld_h, gate_w, (int)M, (int)H, (int)E, status, parts, st);
+    else launch_router_mma<__half>(sh, splits, hidden, ld_h, gate_w, (int)M, (int)H, (int)E, status, parts, st);
   } else {
-    static bool set[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !set[dev]) {
-      cudaFuncSetAttribute(router_logits_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      set[dev] = true;
-    }
-    router_logits_kernel<__half><<<grid, kRtThreads, smem, st>>>(static_cast<const __half*>(hidden), ld_h,
-                                                                 static_cast<const __half*>(gate_w), (int)M, (int)H, (int)E,
-                                                                 logits);
+    if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
+    const int most = (int)((H + 4 * kRgK - 1) / (4 * kRgK));       // at least about four stages per slice
+    if (splits > most) splits = most;
+    CUtensorMap mx, mw;
+    if (!make_rows_map(&mx, hidden, (uint64_t)M, (uint64_t)H * 2, (uint64_t)ld_h * 2, 128, 128) ||
+        !make_rows_map(&mw, gate_w, (uint64_t)E, (uint64_t)H * 2, (uint64_t)H * 2, (uint32_t)sh.bn, 128))
+      return B200FP4_STATUS_INTERNAL_ERROR;
+    const int rc = sh.bn == 128 ? launch_router_gemm<128>(mx, mw, splits, bf, (int)M, (int)H, (int)E, status, parts, st)
+                                : launch_router_gemm<256>(mx, mw, splits, bf, (int)M, (int)H, (int)E, status, parts, st);
+    if (rc != B200FP4_STATUS_SUCCESS) return rc;
   }
-  // the top-k kernel may become resident while the projection drains (programmatic dependent launch)
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((M + 3) / 4));
-  cfg.blockDim = dim3(128);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cfg.numAttrs = (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, router_topk_kernel, (const float*)logits, (int)M, (int)E, (int)topk, renormalize, topk_weights,
-                     topk_ids);
+  auto topk_go = [&](auto kernel) {
+    launch_pdl(kernel, dim3((unsigned)((M + 3) / 4)), dim3(128), 0, st, (const float*)parts, splits, (int)M, (int)E, (int)topk,
+               renormalize, topk_weights, topk_ids);
+  };
+  if (E <= 64) topk_go(router_topk_kernel<2>);
+  else if (E <= 128) topk_go(router_topk_kernel<4>);
+  else if (E <= 256) topk_go(router_topk_kernel<8>);
+  else if (E <= 512) topk_go(router_topk_kernel<16>);
+  else topk_go(router_topk_kernel<kRtPerLane>);
   return finish_launch(2);
 }

@@ -8,6 +8,11 @@
 
 namespace b200fp4 {
 
+// Tensor map of [rows, row_bytes] bytes, rows row_stride bytes apart (multiples of 16); box = box_bytes (128, 64 or 32) x box_rows
+// with the matching swizzle, zeros out of bounds.  Cached per argument list.  (gemm.cu)
+bool make_rows_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t row_stride, uint32_t box_rows,
+                   int box_bytes);
+
 constexpr long long kWaitCycles = 2000000000LL;   // ~1 s at 2 GHz: every barrier wait gives up after this
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

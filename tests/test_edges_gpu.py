@@ -28,3 +28,31 @@ def test_convert_2of4_tile_edges(E, N, K, G):
         np.testing.assert_array_equal(to_np(comp[e]), oc)
         np.testing.assert_array_equal(to_np(meta[e]), om)
         np.testing.assert_array_equal(to_np(scale[e]), sf[e].T)
+
+
+@pytest.mark.parametrize("M,H,E,topk,dtype,renorm", [
+    (1, 8, 1, 1, torch.bfloat16, True),               # smallest: one 16-byte piece of K, one expert
+    (9, 1000, 40, 5, torch.float16, True),            # one past eight tokens, K no multiple of 64, experts past a block of 16
+    (64, 512, 64, 8, torch.bfloat16, True),           # last size of the small-batch kernel
+    (65, 2048, 1024, 32, torch.bfloat16, False),      # first of the tile kernel, largest E and topk
+    (257, 520, 136, 8, torch.float16, True),          # tokens, experts and K past their tiles
+    (1024, 2048, 512, 10, torch.bfloat16, True),      # several K-slices
+    (4864, 1024, 512, 10, torch.bfloat16, False),     # 256-wide expert tiles
+    (4865, 256, 290, 4, torch.float16, True),         # ... past their end, E no multiple of four
+])
+def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
+    from dgx_vllm_b200.router import moe_router
+    g = torch.Generator(device="cuda").manual_seed(M + E)
+    wide = torch.randn(M, H + 8, generator=g, device="cuda").to(dtype)
+    hidden = wide[:, :H]                              # strided rows
+    gate = (torch.randn(E, H, generator=g, device="cuda") / H ** 0.5).to(dtype)
+    tw, ids = moe_router(hidden, gate, topk, renormalize=renorm)
+    logits = hidden.double() @ gate.double().t()
+    w, ref_ids = torch.softmax(logits, dim=-1).topk(topk, dim=-1)
+    if renorm:
+        w = w / w.sum(-1, keepdim=True)
+    srt = torch.cat((logits, torch.full((M, 1), -1e9, device="cuda", dtype=torch.double)), 1).sort(dim=-1, descending=True).values
+    clear = (srt[:, :topk] - srt[:, 1:topk + 1]).min(dim=-1).values > 2e-5
+    assert clear.float().mean() > 0.8
+    assert torch.equal(ids[clear].long(), ref_ids[clear])
+    assert ((tw[clear].double() - w[clear]).abs() / w[clear]).max() < 1e-4
