@@ -5,10 +5,12 @@ non-zero status the call raises."""
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libb200nvfp4.so")
+HOST_PATH = os.path.join(_HERE, "lib", "b200_host.so")
 
 F16, BF16, F32 = 0, 1, 2
 MOE_ROUTER_WEIGHT_ON_INPUT, SPARSE_META_ORDERED, MOE_SEPARATE_LAUNCHES, MOE_HOST_DIRECT_OUT = 1, 2, 4, 8     # flags of the sparse entry points
@@ -41,6 +43,9 @@ SIGNATURES = {
     "b200fp4_grouped_gemm_nvfp4_silu_quant": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64,
                                                      _i64, _vp, _sz, _vp]),
     "b200fp4_moe_unpermute_reduce": (_i32, [_vp, _i32, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
+    "b200fp4_moe_prefill_workspace_bytes": (_sz, [_i64] * 5),
+    "b200fp4_moe_prefill": (_i32, [_vp, _i32, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                                   _i64, _i64, _i64, _i64, _i64, _vp, _sz, _vp]),
     "b200fp4_sparse_workspace_bytes": (_sz, [_i64, _i64, _i64]),
     "b200fp4_sparse_gemv": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp]),
     "b200fp4_sparse_gemv_static": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64, _i64, _i64, _i64, _i64, _vp]),
@@ -88,6 +93,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class B200Fp4Error(RuntimeError):
@@ -111,6 +117,21 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+def host():
+    """The native host path of the torch-facing ops (csrc/torch_host.cpp)."""
+    global _host
+    if _host is None:
+        lib()                               # a missing library raises here, with its own message
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m dgx_vllm_b200.build`. "
+                               "This package has no fallback path.")
+        spec = importlib.util.spec_from_file_location("b200_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 def check(status: int, where: str) -> None:

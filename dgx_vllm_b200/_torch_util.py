@@ -6,7 +6,6 @@ import torch
 from . import _lib
 
 _DT = {torch.float16: _lib.F16, torch.bfloat16: _lib.BF16, torch.float32: _lib.F32}
-_workspaces: dict = {}
 
 
 def dtype_code(t: torch.dtype) -> int:
@@ -39,15 +38,10 @@ def stream_ptr(device: torch.device) -> int:
 
 
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Grow-only scratch buffer per (device, stream).  Calls issued on one stream serialise on the
-    GPU, so sharing it between consecutive ops is safe; its address is stable once large enough,
+    """Grow-only scratch buffer per (device, current stream), shared with the native host path.  Calls issued on one
+    stream serialise on the GPU, so sharing it between consecutive ops is safe; its address is stable once large enough,
     which CUDA-graph capture relies on."""
-    key = (device.index, stream_ptr(device))
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+    return _lib.host().workspace(torch.cuda.current_device() if device.index is None else device.index, nbytes)
 
 
 def ptr(t) -> int:

@@ -1,8 +1,9 @@
-"""In-tree build of libb200nvfp4.so (sm_100a only) with nvcc.  No torch dependency.
+"""In-tree build of libb200nvfp4.so (sm_100a only, nvcc, no torch dependency) and of b200_host.so, the native host path of
+the torch-facing ops (csrc/torch_host.cpp, the host compiler against torch's headers, linked to the former).
 
     python -m dgx_vllm_b200.build [--force] [--verbose]
 
-Objects go to dgx_vllm_b200/build/, the library to dgx_vllm_b200/lib/libb200nvfp4.so.
+Objects go to dgx_vllm_b200/build/, the libraries to dgx_vllm_b200/lib/.
 """
 from __future__ import annotations
 
@@ -12,12 +13,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libb200nvfp4.so")
+HOST_SRC = os.path.join(CSRC, "torch_host.cpp")
+HOST_PATH = os.path.join(LIB_DIR, "b200_host.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -69,7 +73,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_host(force)
     return LIB_PATH
+
+
+def _build_host(force: bool) -> None:
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(HOST_SRC), _deps_mtime()):
+        return
+    import torch
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    inc = [os.path.join(tdir, "include"), os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", HOST_PATH, HOST_SRC]
+    cmd += [f"-isystem{i}" for i in inc]
+    cmd += [f"-L{LIB_DIR}", "-lb200nvfp4", "-Wl,-rpath,$ORIGIN", f"-L{os.path.join(tdir, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {HOST_PATH} failed:\n{r.stdout}\n{r.stderr}")
 
 
 if __name__ == "__main__":

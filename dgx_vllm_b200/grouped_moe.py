@@ -238,15 +238,18 @@ def nvfp4_moe_prefill(hidden, topk_weights, topk_ids, w13_codes, w13_sf, w13_gs,
 
     w13_codes [E,2I,H/2], w13_sf [E, swizzled(2I,H/16)], w13_gs [E] weight global scales (448*6/amax);
     w2_* likewise for [E,H,I/2]; a1_gs / a2_gs [E] activation global scales of the two GEMM inputs."""
-    dev = hidden.device
-    M, H = hidden.shape
     topk = topk_ids.shape[1]
     E, N1, _ = w13_codes.shape
+    alpha1, alpha2 = alphas if alphas is not None else nvfp4_moe_alphas(w13_gs, w2_gs, a1_gs, a2_gs)
+    if topk <= 32 and N1 % 256 == 0:
+        return _lib.host().moe_prefill(hidden, topk_weights, topk_ids, w13_codes, w13_sf, w2_codes, w2_sf, a1_gs, a2_gs,
+                                       alpha1, alpha2, expert_map)
+    dev = hidden.device
+    M, H = hidden.shape
     P = M * topk
     eo = torch.empty(E + 1, dtype=torch.int32, device=dev)
     a_map = torch.empty(P, dtype=torch.int32, device=dev)
     c_map = torch.empty(P, dtype=torch.int32, device=dev)
-    alpha1, alpha2 = alphas if alphas is not None else nvfp4_moe_alphas(w13_gs, w2_gs, a1_gs, a2_gs)
     bso = get_cutlass_moe_mm_data(topk_ids, eo, None, None, a_map, c_map, E, N1 // 2, H, expert_map=expert_map,
                                   pair_indices=topk <= 32)
     if topk <= 32:

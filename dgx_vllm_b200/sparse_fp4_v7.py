@@ -268,40 +268,14 @@ class FusedSparseMoE:
                       ptr(w13_comp), ptr(w13_meta), ptr(w13_scale), ptr(w13_g_scales), w13_scale.shape[1],
                       ptr(w2_comp), ptr(w2_meta), ptr(w2_scale), ptr(w2_g_scales), w2_scale.shape[1])
         self._lib = _lib.lib()
-        self._fn = self._lib.b200fp4_fused_sparse_moe
+        self._call = _lib.host().moe_call
+        self._bound = _lib.host().moe_bind(*self._keep, H, I, E, self._flags)
         self._ws_bytes = {}
         self._host_slots = {}
         self._copy_stream = None
 
     def __call__(self, hidden_states, topk_weights, topk_ids, apply_router_weight_on_input: bool = False, out=None):
-        M, H = hidden_states.shape
-        topk = topk_ids.shape[1]
-        require(hidden_states.is_cuda and H == self.H and hidden_states.is_contiguous() and
-                hidden_states.dtype in (torch.float16, torch.bfloat16), "hidden_states must be a contiguous [M,H] 16-bit CUDA tensor")
-        tw = topk_weights if topk_weights.dtype == torch.float32 else topk_weights.float()
-        ids = topk_ids if topk_ids.dtype == torch.int32 else topk_ids.to(torch.int32)
-        require(tw.is_contiguous() and ids.is_contiguous() and tuple(tw.shape) == (M, topk) and ids.shape[0] == M,
-                "topk_weights / topk_ids must be contiguous [M, topk]")
-        dev = self.device
-        if out is None:
-            out = torch.empty((M, H), dtype=hidden_states.dtype, device=dev)
-        key = (M, topk)
-        nws = self._ws_bytes.get(key)
-        if nws is None:
-            nws = self._ws_bytes[key] = self._lib.b200fp4_fused_moe_workspace_bytes(M, topk, H, self.I, self.E)
-        ws = workspace(dev, nws)
-        code = dtype_code(hidden_states.dtype)
-        flags = self._flags | (_lib.MOE_ROUTER_WEIGHT_ON_INPUT if apply_router_weight_on_input else 0)
-        if torch.cuda.current_device() != dev.index:
-            with torch.cuda.device(dev):
-                rc = self._fn(hidden_states.data_ptr(), code, tw.data_ptr(), ids.data_ptr(), *self._head, out.data_ptr(),
-                              dtype_code(out.dtype), M, topk, H, self.I, self.E, flags, ws.data_ptr(), ws.numel(), stream_ptr(dev))
-        else:
-            rc = self._fn(hidden_states.data_ptr(), code, tw.data_ptr(), ids.data_ptr(), *self._head, out.data_ptr(),
-                          dtype_code(out.dtype), M, topk, H, self.I, self.E, flags, ws.data_ptr(), ws.numel(), stream_ptr(dev))
-        _lib.check(rc, "fused_sparse_moe_v7")
-        return out
-
+        return self._call(self._bound, hidden_states, topk_weights, topk_ids, apply_router_weight_on_input, out)
 
     def forward_host(self, hidden_host, topk_weights_host, topk_ids_host, out_host=None,
                      apply_router_weight_on_input: bool = False):
