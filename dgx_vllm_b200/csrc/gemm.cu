@@ -4,7 +4,7 @@
 // kernels are scalar CUDA-core loops, cutlass_nvfp4/nvfp4_gemm_kernel.cuh:296-345) with a
 // tcgen05 design:
 //   * persistent, warp-specialised CTAs (one per SM): warp 0 issues TMA loads, warp 1 issues
-//     tcgen05.cp / tcgen05.mma, warps 2-5 run the epilogue;
+//     tcgen05.mma, further warps, in groups of four, move scale factors and run the epilogue;
 //   * operands are packed E2M1 bytes, K-major, staged by 2-D TMA (no multicast) into 128-byte
 //     swizzled shared-memory tiles of 128 (A) / BN (B) rows x 256 k; scale factors come from the
 //     128x4-tile swizzled global layout, where the 4 k-blocks x 128 rows an MMA needs are 512
@@ -34,7 +34,10 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const uint8_t
 namespace {
 
 constexpr int kBM = 128;
-constexpr int kGemmThreads = 448;         // warp 0 TMA, warp 1 MMA, warps 2-5 and 10-13 epilogue, warps 6-9 scale factors
+// Warp 0 TMA, warp 1 MMA, warps 6-9 scale factors, the others epilogue in groups of four (one warp per 32-lane quarter of
+// tensor memory): warps 2-5 and 10-13, and in the grouped kernels also 14-17 and 18-21.
+constexpr int gemm_epi_groups(bool grouped) { return grouped ? 4 : 2; }
+constexpr int gemm_threads(bool grouped) { return 32 * (6 + 4 * gemm_epi_groups(grouped)); }
 constexpr uint32_t kTmemCols = 512;
 
 struct GemmParams {
@@ -117,13 +120,13 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int tile, int
   return t;
 }
 
-// 64 gate and 64 up values of one row (as 16-bit pairs) -> SiLU(gate)*up rounded to T -> four NVFP4 blocks:
-// 8 words of codes and 4 scale bytes, with the arithmetic of the stand-alone SiLU-mul quantizer.
-template <typename T>
+// 16 NB gate and as many up values of one row (as 16-bit pairs) -> SiLU(gate)*up rounded to T -> NB NVFP4 blocks:
+// 2 NB words of codes and NB scale bytes, with the arithmetic of the stand-alone SiLU-mul quantizer.
+template <typename T, int NB>
 __device__ __forceinline__ void silu_quant_row(const uint32_t* pg, const uint32_t* pu, float gs, float rcp_gs,
                                                uint32_t* codes, uint32_t& sf4) {
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
+  for (int b = 0; b < NB; ++b) {
     float x[16];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -159,7 +162,8 @@ __device__ __forceinline__ void silu_quant_row(const uint32_t* pg, const uint32_
 
 // BN = tile width; KB = 64-wide k-blocks (MMAs) per shared-memory stage.  Smaller stages do not change
 // the bytes resident in shared memory but refill in finer steps, which keeps more of them in flight.
-template <int BN, int KB, bool kOutTma = false>
+// kOutStage: bytes of shared memory the epilogue stages its output in.
+template <int BN, int KB, int kOutStage = 0>
 struct Cfg {
   static constexpr int kAcc = BN == 128 ? 2 : 1;                    // accumulator buffers in tensor memory
   static constexpr int kSfTiles = BN / 128;                         // 128-row scale tiles on the B side
@@ -169,31 +173,37 @@ struct Cfg {
   static constexpr int kStageSFA = KB * 512;
   static constexpr int kStageSFB = kSfTiles * KB * 512;
   static constexpr int kStageBytes = kStageA + kStageB + kStageSFA + kStageSFB;
-  // BN = 256 gives one of its four stages to the epilogue's staging buffers (tile stores through the copy engine)
-  static constexpr int kStages = (BN == 128 ? 24 : (kOutTma ? 12 : 16)) / KB;
-  static constexpr int kOutStage = kOutTma ? 8 * 4096 : 0;         // 8 epilogue warps x [32 rows x 64 columns] 16-bit
+  // an epilogue that stages its output takes the place of one operand stage
+  static constexpr int kStages = (BN == 128 ? 24 : 16) / KB - (kOutStage > 0 ? 1 : 0);
   // tensor-memory column map: accumulators, then one scale-factor block per shared-memory stage
   // (4 columns per k-block for A, 4*kSfTiles for B)
   static constexpr uint32_t kSfCols = KB * (4 + 4 * kSfTiles);
   static constexpr uint32_t kSfBase = kAcc * BN;
   static_assert(kSfBase + kStages * kSfCols <= 512, "tensor memory budget");
   static constexpr int kBarBytes = 1024;
-  static constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + kOutStage + 1024 /*alignment slack*/ + kBarBytes;
+  static constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + (size_t)kOutStage + 1024 /*alignment slack*/ + kBarBytes;
   // instruction descriptor: E2M1 x E2M1, UE4M3 scales, K-major A and B, N = BN, M = 128, dense K = 64
   static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 };
 
+// Staging: the dense wide-tile kernel hands [32 rows x 64 columns] boxes of 8 warps to the copy engine, the grouped kernel
+// transposes [32 rows x 32 columns] of 16 warps.
+template <int BN, bool kGrouped, bool kSiluQuant>
+constexpr int out_stage_bytes() { return kSiluQuant ? 0 : (kGrouped ? 16 * 2048 : (BN == 256 ? 8 * 4096 : 0)); }
+
 template <int BN, int KB, bool kGrouped, bool kSiluQuant = false>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
   constexpr bool kOutTma = BN == 256 && !kGrouped && !kSiluQuant;     // the dense wide-tile kernel stores tiles through the copy engine
-  using C = Cfg<BN, KB, kOutTma>;
+  constexpr int kOutStage = out_stage_bytes<BN, kGrouped, kSiluQuant>();
+  using C = Cfg<BN, KB, kOutStage>;
+  constexpr int kEpi = gemm_epi_groups(kGrouped);
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment for the 128-byte swizzle atoms
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* out_stage = smem + (size_t)C::kStages * C::kStageBytes;      // 1024-byte aligned (stages are multiples of 1 KiB)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + C::kOutStage);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + kOutStage);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + C::kStages;
   uint64_t* acc_full = bars + 2 * C::kStages;
@@ -218,7 +228,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int a = 0; a < C::kAcc; ++a) {
       mbar_init(smem_u32(&acc_full[a]), 1);
-      mbar_init(smem_u32(&acc_empty[a]), 8);      // one arrival per epilogue warp
+      mbar_init(smem_u32(&acc_empty[a]), 4 * kEpi);      // one arrival per epilogue warp
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -334,13 +344,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5 and 10..13)
-    // Two warps per tensor-memory lane quarter, each draining and storing half of the tile's columns.
+    // ------------------------------------------------------------------ epilogue
+    // kEpi warps per tensor-memory lane quarter, each draining and storing its share of the tile's columns.
     // With long K the epilogue hides behind the next tile either way; with short K (the grouped down
-    // projection: 8 MMAs per tile) the kernel is bound by how fast a tile can be drained and stored.
+    // projection: 8 MMAs per tile) the kernel is bound by how fast a tile can be drained and stored, and with SiLU and
+    // quantization by the epilogue's arithmetic: about 3000 instructions per row and 64 columns keep eight warps busy for
+    // twice the 6600 cycles of the main loop (gate_up of 81,920 rows: 182 us with eight epilogue warps).
     const int quarter = warp & 3;                 // tensor-memory lanes [32*quarter, +32) belong to this warp
-    constexpr int CH = BN / 64;                   // 32-column chunks per warp
-    const int c_first = warp >= 10 ? CH : 0;
+    constexpr int CH = BN / 32 / kEpi;            // 32-column chunks per warp
+    const int grp = warp < 6 ? 0 : (warp - 6) >> 2;
+    const int c_first = grp * CH;
     const float alpha_dense = kGrouped ? 0.f : p.alpha[0];
     uint32_t tcount = 0;
     bool ok = true;
@@ -356,33 +369,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       if constexpr (kSiluQuant) {
         // Tensor-memory columns [0,128) hold the gate half of this thread's row, [128,256) the up half.
-        // This warp takes 64 of the 128 output columns: 4 blocks of 16 -> 32 bytes of codes + 4 scale bytes,
+        // This warp takes 32 of the 128 output columns: 2 blocks of 16 -> 16 bytes of codes + 2 scale bytes,
         // computed exactly as the separate SiLU-mul quantizer does from the 16-bit rounded GEMM output.
-        const int half = warp >= 10 ? 1 : 0;
         const float gs = p.q_gs[ti.expert];
         const float rcp_gs = __frcp_rn(gs + (gs == 0.f ? 1.0e8f : 0.f));
         // drain both halves as 16-bit pairs (the rounding the separate GEMM's output has), hand the accumulator
         // back, and only then do the SiLU / quantization arithmetic, so that it overlaps the next tile's main loop
-        uint32_t pg[32], pu[32];
+        uint32_t pg[16], pu[16];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          uint32_t rg[32], ru[32];
-          tcgen05_ld_32x32(taddr + (half * 2 + c) * 32, rg);
-          tcgen05_ld_32x32(taddr + 128 + (half * 2 + c) * 32, ru);
+          uint32_t r[32];
+          tcgen05_ld_32x32(taddr + c * 128 + grp * 32, r);
           tcgen05_wait_ld();
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float g0 = __uint_as_float(rg[2 * i]) * alpha, g1 = __uint_as_float(rg[2 * i + 1]) * alpha;
-            const float u0 = __uint_as_float(ru[2 * i]) * alpha, u1 = __uint_as_float(ru[2 * i + 1]) * alpha;
+            const float v0 = __uint_as_float(r[2 * i]) * alpha, v1 = __uint_as_float(r[2 * i + 1]) * alpha;
+            uint32_t w;
             if (p.out_bf16) {
-              const __nv_bfloat162 vg = __floats2bfloat162_rn(g0, g1), vu = __floats2bfloat162_rn(u0, u1);
-              pg[c * 16 + i] = *reinterpret_cast<const uint32_t*>(&vg);
-              pu[c * 16 + i] = *reinterpret_cast<const uint32_t*>(&vu);
+              const __nv_bfloat162 v = __floats2bfloat162_rn(v0, v1);
+              w = *reinterpret_cast<const uint32_t*>(&v);
             } else {
-              const __half2 vg = __floats2half2_rn(g0, g1), vu = __floats2half2_rn(u0, u1);
-              pg[c * 16 + i] = *reinterpret_cast<const uint32_t*>(&vg);
-              pu[c * 16 + i] = *reinterpret_cast<const uint32_t*>(&vu);
+              const __half2 v = __floats2half2_rn(v0, v1);
+              w = *reinterpret_cast<const uint32_t*>(&v);
             }
+            (c ? pu : pg)[i] = w;
           }
         }
         tcgen05_fence_before();
@@ -390,15 +400,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
         // rows past the end of the expert are never stored: warps whose 32 rows are all past it skip the arithmetic
         if (row < ti.row_end) {
-          uint32_t codes[8];
-          uint32_t sf4 = 0;
-          if (p.out_bf16) silu_quant_row<__nv_bfloat16>(pg, pu, gs, rcp_gs, codes, sf4);
-          else silu_quant_row<__half>(pg, pu, gs, rcp_gs, codes, sf4);
-          uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + (size_t)row * (size_t)(p.q_inter / 2) + (ti.n0 + half * 64) / 2;
-          st_global_v8(dst, codes);
+          uint32_t codes[4];
+          uint32_t sf2 = 0;
+          if (p.out_bf16) silu_quant_row<__nv_bfloat16, 2>(pg, pu, gs, rcp_gs, codes, sf2);
+          else silu_quant_row<__half, 2>(pg, pu, gs, rcp_gs, codes, sf2);
+          const int col = ti.n0 + grp * 32;
+          uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + (size_t)row * (size_t)(p.q_inter / 2) + col / 2;
+          *reinterpret_cast<uint4*>(dst) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
           const size_t kt2 = (size_t)(p.q_inter / 64);
-          *reinterpret_cast<uint32_t*>(p.q_sf + ((size_t)ti.sfa_tile * kt2 + (size_t)(ti.n0 / 64 + half)) * 512 + lane * 16 +
-                                       quarter * 4) = sf4;
+          *reinterpret_cast<uint16_t*>(p.q_sf + ((size_t)ti.sfa_tile * kt2 + (size_t)(col / 64)) * 512 + lane * 16 + quarter * 4 +
+                                       (grp & 1) * 2) = (uint16_t)sf2;
         }
         continue;
       }
@@ -432,7 +443,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         continue;
       }
       // drain this thread's row of the accumulator into packed 16-bit registers ...
-      uint32_t packed[BN / 4];
+      uint32_t packed[16 * CH];
 #pragma unroll
       for (int c = 0; c < CH; ++c) {
         uint32_t r[32];
@@ -457,12 +468,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
-      if (kOutTma && p.out_tma) {
+      if constexpr (kOutTma) if (p.out_tma) {
         // This warp's 32 rows x 128 columns leave in two halves of 64 columns (128 bytes per row): rows go to a private
         // staging buffer with the 128-byte swizzle of the tensor map (16-byte chunk c of row r at c ^ (r % 8): the
         // lanes of a warp write different banks), one lane hands the box to the copy engine, which writes whole lines
         // and clips rows / columns beyond the tensor.
-        const uint32_t stg = smem_u32(out_stage) + (uint32_t)((warp >= 10 ? 4 : 0) + quarter) * 4096u;
+        const uint32_t stg = smem_u32(out_stage) + (uint32_t)(grp * 4 + quarter) * 4096u;
         const int row0 = ti.a_row0 + quarter * 32;
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
@@ -478,6 +489,32 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           if (lane == 0 && col0 < p.N && row0 < p.M) {
             tma_store_2d(&map_out, col0, row0, stg);
             bulk_commit();
+          }
+        }
+        continue;
+      }
+      if constexpr (kGrouped) if ((p.N % 8) == 0) {
+        // Rows of the next expert must not be touched, so the copy engine's boxes do not fit; a lane that stored its own row
+        // directly would write 32 rows per instruction, 32 bytes each.  Instead the warp turns [32 rows x 32 columns] around
+        // in a private buffer (16-byte chunk c of row r at c ^ (r / 2) % 4: no bank conflicts either way) and stores four
+        // neighbouring lanes to a row.
+        const uint32_t stg = smem_u32(out_stage) + (uint32_t)(grp * 4 + quarter) * 2048u;
+        const int row0 = ti.a_row0 + quarter * 32;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            sts128(stg + (uint32_t)lane * 64u + (uint32_t)((i ^ ((lane >> 1) & 3)) << 4), packed[c * 16 + 4 * i],
+                   packed[c * 16 + 4 * i + 1], packed[c * 16 + 4 * i + 2], packed[c * 16 + 4 * i + 3]);
+          __syncwarp();
+          const int col = ti.n0 + (c_first + c) * 32 + (lane & 3) * 8;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = i * 8 + (lane >> 2);
+            const uint4 v = lds128(stg + (uint32_t)r * 64u + (uint32_t)(((lane & 3) ^ ((r >> 1) & 3)) << 4));
+            if (row0 + r < ti.row_end && col < p.N)
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)(row0 + r) * p.N + col) = v;
           }
         }
         continue;
@@ -511,7 +548,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
   }
   // all roles fall through to here (also after a timed-out wait), so tensor memory is always freed
-  if (kOutTma && p.out_tma && lane == 0 && (warp >= 2 && (warp < 6 || warp >= 10))) bulk_wait0();
+  if (kOutTma && p.out_tma && lane == 0 && warp >= 2 && (warp < 6 || warp >= 10)) bulk_wait0();
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -885,7 +922,7 @@ namespace {
 template <int BN, int KB, bool kGrouped, bool kSiluQuant = false>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int max_m_tiles, cudaStream_t st,
                 const CUtensorMap* mo = nullptr) {
-  using C = Cfg<BN, KB, BN == 256 && !kGrouped && !kSiluQuant>;
+  using C = Cfg<BN, KB, out_stage_bytes<BN, kGrouped, kSiluQuant>()>;
   CUtensorMap dummy = {};
   if (mo == nullptr) {
     mo = &dummy;
@@ -907,7 +944,7 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
   if (grid > sm_count()) grid = sm_count();
   if (grid < 1) grid = 1;
   p.k_stages = (p.K + KB * 64 - 1) / (KB * 64);
-  nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant><<<(unsigned)grid, kGemmThreads, C::kSmemBytes, st>>>(ma, mb, *mo, p);
+  nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant><<<(unsigned)grid, gemm_threads(kGrouped), C::kSmemBytes, st>>>(ma, mb, *mo, p);
   return B200FP4_STATUS_SUCCESS;
 }
 
