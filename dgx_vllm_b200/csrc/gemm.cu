@@ -23,6 +23,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "grouped.cuh"
 #include "sm100_ptx.cuh"
 
 namespace b200fp4 {
@@ -34,6 +35,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const uint8_t
 namespace {
 
 constexpr int kBM = 128;
+static_assert(kBM == kGroupTileRows, "tile list");
 // Warp 0 TMA, warp 1 MMA, warps 6-9 scale factors, the others epilogue in groups of four (one warp per 32-lane quarter of
 // tensor memory): warps 2-5 and 10-13, and in the grouped kernels also 14-17 and 18-21.
 constexpr int gemm_epi_groups(bool grouped) { return grouped ? 4 : 2; }
@@ -213,12 +215,6 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(sf_full + C::kStages);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // dense mode: the status word is cleared here instead of by a separate memset (a wait only writes it after its ~1 s
-  // budget, long after this store); in grouped mode the tile-list kernel has cleared it
-  if (!kGrouped && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
-  const int m_tiles = kGrouped ? p.g_hdr[0] : p.m_tiles;
-  const int n_tiles_total = m_tiles * p.n_tiles;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
@@ -242,6 +238,13 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();                 // everything above overlaps the end of the kernel before this one
+  pdl_launch_dependents();
+  // dense mode: the status word is cleared here instead of by a separate memset (a wait only writes it after its ~1 s
+  // budget, long after this store); in grouped mode whoever made the tile list has cleared it
+  if (!kGrouped && blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;
+  const int m_tiles = kGrouped ? p.g_hdr[0] : p.m_tiles;
+  const int n_tiles_total = m_tiles * p.n_tiles;
   const int KT = (p.K + 63) / 64;   // 64-wide k-blocks = 512-byte scale tiles per 128 rows
 
   if (warp == 0) {
@@ -559,8 +562,6 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
 
 // ---------------------------------------------------------------------------------------- grouped helpers
 
-constexpr int kGroupMaxExperts = 4096;
-constexpr int kPermuteGridMinPairs = 8192;   // below this one block does the whole routing pass
 
 // One block: cuts every expert's row range into 128-row tiles.
 //   hdr[0] = number of tiles; mtiles[t] = {first row, end row of the expert, A scale-tile row, expert}
@@ -604,176 +605,6 @@ __global__ void __launch_bounds__(1024)
   if (tid == 0) hdr[0] = min(s_base, max_tiles);
 }
 
-// Routing metadata for the grouped path (one block): counts pairs per local expert and writes
-//   expert_offsets[E+1]      first permuted row of every expert
-//   blockscale_offsets[E+1]  the same with every expert padded to a multiple of 128 rows
-//   dst2src[P]               permuted row -> pair index (token*topk + slot); -1 past the last valid row
-//   src2dst[P]               pair index -> permuted row, or -1 if the pair's expert is not local
-__global__ void __launch_bounds__(1024)
-    moe_permute_kernel(const int32_t* __restrict__ topk_ids, int P, const int32_t* __restrict__ expert_map, int global_E,
-                       int E, int* expert_offsets, int* blockscale_offsets, int* dst2src, int* src2dst) {
-  __shared__ int s_count[kGroupMaxExperts];
-  __shared__ int s_scan[1024], s_scan2[1024];
-  const int tid = threadIdx.x;
-  for (int e = tid; e < E; e += 1024) s_count[e] = 0;
-  __syncthreads();
-  for (int p = tid; p < P; p += 1024) {
-    int e = topk_ids[p];
-    if (expert_map != nullptr) e = (e >= 0 && e < global_E) ? expert_map[e] : -1;
-    if (e < 0 || e >= E) e = -1;
-    src2dst[p] = e;                      // holds the local expert id until the scatter below
-    dst2src[p] = -1;
-    if (e >= 0) atomicAdd(&s_count[e], 1);
-  }
-  __syncthreads();
-  const int per = (E + 1023) / 1024;
-  int sum = 0, sum_pad = 0;
-  for (int i = 0; i < per; ++i) {
-    const int e = tid * per + i;
-    if (e < E) {
-      sum += s_count[e];
-      sum_pad += (s_count[e] + 127) / 128 * 128;
-    }
-  }
-  s_scan[tid] = sum;
-  s_scan2[tid] = sum_pad;
-  __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int v = tid >= d ? s_scan[tid - d] : 0, v2 = tid >= d ? s_scan2[tid - d] : 0;
-    __syncthreads();
-    s_scan[tid] += v;
-    s_scan2[tid] += v2;
-    __syncthreads();
-  }
-  int base = s_scan[tid] - sum, base_pad = s_scan2[tid] - sum_pad;
-  for (int i = 0; i < per; ++i) {
-    const int e = tid * per + i;
-    if (e < E) {
-      const int c = s_count[e];
-      expert_offsets[e] = base;
-      blockscale_offsets[e] = base_pad;
-      s_count[e] = base;                 // scatter cursor
-      base += c;
-      base_pad += (c + 127) / 128 * 128;
-    }
-  }
-  if (tid == 1023) {
-    expert_offsets[E] = s_scan[1023];
-    blockscale_offsets[E] = s_scan2[1023];
-  }
-  __syncthreads();
-  for (int p = tid; p < P; p += 1024) {
-    const int e = src2dst[p];
-    if (e >= 0) {
-      const int pos = atomicAdd(&s_count[e], 1);
-      src2dst[p] = pos;
-      dst2src[pos] = p;
-    }
-  }
-}
-
-// The same routing metadata for large batches, as three grid-wide steps around global counters kept in
-// expert_offsets itself (no scratch): count pairs per expert, scan, scatter with expert_offsets[e] as
-// the running cursor, then shift the cursors (now each expert's end) back into start offsets.
-// Both grid-wide passes aggregate per block in shared memory first: with skewed routing a popular expert would
-// otherwise take one global atomic per pair on a single address.
-constexpr int kPermuteBlock = 1024;
-
-__global__ void __launch_bounds__(kPermuteBlock)
-    moe_permute_count_kernel(const int32_t* __restrict__ topk_ids, int P, const int32_t* __restrict__ expert_map,
-                             int global_E, int E, int* expert_offsets, int* dst2src, int* src2dst) {
-  __shared__ int s_count[kGroupMaxExperts];
-  for (int e = threadIdx.x; e < E; e += kPermuteBlock) s_count[e] = 0;
-  __syncthreads();
-  const int p = blockIdx.x * kPermuteBlock + threadIdx.x;
-  if (p < P) {
-    int e = topk_ids[p];
-    if (expert_map != nullptr) e = (e >= 0 && e < global_E) ? expert_map[e] : -1;
-    if (e < 0 || e >= E) e = -1;
-    src2dst[p] = e;
-    dst2src[p] = -1;
-    if (e >= 0) atomicAdd(&s_count[e], 1);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += kPermuteBlock) {
-    const int c = s_count[e];
-    if (c > 0) atomicAdd(&expert_offsets[e], c);
-  }
-}
-
-__global__ void __launch_bounds__(1024)
-    moe_permute_scan_kernel(int E, int* expert_offsets, int* blockscale_offsets) {
-  __shared__ int s_scan[1024], s_scan2[1024];
-  const int tid = threadIdx.x;
-  const int per = (E + 1023) / 1024;
-  int sum = 0, sum_pad = 0;
-  for (int i = 0; i < per; ++i) {
-    const int e = tid * per + i;
-    if (e < E) {
-      const int c = expert_offsets[e];
-      sum += c;
-      sum_pad += (c + 127) / 128 * 128;
-    }
-  }
-  s_scan[tid] = sum;
-  s_scan2[tid] = sum_pad;
-  __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int v = tid >= d ? s_scan[tid - d] : 0, v2 = tid >= d ? s_scan2[tid - d] : 0;
-    __syncthreads();
-    s_scan[tid] += v;
-    s_scan2[tid] += v2;
-    __syncthreads();
-  }
-  int base = s_scan[tid] - sum, base_pad = s_scan2[tid] - sum_pad;
-  for (int i = 0; i < per; ++i) {
-    const int e = tid * per + i;
-    if (e < E) {
-      const int c = expert_offsets[e];
-      expert_offsets[e] = base;
-      blockscale_offsets[e] = base_pad;
-      base += c;
-      base_pad += (c + 127) / 128 * 128;
-    }
-  }
-  if (tid == 1023) {
-    expert_offsets[E] = s_scan[1023];
-    blockscale_offsets[E] = s_scan2[1023];
-  }
-}
-
-__global__ void __launch_bounds__(kPermuteBlock)
-    moe_permute_scatter_kernel(int P, int E, int* expert_offsets, int* dst2src, int* src2dst) {
-  __shared__ int s_count[kGroupMaxExperts];     // pairs of this block per expert, then the block's first row
-  for (int e = threadIdx.x; e < E; e += kPermuteBlock) s_count[e] = 0;
-  __syncthreads();
-  const int p = blockIdx.x * kPermuteBlock + threadIdx.x;
-  int e = -1, rank = 0;
-  if (p < P) {
-    e = src2dst[p];
-    if (e >= 0) rank = atomicAdd(&s_count[e], 1);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < E; i += kPermuteBlock) {
-    const int c = s_count[i];
-    if (c > 0) s_count[i] = atomicAdd(&expert_offsets[i], c);
-  }
-  __syncthreads();
-  if (e >= 0) {
-    const int pos = s_count[e] + rank;
-    src2dst[p] = pos;
-    dst2src[pos] = p;
-  }
-}
-
-__global__ void __launch_bounds__(1024) moe_permute_shift_kernel(int E, int* expert_offsets) {
-  __shared__ int s_end[kGroupMaxExperts];
-  for (int e = threadIdx.x; e < E; e += 1024) s_end[e] = expert_offsets[e];
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += 1024) expert_offsets[e + 1] = s_end[e];
-  if (threadIdx.x == 0) expert_offsets[0] = 0;
-}
-
 // out[i, :] = in[dst2src[i] / src_div, :] for 16-byte chunks; rows whose map entry is < 0 become zero.
 __global__ void shuffle_rows_kernel(const uint4* __restrict__ in, const int* __restrict__ dst2src, int src_div,
                                     int64_t chunks_per_row, int64_t n_dst, uint4* __restrict__ out) {
@@ -783,50 +614,6 @@ __global__ void shuffle_rows_kernel(const uint4* __restrict__ in, const int* __r
     const int src = dst2src[r];
     out[i] = src >= 0 ? in[(int64_t)(src / src_div) * chunks_per_row + c] : make_uint4(0, 0, 0, 0);
   }
-}
-
-// out[m, h] = sum over the token's slots of weight * expert_out[src2dst[m*topk + t], h] (local pairs only).
-template <typename T>
-__global__ void unpermute_reduce_kernel(const T* __restrict__ expert_out, const int* __restrict__ src2dst,
-                                        const float* __restrict__ topk_w, int M, int topk, int H, T* __restrict__ out) {
-  const int m = blockIdx.y;
-  for (int h = (blockIdx.x * blockDim.x + threadIdx.x) * 2; h < H; h += gridDim.x * blockDim.x * 2) {
-    float a0 = 0.f, a1 = 0.f;
-    for (int t = 0; t < topk; ++t) {
-      const int r = src2dst[m * topk + t];
-      if (r < 0) continue;
-      const float w = topk_w[m * topk + t];
-      a0 = fmaf(w, to_f32<T>(expert_out[(int64_t)r * H + h]), a0);
-      a1 = fmaf(w, to_f32<T>(expert_out[(int64_t)r * H + h + 1]), a1);
-    }
-    out[(int64_t)m * H + h] = from_f32<T>(a0);
-    out[(int64_t)m * H + h + 1] = from_f32<T>(a1);
-  }
-}
-
-// The same for H % 8 == 0 and 16-byte aligned rows: eight columns per thread, 16-byte loads and stores,
-// same order of additions per output element.
-template <typename T>
-__global__ void unpermute_reduce_vec8_kernel(const T* __restrict__ expert_out, const int* __restrict__ src2dst,
-                                             const float* __restrict__ topk_w, int M, int topk, int H, T* __restrict__ out) {
-  const int m = blockIdx.y;
-  const int h = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (h >= H) return;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int t = 0; t < topk; ++t) {
-    const int r = src2dst[m * topk + t];
-    if (r < 0) continue;
-    const float w = topk_w[m * topk + t];
-    const uint4 raw = *reinterpret_cast<const uint4*>(expert_out + (int64_t)r * H + h);
-    const T* v = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, to_f32<T>(v[i]), acc[i]);
-  }
-  uint4 o;
-  T* ov = reinterpret_cast<T*>(&o);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) ov[i] = from_f32<T>(acc[i]);
-  *reinterpret_cast<uint4*>(out + (int64_t)m * H + h) = o;
 }
 
 // ---------------------------------------------------------------------------------------- host
@@ -944,7 +731,11 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
   if (grid > sm_count()) grid = sm_count();
   if (grid < 1) grid = 1;
   p.k_stages = (p.K + KB * 64 - 1) / (KB * 64);
-  nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant><<<(unsigned)grid, gemm_threads(kGrouped), C::kSmemBytes, st>>>(ma, mb, *mo, p);
+  if (launch_pdl(nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant>, dim3((unsigned)grid), dim3(gemm_threads(kGrouped)), C::kSmemBytes, st,
+                 ma, mb, *mo, p) != cudaSuccess) {
+    cudaGetLastError();
+    return B200FP4_STATUS_EXECUTION_FAILED;
+  }
   return B200FP4_STATUS_SUCCESS;
 }
 
@@ -1068,15 +859,15 @@ extern "C" int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, con
 
 extern "C" size_t b200fp4_grouped_gemm_workspace_bytes(int64_t rows_capacity, int64_t E) {
   if (rows_capacity < 0 || E < 0) return 0;
-  return 256 + (size_t)(rows_capacity / kBM + E + 1) * sizeof(int4);
+  return 256 + (size_t)grouped_max_tiles(rows_capacity, E) * sizeof(int4);
 }
 
-// q_sf / q_gs non-null: the gate_up projection with SiLU(gate)*up and the NVFP4 quantization of the result in the
-// epilogue (out = packed codes [rows_capacity, N/4]).
-static int grouped_gemm_impl(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf,
-                             const float* alphas, const int32_t* expert_offsets, const int32_t* sf_offsets, void* out,
-                             int out_dtype, int64_t rows_capacity, int64_t N, int64_t K, int64_t E, int tile_n,
-                             void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs) {
+namespace b200fp4 {
+
+int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
+                 const int32_t* expert_offsets, const int32_t* sf_offsets, void* out, int out_dtype, int64_t rows_capacity, int64_t N,
+                 int64_t K, int64_t E, int tile_n, void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs,
+                 bool tiles_ready) {
   const bool fused = q_sf != nullptr;
   if (fused && (!q_gs || (N % 256) != 0 || !aligned(out, 32) || !aligned(q_sf, 4))) return B200FP4_STATUS_INVALID_VALUE;
   if (rows_capacity < 0 || N <= 0 || K <= 0 || E <= 0 || (K % 64) != 0) return B200FP4_STATUS_INVALID_VALUE;
@@ -1096,7 +887,7 @@ static int grouped_gemm_impl(const void* a_codes, const void* b_codes, const voi
     return B200FP4_STATUS_ALLOC_FAILED;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
   cudaStream_t st = (cudaStream_t)stream;
-  const int max_tiles = (int)(rows_capacity / kBM + E + 1);
+  const int max_tiles = grouped_max_tiles(rows_capacity, E);
   GemmParams p;
   p.sfa = reinterpret_cast<const uint8_t*>(a_sf);
   p.sfb = reinterpret_cast<const uint8_t*>(b_sf);
@@ -1107,9 +898,9 @@ static int grouped_gemm_impl(const void* a_codes, const void* b_codes, const voi
   p.out_tma = 0;
   p.M = (int)rows_capacity; p.N = (int)N; p.K = (int)K;
   p.m_tiles = max_tiles;
-  p.status = reinterpret_cast<int*>(workspace);
-  p.g_hdr = reinterpret_cast<int*>(workspace) + 4;
-  p.g_mtiles = reinterpret_cast<const int4*>(reinterpret_cast<unsigned char*>(workspace) + 256);
+  p.status = grouped_status(workspace);
+  p.g_hdr = grouped_hdr(workspace);
+  p.g_mtiles = grouped_tiles(workspace);
   p.g_alphas = alphas;
   p.g_sfb_expert_bytes = (long long)b200fp4_sf_swizzled_bytes(N, K / 16);
   p.q_inter = fused ? (int)(N / 2) : 0;
@@ -1129,19 +920,22 @@ static int grouped_gemm_impl(const void* a_codes, const void* b_codes, const voi
   if (!make_map(&ma, a_codes, (uint64_t)rows_capacity, (uint64_t)K / 2, kBM, kb * 32) ||
       !make_map(&mb, b_codes, (uint64_t)(E * N), (uint64_t)K / 2, fused ? 128u : (uint32_t)bn, kb * 32))
     return B200FP4_STATUS_INTERNAL_ERROR;
-  grouped_tiles_kernel<<<1, 1024, 0, st>>>(expert_offsets, sf_offsets, (int)E, const_cast<int*>(p.g_hdr),
-                                           const_cast<int4*>(p.g_mtiles), max_tiles);
+  if (!tiles_ready)
+    grouped_tiles_kernel<<<1, 1024, 0, st>>>(expert_offsets, sf_offsets, (int)E, grouped_hdr(workspace), grouped_tiles(workspace),
+                                             max_tiles);
   int rc = fused ? launch_gemm<256, 4, true, true>(ma, mb, p, max_tiles, st) : dispatch_gemm<true>(bn, kb, ma, mb, p, max_tiles, st);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
-  return finish_launch(2);
+  return finish_launch(tiles_ready ? 1 : 2);
 }
+
+}  // namespace b200fp4
 
 extern "C" int b200fp4_grouped_gemm_nvfp4(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf,
                                           const float* alphas, const int32_t* expert_offsets, const int32_t* sf_offsets,
                                           void* out, int out_dtype, int64_t rows_capacity, int64_t N, int64_t K, int64_t E,
                                           int tile_n, void* workspace, size_t workspace_bytes, void* stream) {
-  return grouped_gemm_impl(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out, out_dtype, rows_capacity,
-                           N, K, E, tile_n, workspace, workspace_bytes, stream, nullptr, nullptr);
+  return grouped_gemm(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out, out_dtype, rows_capacity, N, K, E, tile_n,
+                      workspace, workspace_bytes, stream, nullptr, nullptr, false);
 }
 
 extern "C" int b200fp4_grouped_gemm_nvfp4_silu_quant(const void* a_codes, const void* b_codes, const void* a_sf,
@@ -1151,33 +945,8 @@ extern "C" int b200fp4_grouped_gemm_nvfp4_silu_quant(const void* a_codes, const 
                                                      int64_t N, int64_t K, int64_t E, void* workspace,
                                                      size_t workspace_bytes, void* stream) {
   if (!out_sf || !out_global_scales) return B200FP4_STATUS_INVALID_VALUE;
-  return grouped_gemm_impl(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out_codes, mid_dtype,
-                           rows_capacity, N, K, E, 0, workspace, workspace_bytes, stream, out_sf, out_global_scales);
-}
-
-extern "C" int b200fp4_moe_permute(const int32_t* topk_ids, const int32_t* expert_map, int64_t global_E, int64_t M,
-                                   int64_t topk, int64_t E, int32_t* expert_offsets, int32_t* blockscale_offsets,
-                                   int32_t* dst2src, int32_t* src2dst, void* stream) {
-  if (M < 0 || topk <= 0 || E <= 0 || E > kGroupMaxExperts || M * topk > (1 << 24)) return B200FP4_STATUS_INVALID_VALUE;
-  if (!expert_offsets || !blockscale_offsets) return B200FP4_STATUS_INVALID_VALUE;
-  if (M > 0 && (!topk_ids || !dst2src || !src2dst)) return B200FP4_STATUS_INVALID_VALUE;
-  if (expert_map && global_E <= 0) return B200FP4_STATUS_INVALID_VALUE;
-  const int P = (int)(M * topk);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (P < kPermuteGridMinPairs) {
-    moe_permute_kernel<<<1, 1024, 0, st>>>(topk_ids, P, expert_map, (int)global_E, (int)E, expert_offsets,
-                                           blockscale_offsets, dst2src, src2dst);
-    return finish_launch(1);
-  }
-  if (cudaMemsetAsync(expert_offsets, 0, (size_t)(E + 1) * sizeof(int32_t), st) != cudaSuccess)
-    return B200FP4_STATUS_EXECUTION_FAILED;
-  const int blocks = (P + kPermuteBlock - 1) / kPermuteBlock;
-  moe_permute_count_kernel<<<blocks, kPermuteBlock, 0, st>>>(topk_ids, P, expert_map, (int)global_E, (int)E,
-                                                             expert_offsets, dst2src, src2dst);
-  moe_permute_scan_kernel<<<1, 1024, 0, st>>>((int)E, expert_offsets, blockscale_offsets);
-  moe_permute_scatter_kernel<<<blocks, kPermuteBlock, 0, st>>>(P, (int)E, expert_offsets, dst2src, src2dst);
-  moe_permute_shift_kernel<<<1, 1024, 0, st>>>((int)E, expert_offsets);
-  return finish_launch(4);
+  return grouped_gemm(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out_codes, mid_dtype, rows_capacity, N, K, E, 0,
+                      workspace, workspace_bytes, stream, out_sf, out_global_scales, false);
 }
 
 extern "C" int b200fp4_shuffle_rows(const void* in, int64_t row_bytes, const int32_t* dst2src, int64_t n_dst,
@@ -1193,33 +962,3 @@ extern "C" int b200fp4_shuffle_rows(const void* in, int64_t row_bytes, const int
   return finish_launch(1);
 }
 
-extern "C" int b200fp4_moe_unpermute_reduce(const void* expert_out, int dtype, const int32_t* src2dst,
-                                            const float* topk_weights, int64_t M, int64_t topk, int64_t H, void* out,
-                                            void* stream) {
-  if (M < 0 || topk <= 0 || H <= 0 || (H % 2) != 0 || M > 65535) return B200FP4_STATUS_INVALID_VALUE;
-  if (dtype != B200FP4_DTYPE_BF16 && dtype != B200FP4_DTYPE_F16) return B200FP4_STATUS_NOT_SUPPORTED;
-  if (M == 0) return B200FP4_STATUS_SUCCESS;
-  if (!expert_out || !src2dst || !topk_weights || !out) return B200FP4_STATUS_INVALID_VALUE;
-  if ((H % 8) == 0 && aligned(expert_out, 16) && aligned(out, 16)) {
-    dim3 grid8((unsigned)((H / 8 + 127) / 128), (unsigned)M);
-    if (dtype == B200FP4_DTYPE_BF16)
-      unpermute_reduce_vec8_kernel<__nv_bfloat16><<<grid8, 128, 0, (cudaStream_t)stream>>>(
-          reinterpret_cast<const __nv_bfloat16*>(expert_out), src2dst, topk_weights, (int)M, (int)topk, (int)H,
-          reinterpret_cast<__nv_bfloat16*>(out));
-    else
-      unpermute_reduce_vec8_kernel<__half><<<grid8, 128, 0, (cudaStream_t)stream>>>(
-          reinterpret_cast<const __half*>(expert_out), src2dst, topk_weights, (int)M, (int)topk, (int)H,
-          reinterpret_cast<__half*>(out));
-    return finish_launch(1);
-  }
-  dim3 grid((unsigned)((H / 2 + 127) / 128), (unsigned)M);
-  if (dtype == B200FP4_DTYPE_BF16)
-    unpermute_reduce_kernel<__nv_bfloat16><<<grid, 128, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(expert_out), src2dst, topk_weights, (int)M, (int)topk, (int)H,
-        reinterpret_cast<__nv_bfloat16*>(out));
-  else
-    unpermute_reduce_kernel<__half><<<grid, 128, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const __half*>(expert_out), src2dst, topk_weights, (int)M, (int)topk, (int)H,
-        reinterpret_cast<__half*>(out));
-  return finish_launch(1);
-}

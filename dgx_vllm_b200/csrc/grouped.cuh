@@ -1,0 +1,38 @@
+// What the steps of the grouped (per-expert) path share inside the library.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200fp4 {
+
+constexpr int kGroupMaxExperts = 4096;
+constexpr int kGroupTileRows = 128;            // rows of a grouped-GEMM tile
+
+// The tile list of the grouped GEMM, at the start of its workspace: status word (0 = ok) | ... | hdr (int 4): number of tiles |
+// ... | (byte 256) per tile {first row, end row of its expert, scale-tile row of A, expert}.
+inline int* grouped_status(void* ws) { return static_cast<int*>(ws); }
+inline int* grouped_hdr(void* ws) { return static_cast<int*>(ws) + 4; }
+inline int4* grouped_tiles(void* ws) { return reinterpret_cast<int4*>(static_cast<unsigned char*>(ws) + 256); }
+inline int grouped_max_tiles(int64_t rows, int64_t E) { return (int)(rows / kGroupTileRows + E + 1); }
+
+// Routing metadata; with tile_ws also the tile list.  At most kRouteMaxPairs pairs.  dst2src may be null.  (moe_prefill.cu)
+constexpr int64_t kRouteMaxPairs = 131072;
+void launch_moe_route(const int32_t* topk_ids, int P, const int32_t* expert_map, int global_E, int E, int32_t* expert_offsets,
+                      int32_t* blockscale_offsets, int32_t* dst2src, int32_t* src2dst, void* tile_ws, cudaStream_t st);
+
+// Token-major quantization (b200fp4_experts_quantize_scatter); zero_sf: clear the scale tensor first, as the public entry
+// does.  Without it the scale bytes of padding rows stay undefined, which the grouped GEMM does not mind: they only scale
+// rows that are never stored.  (quant.cu)
+int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
+                             const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                             int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
+                             int64_t global_E, void* codes, void* sf, void* stream, bool zero_sf);
+
+// The grouped GEMM; q_sf / q_gs non-null: the gate_up projection with SiLU(gate)*up and the NVFP4 quantization of the result
+// in the epilogue (out = packed codes [rows_capacity, N/4]).  tiles_ready: the workspace already holds the tile list.  (gemm.cu)
+int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
+                 const int32_t* expert_offsets, const int32_t* sf_offsets, void* out, int out_dtype, int64_t rows_capacity, int64_t N,
+                 int64_t K, int64_t E, int tile_n, void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs,
+                 bool tiles_ready);
+
+}  // namespace b200fp4

@@ -10,7 +10,7 @@
 // bit-identical to the reference's emulation path; the E2M1 rounding itself is the native
 // cvt.rn.satfinite.e2m1x2.f32 that replaces the reference's software routine
 // (patch_nvfp4_utils_sw_e2m1.py:31-63).
-#include "common.cuh"
+#include "grouped.cuh"
 
 namespace b200fp4 {
 
@@ -184,6 +184,11 @@ __global__ void __launch_bounds__(kTX* kTY)
 // `topk` destination rows src2dst[t*topk + s] (negative = no destination), each with the global scale of the
 // expert that owns the destination row.  Same bytes as quantizing the gathered rows one by one; the source is
 // read once instead of topk times.
+// One thread = one block of 16 elements (the block maximum needs no other lane, the scale arithmetic is done once): with two
+// lanes per block the kernel issued 70 instructions per 8 elements and destination and was bound by that (8192 x 2048, ten
+// destinations: 51-58 us, 82 % of the issue slots).  Slots whose expert has the global scale of the slot before share its
+// codes -- the arithmetic depends on nothing else -- and only store them again.  Four lanes put their scale bytes together for
+// one 4-byte store.
 constexpr int kScatterMaxTopk = 32;
 constexpr int kScatterThreads = 256;
 
@@ -197,11 +202,18 @@ __global__ void __launch_bounds__(kScatterThreads)
   __shared__ float s_gs[kScatterMaxTopk], s_rcp[kScatterMaxTopk];
   __shared__ long long s_sfrow[kScatterMaxTopk], s_code[kScatterMaxTopk];
   __shared__ int s_dst[kScatterMaxTopk];
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t t = blockIdx.x;
-  const int64_t CPR = K >> 3, KB = K >> 4, KT = (KB + 3) >> 2;
-  // the first chunk of the row is requested before the destination lookup, so the two latencies overlap
-  uint4 raw_first = make_uint4(0, 0, 0, 0);
-  if ((int64_t)threadIdx.x < CPR) raw_first = *reinterpret_cast<const uint4*>(x + t * K + (int64_t)threadIdx.x * 8);
+  const int KB = (int)(K >> 4);
+  const int64_t KT = (KB + 3) >> 2;
+  const T* row_src = x + t * K;
+  // the first piece of the row is requested before the destination lookup, so the two latencies overlap
+  uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
+  if ((int)threadIdx.x < KB) {
+    r0 = reinterpret_cast<const uint4*>(row_src)[2 * threadIdx.x];
+    r1 = reinterpret_cast<const uint4*>(row_src)[2 * threadIdx.x + 1];
+  }
   if ((int)threadIdx.x < topk) {
     const int dst = src2dst[t * topk + threadIdx.x];
     float gs = 0.f;
@@ -233,32 +245,42 @@ __global__ void __launch_bounds__(kScatterThreads)
     s_code[threadIdx.x] = (long long)dst * (long long)(K >> 1);
   }
   __syncthreads();
-  for (int64_t base = 0; base < CPR; base += kScatterThreads) {
-    const int64_t kc = base + threadIdx.x;
-    const bool ok = kc < CPR;
-    uint4 raw = raw_first;
-    if (base > 0) {
-      raw = make_uint4(0, 0, 0, 0);
-      if (ok) raw = *reinterpret_cast<const uint4*>(x + t * K + kc * 8);
+  const bool sf_words = (KB & 3) == 0;         // the four lanes of a scale word are then all inside the row
+  for (int kb0 = 0; kb0 < KB; kb0 += blockDim.x) {
+    const int kb = kb0 + threadIdx.x;
+    const bool ok = kb < KB;
+    if (kb0 > 0 && ok) {
+      r0 = reinterpret_cast<const uint4*>(row_src)[2 * kb];
+      r1 = reinterpret_cast<const uint4*>(row_src)[2 * kb + 1];
     }
-    float amax = amax8<T>(raw);
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    float v[8];
-    unpack8<T>(raw, v);
-    const float sixth = __fmul_rn(amax, 0.16666667163372039794921875f);
-    const int64_t kb = kc >> 1;
-    const int64_t sf_col = (kb >> 2) * 512 + (kb & 3);     // scale byte of this block of 16 relative to its row's first
+    float v[16];
+    unpack8<T>(r0, v);
+    unpack8<T>(r1, v + 8);
+    const float sixth = __fmul_rn(fmaxf(amax8<T>(r0), amax8<T>(r1)), 0.16666667163372039794921875f);
+    const int64_t sf_col = (int64_t)(kb >> 2) * 512 + (kb & 3);     // scale byte of this block of 16 relative to its row's first
+    uint2 packed = make_uint2(0, 0);
+    uint32_t sfb = 0, sf4 = 0;
+    float last_gs = __int_as_float(0x7FFFFFFF);                     // a NaN: equal to nothing
     for (int sl = 0; sl < topk; ++sl) {
-      const int dst = s_dst[sl];
-      if (dst < 0 || !ok) continue;
-      const float scale = fminf(__fmul_rn(s_gs[sl], sixth), 448.f);
-      const uint8_t sfb = f32_to_e4m3(scale);
-      const float os = out_scale_of(sfb, s_rcp[sl]);
-      const uint32_t packed =
-          f32x8_to_e2m1(__fmul_rn(v[0], os), __fmul_rn(v[1], os), __fmul_rn(v[2], os), __fmul_rn(v[3], os),
-                        __fmul_rn(v[4], os), __fmul_rn(v[5], os), __fmul_rn(v[6], os), __fmul_rn(v[7], os));
-      *reinterpret_cast<uint32_t*>(codes + s_code[sl] + kc * 4) = packed;
-      if ((kc & 1) == 0) sf[s_sfrow[sl] + sf_col] = sfb;
+      if (s_dst[sl] < 0) continue;
+      const float gs = s_gs[sl];
+      if (gs != last_gs) {
+        last_gs = gs;
+        sfb = f32_to_e4m3(fminf(__fmul_rn(gs, sixth), 448.f));
+        const float os = out_scale_of((uint8_t)sfb, s_rcp[sl]);
+        packed.x = f32x8_to_e2m1(__fmul_rn(v[0], os), __fmul_rn(v[1], os), __fmul_rn(v[2], os), __fmul_rn(v[3], os),
+                                 __fmul_rn(v[4], os), __fmul_rn(v[5], os), __fmul_rn(v[6], os), __fmul_rn(v[7], os));
+        packed.y = f32x8_to_e2m1(__fmul_rn(v[8], os), __fmul_rn(v[9], os), __fmul_rn(v[10], os), __fmul_rn(v[11], os),
+                                 __fmul_rn(v[12], os), __fmul_rn(v[13], os), __fmul_rn(v[14], os), __fmul_rn(v[15], os));
+        sf4 = sfb << (8 * (threadIdx.x & 3));
+        sf4 |= __shfl_xor_sync(0xffffffffu, sf4, 1);
+        sf4 |= __shfl_xor_sync(0xffffffffu, sf4, 2);
+      }
+      if (ok) {
+        *reinterpret_cast<uint2*>(codes + s_code[sl] + kb * 8) = packed;
+        if (!sf_words) sf[s_sfrow[sl] + sf_col] = (uint8_t)sfb;
+        else if ((threadIdx.x & 3) == 0) *reinterpret_cast<uint32_t*>(sf + s_sfrow[sl] + sf_col) = sf4;
+      }
     }
   }
 }
@@ -348,12 +370,12 @@ extern "C" int b200fp4_experts_quantize(const void* x, int in_dtype, int64_t M, 
                                sf_rows_padded, silu_mul, codes, sf, stream, nullptr, 1);
 }
 
-extern "C" int b200fp4_experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk,
-                                                const int32_t* src2dst, const float* global_scales,
-                                                const int32_t* expert_offsets, const int32_t* blockscale_offsets,
-                                                int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids,
-                                                const int32_t* expert_map, int64_t global_E, void* codes, void* sf,
-                                                void* stream) {
+namespace b200fp4 {
+
+int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
+                             const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                             int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
+                             int64_t global_E, void* codes, void* sf, void* stream, bool zero_sf) {
   if (expert_map && (!topk_ids || global_E <= 0)) return B200FP4_STATUS_INVALID_VALUE;
   if (n_src < 0 || K <= 0 || (K % 16) != 0 || topk <= 0 || num_experts <= 0 || sf_rows_padded < 0 ||
       (sf_rows_padded % 128) != 0)
@@ -361,23 +383,37 @@ extern "C" int b200fp4_experts_quantize_scatter(const void* x, int in_dtype, int
   if (in_dtype != B200FP4_DTYPE_F16 && in_dtype != B200FP4_DTYPE_BF16) return B200FP4_STATUS_NOT_SUPPORTED;
   if (topk > kScatterMaxTopk || n_src > 0x7FFFFFFF) return B200FP4_STATUS_NOT_SUPPORTED;
   if (!global_scales || !expert_offsets || !blockscale_offsets || !sf) return B200FP4_STATUS_INVALID_VALUE;
-  if (n_src > 0 && (!x || !codes || !src2dst || !aligned(x, 16) || !aligned(codes, 4))) return B200FP4_STATUS_INVALID_VALUE;
+  if (n_src > 0 && (!x || !codes || !src2dst || !aligned(x, 16) || !aligned(codes, 8) || !aligned(sf, 4)))
+    return B200FP4_STATUS_INVALID_VALUE;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t KB = K / 16;
-  if (cudaMemsetAsync(sf, 0, (size_t)(sf_rows_padded * (((KB + 3) / 4) * 4)), st) != cudaSuccess) {
+  if (zero_sf && cudaMemsetAsync(sf, 0, (size_t)(sf_rows_padded * (((KB + 3) / 4) * 4)), st) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;
   }
   if (n_src == 0) return finish_launch(1);
+  const unsigned threads = (unsigned)(KB >= kScatterThreads ? kScatterThreads : (KB + 31) / 32 * 32);
   if (in_dtype == B200FP4_DTYPE_BF16)
-    experts_quantize_scatter_kernel<__nv_bfloat16><<<(unsigned)n_src, kScatterThreads, 0, st>>>(
-        reinterpret_cast<const __nv_bfloat16*>(x), K, (int)topk, src2dst, global_scales, expert_offsets, blockscale_offsets,
-        num_experts, topk_ids, expert_map, (int)global_E, (uint8_t*)codes, (uint8_t*)sf);
+    launch_pdl(experts_quantize_scatter_kernel<__nv_bfloat16>, dim3((unsigned)n_src), dim3(threads), 0, st,
+               reinterpret_cast<const __nv_bfloat16*>(x), K, (int)topk, src2dst, global_scales, expert_offsets, blockscale_offsets,
+               num_experts, topk_ids, expert_map, (int)global_E, (uint8_t*)codes, (uint8_t*)sf);
   else
-    experts_quantize_scatter_kernel<__half><<<(unsigned)n_src, kScatterThreads, 0, st>>>(
-        reinterpret_cast<const __half*>(x), K, (int)topk, src2dst, global_scales, expert_offsets, blockscale_offsets,
-        num_experts, topk_ids, expert_map, (int)global_E, (uint8_t*)codes, (uint8_t*)sf);
-  return finish_launch(2);
+    launch_pdl(experts_quantize_scatter_kernel<__half>, dim3((unsigned)n_src), dim3(threads), 0, st, reinterpret_cast<const __half*>(x), K,
+               (int)topk, src2dst, global_scales, expert_offsets, blockscale_offsets, num_experts, topk_ids, expert_map, (int)global_E,
+               (uint8_t*)codes, (uint8_t*)sf);
+  return finish_launch(zero_sf ? 2 : 1);
+}
+
+}  // namespace b200fp4
+
+extern "C" int b200fp4_experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk,
+                                                const int32_t* src2dst, const float* global_scales,
+                                                const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                                                int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids,
+                                                const int32_t* expert_map, int64_t global_E, void* codes, void* sf,
+                                                void* stream) {
+  return experts_quantize_scatter(x, in_dtype, n_src, K, topk, src2dst, global_scales, expert_offsets, blockscale_offsets, num_experts,
+                                  sf_rows_padded, topk_ids, expert_map, global_E, codes, sf, stream, true);
 }
 
 extern "C" int b200fp4_experts_quantize_gather(const void* x, int in_dtype, int64_t M, int64_t K, const float* global_scales,
