@@ -3,7 +3,7 @@
 // Replaces the GEMM behind cuda_fp4_gemm.h / cutlass_scaled_fp4_mm in the reference (whose own
 // kernels are scalar CUDA-core loops, cutlass_nvfp4/nvfp4_gemm_kernel.cuh:296-345) with a
 // tcgen05 design:
-//   * persistent, warp-specialised CTAs (one per SM): warp 0 issues TMA loads, warp 1 issues
+//   * persistent, warp-specialised CTAs (one per SM): three warps issue the copies, one issues
 //     tcgen05.mma, further warps, in groups of four, move scale factors and run the epilogue;
 //   * operands are packed E2M1 bytes, K-major, staged by 2-D TMA (no multicast) into 128-byte
 //     swizzled shared-memory tiles of 128 (A) / BN (B) rows x 256 k; scale factors come from the
@@ -36,10 +36,13 @@ namespace {
 
 constexpr int kBM = 128;
 static_assert(kBM == kGroupTileRows, "tile list");
-// Warp 0 TMA, warp 1 MMA, warps 6-9 scale factors, the others epilogue in groups of four (one warp per 32-lane quarter of
+// Warp 0 copies of the operands, warp 1 MMA, warps 6-9 scale factors into tensor memory, the others epilogue in groups of four (one warp per 32-lane quarter of
 // tensor memory): warps 2-5 and 10-13, and in the grouped kernels also 14-17 and 18-21.
 constexpr int gemm_epi_groups(bool grouped) { return grouped ? 4 : 2; }
-constexpr int gemm_threads(bool grouped) { return 32 * (6 + 4 * gemm_epi_groups(grouped)); }
+// The last warp issues the copies of scale factors (one thread issues a copy every 70-80 cycles and spends about 300 more per
+// stage on its barriers).
+constexpr int gemm_warps(bool grouped) { return 7 + 4 * gemm_epi_groups(grouped); }
+constexpr int gemm_threads(bool grouped) { return 32 * gemm_warps(grouped); }
 constexpr uint32_t kTmemCols = 512;
 
 struct GemmParams {
@@ -210,16 +213,14 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   uint64_t* empty_bar = bars + C::kStages;
   uint64_t* acc_full = bars + 2 * C::kStages;
   uint64_t* acc_empty = acc_full + C::kAcc;
-  uint64_t* sf_ready = acc_empty + C::kAcc;
-  uint64_t* sf_full = sf_ready + C::kStages;     // scale factors of the stage have landed (before the operands)
+  uint64_t* sf_full = acc_empty + C::kAcc;     // scale factors of the stage have landed (before the operands)
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(sf_full + C::kStages);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&full_bar[s]), 5);       // the operand copies, and each scale-factor warp
       mbar_init(smem_u32(&empty_bar[s]), 1);
-      mbar_init(smem_u32(&sf_ready[s]), 4);       // one arrival per scale-factor warp
       mbar_init(smem_u32(&sf_full[s]), 1);
     }
     for (int a = 0; a < C::kAcc; ++a) {
@@ -247,70 +248,85 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   const int n_tiles_total = m_tiles * p.n_tiles;
   const int KT = (p.K + 63) / 64;   // 64-wide k-blocks = 512-byte scale tiles per 128 rows
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  constexpr int kWarpSf = gemm_warps(kGrouped) - 1;
+  if (warp == 0 || warp == kWarpSf) {
+    // ------------------------------------------------------------------ copies into shared memory: operands, scale factors
     if (lane == 0) {
-      uint32_t it = 0;
+      uint32_t s = 0, ph = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x) {
         const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, tile, m_tiles);
-        const uint8_t* sfb_base = p.sfb + (kGrouped ? (size_t)ti.expert * (size_t)p.g_sfb_expert_bytes : (size_t)0);
-        for (int ks = 0; ks < p.k_stages; ++ks, ++it) {
-          const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1;
+        const uint8_t* sfa = p.sfa + (size_t)ti.sfa_tile * KT * 512;
+        const uint8_t* sfb = p.sfb + (kGrouped ? (size_t)ti.expert * (size_t)p.g_sfb_expert_bytes : (size_t)0);
+        const uint8_t* sfb0 = sfb + (size_t)ti.sfb_tile0 * KT * 512;
+        const uint8_t* sfb1 = sfb + (size_t)ti.sfb_tile1 * KT * 512;
+        const int sf_tiles = C::kSfTiles == 1 || ti.sfb_tile1 * 128 >= p.N ? 1 : 2;      // the second 128 columns may lie past N
+        for (int ks = 0; ks < p.k_stages; ++ks) {
           if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, p.status, 1)) { ok = false; break; }
-          unsigned char* st = smem + (size_t)s * C::kStageBytes;
-          const int kblocks = min(KB, KT - ks * KB);
-          int sf_tiles = 0;
-          for (int j = 0; j < C::kSfTiles; ++j) sf_tiles += ((j == 0 ? ti.sfb_tile0 : ti.sfb_tile1) * 128 < p.N) ? 1 : 0;
-          // the small scale-factor copies go first and on their own barrier, so the scale warps can
-          // move them into tensor memory while the operand tiles are still in flight
-          const uint32_t sbar = smem_u32(&sf_full[s]);
-          mbar_expect_tx(sbar, (uint32_t)(kblocks * 512 * (1 + sf_tiles)));
-          bulk_load_1d(smem_u32(st + C::kStageA + C::kStageB), p.sfa + ((size_t)ti.sfa_tile * KT + (size_t)ks * KB) * 512,
-                       (uint32_t)kblocks * 512, sbar);
-          for (int j = 0; j < sf_tiles; ++j)
-            bulk_load_1d(smem_u32(st + C::kStageA + C::kStageB + C::kStageSFA + j * (KB * 512)),
-                         sfb_base + ((size_t)(j == 0 ? ti.sfb_tile0 : ti.sfb_tile1) * KT + (size_t)ks * KB) * 512,
-                         (uint32_t)kblocks * 512, sbar);
-          const uint32_t bar = smem_u32(&full_bar[s]);
-          mbar_expect_tx(bar, (uint32_t)(C::kStageA + C::kStageB));
-          tma_load_2d(smem_u32(st), &map_a, ks * C::kRowBytes, ti.a_row0, bar);
-          if (kSiluQuant) {
-            // map_b's box is 128 rows here: the gate rows and the up rows of the tile land one after the other
-            tma_load_2d(smem_u32(st + C::kStageA), &map_b, ks * C::kRowBytes, ti.b_row0, bar);
-            tma_load_2d(smem_u32(st + C::kStageA + 128 * C::kRowBytes), &map_b, ks * C::kRowBytes, ti.b_row1, bar);
+          const uint32_t st = smem_u32(smem) + s * C::kStageBytes, bar = smem_u32(&full_bar[s]);
+          if (warp == 0) {
+            mbar_expect_tx(bar, (uint32_t)(C::kStageA + C::kStageB));
+            tma_load_2d(st, &map_a, ks * C::kRowBytes, ti.a_row0, bar);
+            tma_load_2d(st + C::kStageA, &map_b, ks * C::kRowBytes, ti.b_row0, bar);
+            // with SiLU map_b's box is 128 rows: the gate rows and the up rows of the tile land one after the other
+            if (kSiluQuant) tma_load_2d(st + C::kStageA + 128 * C::kRowBytes, &map_b, ks * C::kRowBytes, ti.b_row1, bar);
           } else {
-            tma_load_2d(smem_u32(st + C::kStageA), &map_b, ks * C::kRowBytes, ti.b_row0, bar);
+            // scale factors have their own barrier, so that the scale warps can move them into tensor memory while the
+            // operand tiles are still in flight
+            const uint32_t bytes = (uint32_t)min(KB, KT - ks * KB) * 512, off = (uint32_t)ks * (KB * 512);
+            const uint32_t sbar = smem_u32(&sf_full[s]), dst = st + C::kStageA + C::kStageB;
+            mbar_expect_tx(sbar, bytes * (1 + sf_tiles));
+            bulk_load_1d(dst, sfa + off, bytes, sbar);
+            bulk_load_1d(dst + C::kStageSFA, sfb0 + off, bytes, sbar);
+            if (sf_tiles > 1) bulk_load_1d(dst + C::kStageSFA + KB * 512, sfb1 + off, bytes, sbar);
+          }
+          if (++s == C::kStages) {
+            s = 0;
+            ph ^= 1;
           }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
+    // The thread can run only one or two MMAs ahead of the tensor core, so whatever it does between stages leaves the tensor
+    // core idle: with two barriers per stage, descriptors built per MMA and the wait after the fourth MMA it spent 280 cycles
+    // per stage on that (a stage of four 128 x 256 x 64 MMAs is 512 cycles).  Hence one barrier per stage (operands landed and
+    // scales in tensor memory), descriptors by addition, and a look at the next stage's barrier before the last MMA.
     if (lane == 0) {
-      uint32_t it = 0, tcount = 0;
-      bool ok = true;
+      const uint64_t a_desc0 = desc_kmajor<C::kRowBytes>(smem_u32(smem)), b_desc0 = desc_kmajor<C::kRowBytes>(smem_u32(smem) + C::kStageA);
+      const uint32_t full0 = smem_u32(full_bar);
+      uint32_t s = 0, ph = 0, tcount = 0;
+      bool ok = true, ready = false;
       for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x, ++tcount) {
         const uint32_t acc = tcount % C::kAcc, aph = (tcount / C::kAcc) & 1;
         if (!mbar_wait(smem_u32(&acc_empty[acc]), aph ^ 1, p.status, 2)) { ok = false; break; }
-        tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int ks = 0; ks < p.k_stages; ++ks, ++it) {
-          const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1;
-          if (!mbar_wait(smem_u32(&full_bar[s]), ph, p.status, 3)) { ok = false; break; }
+        for (int ks = 0; ks < p.k_stages; ++ks) {
+          if (!ready && !mbar_wait(full0 + s * 8, ph, p.status, 3)) { ok = false; break; }
           tcgen05_fence_after();
-          unsigned char* st = smem + (size_t)s * C::kStageBytes;
-          const int kblocks = min(KB, KT - ks * KB);
-          const uint32_t a_addr = smem_u32(st), b_addr = smem_u32(st + C::kStageA);
+          // each 64-wide k-block is 32 bytes further along the swizzled 128-byte rows (descriptors count 16 bytes)
+          const uint64_t a_desc = a_desc0 + s * (C::kStageBytes >> 4), b_desc = b_desc0 + s * (C::kStageBytes >> 4);
           const uint32_t sfa_tmem = tmem_base + C::kSfBase + s * C::kSfCols, sfb_tmem = sfa_tmem + 4 * KB;
-          if (!mbar_wait(smem_u32(&sf_ready[s]), ph, p.status, 5)) { ok = false; break; }
-          tcgen05_fence_after();
-          for (int kb = 0; kb < kblocks; ++kb) {
-            // each 64-wide k-block is 32 bytes further along the swizzled 128-byte rows
-            tcgen05_mma_nvf4(d_tmem, desc_kmajor<C::kRowBytes>(a_addr + kb * 32), desc_kmajor<C::kRowBytes>(b_addr + kb * 32),
-                             C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles), (ks > 0 || kb > 0) ? 1u : 0u);
+          const uint32_t empty = smem_u32(&empty_bar[s]);
+          const uint32_t s_next = s + 1 == C::kStages ? 0 : s + 1, ph_next = s + 1 == C::kStages ? ph ^ 1 : ph;
+          const int kblocks = min(KB, KT - ks * KB);
+          if (kblocks == KB) {
+#pragma unroll
+            for (int kb = 0; kb < KB; ++kb) {
+              if (kb == KB - 1) ready = mbar_test_wait(full0 + s_next * 8, ph_next);
+              tcgen05_mma_nvf4(d_tmem, a_desc + kb * 2, b_desc + kb * 2, C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles),
+                               (ks > 0 || kb > 0) ? 1u : 0u);
+            }
+          } else {
+            ready = false;
+            for (int kb = 0; kb < kblocks; ++kb)
+              tcgen05_mma_nvf4(d_tmem, a_desc + kb * 2, b_desc + kb * 2, C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles),
+                               (ks > 0 || kb > 0) ? 1u : 0u);
           }
-          tcgen05_commit(smem_u32(&empty_bar[s]));    // frees the stage when these MMAs have read it
+          tcgen05_commit(empty);    // frees the stage when these MMAs have read it
+          s = s_next;
+          ph = ph_next;
         }
         if (ok) tcgen05_commit(smem_u32(&acc_full[acc]));
       }
@@ -343,7 +359,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         tcgen05_wait_st();
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sf_ready[s]));
+        if (lane == 0) mbar_arrive(smem_u32(&full_bar[s]));
       }
     }
   } else {
@@ -376,31 +392,18 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         // computed exactly as the separate SiLU-mul quantizer does from the 16-bit rounded GEMM output.
         const float gs = p.q_gs[ti.expert];
         const float rcp_gs = __frcp_rn(gs + (gs == 0.f ? 1.0e8f : 0.f));
-        // drain both halves as 16-bit pairs (the rounding the separate GEMM's output has), hand the accumulator
-        // back, and only then do the SiLU / quantization arithmetic, so that it overlaps the next tile's main loop
-        uint32_t pg[16], pu[16];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t r[32];
-          tcgen05_ld_32x32(taddr + c * 128 + grp * 32, r);
-          tcgen05_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float v0 = __uint_as_float(r[2 * i]) * alpha, v1 = __uint_as_float(r[2 * i + 1]) * alpha;
-            uint32_t w;
-            if (p.out_bf16) {
-              const __nv_bfloat162 v = __floats2bfloat162_rn(v0, v1);
-              w = *reinterpret_cast<const uint32_t*>(&v);
-            } else {
-              const __half2 v = __floats2half2_rn(v0, v1);
-              w = *reinterpret_cast<const uint32_t*>(&v);
-            }
-            (c ? pu : pg)[i] = w;
-          }
-        }
+        // read both halves, hand the accumulator back, and only then round to 16-bit pairs (as the separate GEMM's output is)
+        // and do the SiLU / quantization arithmetic, so that all of it overlaps the next tile's main loop
+        uint32_t rg[32], ru[32];
+        tcgen05_ld_32x32(taddr + grp * 32, rg);
+        tcgen05_ld_32x32(taddr + 128 + grp * 32, ru);
+        tcgen05_wait_ld();
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
+        uint32_t pg[16], pu[16];
+        pack_row(rg, alpha, p.out_bf16 != 0, pg);
+        pack_row(ru, alpha, p.out_bf16 != 0, pu);
         // rows past the end of the expert are never stored: warps whose 32 rows are all past it skip the arithmetic
         if (row < ti.row_end) {
           uint32_t codes[4];
@@ -445,32 +448,24 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
         continue;
       }
-      // drain this thread's row of the accumulator into packed 16-bit registers ...
+      // Drain this thread's row of the accumulator into packed 16-bit registers, two loads of 32 columns in flight; the
+      // accumulator goes back to the MMA warp after the last loads, before their conversion and the stores, which then
+      // overlap the next tile's main loop.
       uint32_t packed[16 * CH];
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        uint32_t r[32];
-        tcgen05_ld_32x32(taddr + (c_first + c) * 32, r);
+      for (int c = 0; c < CH; c += 2) {
+        uint32_t r0[32], r1[32];
+        tcgen05_ld_32x32(taddr + (c_first + c) * 32, r0);
+        if (c + 1 < CH) tcgen05_ld_32x32(taddr + (c_first + c + 1) * 32, r1);
         tcgen05_wait_ld();
-        if (p.out_bf16) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
-            packed[c * 16 + i] = *reinterpret_cast<uint32_t*>(&v);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            __half2 v = __floats2half2_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
-            packed[c * 16 + i] = *reinterpret_cast<uint32_t*>(&v);
-          }
+        if (c + 2 >= CH) {
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
         }
+        pack_row(r0, alpha, p.out_bf16 != 0, packed + c * 16);
+        if (c + 1 < CH) pack_row(r1, alpha, p.out_bf16 != 0, packed + (c + 1) * 16);
       }
-      // ... hand the accumulator back to the MMA warp, and only then write to global memory, so
-      // that the stores overlap the next tile's main loop
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
       if constexpr (kOutTma) if (p.out_tma) {
         // This warp's 32 rows x 128 columns leave in two halves of 64 columns (128 bytes per row): rows go to a private
         // staging buffer with the 128-byte swizzle of the tensor map (16-byte chunk c of row r at c ^ (r % 8): the

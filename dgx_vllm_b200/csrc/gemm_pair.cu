@@ -8,7 +8,7 @@
 //
 // Roles per CTA (23 warps): warp 0 loads operands, warp 1 issues the MMAs (leader CTA only) and owns tensor memory,
 // warps 2-5, 10-13 and 15-22 drain and store the CTA's 128 accumulator rows (four warps per tensor-memory lane quarter, 64
-// columns each: the one accumulator is handed back after two tcgen05.ld per warp), warps 6-9 move scale factors from
+// columns each: the one accumulator is handed back after two tcgen05.ld per warp, before their conversion), warps 6-9 move scale factors from
 // shared memory into tensor memory, warp 14 loads scale factors.
 //
 // What keeps the stage loop short (a stage = 256 k = 4 MMAs = about 700 cycles, less than the latency of a load, so
@@ -18,11 +18,11 @@
 //   * tcgen05.commit with a CTA mask frees the stage (`empty`) and publishes the accumulator (`acc_full`) in both CTAs;
 //   * scale factors have their own, deeper ring in shared memory (10 stages of 6 KiB, loaded well ahead of the operands),
 //     so that when a scale slot of tensor memory frees up its data is already on chip: the scale warps copy it with
-//     three 16-column tcgen05.st and arrive on the leader's `sf_ready` (remotely from the peer);
+//     three 16-column tcgen05.st and arrive on the leader's `full` (remotely from the peer);
 //   * arrivals on a barrier of the other CTA are RELAXED at cluster scope: with release semantics each one stalled the
 //     arriving warp for about 1100 cycles and the whole kernel ran at one stage per 2000 cycles (242 us).
-// Where the cycles of the MMA thread go (M=4096, per pair): issuing 75 %, waiting for scales 10 %, for operands 7 %, for
-// the single accumulator to be drained 8 %.
+// The MMA thread waits on one barrier per stage and looks at the next one before a stage's last MMA (M=4096, quantizer
+// included, under the power cap: 149 us with two barriers per stage and descriptors built per MMA, 139 us so).
 // No copy uses cluster multicast.  Every wait is bounded and reports through the status word; the pair leaves through a
 // cluster barrier so neither CTA frees tensor memory or exits while the other may still signal it.
 #include "sm100_ptx.cuh"
@@ -120,10 +120,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* sf_ring = smem + (size_t)kPStages * kPStageOp;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sf_ring + (size_t)kPSfStages * kPSfStage);
-  uint64_t* full_bar = bars;                         // leader's: the operands of both CTAs have landed
+  uint64_t* full_bar = bars;                         // leader's: operands of both CTAs have landed, their scales are in tensor memory
   uint64_t* empty_bar = full_bar + kPStages;         // own: the MMAs that read the stage (and its scale slot) are done
-  uint64_t* sf_ready = empty_bar + kPStages;         // leader's: both CTAs' scales of the stage are in tensor memory
-  uint64_t* sf_full = sf_ready + kPStages;           // own: scale-factor slot has landed in shared memory
+  uint64_t* sf_full = empty_bar + kPStages;          // own: scale-factor slot has landed in shared memory
   uint64_t* sf_free = sf_full + kPSfStages;          // own: scale-factor slot has been copied to tensor memory
   uint64_t* acc_full = sf_free + kPSfStages;         // own: accumulator complete
   uint64_t* acc_empty = acc_full + 1;                // leader's: both epilogues have drained
@@ -138,9 +137,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPStages; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&full_bar[s]), 9);       // the operand copies, and each scale warp of both CTAs
       mbar_init(smem_u32(&empty_bar[s]), 1);
-      mbar_init(smem_u32(&sf_ready[s]), 8);       // one arrival per scale warp of both CTAs
     }
     for (int j = 0; j < kPSfStages; ++j) {
       mbar_init(smem_u32(&sf_full[j]), 1);
@@ -209,25 +207,40 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
+    // The thread runs only one or two MMAs ahead of the tensor cores, so what it does between stages leaves them idle: one
+    // barrier per stage, descriptors by addition, and a look at the next stage's barrier before the last MMA of a stage.
     if (leader && lane == 0) {
-      uint32_t it = 0, tcount = 0;
-      bool ok = true;
+      const uint64_t a_desc0 = desc_kmajor<128>(smem_u32(smem)), b_desc0 = desc_kmajor<128>(smem_u32(smem) + kPStageA);
+      const uint32_t full0 = smem_u32(full_bar);
+      uint32_t s = 0, ph = 0, tcount = 0;
+      bool ok = true, ready = false;
       for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs, ++tcount) {
         if (!mbar_wait(smem_u32(acc_empty), (tcount & 1) ^ 1, p.status, 23)) { ok = false; break; }
-        tcgen05_fence_after();
-        for (int ks = 0; ks < p.k_stages; ++ks, ++it) {
-          const uint32_t s = it % kPStages, ph = (it / kPStages) & 1;
-          if (!mbar_wait(smem_u32(&sf_ready[s]), ph, p.status, 24)) { ok = false; break; }
-          if (!mbar_wait(smem_u32(&full_bar[s]), ph, p.status, 25)) { ok = false; break; }
+        for (int ks = 0; ks < p.k_stages; ++ks) {
+          if (!ready && !mbar_wait(full0 + s * 8, ph, p.status, 25)) { ok = false; break; }
           tcgen05_fence_after();
-          unsigned char* st = smem + (size_t)s * kPStageOp;
-          const int kblocks = min(4, KT - ks * 4);
-          const uint32_t a_addr = smem_u32(st), b_addr = smem_u32(st + kPStageA);
+          const uint64_t a_desc = a_desc0 + s * (kPStageOp >> 4), b_desc = b_desc0 + s * (kPStageOp >> 4);
           const uint32_t sfa_tmem = tmem_base + kPSfBase + s * kPSfCols, sfb_tmem = sfa_tmem + 16;
-          for (int kb = 0; kb < kblocks; ++kb)
-            tcgen05_mma_nvf4_pair(tmem_base, desc_kmajor<128>(a_addr + kb * 32), desc_kmajor<128>(b_addr + kb * 32), kPIdesc,
-                                  sfa_tmem + kb * 4, sfb_tmem + kb * 8, (ks > 0 || kb > 0) ? 1u : 0u);
-          tcgen05_commit_pair(smem_u32(&empty_bar[s]), 3);     // both CTAs may refill this stage and its scale slot
+          const uint32_t empty = smem_u32(&empty_bar[s]);
+          const bool wrap = s + 1 == kPStages;
+          const uint32_t s_next = wrap ? 0 : s + 1, ph_next = wrap ? ph ^ 1 : ph;
+          const int kblocks = min(4, KT - ks * 4);
+          if (kblocks == 4) {
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+              if (kb == 3) ready = mbar_test_wait(full0 + s_next * 8, ph_next);
+              tcgen05_mma_nvf4_pair(tmem_base, a_desc + kb * 2, b_desc + kb * 2, kPIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * 8,
+                                    (ks > 0 || kb > 0) ? 1u : 0u);
+            }
+          } else {
+            ready = false;
+            for (int kb = 0; kb < kblocks; ++kb)
+              tcgen05_mma_nvf4_pair(tmem_base, a_desc + kb * 2, b_desc + kb * 2, kPIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * 8,
+                                    (ks > 0 || kb > 0) ? 1u : 0u);
+          }
+          tcgen05_commit_pair(empty, 3);                          // both CTAs may refill this stage and its scale slot
+          s = s_next;
+          ph = ph_next;
         }
         if (ok) tcgen05_commit_pair(smem_u32(acc_full), 3);     // both epilogues may start
       }
@@ -237,7 +250,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     // One warp per tensor-memory lane quarter.  (A second group of four warps taking alternate stages, and stores left
     // in flight across the next stage's waits, were both measured: no gain.)
     const int quarter = warp & 3;
-    const uint32_t ready_leader = map_to_cta(smem_u32(&sf_ready[0]), 0);
+    const uint32_t ready_leader = map_to_cta(smem_u32(&full_bar[0]), 0);
     uint32_t it = 0;
     bool ok = true;
     for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs) {
@@ -287,30 +300,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       tcgen05_fence_after();
       const int row = mp * 256 + (int)rank * 128 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-      uint32_t packed[32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t r[32];
-        tcgen05_ld_32x32(taddr + (c_first + c) * 32, r);
-        tcgen05_wait_ld();
-        if (p.out_bf16) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
-            packed[c * 16 + i] = *reinterpret_cast<uint32_t*>(&v);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            __half2 v = __floats2half2_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
-            packed[c * 16 + i] = *reinterpret_cast<uint32_t*>(&v);
-          }
-        }
-      }
-      // hand the accumulator back before the global stores, which then overlap the next tile's main loop
+      // both loads in flight; the accumulator goes back before the conversion and the global stores, which then overlap
+      // the next tile's main loop
+      uint32_t packed[32], r0[32], r1[32];
+      tcgen05_ld_32x32(taddr + c_first * 32, r0);
+      tcgen05_ld_32x32(taddr + (c_first + 1) * 32, r1);
+      tcgen05_wait_ld();
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
+      pack_row(r0, alpha, p.out_bf16 != 0, packed);
+      pack_row(r1, alpha, p.out_bf16 != 0, packed + 16);
       if (row < p.M) {
         uint16_t* dst_row = reinterpret_cast<uint16_t*>(p.out) + (size_t)row * p.N;
 #pragma unroll

@@ -52,9 +52,14 @@ __global__ void __cluster_dims__(kRouteBlocks, 1, 1) __launch_bounds__(kRouteThr
 #pragma unroll
   for (int i = 0; i < kRoutePer; ++i) {
     const int p = (i * kRouteBlocks + (int)rank) * kRouteThreads + tid;
-    er[i] = -1;
+    er[i] = p < P ? topk_ids[p] : -1;            // all in flight together
+  }
+#pragma unroll
+  for (int i = 0; i < kRoutePer; ++i) {
+    const int p = (i * kRouteBlocks + (int)rank) * kRouteThreads + tid;
     if (p < P) {
-      int e = topk_ids[p];
+      int e = er[i];
+      er[i] = -1;
       if (expert_map != nullptr) e = (e >= 0 && e < global_E) ? expert_map[e] : -1;
       if (e >= 0 && e < E) er[i] = e << 16 | atomicAdd(&s_count[e], 1);
     }

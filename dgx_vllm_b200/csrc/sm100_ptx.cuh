@@ -39,6 +39,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// one look, without waiting
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait: returns false (and records `code`) if the phase does not complete in ~1 s.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -129,6 +143,23 @@ __device__ __forceinline__ void tcgen05_st_32x32_x4(uint32_t taddr, const uint4&
                : "memory");
 }
 __device__ __forceinline__ void tcgen05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// 32 accumulator columns times alpha -> 16 pairs of 16-bit values
+__device__ __forceinline__ void pack_row(const uint32_t (&r)[32], float alpha, bool bf16, uint32_t* out) {
+  if (bf16) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
+      out[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const __half2 v = __floats2half2_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
+      out[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  }
+}
 
 // Shared-memory matrix descriptors (K-major).  Fields: start address >> 4 in bits [0,14), leading
 // byte offset >> 4 in [16,30), stride byte offset >> 4 in [32,46), descriptor version 1 in
