@@ -133,8 +133,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   const bool leader = rank == 0;
   const int n_pairs = gridDim.x >> 1, pair = blockIdx.x >> 1;
   const int n_tiles_total = p.m_pairs * p.n_tiles;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;    // a wait writes it only after its ~1 s budget
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPStages; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 9);       // the operand copies, and each scale warp of both CTAs
@@ -158,6 +156,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   const int KT = (p.K + 63) / 64;
+  pdl_wait();                 // everything above overlaps the end of the kernel before this one
+  pdl_launch_dependents();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *p.status = 0;    // a wait writes it only after its ~1 s budget
 
   if (warp == 0) {
     // ------------------------------------------------------------------ operand loads (both CTAs)
@@ -361,7 +362,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const uint8_t
   cfg.blockDim = dim3(kPairThreads);
   cfg.dynamicSmemBytes = kPairSmemBytes;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -393,6 +394,10 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const uint8_t
   if (pairs > max_pairs_of[dev]) pairs = max_pairs_of[dev];
   if (pairs < 1) pairs = 1;
   cfg.gridDim = dim3((unsigned)(2 * pairs));
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // as in launch_pdl
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cfg.numAttrs = (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel, ma, mb, p) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;

@@ -56,3 +56,23 @@ def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
     assert clear.float().mean() > 0.8
     assert torch.equal(ids[clear].long(), ref_ids[clear])
     assert ((tw[clear].double() - w[clear]).abs() / w[clear]).max() < 1e-4
+
+
+@pytest.mark.parametrize("M,K", [(1, 16), (31, 48), (33, 512), (97, 528), (129, 80), (200, 2064)])
+@pytest.mark.parametrize("swizzled", [True, False])
+@pytest.mark.parametrize("offset", [0, 8])            # elements: rows on 32-byte and only on 16-byte boundaries
+def test_quantizer_tile_edges(M, K, swizzled, offset):
+    from dgx_vllm_b200 import scaled_fp4_quant
+    from util import bf16_bits
+    g = torch.Generator().manual_seed(M * K)
+    wide = torch.randn(M, K + 16, generator=g).to(torch.bfloat16)
+    wide[0, offset:offset + 16] = 0.0                 # a block of zeros
+    x = wide[:, offset:offset + K]
+    gs = torch.tensor([448.0 * 6.0 / 4.0])
+    codes, sf = scaled_fp4_quant(wide.cuda()[:, offset:offset + K], gs.cuda(), swizzled)
+    ref_codes, ref_sf = oracle.quantize_bf16(bf16_bits(x.contiguous()), float(gs[0]))
+    np.testing.assert_array_equal(to_np(codes), ref_codes)
+    got = to_np(sf)
+    if swizzled:                                      # padding included: zeros past M and past K / 16
+        ref_sf = np.asarray(oracle.sf_linear_to_swizzled(ref_sf)).reshape(got.shape)
+    np.testing.assert_array_equal(got, ref_sf)
