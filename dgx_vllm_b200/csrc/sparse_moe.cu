@@ -23,7 +23,7 @@
 
 #include <mutex>
 
-#include "common.cuh"
+#include "sparse_mma.cuh"
 
 extern "C" size_t b200fp4_sparse_workspace_bytes(int64_t P, int64_t K, int64_t E);
 
@@ -35,22 +35,6 @@ constexpr int kMaxTok = 4;       // tokens of one expert processed per pass over
 constexpr int kPlanThreads = 1024;
 constexpr int kPlanMaxExperts = 4096;
 constexpr int kLutBytes = 256 * 256;   // 256 rows of [32 x comp entry | 32 x meta entry]
-
-// Where one projection's weights live.  Row r of the compressed tensor for expert e and column n:
-//   comp  + e*comp_e  + (r/2)*comp_pair + (r&1)*comp_odd + n
-//   meta  + e*meta_e  + (r/2)*meta_row + n            (one metadata row per two compressed rows)
-//   scale + e*scale_e + srow*scale_row + n
-// which covers both the separate tensors (sparse_fp4_v7.cu:158-167) and the interleaved
-// [E, K/8, 4N] tensor (sparse_fp4_v7.cu:246-251).
-struct SparseWeights {
-  const uint8_t* comp;
-  const uint8_t* meta;
-  const uint8_t* scale;
-  const float* g;
-  int64_t comp_e, comp_pair, comp_odd;
-  int64_t meta_e, meta_row;
-  int64_t scale_e, scale_row;
-};
 
 struct Plan {
   int* hdr;        // [0] = number of unique experts, [1] = number of passes, [2] and [4] = work-item counters of the
@@ -93,6 +77,88 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+
+// The plan of few pairs, one pair per thread of the first eight warps: ranks by warp-wide matching, one warp after the other,
+// and passes numbered by the first pair of their expert, so that nothing is as long as the number of experts (a decode step
+// waits for this kernel from end to end: 4.6 us with the general path below, 2.7 us so at 10 pairs and 512 experts).
+constexpr int kPlanSmallPairs = 256;
+__device__ __forceinline__ void plan_small(const int32_t* __restrict__ ids, int P, const int32_t* __restrict__ expert_map, int global_E,
+                                           int E, const Plan& plan, int ids_topk, int64_t ids_ld, int* zero_buf, int zero_count,
+                                           int* s_count, int (*s_warp)[32]) {
+  constexpr int kThr = kPlanSmallPairs;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid >= kThr) {                           // the other warps clear the counters and are done
+    for (int i = tid - kThr; i < zero_count; i += kPlanThreads - kThr) zero_buf[i] = 0;
+    return;
+  }
+  auto barrier = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(kThr) : "memory"); };
+  if (tid == 0) plan.hdr[2] = plan.hdr[3] = plan.hdr[4] = 0;
+  int e = -1;
+  if (tid < P) {
+    e = ids[(int64_t)(tid / ids_topk) * ids_ld + (tid % ids_topk)];
+    if (expert_map != nullptr) e = (e >= 0 && e < global_E) ? expert_map[e] : -1;
+    if (e < 0 || e >= E) e = -1;
+    plan.mapped[tid] = e;
+    if (e >= 0) s_count[e] = 0;
+  }
+  __syncwarp();
+  barrier();
+  int rank = 0;                                // among the pairs of the same expert
+  for (int w = 0; w * 32 < P; ++w) {
+    if (warp == w) {
+      const uint32_t same = __match_any_sync(0xffffffffu, e);
+      const int base = e >= 0 ? s_count[e] : 0;
+      rank = base + __popc(same & ((1u << lane) - 1));
+      __syncwarp();
+      if (e >= 0 && (same >> lane) == 1u) s_count[e] = base + __popc(same);        // the highest lane of the group
+      __syncwarp();
+    }
+    barrier();
+  }
+  // scans over the experts' first pairs: (pairs, experts, passes)
+  const int count = e >= 0 ? s_count[e] : 0;
+  const bool first = e >= 0 && rank == 0;
+  const int sum[3] = {first ? count : 0, first ? 1 : 0, first ? (count + 7) >> 3 : 0};
+  int inc[3] = {sum[0], sum[1], sum[2]};
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int v = __shfl_up_sync(0xffffffffu, inc[k], d);
+      if (lane >= d) inc[k] += v;
+    }
+  if (lane == 31)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s_warp[k][warp] = inc[k];
+  __syncwarp();
+  barrier();
+  int start[3] = {inc[0] - sum[0], inc[1] - sum[1], inc[2] - sum[2]}, total[3] = {0, 0, 0};
+#pragma unroll
+  for (int w = 0; w < kThr / 32; ++w)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (w < warp) start[k] += s_warp[k][w];
+      total[k] += s_warp[k][w];
+    }
+  if (tid == 0) {
+    plan.hdr[0] = total[1];
+    plan.hdr[1] = total[2];
+  }
+  if (first) s_count[e] = start[0] | (start[2] << 16);        // first position in pairs[], first pass
+  __syncwarp();
+  barrier();
+  if (e >= 0) {
+    const int pos = (s_count[e] & 0xFFFF) + rank, pass = (s_count[e] >> 16) + (rank >> 3), slot = rank & 7;
+    plan.pairs[pos] = tid;
+    int* rec = reinterpret_cast<int*>(plan.pass_rec + 2 * pass);        // {expert, tokens, pair0, pair1, pair2, pair3, position, -}
+    if (slot < 4) rec[2 + slot] = tid;
+    if (slot == 0) {
+      rec[0] = e;
+      rec[1] = min(8, count - rank);
+      rec[6] = pos;
+    }
+  }
+}
 
 // Block 0 builds the plan; the remaining blocks (if any) copy / convert the activation matrix to fp16.
 __global__ void __launch_bounds__(kPlanThreads)
@@ -137,6 +203,10 @@ __global__ void __launch_bounds__(kPlanThreads)
   __shared__ int s_count[kPlanMaxExperts];
   __shared__ int s_warp[3][32];
   const int tid = threadIdx.x;
+  if (P <= kPlanSmallPairs && max_tok == 8) {
+    plan_small(ids, P, expert_map, global_E, E, plan, ids_topk, ids_ld, zero_buf, zero_count, s_count, s_warp);
+    return;
+  }
   for (int e = tid; e < E; e += kPlanThreads) s_count[e] = 0;
   for (int i = tid; i < zero_count; i += kPlanThreads) zero_buf[i] = 0;   // per-pass counters of the one-launch layer
   if (tid == 0) plan.hdr[2] = plan.hdr[3] = plan.hdr[4] = 0;
@@ -280,16 +350,6 @@ __device__ __forceinline__ void cp_async_cols(void* smem_dst, const void* gmem_s
   if (COLS == 16) cp_async16(smem_dst, gmem_src);
   else cp_async8(smem_dst, gmem_src);
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ uint32_t word_of(const uint4& v, int q) {
-  return q == 0 ? v.x : (q == 1 ? v.y : (q == 2 ? v.z : v.w));
-}
-__device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t lds32(const unsigned char* p) { return *reinterpret_cast<const uint32_t*>(p); }
 
 // One scale block (16 k) x 16 columns for T tokens.  v[] = 4 compressed rows, 2 metadata rows,
@@ -584,6 +644,21 @@ __global__ void zero_unmapped_rows_kernel(const int* __restrict__ mapped, int P,
   for (int n = threadIdx.x; n < N; n += blockDim.x) store_out(out, out_dtype, (int64_t)p * ldo + n, 0.f);
 }
 
+// four neighbouring results
+__device__ __forceinline__ void store_out4(void* out, int dtype, int64_t idx, const float4& v) {
+  if (dtype == B200FP4_DTYPE_F32) {
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + idx) = v;
+  } else if (dtype == B200FP4_DTYPE_F16) {
+    const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(out) + idx) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  } else {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + idx) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  }
+}
+
 // Pass record of the tensor-core kernel: up to TM (4 or 8) pairs.
 template <int TM>
 struct RecT {
@@ -645,75 +720,11 @@ constexpr int kMmaWarps = 16;
 constexpr int kMmaStageBytes = 1792;
 constexpr int kMmaRedBytes = kMmaWarps * 128 * 4 * 4;   // K-slice partial sums [warp][column][token] fp32
 
-__device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint32_t lds32_at(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint2 lds64_at(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint4 lds128_at(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 lds128f_at(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void sts64f_at(uint32_t a, float x, float y) {
-  asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(a), "f"(x), "f"(y) : "memory");
-}
-__device__ __forceinline__ void cp_async16_s(uint32_t smem_dst, const void* gmem_src) {
-  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(smem_dst), "l"(gmem_src) : "memory");
-}
-
-__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-template <int SEL>
-__device__ __forceinline__ void mma_sp_m16n8k32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                                const uint32_t (&b)[4], uint32_t e) {
-  asm volatile(
-      "mma.sp::ordered_metadata.sync.aligned.m16n8k32.row.col.f32.f16.f16.f32 "
-      "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9,%10,%11}, {%0,%1,%2,%3}, %12, %13;"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(e), "n"(SEL));
-}
-
-// byte B of a word holds two E2M1 values -> half2 (low nibble in the low half)
-template <int B>
-__device__ __forceinline__ __half2 e2m1x2_to_h2(uint32_t w) {
-  uint32_t r;
-  if (B == 0) asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %1; cvt.rn.f16x2.e2m1x2 %0, b0; }" : "=r"(r) : "r"(w));
-  else if (B == 1) asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %1; cvt.rn.f16x2.e2m1x2 %0, b1; }" : "=r"(r) : "r"(w));
-  else if (B == 2) asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %1; cvt.rn.f16x2.e2m1x2 %0, b2; }" : "=r"(r) : "r"(w));
-  else asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %1; cvt.rn.f16x2.e2m1x2 %0, b3; }" : "=r"(r) : "r"(w));
-  return as_h2(r);
-}
-// half H (16 bits) of a word holds two E4M3 values -> half2
-template <int H>
-__device__ __forceinline__ __half2 e4m3x2_to_h2(uint32_t w) {
-  uint32_t r;
-  if (H == 0) asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; cvt.rn.f16x2.e4m3x2 %0, lo; }" : "=r"(r) : "r"(w));
-  else asm("{ .reg .b16 lo, hi; mov.b32 {lo, hi}, %1; cvt.rn.f16x2.e4m3x2 %0, hi; }" : "=r"(r) : "r"(w));
-  return as_h2(r);
-}
-
-// One projection over all items of this block.  kDep links the two projections of the MoE layer when
-// they run in one launch: 1 = producer (done[pass] is incremented once an item's output is stored and
-// fenced), 2 = consumer (the activations of a pass are staged only after done[pass] has reached
-// `need` = producer slabs per pass), 0 = stand-alone.
+// One projection over all items of this block.
 // TM = tokens per pass (4 or 8; the instruction's B operand has 8 columns either way, but the
 // activation buffers and the partial-sum scratch double with 8).
-template <int CG, int S, bool kSilu, int kDep, int TM>
-__device__ __forceinline__ void gemv_mma_phase(const GemvArgs& g, unsigned char* smem, int* done, int need) {
+template <int CG, int S, bool kSilu, int TM>
+__device__ __forceinline__ void gemv_mma_phase(const GemvArgs& g, unsigned char* smem) {
   using Rec = RecT<TM>;
   constexpr int KSL = kMmaWarps / CG;          // K-slices per item
   constexpr int VCOLS = 128 * CG;              // columns of a slab (SiLU: 64*CG gate + 64*CG up)
@@ -800,44 +811,6 @@ __device__ __forceinline__ void gemv_mma_phase(const GemvArgs& g, unsigned char*
     if (f_dst >= ring_end) f_dst -= ring_bytes;
   };
 
-  // consumer side of the dependency: thread 0 reads a pass's counter (acquire) one item ahead, so the
-  // load's latency is hidden; only a counter that is still short is polled (bounded), and the block's
-  // next barrier releases the other threads
-  auto load_count = [&](int pass) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(done + pass) : "memory");
-    return v;
-  };
-  // A wait that runs out of its clock budget records B200FP4_MOE_STATUS_WAIT_EXPIRED in the plan header (the layer's
-  // status word) and carries on with whatever the activation buffer holds; once the word is set no later wait of the
-  // launch polls at all, so a broken launch still ends promptly.
-  auto wait_pass = [&](int pass, int seen) {
-    if (kDep == 2 && tid == 0 && pass >= 0 && seen < need) {
-      volatile int* status = g.plan.hdr + 3;
-      if (*status == 0) {
-        const long long t0 = clock64();
-        while (load_count(pass) < need) {
-          if (clock64() - t0 > g.wait_cycles) {
-            *status = B200FP4_MOE_STATUS_WAIT_EXPIRED;
-            break;
-          }
-        }
-      }
-    }
-  };
-  // producer side: an item's output is complete for the whole block at the next block-wide barrier;
-  // thread 0 then fences (cumulative over the barrier) and counts the item
-  int finished_pass = -1;
-  auto signal_finished = [&]() {
-    if (kDep == 1 && tid == 0 && finished_pass >= 0) {
-      __threadfence();
-      atomicAdd(done + finished_pass, 1);
-    }
-  };
-  int seen_next = 0;      // thread 0: counter of the next item's pass, read during the previous item
-  wait_pass(pass_of(0), 0);
-  if (kDep == 2) __syncthreads();
-  if (kDep == 2 && tid == 0 && my_items > 1) seen_next = load_count(pass_of(1));
   issue_A(rc, 0);
   cp_async_commit();
 #pragma unroll
@@ -867,11 +840,8 @@ __device__ __forceinline__ void gemv_mma_phase(const GemvArgs& g, unsigned char*
     if (nstep >= S - 1) cp_async_wait<S - 2>();
     else if (nstep == 2) cp_async_wait<1>();
     else cp_async_wait<(S > 3 ? 2 : 1)>();
-    wait_pass(i_cur + 1 < my_items ? pass_of(i_cur + 1) : -1, seen_next);
     __syncthreads();   // activations of this pass complete for all threads; scratch and the other buffer free
-    signal_finished();
     issue_A(rn, abuf ^ 1);   // rides on the next committed weight stage
-    if (kDep == 2 && tid == 0 && i_cur + 2 < my_items) seen_next = load_count(pass_of(i_cur + 2));
 
     float acc[8][4];
 #pragma unroll
@@ -965,17 +935,12 @@ __device__ __forceinline__ void gemv_mma_phase(const GemvArgs& g, unsigned char*
         if (tok < rc.nt) store_out(g.out, g.out_dtype, (int64_t)rc.pair(tok) * g.ldo + slab * VCOLS + v, sum * gmul);
       }
     }
-    if (kDep == 1) finished_pass = pass_of(i_cur);   // counted after the next block-wide barrier
     rc = rn;
     rn = rnn;
     e_nn = e_n3;
     abuf ^= 1;
   }
   cp_async_wait<0>();
-  if (kDep == 1) {
-    __syncthreads();
-    signal_finished();
-  }
 }
 
 // Programmatic dependent launch: the GEMV and reduce kernels of a layer are launched with the stream-serialization
@@ -988,21 +953,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) sparse_gemv_mma_kernel(const G
   extern __shared__ __align__(16) unsigned char smem[];
   pdl_wait();
   pdl_launch_dependents();
-  gemv_mma_phase<CG, S, kSilu, 0, TM>(g, smem, nullptr, 0);
-}
-
-// Both projections of the MoE layer in one launch: every block first walks its gate_up items, then its
-// down items.  A down item only needs the activations of its own pass, so blocks that run out of
-// gate_up items start on the down projection of passes finished long ago instead of idling through
-// the last, partial round and a second kernel's ramp-up.  Launched cooperatively (all blocks
-// co-resident), so a block polling for a pass can never keep the block that produces it off the GPU.
-template <int CGA, int SA, int CGB, int SB, int TM>
-__global__ void __launch_bounds__(kMmaThreads, 1)
-    fused_moe_mma_kernel(const GemvArgs ga, const GemvArgs gb, int* done, int need) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  gemv_mma_phase<CGA, SA, true, 1, TM>(ga, smem, done, need);
-  __syncthreads();              // the second phase lays shared memory out anew
-  gemv_mma_phase<CGB, SB, false, 2, TM>(gb, smem, done, need);
+  gemv_mma_phase<CG, S, kSilu, TM>(g, smem);
 }
 
 // ------------------------------------------------------------------------------------------ warp-scheduled tensor-core GEMV
@@ -1028,44 +979,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
 // token's values through shuffles, and SiLU(gate)*up leaves in fragment order for the down projection.
 // Two shapes of the same ring budget: 8 warps x 8 stages per block (the default where K is a multiple of 256: two warps
 // per scheduler, each with twice the bytes in flight, measured faster at every batch size tried), or 16 warps x 4 stages.
-constexpr int kWsStages = 4;
-constexpr int kWsWarps = 16;
-constexpr int kWsThreads = 32 * kWsWarps;
-constexpr int kWsStageBytes = 14 * 128 + 512;     // 8 compressed + 4 metadata + 2 scale rows of 128 bytes, B fragments of 8 tokens
-constexpr size_t kWsSmemBytes = (size_t)kWsWarps * kWsStages * kWsStageBytes + 128;
-// (warps per block = 64 / stages, so both shapes use the same shared memory)
-
-// Lane-constant shared-memory offsets of the warp-scheduled kernel.
-// Stage layout: compressed rows 0..7 | metadata rows 0..3 | scale rows 0..1 (128 bytes each) | B fragments.  The 16-byte
-// chunks of a compressed row r sit at chunk ^ 2(r%4), those of a metadata row at chunk ^ 4(r/2), so that the fragment
-// loads (rows t and t+4 for lane t of a quad; metadata rows 2(t%2), 2(t%2)+1) spread over all banks.
-struct WsLane {
-  uint32_t ring;                                   // this warp's ring
-  uint32_t d_comp, d_meta, d_scale, d_b;           // where this lane's copies land (compressed rows fr and fr+4, metadata / scale row fr)
-  uint32_t off_comp, off_meta, off_scale;          // where its fragments are read from
-  int lane, q, t, fr, fc;
-};
-
-template <int kS = kWsStages>
-__device__ __forceinline__ WsLane ws_lane(unsigned char* smem) {
-  WsLane L;
-  L.lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  L.q = L.lane >> 2;
-  L.t = L.lane & 3;
-  L.fr = L.lane >> 3;
-  L.fc = L.lane & 7;
-  L.ring = ((shared_addr(smem) + 127u) & ~127u) + (uint32_t)warp * (kS * kWsStageBytes);
-  L.d_comp = (uint32_t)L.fr * 128u + (uint32_t)((L.fc ^ (2 * (L.fr & 3))) << 4);
-  L.d_meta = 1024u + (uint32_t)L.fr * 128u + (uint32_t)((L.fc ^ (4 * (L.fr >> 1))) << 4);
-  L.d_scale = 1536u + (uint32_t)L.fr * 128u + (uint32_t)L.fc * 16u;
-  L.d_b = 1792u + (uint32_t)L.lane * 16u;
-  L.off_comp = (uint32_t)L.t * 128u + (uint32_t)((L.q ^ (2 * L.t)) << 4);
-  L.off_meta = 1024u + (uint32_t)(2 * (L.t & 1)) * 128u + (uint32_t)((L.q ^ (4 * (L.t & 1))) << 4) + (uint32_t)(L.t >> 1) * 8u;
-  L.off_scale = 1536u + (uint32_t)L.q * 16u;
-  return L;
-}
-
 // One projection for this warp: the items [base, base + passes * groups) of the claim sequence that `counter` hands out.
 // `first` is an index this warp has already claimed; the return value is the first index it claimed that lies past
 // this projection (the caller passes it on to the next one).
@@ -1076,22 +989,33 @@ __device__ __forceinline__ WsLane ws_lane(unsigned char* smem) {
 // was claimed before any item of the second projection) or by the warp of this grid it is statically assigned to (index <
 // number of warps; the grid has at most one block per SM, so that warp becomes resident without anyone's help): the wait
 // cannot deadlock; it is bounded all the same and reports through the status word.
-template <bool kSilu, int kN, int kDep, int kS = kWsStages>
-__device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const int base, int first, const WsLane& L,
-                                        int* done, const int need) {
+// KS > 1: a unit of KS warps shares an item, each warp walking 1/KS of K through its own ring; at the end of an item the
+// warps add their accumulators through shared memory and each stores its share of the columns.  With one warp per item a
+// step takes a warp about 630 cycles at two warps per scheduler -- instruction latency, not memory: it waits 20 cycles of
+// them for data -- so a gate_up item of K = 2048 is 21 us, which is also the grain of the schedule.
+struct WsUnit {
+  int ks, bar, n_units;              // slice, named barrier, units in the grid
+  uint32_t red;                      // partial sums of the unit's first warp: [warp][mma][lane] float4
+  uint32_t next_slot;                // where the unit's first warp publishes claimed items
+};
+struct WsClaims {
+  int cur, nxt;                      // KS == 1: cur only
+};
+template <bool kSilu, int kN, int kDep, int kS = kWsStages, int KS = 1>
+__device__ __forceinline__ void ws_phase(const GemvArgs& g, int* counter, const int base, WsClaims& claims, const WsLane& L, const WsUnit& U,
+                                         int* done, const int need) {
   const int lane = L.lane, q = L.q, t = L.t;
   const int N = kN ? kN : g.N;
-  const int nblk = g.K / (32 * kS);          // blocks of kS 32-wide k-steps (one turn of the ring)
+  const int nblk = g.K / (32 * kS * KS);     // blocks of kS 32-wide k-steps (one turn of the ring)
   const int groups = g.n_slabs;              // 128-column groups per pass
   const int n_items = g.plan.hdr[1] * groups;
-  if (first - base >= n_items) return first;
+  if (claims.cur - base >= n_items) return;
 
-  // warp w of the grid starts on item w without asking (one round trip to the counter less before the first byte is
-  // requested); the counter hands out the items after those
-  const int n_warps = (int)(gridDim.x * (blockDim.x >> 5));
+  // unit w of the grid starts on item w (KS > 1: and goes on to w + units) without asking (one round trip to the counter less
+  // before the first byte is requested); the counter hands out the items after those
   auto claim = [&]() {
     int v = 0;
-    if (lane == 0) v = atomicAdd(counter, 1) + n_warps;
+    if (lane == 0) v = atomicAdd(counter, 1) + U.n_units;
     return __shfl_sync(0xffffffffu, v, 0);
   };
   // An item as read from its pass record: expert, group, and the pairs this lane deals with (B column q; the one or two
@@ -1123,20 +1047,9 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
     if (!kSilu && s0 + 1 < nt) d.ps1 = pair_of(x, y, s0 + 1);
     return d;
   };
-  // this lane's copy sources at k-step 0 of an item
-  struct Fetch {
-    const uint8_t *pc, *pm, *ps;
-    const __half* pb;
-    bool valid;
-  };
-  auto sources = [&](const Item& d) {
-    Fetch f;
-    f.valid = d.valid;
-    f.pc = f.pm = f.ps = nullptr;
-    f.pb = nullptr;
-    if (!d.valid) return f;
-    if (kDep == 2) {
-      // the activations of this pass must be complete before any lane asks for them
+  // consumer: the activations of an item's pass must be complete before any lane asks for them
+  auto wait_pass = [&](const Item& d) {
+    if (kDep == 2 && d.valid) {
       if (lane == 0) {
         volatile int* status = g.plan.hdr + 3;
         int v;
@@ -1154,6 +1067,19 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
       }
       __syncwarp();
     }
+  };
+  // this lane's copy sources at k-step 0 of an item
+  struct Fetch {
+    const uint8_t *pc, *pm, *ps;
+    const __half* pb;
+    bool valid;
+  };
+  auto sources = [&](const Item& d) {
+    Fetch f;
+    f.valid = d.valid;
+    f.pc = f.pm = f.ps = nullptr;
+    f.pb = nullptr;
+    if (!d.valid) return f;
     const uint32_t pr = (uint32_t)d.pb;
     const int64_t row = g.a_magic ? (int64_t)__umulhi(pr, g.a_magic) : (int64_t)pr;
     f.pb = g.A + row * g.lda + t * 8;
@@ -1161,13 +1087,15 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
     if (kSilu) col = L.fc < 4 ? d.grp * 64 + L.fc * 16 : g.inter + d.grp * 64 + (L.fc - 4) * 16;
     else col = d.grp * 128 + L.fc * 16;
     const int64_t lane_off = (int64_t)L.fr * N + col;
-    f.pc = g.w.comp + ((int64_t)d.e * g.w.comp_e + lane_off);
-    f.pm = g.w.meta + ((int64_t)d.e * g.w.meta_e + lane_off);
-    f.ps = g.w.scale + ((int64_t)d.e * g.w.scale_e + lane_off);
+    const int step0 = KS > 1 ? U.ks * (nblk * kS) : 0;       // first k-step of this warp's slice
+    f.pb += step0 * 32;
+    f.pc = g.w.comp + ((int64_t)d.e * g.w.comp_e + (int64_t)step0 * 8 * N + lane_off);
+    f.pm = g.w.meta + ((int64_t)d.e * g.w.meta_e + (int64_t)step0 * 4 * N + lane_off);
+    f.ps = g.w.scale + ((int64_t)d.e * g.w.scale_e + (int64_t)step0 * 2 * N + lane_off);
     return f;
   };
   // copies of k-step `u` (relative to f) into ring slot u; always one commit group, so that the wait counts stay fixed
-  auto fetch = [&](const Fetch& f, int u) {
+  auto fetch_weights = [&](const Fetch& f, int u) {
     if (f.valid) {
       const uint32_t dst = L.ring + (uint32_t)u * kWsStageBytes;
       const uint8_t* c = f.pc + (int64_t)u * 8 * N;
@@ -1175,9 +1103,15 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
       cp_async16_s(dst + 512u + L.d_comp, c + (int64_t)4 * N);
       cp_async16_s(dst + L.d_meta, f.pm + (int64_t)u * 4 * N);
       if (lane < 16) cp_async16_s(dst + L.d_scale, f.ps + (int64_t)u * 2 * N);
-      cp_async16_s(dst + L.d_b, f.pb + u * 32);
     }
+  };
+  auto fetch_b = [&](const Fetch& f, int u) {
+    if (f.valid) cp_async16_s(L.ring + (uint32_t)u * kWsStageBytes + L.d_b, f.pb + u * 32);
     cp_async_commit();
+  };
+  auto fetch = [&](const Fetch& f, int u) {
+    fetch_weights(f, u);
+    fetch_b(f, u);
   };
   auto advance = [&](Fetch& f) {     // kS k-steps on
     f.pc += (int64_t)(8 * kS) * N;
@@ -1186,16 +1120,21 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
     f.pb += 32 * kS;
   };
 
-  Item cur = describe(first);
+  // The first kS k-steps of the first item.  Weights are requested before the activations they meet are known to be there.
+  Item cur = describe(claims.cur);
   Fetch F = sources(cur);
 #pragma unroll
-  for (int u = 0; u < kS; ++u) fetch(F, u);     // the first kS k-steps of the first item
+  for (int u = 0; u < kS; ++u) fetch_weights(F, u);
+  wait_pass(cur);
+#pragma unroll
+  for (int u = 0; u < kS; ++u) fetch_b(F, u);
   advance(F);
-  int carry;
 
   while (true) {
-    carry = claim();
-    const Item nxt = describe(carry);
+    int pending = 0;                           // the item after the next, on its way to the unit's first warp
+    if constexpr (KS == 1) claims.nxt = claim();
+    else if (U.ks == 0 && lane == 0) pending = atomicAdd(counter, 1) + 2 * U.n_units;
+    const Item nxt = describe(claims.nxt);
     const float gmul = g.w.g[cur.e];
     float acc[8][4];
 #pragma unroll
@@ -1204,48 +1143,91 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
       for (int k = 0; k < 4; ++k) acc[j][k] = 0.f;
 
     for (int b = 0; b < nblk; ++b) {
-      if (b == nblk - 1) F = sources(nxt);     // the last block of an item prefetches the first block of the next one
+      if (b == nblk - 1) {                     // the last block of an item prefetches the first block of the next one
+        wait_pass(nxt);
+        F = sources(nxt);
+      }
 #pragma unroll
       for (int u = 0; u < kS; ++u) {
         cp_async_wait<kS - 1>();
         __syncwarp();
-        const uint32_t st = L.ring + (uint32_t)u * kWsStageBytes;
-        const uint4 v0 = lds128_at(st + L.off_comp), v1 = lds128_at(st + L.off_comp + 512u);
-        const uint2 m0 = lds64_at(st + L.off_meta), m1 = lds64_at(st + L.off_meta + 128u);
-        const uint4 s0 = lds128_at(st + L.off_scale), s1 = lds128_at(st + L.off_scale + 128u);
-        const uint4 bv = lds128_at(st + L.d_b);
-        const uint32_t bf[4] = {bv.x, bv.y, bv.z, bv.w};
+        const WsStep w = ws_load_step(L, L.ring + (uint32_t)u * kWsStageBytes);
+        __syncwarp();                // lane 0 may come from a branch of its own: no lane refills the slot before all have read it
         fetch(F, u);                 // k-step kS ahead, into the slot that was just read
-        uint32_t em[4];
-        em[0] = prmt(m0.x, m1.x, 0x5140u);
-        em[1] = prmt(m0.x, m1.x, 0x7362u);
-        em[2] = prmt(m0.y, m1.y, 0x5140u);
-        em[3] = prmt(m0.y, m1.y, 0x7362u);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          // mma j takes columns 2h, 2h+1 of every quad as its rows q and q+8: bytes (2hf, 2hf+1) of word wi of the
-          // loaded vectors.  Even j: metadata from lanes t = 0, 1 (first half of the quad's columns), odd j: t = 2, 3.
-          constexpr int kH[8] = {0, 4, 1, 5, 2, 6, 3, 7};
-          const int h = kH[j];
-          const int wi = h >> 1, hf = h & 1;
-          const uint32_t c0 = word_of(v0, wi), c1 = word_of(v1, wi);
-          const __half2 sc0 = hf ? e4m3x2_to_h2<1>(word_of(s0, wi)) : e4m3x2_to_h2<0>(word_of(s0, wi));
-          const __half2 sc1 = hf ? e4m3x2_to_h2<1>(word_of(s1, wi)) : e4m3x2_to_h2<0>(word_of(s1, wi));
-          const __half2 a0 = __hmul2(hf ? e2m1x2_to_h2<2>(c0) : e2m1x2_to_h2<0>(c0), __low2half2(sc0));
-          const __half2 a1 = __hmul2(hf ? e2m1x2_to_h2<3>(c0) : e2m1x2_to_h2<1>(c0), __high2half2(sc0));
-          const __half2 a2 = __hmul2(hf ? e2m1x2_to_h2<2>(c1) : e2m1x2_to_h2<0>(c1), __low2half2(sc1));
-          const __half2 a3 = __hmul2(hf ? e2m1x2_to_h2<3>(c1) : e2m1x2_to_h2<1>(c1), __high2half2(sc1));
-          if ((j & 1) == 0)
-            mma_sp_m16n8k32<0>(acc[j], *reinterpret_cast<const uint32_t*>(&a0), *reinterpret_cast<const uint32_t*>(&a1),
-                               *reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&a3), bf, em[j >> 1]);
-          else
-            mma_sp_m16n8k32<1>(acc[j], *reinterpret_cast<const uint32_t*>(&a0), *reinterpret_cast<const uint32_t*>(&a1),
-                               *reinterpret_cast<const uint32_t*>(&a2), *reinterpret_cast<const uint32_t*>(&a3), bf, em[j >> 1]);
-        }
+        ws_mma_step(acc, w);
       }
       advance(F);
     }
 
+    int after_next = 0;
+    if constexpr (KS > 1) {
+      // add the K-slices; this warp ends up with the mmas [ks * 8 / KS, +8 / KS), that is column pairs m and m + 4 of every
+      // quad's eight for m in [ks * 4 / KS, +4 / KS)
+      constexpr int kM = 4 / KS;
+      auto unit_barrier = [&]() {
+        __syncwarp();                          // bar.sync takes whole warps
+        asm volatile("bar.sync %0, %1;" ::"r"(U.bar), "n"(32 * KS) : "memory");
+      };
+      const uint32_t mine = U.red + (uint32_t)U.ks * 4096u + (uint32_t)lane * 16u;
+      unit_barrier();                          // the sums of the item before have been read
+      if (U.ks == 0 && lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(U.next_slot), "r"(pending) : "memory");
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sts128f_at(mine + (uint32_t)j * 512u, acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+      unit_barrier();
+      after_next = (int)lds32_at(U.next_slot);
+      float v[2 * kM][4];
+#pragma unroll
+      for (int jj = 0; jj < 2 * kM; ++jj) {
+        const uint32_t at = U.red + (uint32_t)(U.ks * 2 * kM + jj) * 512u + (uint32_t)lane * 16u;
+        float4 sum = lds128f_at(at);
+#pragma unroll
+        for (int s = 1; s < KS; ++s) {
+          const float4 x = lds128f_at(at + (uint32_t)s * 4096u);
+          sum.x += x.x;
+          sum.y += x.y;
+          sum.z += x.z;
+          sum.w += x.w;
+        }
+        v[jj][0] = sum.x * gmul; v[jj][1] = sum.y * gmul; v[jj][2] = sum.z * gmul; v[jj][3] = sum.w * gmul;
+      }
+      const int m0 = U.ks * kM;
+      if (kSilu) {
+        const int hi = lane >> 4;              // as below: the half-warps swap one token's values
+        uint32_t words[2 * kM];
+#pragma unroll
+        for (int jj = 0; jj < 2 * kM; ++jj) {
+          float a[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float keep = hi ? v[jj][2 * r + 1] : v[jj][2 * r], send = hi ? v[jj][2 * r] : v[jj][2 * r + 1];
+            const float recv = __shfl_xor_sync(0xffffffffu, send, 16);
+            const float gate = hi ? recv : keep, up = hi ? keep : recv;
+            a[r] = gate / (1.0f + __expf(-gate)) * up;
+          }
+          const __half2 hv = __floats2half2_rn(a[0], a[1]);
+          words[jj] = *reinterpret_cast<const uint32_t*>(&hv);
+        }
+        if (cur.ps0 >= 0) {
+          __half* dst = reinterpret_cast<__half*>(g.out) + (int64_t)cur.ps0 * g.ldo + (cur.grp * 2 + ((q & 3) >> 1)) * 32 + 4 * (q & 1) + 8 * m0;
+#pragma unroll
+          for (int i = 0; i < kM; ++i) *reinterpret_cast<uint2*>(dst + 8 * i) = make_uint2(words[2 * i], words[2 * i + 1]);
+        }
+      } else {
+#pragma unroll
+        for (int b2 = 0; b2 < 2; ++b2) {
+          const int pair = b2 ? cur.ps1 : cur.ps0;
+          if (pair < 0) continue;
+          float* dst = reinterpret_cast<float*>(g.out) + (int64_t)pair * g.ldo + cur.grp * 128 + q * 16 + 2 * m0;     // fp32 results only
+          if constexpr (KS == 2) {
+            *reinterpret_cast<float4*>(dst) = make_float4(v[0][b2], v[0][2 + b2], v[2][b2], v[2][2 + b2]);
+            *reinterpret_cast<float4*>(dst + 8) = make_float4(v[1][b2], v[1][2 + b2], v[3][b2], v[3][2 + b2]);
+          } else {
+            *reinterpret_cast<float2*>(dst) = make_float2(v[0][b2], v[0][2 + b2]);
+            *reinterpret_cast<float2*>(dst + 8) = make_float2(v[1][b2], v[1][2 + b2]);
+          }
+        }
+      }
+    } else {
     // ---- epilogue from registers.  Column 2h + r of the quad's 16 columns for token 2t + b is acc[kJ[h]][2r + b].
     constexpr int kJ[8] = {0, 2, 4, 6, 1, 3, 5, 7};
     if (kSilu) {
@@ -1309,21 +1291,41 @@ __device__ __forceinline__ int ws_phase(const GemvArgs& g, int* counter, const i
         }
       }
     }
+    }
     if (kDep == 1) {
-      // this item's activations are stored: make them visible, then count the item for its pass
+      // this warp's activations are stored: make them visible, then count them for the pass
       __syncwarp();
       if (lane == 0) {
         __threadfence();
         atomicAdd(done + cur.pass, 1);
       }
     }
+    claims.cur = claims.nxt;
+    claims.nxt = after_next;
     if (!nxt.valid) break;
     cur = nxt;
   }
   cp_async_wait<0>();
   __syncwarp();
-  return carry;
 }
+
+// The unit of this warp and its first item(s).  Units are numbered across the blocks, so that few items sit on many SMs.
+template <int kS, int kW, int KS>
+__device__ __forceinline__ WsUnit ws_unit(const WsLane& L, WsClaims& claims) {
+  const int warp = threadIdx.x >> 5, unit = warp / KS;
+  const uint32_t ring0 = L.ring - (uint32_t)warp * (kS * kWsStageBytes), red0 = ring0 + (uint32_t)kW * (kS * kWsStageBytes);
+  WsUnit u;
+  u.ks = warp - unit * KS;
+  u.bar = 1 + unit;
+  u.n_units = (int)gridDim.x * (kW / KS);
+  u.red = red0 + (uint32_t)unit * (KS * 4096u);
+  u.next_slot = red0 + (uint32_t)kW * 4096u + (uint32_t)unit * 4u;
+  claims.cur = unit * (int)gridDim.x + (int)blockIdx.x;
+  claims.nxt = claims.cur + u.n_units;
+  return u;
+}
+template <int kS, int kW, int KS>
+constexpr size_t ws_smem_bytes() { return (size_t)kW * kS * kWsStageBytes + 128 + (KS > 1 ? (size_t)kW * 4096 + 4 * (kW / KS) : 0); }
 
 template <bool kSilu, int kN, int kS = kWsStages, int kW = kWsWarps>
 __global__ void __launch_bounds__(32 * kW, 1) sparse_gemv_ws_kernel(const GemvArgs g, int* counter) {
@@ -1331,24 +1333,26 @@ __global__ void __launch_bounds__(32 * kW, 1) sparse_gemv_ws_kernel(const GemvAr
   pdl_wait();
   pdl_launch_dependents();
   const WsLane L = ws_lane<kS>(smem);
-  int first = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
-  ws_phase<kSilu, kN, 0, kS>(g, counter, 0, first, L, nullptr, 0);
+  WsClaims claims;
+  const WsUnit U = ws_unit<kS, kW, 1>(L, claims);
+  ws_phase<kSilu, kN, 0, kS>(g, counter, 0, claims, L, U, nullptr, 0);
 }
 
 // Both projections of the MoE layer in one launch: the claim sequence runs through the gate_up items and on into the
 // down items, so a warp that finds no gate_up item left starts on the down projection of passes that are complete
 // instead of idling until the slowest warp of a first launch has finished and a second launch has ramped up.
-template <int kNA, int kNB, int kS = kWsStages, int kW = kWsWarps>
+template <int kNA, int kNB, int kS, int kW, int KS>
 __global__ void __launch_bounds__(32 * kW, 1)
     fused_moe_ws_kernel(const GemvArgs ga, const GemvArgs gb, int* counter, int* done, int need) {
   extern __shared__ __align__(16) unsigned char smem[];
   pdl_wait();
   pdl_launch_dependents();
   const WsLane L = ws_lane<kS>(smem);
-  int first = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  WsClaims claims;
+  const WsUnit U = ws_unit<kS, kW, KS>(L, claims);
   const int n_a = ga.plan.hdr[1] * ga.n_slabs;
-  first = ws_phase<true, kNA, 1, kS>(ga, counter, 0, first, L, done, need);
-  ws_phase<false, kNB, 2, kS>(gb, counter, n_a, first, L, done, need);
+  ws_phase<true, kNA, 1, kS, KS>(ga, counter, 0, claims, L, U, done, need);
+  ws_phase<false, kNB, 2, kS, KS>(gb, counter, n_a, claims, L, U, done, need);
 }
 
 // ------------------------------------------------------------------------------------------ generic
@@ -1450,18 +1454,7 @@ __global__ void __launch_bounds__(kRedThreads)
       a.w += v[i].w * w[i];
     }
   }
-  const int64_t o = (int64_t)m * H + h;
-  if (out_dtype == B200FP4_DTYPE_F32) {
-    *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + o) = a;
-  } else if (out_dtype == B200FP4_DTYPE_F16) {
-    const __half2 lo = __floats2half2_rn(a.x, a.y), hi = __floats2half2_rn(a.z, a.w);
-    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(out) + o) =
-        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-  } else {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
-    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + o) =
-        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-  }
+  store_out4(out, out_dtype, (int64_t)m * H + h, a);
 }
 
 inline dim3 reduce_grid(int64_t H, int64_t M) { return dim3((unsigned)((H + 4 * kRedThreads - 1) / (4 * kRedThreads)), (unsigned)M); }
@@ -1696,18 +1689,33 @@ int run_projection_ws(const SparseWeights& w, const Plan& plan, const __half* A,
   return N == 2048 ? launch_ws_t<false, 2048>(g, counter, items, st) : launch_ws_t<false, 0>(g, counter, items, st);
 }
 
-template <int kNA, int kNB, int kS = kWsStages, int kW = kWsWarps>
-int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int need, int64_t max_items,
-                      cudaStream_t st) {
+template <int kNA, int kNB, int kS, int kW, int KS>
+int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int need, cudaStream_t st) {
   static bool attr_set[64] = {false};
-  constexpr size_t smem = (size_t)kW * kS * kWsStageBytes + 128;
+  constexpr size_t smem = ws_smem_bytes<kS, kW, KS>();
   static_assert(smem <= 227 * 1024, "shared memory of the ring");
-  if (!ws_prepare(fused_moe_ws_kernel<kNA, kNB, kS, kW>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
-  int64_t grid = (max_items + kW - 1) / kW;
-  if (grid > (int64_t)sm_count()) grid = sm_count();
-  if (grid < 1) grid = 1;
-  launch_pdl(fused_moe_ws_kernel<kNA, kNB, kS, kW>, dim3((unsigned)grid), dim3(32 * kW), smem, st, ga, gb, counter, done, need);
+  if (!ws_prepare(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
+  launch_pdl(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS>, dim3((unsigned)sm_count()), dim3(32 * kW), smem, st, ga, gb, counter, done, need);
   return B200FP4_STATUS_SUCCESS;
+}
+
+// Block shape of the one-launch layer by the number of gate_up items (at most one pass per local pair or expert, times 64-column
+// groups).  Measured on B200, 512 experts, H=2048, I=512, top-10, us per layer at M = 1 / 4 / 8 / 16 / 24 / 32 / 64 / 128:
+//   12 warps x 4 stages, four per item    18.3  27.5  34.5  50.0  63.3  73.9  107   142
+//    8 warps x 8 stages, one per item     26.5  28.8  33.3  47.8  61.8  68.7  97.4  127
+//   12 warps x 4 stages, two per item     21.5  27.9  35.7  50.1  58.0  67.6  96.6  128
+//   16 warps x 4 stages, one per item     28.5  31.0  36.4  50.3  60.3  68.5  104   121
+// (K-sliced blocks of the former small-batch kernel: 22.6  34.7  43.6  66.1  86.1).  With the 64 local experts of one of eight
+// expert-parallel ranks the launch alone is 37.6 us with 8 x 8 and 49.7 us with 16 x 4.
+template <int kNA, int kNB>
+int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int64_t local_pairs, int64_t E, cudaStream_t st) {
+  const int64_t items = (local_pairs < E ? local_pairs : E) * ga.n_slabs, sms = sm_count();
+  const bool k256 = ga.K % 256 == 0 && gb.K % 256 == 0, k512 = ga.K % 512 == 0 && gb.K % 512 == 0;
+  const int need = ga.n_slabs, more = g_wait_extra_need;       // per warp of an item: counts a pass's down items wait for
+  if (k512 && items <= 3 * sms) return launch_fused_ws_t<kNA, kNB, 4, 12, 4>(ga, gb, counter, done, 4 * need + more, st);
+  if (k256 && items <= 10 * sms) return launch_fused_ws_t<kNA, kNB, 8, 8, 1>(ga, gb, counter, done, need + more, st);
+  if (k256 && local_pairs < 2 * E) return launch_fused_ws_t<kNA, kNB, 4, 12, 2>(ga, gb, counter, done, 2 * need + more, st);
+  return launch_fused_ws_t<kNA, kNB, 4, 16, 1>(ga, gb, counter, done, need + more, st);
 }
 
 template <bool kScale8, bool kSilu>
@@ -1784,42 +1792,6 @@ GemvArgs make_args(const SparseWeights& w, const Plan& plan, const __half* A, in
   g.n_slabs = 1;
   g.wait_cycles = g_wait_cycles;
   return g;
-}
-
-// Both projections of the layer in one cooperative launch (tensor-core kernel).  Returns
-// NOT_SUPPORTED when the shapes do not map to one of the instantiated pairs of configurations or the
-// device cannot keep all blocks resident; the caller then launches the projections one by one.
-template <int CGA, int SA, int CGB, int SB, int TM>
-int launch_fused_pair(GemvArgs ga, GemvArgs gb, int* done, int64_t P, int64_t E, cudaStream_t st) {
-  const void* fn = reinterpret_cast<const void*>(&fused_moe_mma_kernel<CGA, SA, CGB, SB, TM>);
-  const size_t sa = mma_smem_bytes(ga.K, SA, TM), sb = mma_smem_bytes(gb.K, SB, TM);
-  const size_t smem = sa > sb ? sa : sb;
-  static int state[64] = {0};     // per device: 0 unknown, 1 usable, -1 not usable
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return B200FP4_STATUS_NOT_SUPPORTED;
-  if (state[dev] == 0) {
-    int coop = 0, per_sm = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    bool ok = coop != 0 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess &&
-              cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMmaThreads, 227 * 1024) == cudaSuccess && per_sm >= 1;
-    if (!ok) cudaGetLastError();
-    state[dev] = ok ? 1 : -1;
-  }
-  if (state[dev] < 0) return B200FP4_STATUS_NOT_SUPPORTED;
-  ga.n_slabs = ga.inter / (64 * CGA);
-  gb.n_slabs = gb.N / (128 * CGB);
-  int need = ga.n_slabs + g_wait_extra_need;
-  const int64_t slabs = ga.n_slabs > gb.n_slabs ? ga.n_slabs : gb.n_slabs;
-  int64_t grid = max_passes(P, E) * slabs;
-  if (grid > (int64_t)sm_count()) grid = sm_count();
-  if (grid < 1) grid = 1;
-  void* args[4] = {&ga, &gb, &done, &need};
-  if (cudaLaunchCooperativeKernel(fn, dim3((unsigned)grid), dim3(kMmaThreads), args, smem, st) != cudaSuccess) {
-    cudaGetLastError();
-    return B200FP4_STATUS_NOT_SUPPORTED;
-  }
-  return B200FP4_STATUS_SUCCESS;
 }
 
 int run_projection(const SparseWeights& w, const Plan& plan, const __half* A, int64_t lda, int a_div, void* out,
@@ -2100,11 +2072,12 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   off += align_up((size_t)P * H * sizeof(float), 256);
   int* done = reinterpret_cast<int*>(ws + off);
   const int64_t n_done = max_passes(P, E);
+  const int64_t local_pairs = (expert_map && global_E > 0) ? P * E / global_E : P;      // expected
 
-  // More than 256 pairs: the warp-scheduled tensor-core kernel (passes of eight tokens, activations in fragment order
-  // from the plan kernel and from the gate_up epilogue).  Both projections share one launch and one claim sequence
-  // unless B200FP4_MOE_SEPARATE_LAUNCHES asks for one launch each.
-  if (ordered && P > 256 && ws_ok(2 * I, H, G13, I, w13) && ws_ok(H, I, G2, 0, w2)) {
+  // The warp-scheduled tensor-core kernel (passes of eight tokens, activations in fragment order from the plan kernel and
+  // from the gate_up epilogue).  Both projections share one launch and one claim sequence unless
+  // B200FP4_MOE_SEPARATE_LAUNCHES asks for one launch each (which takes other kernels up to 256 pairs).
+  if (ordered && (P > 256 || !(flags & B200FP4_MOE_SEPARATE_LAUNCHES)) && ws_ok(2 * I, H, G13, I, w13) && ws_ok(H, I, G2, 0, w2)) {
     launch_plan(topk_ids, P, topk, ld_ids, expert_map, global_E, E, plan, hidden, h16, M, H, ld_h, st, done, (int)n_done, 8,
                 bf ? kConvBf16Frag : kConvF16Frag);
     if (g_prof_events[0]) cudaEventRecord(g_prof_events[0], st);
@@ -2113,21 +2086,8 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
       GemvArgs gb = make_args(w2, plan, act, I, 1, down, B200FP4_DTYPE_F32, H, H, I, 0);
       ga.n_slabs = (int)(I / 64);
       gb.n_slabs = (int)(H / 128);
-      const int need = ga.n_slabs + g_wait_extra_need;
-      const int64_t items = max_passes(P, E) * (ga.n_slabs + gb.n_slabs);
-      // Block shape: 8 warps with 8-stage rings where K allows (both K multiples of 256), else 16 warps x 4 stages.
-      // Measured on B200 (layer step / fraction of the copy bandwidth of the launch, batch 32, 512 experts):
-      // 8 x 8: 72.4 us / 0.745; 7 x 8: 73.5 / 0.73; 8 warps x 4 stages: 73.7 / 0.72; 16 x 4: 76.0 / 0.705; 6 x 8: 78.2; 12 x 4:
-      // 79.6; 9, 10, 12 warps x 8: 79-82; 6 or 5 warps x 16 stages: 78.5 / 82.5; 4 x 8: 87.4; 24 x 4: 93.7.  With the 64
-      // local experts of one of eight expert-parallel ranks: 16 x 4 49.7 us for the launch, 8 x 8 37.6 us, 4 x 16 44.7 us.
-      const bool deep = H % 256 == 0 && I % 256 == 0;
-      if (2 * I == 1024 && H == 2048) {
-        rc = deep ? launch_fused_ws_t<1024, 2048, 8, 8>(ga, gb, plan.hdr + 2, done, need, items, st)
-                  : launch_fused_ws_t<1024, 2048>(ga, gb, plan.hdr + 2, done, need, items, st);
-      } else {
-        rc = deep ? launch_fused_ws_t<0, 0, 8, 8>(ga, gb, plan.hdr + 2, done, need, items, st)
-                  : launch_fused_ws_t<0, 0>(ga, gb, plan.hdr + 2, done, need, items, st);
-      }
+      rc = (2 * I == 1024 && H == 2048) ? launch_fused_ws<1024, 2048>(ga, gb, plan.hdr + 2, done, local_pairs, E, st)
+                                        : launch_fused_ws<0, 0>(ga, gb, plan.hdr + 2, done, local_pairs, E, st);
       if (rc != B200FP4_STATUS_SUCCESS) return rc;
       if (g_prof_events[1]) cudaEventRecord(g_prof_events[1], st);
     } else {
@@ -2147,7 +2107,6 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   // batches, expert parallelism with many source ranks) and both projections have a tensor-core
   // configuration for it; four otherwise.
   const int64_t pb = P < E ? P : E;
-  const int64_t local_pairs = (expert_map && global_E > 0) ? P * E / global_E : P;
   int tm = kMaxTok;
   if (ordered && local_pairs >= 4 * E) {
     const MmaCfg a8 = pick_mma_cfg(2 * I, H, G13, (int)I, pb, 8), b8 = pick_mma_cfg(H, I, G2, 0, pb, 8);
@@ -2156,32 +2115,6 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   launch_plan(topk_ids, P, topk, ld_ids, expert_map, global_E, E, plan, bf ? hidden : nullptr, h16, M, H, ld_h, st, done,
               (int)n_done, tm);
   if (g_prof_events[0]) cudaEventRecord(g_prof_events[0], st);
-  // One cooperative launch for both projections pays for small batches (measured on B200: 24.6 vs 27.2 us
-  // per layer at 10 pairs, 67.7 vs 68.2 us at 160); from 320 pairs on two launches are faster (100.6 vs
-  // 102.3 us, 185.6 vs 193.8 us at 1280 pairs), so it is used up to 256 pairs.
-  if (ordered && !(flags & B200FP4_MOE_SEPARATE_LAUNCHES) && P <= 256) {
-    const MmaCfg ca = pick_mma_cfg(2 * I, H, G13, (int)I, pb, tm), cb = pick_mma_cfg(H, I, G2, 0, pb, tm);
-    if (ca.ok && cb.ok) {
-      const GemvArgs ga = make_args(w13, plan, bf ? h16 : reinterpret_cast<const __half*>(hidden), bf ? H : ld_h, (int)topk,
-                                    act, B200FP4_DTYPE_F16, I, 2 * I, H, (int)I);
-      const GemvArgs gb = make_args(w2, plan, act, I, 1, down, B200FP4_DTYPE_F32, H, H, I, 0);
-      int frc = B200FP4_STATUS_NOT_SUPPORTED;
-      if (tm == 4 && ca.stages == 5 && cb.stages == 5) {
-        if (ca.cg == 2 && cb.cg == 4) frc = launch_fused_pair<2, 5, 4, 5, 4>(ga, gb, done, P, E, st);
-        else if (ca.cg == 1 && cb.cg == 2) frc = launch_fused_pair<1, 5, 2, 5, 4>(ga, gb, done, P, E, st);
-      } else if (tm == 8 && ca.stages == 3 && cb.stages == 5) {
-        if (ca.cg == 2 && cb.cg == 4) frc = launch_fused_pair<2, 3, 4, 5, 8>(ga, gb, done, P, E, st);
-        else if (ca.cg == 1 && cb.cg == 2) frc = launch_fused_pair<1, 3, 2, 5, 8>(ga, gb, done, P, E, st);
-      }
-      if (frc == B200FP4_STATUS_SUCCESS) {
-        if (g_prof_events[1]) cudaEventRecord(g_prof_events[1], st);
-        if (g_prof_events[2]) cudaEventRecord(g_prof_events[2], st);
-        weighted_reduce_kernel<<<reduce_grid(H, M), kRedThreads, 0, st>>>(down, topk_weights, plan.mapped, out, out_dtype, (int)M, (int)topk,
-                                                      (int)H, (flags & B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT) ? 1 : 0, ld_w, sc);
-        return finish_launch(3);
-      }
-    }
-  }
   rc = run_projection(w13, plan, bf ? h16 : reinterpret_cast<const __half*>(hidden), bf ? H : ld_h, (int)topk, act,
                       B200FP4_DTYPE_F16, I, P, 2 * I, H, G13, E, (int)I, ordered, st, tm);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;

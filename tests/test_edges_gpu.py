@@ -76,3 +76,31 @@ def test_quantizer_tile_edges(M, K, swizzled, offset):
     if swizzled:                                      # padding included: zeros past M and past K / 16
         ref_sf = np.asarray(oracle.sf_linear_to_swizzled(ref_sf)).reshape(got.shape)
     np.testing.assert_array_equal(got, ref_sf)
+
+
+@pytest.mark.parametrize("E,H,I,M,topk", [
+    (4, 256, 128, 1, 1),          # smallest: one item, K = 128 on the down side
+    (8, 512, 512, 3, 4),          # four warps per item
+    (16, 256, 256, 32, 8),        # 256 pairs: last size of the small plan; several passes per expert
+    (16, 256, 256, 33, 8),        # 264 pairs
+    (128, 1024, 768, 25, 10),     # eight warps, one per item
+    (512, 512, 512, 64, 8),       # 12 warps, two per item
+    (8, 384, 128, 200, 4),        # 16 warps, one per item: K no multiple of 256, many pairs per expert
+])
+def test_fused_moe_block_shapes(E, H, I, M, topk):
+    import synth
+    from dgx_vllm_b200 import sparse_fp4_v7 as sp7
+    from util import expert_fetch, gpu_quantize_fn, rel_err
+    keys = ("comp_T", "meta_T", "scale_T", "g_scales")
+    w13 = synth.make_sparse_experts(E, 2 * I, H, 1, "cuda", gpu_quantize_fn)
+    w2 = synth.make_sparse_experts(E, H, I, 2, "cuda", gpu_quantize_fn)
+    tw, ids = synth.make_routing(M, E, topk, 3, "cuda")
+    ids[0, 0] = -1                                    # not local
+    hidden = synth.make_hidden(M, H, 4, "cuda")
+    args = (hidden, tw, ids, None, *[w13[k] for k in keys], *[w2[k] for k in keys], I, False)
+    out = sp7.fused_sparse_moe_v7(*args)
+    again = sp7.fused_sparse_moe_v7(*args)
+    assert sp7.last_moe_status() == 0
+    assert torch.equal(out, again)
+    ref = oracle.fused_sparse_moe_by_expert(hidden.float().cpu().numpy(), tw.cpu().numpy(), ids.cpu().numpy(), expert_fetch(w13, w2), I)
+    assert rel_err(to_np(out), ref) < 1e-2
