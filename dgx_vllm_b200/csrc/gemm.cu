@@ -163,6 +163,44 @@ __device__ __forceinline__ void silu_quant_row(const uint32_t* pg, const uint32_
   }
 }
 
+// 32 finished columns of one row of the dense output
+__device__ __forceinline__ void store_row32(const GemmParams& p, int row, int col0, const float (&v)[32]) {
+  if (col0 >= p.N) return;
+  const bool whole = col0 + 32 <= p.N;
+  if (p.out_f32) {
+    float* dst = reinterpret_cast<float*>(p.out) + (size_t)row * p.N + col0;
+    if (whole && (p.N % 4) == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) reinterpret_cast<float4*>(dst)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (col0 + i < p.N) dst[i] = v[i];
+    }
+    return;
+  }
+  uint32_t w[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if (p.out_bf16) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    } else {
+      const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+  }
+  uint16_t* dst = reinterpret_cast<uint16_t*>(p.out) + (size_t)row * p.N + col0;
+  if (whole && (p.N % 8) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(dst)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (col0 + i < p.N) dst[i] = (uint16_t)((i & 1) ? (w[i >> 1] >> 16) : (w[i >> 1] & 0xFFFFu));
+  }
+}
+
 // ---------------------------------------------------------------------------------------- kernel
 
 // BN = tile width; KB = 64-wide k-blocks (MMAs) per shared-memory stage.  Smaller stages do not change
@@ -178,8 +216,9 @@ struct Cfg {
   static constexpr int kStageSFA = KB * 512;
   static constexpr int kStageSFB = kSfTiles * KB * 512;
   static constexpr int kStageBytes = kStageA + kStageB + kStageSFA + kStageSFB;
-  // an epilogue that stages its output takes the place of one operand stage
-  static constexpr int kStages = (BN == 128 ? 24 : 16) / KB - (kOutStage > 0 ? 1 : 0);
+  // as many stages as fit beside what the epilogue stages
+  static constexpr int kFit = (227 * 1024 - 2048 - kOutStage) / kStageBytes, kMost = (BN == 128 ? 24 : 16) / KB;
+  static constexpr int kStages = kFit < kMost ? kFit : kMost;
   // tensor-memory column map: accumulators, then one scale-factor block per shared-memory stage
   // (4 columns per k-block for A, 4*kSfTiles for B)
   static constexpr uint32_t kSfCols = KB * (4 + 4 * kSfTiles);
@@ -193,15 +232,21 @@ struct Cfg {
 
 // Staging: the dense wide-tile kernel hands [32 rows x 64 columns] boxes of 8 warps to the copy engine, the grouped kernel
 // transposes [32 rows x 32 columns] of 16 warps.
-template <int BN, bool kGrouped, bool kSiluQuant>
-constexpr int out_stage_bytes() { return kSiluQuant ? 0 : (kGrouped ? 16 * 2048 : (BN == 256 ? 8 * 4096 : 0)); }
+// kSplit > 1: partial sums from the other CTAs of the cluster, 128 rows x 128 / kSplit columns fp32 each.
+template <int BN, bool kGrouped, bool kSiluQuant, int kSplit = 1>
+constexpr int out_stage_bytes() {
+  return kSplit > 1 ? (kSplit - 1) * (4 / kSplit) * 16384 : (kSiluQuant ? 0 : (kGrouped ? 16 * 2048 : (BN == 256 ? 8 * 4096 : 0)));
+}
 
-template <int BN, int KB, bool kGrouped, bool kSiluQuant = false>
+// kSplit > 1 (dense, 128-wide tiles, fewer tiles than SMs): the kSplit CTAs of a cluster each take a part of K of one tile; each
+// then finishes 128 / kSplit of its columns, with the other CTAs' sums of them arriving through distributed shared memory.
+template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1>
 __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
   constexpr bool kOutTma = BN == 256 && !kGrouped && !kSiluQuant;     // the dense wide-tile kernel stores tiles through the copy engine
-  constexpr int kOutStage = out_stage_bytes<BN, kGrouped, kSiluQuant>();
+  constexpr int kOutStage = out_stage_bytes<BN, kGrouped, kSiluQuant, kSplit>();
+  static_assert(kSplit == 1 || (BN == 128 && !kGrouped && (kSplit == 2 || kSplit == 4)), "split K");
   using C = Cfg<BN, KB, kOutStage>;
   constexpr int kEpi = gemm_epi_groups(kGrouped);
   extern __shared__ unsigned char smem_raw[];
@@ -236,7 +281,8 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tcgen05_fence_before();
-  __syncthreads();
+  if constexpr (kSplit > 1) cluster_sync_any();      // the other CTAs run before anything is sent to them
+  else __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   pdl_wait();                 // everything above overlaps the end of the kernel before this one
@@ -247,6 +293,10 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   const int m_tiles = kGrouped ? p.g_hdr[0] : p.m_tiles;
   const int n_tiles_total = m_tiles * p.n_tiles;
   const int KT = (p.K + 63) / 64;   // 64-wide k-blocks = 512-byte scale tiles per 128 rows
+  const int rank = kSplit > 1 ? (int)(blockIdx.x % kSplit) : 0;      // in the cluster
+  const int first_tile = blockIdx.x / kSplit, tile_stride = gridDim.x / kSplit;
+  const int ks_begin = p.k_stages * rank / kSplit, ks_end = p.k_stages * (rank + 1) / kSplit;
+  float keep[kSplit > 1 ? 128 / kSplit : 1];                          // this thread's row of the columns its CTA finishes
 
   constexpr int kWarpSf = gemm_warps(kGrouped) - 1;
   if (warp == 0 || warp == kWarpSf) {
@@ -254,14 +304,14 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     if (lane == 0) {
       uint32_t s = 0, ph = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x) {
+      for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride) {
         const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, tile, m_tiles);
         const uint8_t* sfa = p.sfa + (size_t)ti.sfa_tile * KT * 512;
         const uint8_t* sfb = p.sfb + (kGrouped ? (size_t)ti.expert * (size_t)p.g_sfb_expert_bytes : (size_t)0);
         const uint8_t* sfb0 = sfb + (size_t)ti.sfb_tile0 * KT * 512;
         const uint8_t* sfb1 = sfb + (size_t)ti.sfb_tile1 * KT * 512;
         const int sf_tiles = C::kSfTiles == 1 || ti.sfb_tile1 * 128 >= p.N ? 1 : 2;      // the second 128 columns may lie past N
-        for (int ks = 0; ks < p.k_stages; ++ks) {
+        for (int ks = ks_begin; ks < ks_end; ++ks) {
           if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, p.status, 1)) { ok = false; break; }
           const uint32_t st = smem_u32(smem) + s * C::kStageBytes, bar = smem_u32(&full_bar[s]);
           if (warp == 0) {
@@ -298,11 +348,11 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
       const uint32_t full0 = smem_u32(full_bar);
       uint32_t s = 0, ph = 0, tcount = 0;
       bool ok = true, ready = false;
-      for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x, ++tcount) {
+      for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride, ++tcount) {
         const uint32_t acc = tcount % C::kAcc, aph = (tcount / C::kAcc) & 1;
         if (!mbar_wait(smem_u32(&acc_empty[acc]), aph ^ 1, p.status, 2)) { ok = false; break; }
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int ks = 0; ks < p.k_stages; ++ks) {
+        for (int ks = ks_begin; ks < ks_end; ++ks) {
           if (!ready && !mbar_wait(full0 + s * 8, ph, p.status, 3)) { ok = false; break; }
           tcgen05_fence_after();
           // each 64-wide k-block is 32 bytes further along the swizzled 128-byte rows (descriptors count 16 bytes)
@@ -316,13 +366,13 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
             for (int kb = 0; kb < KB; ++kb) {
               if (kb == KB - 1) ready = mbar_test_wait(full0 + s_next * 8, ph_next);
               tcgen05_mma_nvf4(d_tmem, a_desc + kb * 2, b_desc + kb * 2, C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles),
-                               (ks > 0 || kb > 0) ? 1u : 0u);
+                               (ks > ks_begin || kb > 0) ? 1u : 0u);
             }
           } else {
             ready = false;
             for (int kb = 0; kb < kblocks; ++kb)
               tcgen05_mma_nvf4(d_tmem, a_desc + kb * 2, b_desc + kb * 2, C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles),
-                               (ks > 0 || kb > 0) ? 1u : 0u);
+                               (ks > ks_begin || kb > 0) ? 1u : 0u);
           }
           tcgen05_commit(empty);    // frees the stage when these MMAs have read it
           s = s_next;
@@ -340,8 +390,8 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     const int quarter = warp & 3;
     uint32_t it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x) {
-      for (int ks = 0; ks < p.k_stages; ++ks, ++it) {
+    for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride) {
+      for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
         const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1;
         ok = mbar_wait(smem_u32(&sf_full[s]), ph, p.status, 6);
         ok = __all_sync(0xffffffffu, ok);
@@ -376,7 +426,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     const float alpha_dense = kGrouped ? 0.f : p.alpha[0];
     uint32_t tcount = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x, ++tcount) {
+    for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride, ++tcount) {
       const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, tile, m_tiles);
       const float alpha = kGrouped ? p.g_alphas[ti.expert] : alpha_dense;
       const uint32_t acc = tcount % C::kAcc, aph = (tcount / C::kAcc) & 1;
@@ -416,6 +466,29 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
           const size_t kt2 = (size_t)(p.q_inter / 64);
           *reinterpret_cast<uint16_t*>(p.q_sf + ((size_t)ti.sfa_tile * kt2 + (size_t)(col / 64)) * 512 + lane * 16 + quarter * 4 +
                                        (grp & 1) * 2) = (uint16_t)sf2;
+        }
+        continue;
+      }
+      if constexpr (kSplit > 1) {
+        // 32-column chunk c of the tile belongs to CTA c * kSplit / 4: kept if that is this one, sent there otherwise as
+        // [sender][chunk][quarter][column][row] so that a warp's store of one column is 128 contiguous bytes
+        constexpr int kOwn = 4 / kSplit;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          const int chunk = c_first + c, owner = chunk / kOwn;
+          uint32_t r[32];
+          tcgen05_ld_32x32(taddr + chunk * 32, r);
+          tcgen05_wait_ld();
+          if (owner == rank) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) keep[(kOwn == 1 ? 0 : c * 32) + i] = __uint_as_float(r[i]);
+          } else if (row < ti.row_end) {
+            const int slot = rank < owner ? rank : rank - 1;
+            const uint32_t dst = map_to_cta(smem_u32(out_stage) + (uint32_t)((slot * kOwn + chunk % kOwn) * 4 + quarter) * 4096u + lane * 4u,
+                                            (uint32_t)owner);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + i * 128u), "r"(r[i]) : "memory");
+          }
         }
         continue;
       }
@@ -541,6 +614,38 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
                   dst[i] = (uint16_t)((i & 1) ? (packed[c * 16 + (i >> 1)] >> 16) : (packed[c * 16 + (i >> 1)] & 0xFFFFu));
             }
           }
+        }
+      }
+    }
+  }
+  if constexpr (kSplit > 1) {
+    // every CTA's sums have arrived (also after a timed-out wait: the status word then says that the result is not valid)
+    __syncwarp();
+    cluster_sync_any();
+    constexpr int kOwn = 4 / kSplit;
+    const int quarter = warp & 3, grp = warp < 6 ? 0 : (warp - 6) >> 2;
+    const bool epilogue = warp >= 2 && (warp < 6 || (warp >= 10 && warp < 14));
+    if (epilogue && grp == rank * 2 / kSplit && first_tile < n_tiles_total) {
+      const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, first_tile, m_tiles);
+      const int row = ti.a_row0 + quarter * 32 + lane;
+      const float alpha = p.alpha[0];
+      if (row < ti.row_end) {
+#pragma unroll
+        for (int c = 0; c < kOwn; ++c) {
+          float v[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            float sum = 0.f;
+#pragma unroll
+            for (int src = 0; src < kSplit; ++src) {         // in the order of K
+              const int slot = src < rank ? src : src - 1;
+              sum += src == rank ? keep[c * 32 + i]
+                                 : __uint_as_float(lds32(smem_u32(out_stage) + (uint32_t)((slot * kOwn + c) * 4 + quarter) * 4096u +
+                                                         (uint32_t)i * 128u + lane * 4u));
+            }
+            v[i] = sum * alpha;
+          }
+          store_row32(p, row, ti.n0 + (rank * kOwn + c) * 32, v);
         }
       }
     }
@@ -701,10 +806,10 @@ bool make_rows_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t r
 
 namespace {
 
-template <int BN, int KB, bool kGrouped, bool kSiluQuant = false>
+template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int max_m_tiles, cudaStream_t st,
                 const CUtensorMap* mo = nullptr) {
-  using C = Cfg<BN, KB, out_stage_bytes<BN, kGrouped, kSiluQuant>()>;
+  using C = Cfg<BN, KB, out_stage_bytes<BN, kGrouped, kSiluQuant, kSplit>()>;
   CUtensorMap dummy = {};
   if (mo == nullptr) {
     mo = &dummy;
@@ -714,7 +819,7 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)C::kSmemBytes) != cudaSuccess) {
       cudaGetLastError();
       return B200FP4_STATUS_EXECUTION_FAILED;
@@ -723,11 +828,11 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
   }
   p.n_tiles = kSiluQuant ? p.q_inter / 128 : (p.N + BN - 1) / BN;
   long long grid = (long long)max_m_tiles * p.n_tiles;
-  if (grid > sm_count()) grid = sm_count();
+  if (kSplit == 1 && grid > sm_count()) grid = sm_count();
   if (grid < 1) grid = 1;
   p.k_stages = (p.K + KB * 64 - 1) / (KB * 64);
-  if (launch_pdl(nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant>, dim3((unsigned)grid), dim3(gemm_threads(kGrouped)), C::kSmemBytes, st,
-                 ma, mb, *mo, p) != cudaSuccess) {
+  if (launch_pdl_cluster(kSplit, nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant, kSplit>, dim3((unsigned)grid * kSplit),
+                         dim3(gemm_threads(kGrouped)), C::kSmemBytes, st, ma, mb, *mo, p) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;
   }
@@ -738,6 +843,30 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
 // 32-byte swizzled rows, 8 or 16 stages); on B200 those measured 190 and 317 us against 150 us at
 // M=4096 (TMA issues one request per box row, so narrower rows double and quadruple the requests).
 int stage_kblocks() { return 4; }
+
+// Tile of the dense GEMM: 128- or 256-wide on single CTAs (one per SM), 256 x 256 on CTA pairs, and for few tiles the split of K
+// over clusters of two or four.  Each takes whole rounds over the SMs, so the choice is the least of
+//   fixed + rounds x (stages x time per 256-k stage + tile)
+// with times in us fitted to sweeps on B200 (weights cold, M 128..4096, N 2048..16000, K 512..8192; within 10 % of all but the
+// ragged sizes).  What the former rule (256-wide once there are as many of them as SMs, pairs likewise) cost: M=777, N=3000,
+// K=4160 168 narrow tiles on 148 SMs 20.7 us, 84 wide ones 13.4; M=1024, N=4096, K=4096 17.8 / 12.4; M=600, N=6000, K=8192
+// 30.5 us, pairs 19.3.
+void pick_dense_tile(int64_t M, int64_t N, int64_t stages, bool f32, int& bn, int& split) {
+  const int64_t sms = sm_count(), m128 = (M + 127) / 128, m256 = (M + 255) / 256, n128 = (N + 127) / 128, n256 = (N + 255) / 256;
+  auto rounds = [](int64_t tiles, int64_t places) { return (double)((tiles + places - 1) / places); };
+  const double S = (double)stages;
+  const double narrow = 3.3 + rounds(m128 * n128, sms) * (0.42 * S + 0.6);
+  const double wide = 3.3 + rounds(m128 * n256, sms) * (0.56 * S + 0.6);
+  // a row pitch that is no multiple of 32 bytes slows the pair kernel's direct stores
+  const double pair = 3.8 + rounds(m256 * n256, sms / 2) * (0.46 * S + 1.6 + (N % 16 != 0 ? 1.5 : 0.0));
+  bn = wide < narrow ? 256 : 128;
+  if (!f32 && pair < (wide < narrow ? wide : narrow)) bn = 512;
+  split = 1;
+  if (bn == 128 && stages >= 4) {
+    if (m128 * n128 * 4 <= sms && stages >= 8) split = 4;
+    else if (m128 * n128 * 2 <= sms) split = 2;
+  }
+}
 
 template <bool kGrouped>
 int dispatch_gemm(int bn, int kb, const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int max_m_tiles,
@@ -784,15 +913,8 @@ extern "C" int b200fp4_gemm_nvfp4(const void* a_codes, const void* b_codes, cons
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.m_tiles = (int)((M + kBM - 1) / kBM);
   p.status = reinterpret_cast<int*>(workspace);
-  // Wide tiles once there are enough of them to fill the GPU; narrow tiles (double-buffered
-  // accumulator, twice the CTAs) for small problems.
-  // ... and 256 x 256 tiles on pairs of CTAs (gemm_pair.cu) once there are two rounds of those for every pair of SMs
-  // (measured at N=14336, K=4096: M=1024 46 us against 48 us, M=4096 123 us against 129 us; M=128 stays with 128-wide tiles).
-  int bn = tile_n;
-  if (bn == 0) {
-    bn = (p.m_tiles * ((N + 255) / 256) >= sm_count()) ? 256 : 128;
-    if (bn == 256 && !p.out_f32 && ((M + 255) / 256) * ((N + 255) / 256) >= sm_count()) bn = 512;
-  }
+  int bn = tile_n, split = 1;
+  if (bn == 0) pick_dense_tile(M, N, (K + 255) / 256, p.out_f32 != 0, bn, split);
   const int kb = stage_kblocks();
   if (bn == 512) {
     // 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2)
@@ -816,7 +938,9 @@ extern "C" int b200fp4_gemm_nvfp4(const void* a_codes, const void* b_codes, cons
   CUtensorMap mo;
   const bool tma_out = bn == 256 && !p.out_f32 && (N % 8) == 0 && make_out_map(&mo, out, (uint64_t)M, (uint64_t)N);
   p.out_tma = tma_out ? 1 : 0;
-  int rc = dispatch_gemm<false>(bn, kb, ma, mb, p, p.m_tiles, st, tma_out ? &mo : nullptr);
+  int rc = split == 4   ? launch_gemm<128, 4, false, false, 4>(ma, mb, p, p.m_tiles, st)
+           : split == 2 ? launch_gemm<128, 4, false, false, 2>(ma, mb, p, p.m_tiles, st)
+                        : dispatch_gemm<false>(bn, kb, ma, mb, p, p.m_tiles, st, tma_out ? &mo : nullptr);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   return finish_launch(1);
 }

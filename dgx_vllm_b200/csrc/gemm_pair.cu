@@ -63,12 +63,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// shared::cluster address of the same shared-memory offset in CTA `rank` of this cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 // Arrival on a barrier of any CTA of the cluster.  Relaxed: what it publishes are tensor-memory accesses, which the
 // tcgen05 wait and fence before it have completed and ordered; a release at cluster scope costs the arriving thread
 // about 1100 cycles here, more than a whole stage of MMAs.

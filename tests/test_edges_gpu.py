@@ -104,3 +104,36 @@ def test_fused_moe_block_shapes(E, H, I, M, topk):
     assert torch.equal(out, again)
     ref = oracle.fused_sparse_moe_by_expert(hidden.float().cpu().numpy(), tw.cpu().numpy(), ids.cpu().numpy(), expert_fetch(w13, w2), I)
     assert rel_err(to_np(out), ref) < 1e-2
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 2048),             # split of K over four CTAs, one row and less than a 32-column piece
+    (33, 136, 2112),          # ... ragged everywhere, last k-stage short
+    (129, 1000, 4096),        # ... two row tiles
+    (5, 5000, 1024),          # split over two
+    (200, 4096, 1088),        # ... two row tiles
+    (8, 264, 768),            # three stages: no split
+    (385, 6000, 1024),        # wide tiles, ragged
+    (520, 7000, 2048),        # pairs of CTAs, ragged
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dense_gemm_tile_choice(M, N, K, dtype):
+    from dgx_vllm_b200 import cutlass_scaled_fp4_mm, scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").mul_(0.02).to(torch.bfloat16)
+    gx, gw = torch.full((1,), 2688 / 6.5, device="cuda"), torch.full((1,), 2688 / 0.13, device="cuda")
+    (xc, xs), (wc, ws) = scaled_fp4_quant(x, gx), scaled_fp4_quant(w, gw)
+    alpha = 1.0 / (gx * gw)
+    guard = torch.full((M * N + 64,), 7.0, dtype=dtype, device="cuda")       # nothing past the result is touched
+    out = guard[:M * N].view(M, N)
+    cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype, out=out)
+    assert last_gemm_status() == 0
+    assert bool((guard[M * N:] == 7.0).all())
+
+    def deq(codes, sf, gs, rows):
+        lin = oracle.sf_swizzled_to_linear(to_np(sf).reshape(-1), rows, K // 16)
+        return torch.from_numpy(oracle.dequantize(to_np(codes), lin, float(gs[0]))).cuda().double()
+    ref = (deq(xc, xs, gx, M) @ deq(wc, ws, gw, N).t()).float()
+    assert ((out.float() - ref).abs().max() / ref.abs().max()).item() < 5e-3
