@@ -1341,7 +1341,8 @@ __global__ void __launch_bounds__(32 * kW, 1) sparse_gemv_ws_kernel(const GemvAr
 // Both projections of the MoE layer in one launch: the claim sequence runs through the gate_up items and on into the
 // down items, so a warp that finds no gate_up item left starts on the down projection of passes that are complete
 // instead of idling until the slowest warp of a first launch has finished and a second launch has ramped up.
-template <int kNA, int kNB, int kS, int kW, int KS>
+// kSB: ring slots the down projection turns through (its slice of K may be shorter than a ring).
+template <int kNA, int kNB, int kS, int kW, int KS, int kSB>
 __global__ void __launch_bounds__(32 * kW, 1)
     fused_moe_ws_kernel(const GemvArgs ga, const GemvArgs gb, int* counter, int* done, int need) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1352,7 +1353,7 @@ __global__ void __launch_bounds__(32 * kW, 1)
   const WsUnit U = ws_unit<kS, kW, KS>(L, claims);
   const int n_a = ga.plan.hdr[1] * ga.n_slabs;
   ws_phase<true, kNA, 1, kS, KS>(ga, counter, 0, claims, L, U, done, need);
-  ws_phase<false, kNB, 2, kS, KS>(gb, counter, n_a, claims, L, U, done, need);
+  ws_phase<false, kNB, 2, kSB, KS>(gb, counter, n_a, claims, L, U, done, need);
 }
 
 // ------------------------------------------------------------------------------------------ generic
@@ -1689,32 +1690,57 @@ int run_projection_ws(const SparseWeights& w, const Plan& plan, const __half* A,
   return N == 2048 ? launch_ws_t<false, 2048>(g, counter, items, st) : launch_ws_t<false, 0>(g, counter, items, st);
 }
 
-template <int kNA, int kNB, int kS, int kW, int KS>
+template <int kNA, int kNB, int kS, int kW, int KS, int kSB = kS>
 int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int need, cudaStream_t st) {
   static bool attr_set[64] = {false};
   constexpr size_t smem = ws_smem_bytes<kS, kW, KS>();
   static_assert(smem <= 227 * 1024, "shared memory of the ring");
-  if (!ws_prepare(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
-  launch_pdl(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS>, dim3((unsigned)sm_count()), dim3(32 * kW), smem, st, ga, gb, counter, done, need);
+  if (!ws_prepare(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS, kSB>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
+  launch_pdl(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS, kSB>, dim3((unsigned)sm_count()), dim3(32 * kW), smem, st, ga, gb, counter, done, need);
   return B200FP4_STATUS_SUCCESS;
 }
 
-// Block shape of the one-launch layer by the number of gate_up items (at most one pass per local pair or expert, times 64-column
-// groups).  Measured on B200, 512 experts, H=2048, I=512, top-10, us per layer at M = 1 / 4 / 8 / 16 / 24 / 32 / 64 / 128:
-//   12 warps x 4 stages, four per item    18.3  27.5  34.5  50.0  63.3  73.9  107   142
-//    8 warps x 8 stages, one per item     26.5  28.8  33.3  47.8  61.8  68.7  97.4  127
-//   12 warps x 4 stages, two per item     21.5  27.9  35.7  50.1  58.0  67.6  96.6  128
-//   16 warps x 4 stages, one per item     28.5  31.0  36.4  50.3  60.3  68.5  104   121
-// (K-sliced blocks of the former small-batch kernel: 22.6  34.7  43.6  66.1  86.1).  With the 64 local experts of one of eight
-// expert-parallel ranks the launch alone is 37.6 us with 8 x 8 and 49.7 us with 16 x 4.
+// Block shape of the one-launch layer by the number of gate_up items (expected passes if every expert is hit, times 64-column
+// groups).  Measured on B200, top-10, us per layer; the former K-sliced and 8 x 8 kernels in the last row:
+//   experts, H, I             512, 2048, 512                    128, 4096, 1024                16, 4096, 1024
+//   M                         8     16    32    64    128  256   8     32    64    128  256    8     32    64    128  256
+//   12 warps, four per item   34.2  50.2  75.3  109   140  159   73.4  124   140   206  348    32.1  55.3  88.1  159  300
+//    8 warps, one per item    33.0  47.0  67.9  96.6  125  142   72.9  118   130   189  312    40.5  57.7  93.2  142  262
+//   12 warps, two per item    34.6  49.8  67.9  96.1  125  141   80.2  120   128   189  312    33.8  54.7  79.5  137  255
+//   16 warps, one per item    35.6  49.5  67.2  102   120  134   95.1  125   133   195  306    46.7  66.3  86.1  159  247
+//   before                    43.2  65.6  68.4  97.2  125  142   95.9  119   133   189  320    54.5  66.4  95.2  144  267
+// Under three items an SM four warps share one; while single-pass items last about a round of the warps, eight warps with the
+// deepest rings stream best; in between two warps an item level the last round; sixteen warps need enough items that their
+// last round is short beside the rest, twice as many where an item is twice as long.
 template <int kNA, int kNB>
 int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int64_t local_pairs, int64_t E, cudaStream_t st) {
-  const int64_t items = (local_pairs < E ? local_pairs : E) * ga.n_slabs, sms = sm_count();
-  const bool k256 = ga.K % 256 == 0 && gb.K % 256 == 0, k512 = ga.K % 512 == 0 && gb.K % 512 == 0;
+  const int64_t passes = (local_pairs < E ? local_pairs : E) * ((local_pairs + 8 * E - 1) / (8 * E));
+  const int64_t items = passes * ga.n_slabs, sms = sm_count();
   const int need = ga.n_slabs, more = g_wait_extra_need;       // per warp of an item: counts a pass's down items wait for
-  if (k512 && items <= 3 * sms) return launch_fused_ws_t<kNA, kNB, 4, 12, 4>(ga, gb, counter, done, 4 * need + more, st);
-  if (k256 && items <= 10 * sms) return launch_fused_ws_t<kNA, kNB, 8, 8, 1>(ga, gb, counter, done, need + more, st);
-  if (k256 && local_pairs < 2 * E) return launch_fused_ws_t<kNA, kNB, 4, 12, 2>(ga, gb, counter, done, 2 * need + more, st);
+  // 32-wide steps per warp with the item shared by KS warps; whole turns of a 4-slot ring in the gate_up projection, of 4, 3 or
+  // 2 slots in the down projection
+  auto turns = [&](int KS) {
+    const int a = ga.K / 32, b = gb.K / 32;
+    if (a % (4 * KS) != 0 || b % KS != 0) return 0;
+    return b / KS % 4 == 0 ? 4 : (b / KS % 3 == 0 ? 3 : (b / KS % 2 == 0 ? 2 : 0));
+  };
+  constexpr bool kAny = kNA == 0;              // the instantiation for one model's widths has K = 2048 and 512 only
+  if (items <= 3 * sms) {
+    const int t = turns(4), n = 4 * need + more;
+    if (t == 4) return launch_fused_ws_t<kNA, kNB, 4, 12, 4>(ga, gb, counter, done, n, st);
+    if (kAny && t == 3) return launch_fused_ws_t<0, 0, 4, 12, 4, 3>(ga, gb, counter, done, n, st);
+    if (kAny && t == 2) return launch_fused_ws_t<0, 0, 4, 12, 4, 2>(ga, gb, counter, done, n, st);
+  }
+  if (items <= 10 * sms && local_pairs <= E && ga.K % 256 == 0) {
+    if (gb.K % 256 == 0) return launch_fused_ws_t<kNA, kNB, 8, 8, 1>(ga, gb, counter, done, need + more, st);
+    if (kAny) return launch_fused_ws_t<0, 0, 8, 8, 1, 4>(ga, gb, counter, done, need + more, st);
+  }
+  if (items * 2048 <= 24 * sms * (ga.K > 2048 ? ga.K : 2048)) {
+    const int t = turns(2), n = 2 * need + more;
+    if (t == 4) return launch_fused_ws_t<kNA, kNB, 4, 12, 2>(ga, gb, counter, done, n, st);
+    if (kAny && t == 3) return launch_fused_ws_t<0, 0, 4, 12, 2, 3>(ga, gb, counter, done, n, st);
+    if (kAny && t == 2) return launch_fused_ws_t<0, 0, 4, 12, 2, 2>(ga, gb, counter, done, n, st);
+  }
   return launch_fused_ws_t<kNA, kNB, 4, 16, 1>(ga, gb, counter, done, need + more, st);
 }
 

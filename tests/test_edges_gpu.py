@@ -85,6 +85,10 @@ def test_quantizer_tile_edges(M, K, swizzled, offset):
     (16, 256, 256, 33, 8),        # 264 pairs
     (128, 1024, 768, 25, 10),     # eight warps, one per item
     (512, 512, 512, 64, 8),       # 12 warps, two per item
+    (8, 512, 384, 3, 4),          # four warps per item, down slices of three steps
+    (8, 1024, 256, 3, 4),         # ... of two
+    (128, 512, 384, 40, 4),       # eight warps, down turns of four
+    (256, 512, 384, 64, 4),       # 12 warps, two per item, down turns of three
     (8, 384, 128, 200, 4),        # 16 warps, one per item: K no multiple of 256, many pairs per expert
 ])
 def test_fused_moe_block_shapes(E, H, I, M, topk):
