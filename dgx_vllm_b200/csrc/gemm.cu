@@ -240,7 +240,19 @@ constexpr int out_stage_bytes() {
 
 // kSplit > 1 (dense, 128-wide tiles, fewer tiles than SMs): the kSplit CTAs of a cluster each take a part of K of one tile; each
 // then finishes 128 / kSplit of its columns, with the other CTAs' sums of them arriving through distributed shared memory.
-template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1>
+// The KB scale tiles of a stage to tensor memory, `step` columns apart: all loads before the first store (one after the other
+// they were on the path of short main loops: grouped down projection of 64 x 1280 rows, K = 1024, 96 us, 85 so)
+template <int KB>
+__device__ __forceinline__ void copy_sf(uint32_t tmem, uint32_t step, const unsigned char* sf, int lane) {
+  uint4 w[KB];
+#pragma unroll
+  for (int kb = 0; kb < KB; ++kb) w[kb] = *reinterpret_cast<const uint4*>(sf + kb * 512 + lane * 16);
+#pragma unroll
+  for (int kb = 0; kb < KB; ++kb) tcgen05_st_32x32_x4(tmem + kb * step, w[kb]);
+}
+
+// kStageSf: the scales of A come as [128-row tile][256 of k][row][16 bytes]
+template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1, bool kStageSf = false>
 __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_out, const GemmParams p) {
@@ -306,7 +318,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
       bool ok = true;
       for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride) {
         const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, tile, m_tiles);
-        const uint8_t* sfa = p.sfa + (size_t)ti.sfa_tile * KT * 512;
+        const uint8_t* sfa = p.sfa + (size_t)ti.sfa_tile * (kStageSf ? p.k_stages * KB : KT) * 512;
         const uint8_t* sfb = p.sfb + (kGrouped ? (size_t)ti.expert * (size_t)p.g_sfb_expert_bytes : (size_t)0);
         const uint8_t* sfb0 = sfb + (size_t)ti.sfb_tile0 * KT * 512;
         const uint8_t* sfb1 = sfb + (size_t)ti.sfb_tile1 * KT * 512;
@@ -325,8 +337,9 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
             // operand tiles are still in flight
             const uint32_t bytes = (uint32_t)min(KB, KT - ks * KB) * 512, off = (uint32_t)ks * (KB * 512);
             const uint32_t sbar = smem_u32(&sf_full[s]), dst = st + C::kStageA + C::kStageB;
-            mbar_expect_tx(sbar, bytes * (1 + sf_tiles));
-            bulk_load_1d(dst, sfa + off, bytes, sbar);
+            const uint32_t bytes_a = kStageSf ? KB * 512 : bytes;
+            mbar_expect_tx(sbar, bytes_a + bytes * sf_tiles);
+            bulk_load_1d(dst, sfa + off, bytes_a, sbar);
             bulk_load_1d(dst + C::kStageSFA, sfb0 + off, bytes, sbar);
             if (sf_tiles > 1) bulk_load_1d(dst + C::kStageSFA + KB * 512, sfb1 + off, bytes, sbar);
           }
@@ -399,12 +412,37 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         const unsigned char* sf = smem + (size_t)s * C::kStageBytes + C::kStageA + C::kStageB;
         const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + C::kSfBase + s * C::kSfCols;
         const int kblocks = min(KB, KT - ks * KB);
-        for (int kb = 0; kb < kblocks; ++kb) {
-          tcgen05_st_32x32_x4(t0 + kb * 4, *reinterpret_cast<const uint4*>(sf + kb * 512 + lane * 16));
+        if (kblocks == KB) {
+          if constexpr (kStageSf) {
+            // 16 bytes of each of the rows lane, lane + 32, ...: a word per k-block
+            static_assert(KB == 4, "stage of 256 k");
+            uint4 w[4];
 #pragma unroll
-          for (int j = 0; j < C::kSfTiles; ++j)
-            tcgen05_st_32x32_x4(t0 + 4 * KB + kb * (4 * C::kSfTiles) + j * 4,
-                                *reinterpret_cast<const uint4*>(sf + C::kStageSFA + j * (KB * 512) + kb * 512 + lane * 16));
+            for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const uint4*>(sf + j * 512 + lane * 16);
+            tcgen05_st_32x32_x4(t0, make_uint4(w[0].x, w[1].x, w[2].x, w[3].x));
+            tcgen05_st_32x32_x4(t0 + 4, make_uint4(w[0].y, w[1].y, w[2].y, w[3].y));
+            tcgen05_st_32x32_x4(t0 + 8, make_uint4(w[0].z, w[1].z, w[2].z, w[3].z));
+            tcgen05_st_32x32_x4(t0 + 12, make_uint4(w[0].w, w[1].w, w[2].w, w[3].w));
+          } else {
+            copy_sf<KB>(t0, 4, sf, lane);
+          }
+#pragma unroll
+          for (int j = 0; j < C::kSfTiles; ++j) copy_sf<KB>(t0 + 4 * KB + j * 4, 4 * C::kSfTiles, sf + C::kStageSFA + j * (KB * 512), lane);
+        } else {
+          for (int kb = 0; kb < kblocks; ++kb) {
+            uint4 a;
+            if constexpr (kStageSf) {
+              const uint32_t* w = reinterpret_cast<const uint32_t*>(sf) + lane * 4 + kb;
+              a = make_uint4(w[0], w[128], w[256], w[384]);
+            } else {
+              a = *reinterpret_cast<const uint4*>(sf + kb * 512 + lane * 16);
+            }
+            tcgen05_st_32x32_x4(t0 + kb * 4, a);
+#pragma unroll
+            for (int j = 0; j < C::kSfTiles; ++j)
+              tcgen05_st_32x32_x4(t0 + 4 * KB + kb * (4 * C::kSfTiles) + j * 4,
+                                  *reinterpret_cast<const uint4*>(sf + C::kStageSFA + j * (KB * 512) + kb * 512 + lane * 16));
+          }
         }
         tcgen05_wait_st();
         tcgen05_fence_before();
@@ -806,7 +844,7 @@ bool make_rows_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t r
 
 namespace {
 
-template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1>
+template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1, bool kStageSf = false>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int max_m_tiles, cudaStream_t st,
                 const CUtensorMap* mo = nullptr) {
   using C = Cfg<BN, KB, out_stage_bytes<BN, kGrouped, kSiluQuant, kSplit>()>;
@@ -819,7 +857,7 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant, kSplit, kStageSf>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)C::kSmemBytes) != cudaSuccess) {
       cudaGetLastError();
       return B200FP4_STATUS_EXECUTION_FAILED;
@@ -831,7 +869,7 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
   if (kSplit == 1 && grid > sm_count()) grid = sm_count();
   if (grid < 1) grid = 1;
   p.k_stages = (p.K + KB * 64 - 1) / (KB * 64);
-  if (launch_pdl_cluster(kSplit, nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant, kSplit>, dim3((unsigned)grid * kSplit),
+  if (launch_pdl_cluster(kSplit, nvfp4_gemm_kernel<BN, KB, kGrouped, kSiluQuant, kSplit, kStageSf>, dim3((unsigned)grid * kSplit),
                          dim3(gemm_threads(kGrouped)), C::kSmemBytes, st, ma, mb, *mo, p) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;
@@ -986,8 +1024,9 @@ namespace b200fp4 {
 int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
                  const int32_t* expert_offsets, const int32_t* sf_offsets, void* out, int out_dtype, int64_t rows_capacity, int64_t N,
                  int64_t K, int64_t E, int tile_n, void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs,
-                 bool tiles_ready) {
+                 bool tiles_ready, bool stage_sf) {
   const bool fused = q_sf != nullptr;
+  if (stage_sf && !fused) return B200FP4_STATUS_INVALID_VALUE;
   if (fused && (!q_gs || (N % 256) != 0 || !aligned(out, 32) || !aligned(q_sf, 4))) return B200FP4_STATUS_INVALID_VALUE;
   if (rows_capacity < 0 || N <= 0 || K <= 0 || E <= 0 || (K % 64) != 0) return B200FP4_STATUS_INVALID_VALUE;
   if (out_dtype != B200FP4_DTYPE_BF16 && out_dtype != B200FP4_DTYPE_F16) return B200FP4_STATUS_NOT_SUPPORTED;
@@ -1042,7 +1081,9 @@ int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, con
   if (!tiles_ready)
     grouped_tiles_kernel<<<1, 1024, 0, st>>>(expert_offsets, sf_offsets, (int)E, grouped_hdr(workspace), grouped_tiles(workspace),
                                              max_tiles);
-  int rc = fused ? launch_gemm<256, 4, true, true>(ma, mb, p, max_tiles, st) : dispatch_gemm<true>(bn, kb, ma, mb, p, max_tiles, st);
+  int rc = stage_sf ? launch_gemm<256, 4, true, true, 1, true>(ma, mb, p, max_tiles, st)
+           : fused  ? launch_gemm<256, 4, true, true>(ma, mb, p, max_tiles, st)
+                    : dispatch_gemm<true>(bn, kb, ma, mb, p, max_tiles, st);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   return finish_launch(tiles_ready ? 1 : 2);
 }
@@ -1054,7 +1095,7 @@ extern "C" int b200fp4_grouped_gemm_nvfp4(const void* a_codes, const void* b_cod
                                           void* out, int out_dtype, int64_t rows_capacity, int64_t N, int64_t K, int64_t E,
                                           int tile_n, void* workspace, size_t workspace_bytes, void* stream) {
   return grouped_gemm(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out, out_dtype, rows_capacity, N, K, E, tile_n,
-                      workspace, workspace_bytes, stream, nullptr, nullptr, false);
+                      workspace, workspace_bytes, stream, nullptr, nullptr, false, false);
 }
 
 extern "C" int b200fp4_grouped_gemm_nvfp4_silu_quant(const void* a_codes, const void* b_codes, const void* a_sf,
@@ -1065,7 +1106,7 @@ extern "C" int b200fp4_grouped_gemm_nvfp4_silu_quant(const void* a_codes, const 
                                                      size_t workspace_bytes, void* stream) {
   if (!out_sf || !out_global_scales) return B200FP4_STATUS_INVALID_VALUE;
   return grouped_gemm(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out_codes, mid_dtype, rows_capacity, N, K, E, 0,
-                      workspace, workspace_bytes, stream, out_sf, out_global_scales, false);
+                      workspace, workspace_bytes, stream, out_sf, out_global_scales, false, false);
 }
 
 extern "C" int b200fp4_shuffle_rows(const void* in, int64_t row_bytes, const int32_t* dst2src, int64_t n_dst,

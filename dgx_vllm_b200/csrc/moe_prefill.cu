@@ -280,8 +280,9 @@ __global__ void unpermute_reduce_kernel(const T* __restrict__ expert_out, const 
 
 // The same for H % 8 == 0 and 16-byte aligned rows: eight columns per thread, 16-byte loads and stores, same order of
 // additions per output element.  Bound by HBM (the rows of a large prompt do not fit L2) or, for small prompts, by the latency
-// of a token's rows: those of eight slots are requested before the first is used.
-constexpr int kUnpermuteThreads = 128;
+// of a token's rows: those of four slots are requested before the first is used (8192 x 2048, ten slots: four 68 us, five 67.5,
+// eight 73.5, twelve 84.6 -- their registers cost more warps than they keep requests in flight).
+constexpr int kUnpermuteThreads = 128, kUnpermuteBatch = 4;
 
 template <typename T>
 __global__ void __launch_bounds__(kUnpermuteThreads)
@@ -293,11 +294,11 @@ __global__ void __launch_bounds__(kUnpermuteThreads)
   const int h = (blockIdx.x * kUnpermuteThreads + threadIdx.x) * 8;
   if (h >= H) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int t0 = 0; t0 < topk; t0 += 8) {
-    uint4 raw[8];
-    float w[8];
+  for (int t0 = 0; t0 < topk; t0 += kUnpermuteBatch) {
+    uint4 raw[kUnpermuteBatch];
+    float w[kUnpermuteBatch];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kUnpermuteBatch; ++i) {
       const int r = t0 + i < topk ? src2dst[m * topk + t0 + i] : -1;
       raw[i] = make_uint4(0, 0, 0, 0);
       w[i] = 0.f;
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kUnpermuteThreads)
       }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kUnpermuteBatch; ++i) {
       const T* v = reinterpret_cast<const T*>(&raw[i]);
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc[k] = fmaf(w[i], to_f32<T>(v[k]), acc[k]);
@@ -344,7 +345,7 @@ PrefillLayout prefill_layout(int64_t M, int64_t topk, int64_t H, int64_t I, int6
   l.dst2src = take((size_t)l.P * 4);
   l.src2dst = take((size_t)l.P * 4);
   l.xq = take((size_t)l.P * H / 2);
-  l.xsf = take((size_t)l.sf_rows * ((H / 16 + 3) / 4 * 4));
+  l.xsf = take(stage_sf_bytes(l.sf_rows, H));
   l.hq = take((size_t)l.P * I / 2);
   l.hsf = take((size_t)l.sf_rows * ((I / 16 + 3) / 4 * 4));
   l.c2 = take((size_t)l.P * H * 2);
@@ -453,13 +454,13 @@ extern "C" int b200fp4_moe_prefill(const void* hidden, int dtype, const float* t
   }
   if (rc == B200FP4_STATUS_SUCCESS)
     rc = experts_quantize_scatter(hidden, dtype, M, H, topk, src2dst, a1_gs, eo, bso, (int32_t)E, l.sf_rows, topk_ids, expert_map, global_E,
-                                  ws + l.xq, ws + l.xsf, stream, false);
+                                  ws + l.xq, ws + l.xsf, stream, true);
   if (rc == B200FP4_STATUS_SUCCESS)
     rc = grouped_gemm(ws + l.xq, w13_codes, ws + l.xsf, w13_sf, alpha1, eo, bso, ws + l.hq, dtype, l.P, 2 * I, H, E, 0, ws + l.gemm,
-                      gemm_bytes, stream, ws + l.hsf, a2_gs, one_launch);
+                      gemm_bytes, stream, ws + l.hsf, a2_gs, one_launch, true);
   if (rc == B200FP4_STATUS_SUCCESS)
     rc = grouped_gemm(ws + l.hq, w2_codes, ws + l.hsf, w2_sf, alpha2, eo, bso, ws + l.c2, dtype, l.P, H, I, E, 0, ws + l.gemm, gemm_bytes,
-                      stream, nullptr, nullptr, true);
+                      stream, nullptr, nullptr, true, false);
   if (rc == B200FP4_STATUS_SUCCESS)
     rc = b200fp4_moe_unpermute_reduce(ws + l.c2, dtype, src2dst, topk_weights, M, topk, H, out, stream);
   return rc;

@@ -260,11 +260,12 @@ __global__ void __launch_bounds__(kTX* kTY)
 // lanes per block the kernel issued 70 instructions per 8 elements and destination and was bound by that (8192 x 2048, ten
 // destinations: 51-58 us, 82 % of the issue slots).  Slots whose expert has the global scale of the slot before share its
 // codes -- the arithmetic depends on nothing else -- and only store them again.  Four lanes put their scale bytes together for
-// one 4-byte store.
+// one 4-byte store; with kStageSf (the grouped GEMM's own layout) sixteen lanes for one of 16 bytes: the 4-byte stores, each to
+// a sector of its own, were half of all sectors written (8192 x 2048, ten destinations: 45.3 us, 35.5 so, 33.2 without scales).
 constexpr int kScatterMaxTopk = 32;
 constexpr int kScatterThreads = 256;
 
-template <typename T>
+template <typename T, bool kStageSf>
 __global__ void __launch_bounds__(kScatterThreads)
     experts_quantize_scatter_kernel(const T* __restrict__ x, int64_t K, int topk, const int32_t* __restrict__ src2dst,
                                     const float* __restrict__ gs_ptr, const int32_t* __restrict__ expert_offsets,
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kScatterThreads)
     s_gs[threadIdx.x] = gs;
     s_rcp[threadIdx.x] = __frcp_rn(gs + (gs == 0.f ? 1.0e8f : 0.f));
     // byte offsets of the destination row in the code tensor and of its first scale byte, computed once per block
-    s_sfrow[threadIdx.x] = sf_swizzled_offset(row, 0, KT);
+    s_sfrow[threadIdx.x] = kStageSf ? (row >> 7) * ((KB + 15) >> 4) * 2048 + (row & 127) * 16 : sf_swizzled_offset(row, 0, KT);
     s_code[threadIdx.x] = (long long)dst * (long long)(K >> 1);
   }
   __syncthreads();
@@ -329,9 +330,11 @@ __global__ void __launch_bounds__(kScatterThreads)
     unpack8<T>(r0, v);
     unpack8<T>(r1, v + 8);
     const float sixth = __fmul_rn(fmaxf(amax8<T>(r0), amax8<T>(r1)), 0.16666667163372039794921875f);
-    const int64_t sf_col = (int64_t)(kb >> 2) * 512 + (kb & 3);     // scale byte of this block of 16 relative to its row's first
+    // scale byte of this block of 16 relative to its row's first
+    const int64_t sf_col = kStageSf ? (int64_t)(kb >> 4) * 2048 + (kb & 15) : (int64_t)(kb >> 2) * 512 + (kb & 3);
     uint2 packed = make_uint2(0, 0);
     uint32_t sfb = 0, sf4 = 0;
+    uint4 sf16 = make_uint4(0, 0, 0, 0);
     float last_gs = __int_as_float(0x7FFFFFFF);                     // a NaN: equal to nothing
     for (int sl = 0; sl < topk; ++sl) {
       if (s_dst[sl] < 0) continue;
@@ -347,10 +350,15 @@ __global__ void __launch_bounds__(kScatterThreads)
         sf4 = sfb << (8 * (threadIdx.x & 3));
         sf4 |= __shfl_xor_sync(0xffffffffu, sf4, 1);
         sf4 |= __shfl_xor_sync(0xffffffffu, sf4, 2);
+        if (kStageSf)
+          sf16 = make_uint4(sf4, __shfl_down_sync(0xffffffffu, sf4, 4), __shfl_down_sync(0xffffffffu, sf4, 8),
+                            __shfl_down_sync(0xffffffffu, sf4, 12));
       }
       if (ok) {
         *reinterpret_cast<uint2*>(codes + s_code[sl] + kb * 8) = packed;
-        if (!sf_words) sf[s_sfrow[sl] + sf_col] = (uint8_t)sfb;
+        if (kStageSf) {
+          if ((threadIdx.x & 15) == 0) *reinterpret_cast<uint4*>(sf + s_sfrow[sl] + sf_col) = sf16;
+        } else if (!sf_words) sf[s_sfrow[sl] + sf_col] = (uint8_t)sfb;
         else if ((threadIdx.x & 3) == 0) *reinterpret_cast<uint32_t*>(sf + s_sfrow[sl] + sf_col) = sf4;
       }
     }
@@ -451,7 +459,7 @@ namespace b200fp4 {
 int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
                              const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
                              int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
-                             int64_t global_E, void* codes, void* sf, void* stream, bool zero_sf) {
+                             int64_t global_E, void* codes, void* sf, void* stream, bool stage_sf) {
   if (expert_map && (!topk_ids || global_E <= 0)) return B200FP4_STATUS_INVALID_VALUE;
   if (n_src < 0 || K <= 0 || (K % 16) != 0 || topk <= 0 || num_experts <= 0 || sf_rows_padded < 0 ||
       (sf_rows_padded % 128) != 0)
@@ -463,21 +471,24 @@ int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t
     return B200FP4_STATUS_INVALID_VALUE;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t KB = K / 16;
-  if (zero_sf && cudaMemsetAsync(sf, 0, (size_t)(sf_rows_padded * (((KB + 3) / 4) * 4)), st) != cudaSuccess) {
+  if (stage_sf && ((K % 64) != 0 || !aligned(sf, 16))) return B200FP4_STATUS_INVALID_VALUE;
+  if (!stage_sf && cudaMemsetAsync(sf, 0, (size_t)(sf_rows_padded * (((KB + 3) / 4) * 4)), st) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;
   }
   if (n_src == 0) return finish_launch(1);
   const unsigned threads = (unsigned)(KB >= kScatterThreads ? kScatterThreads : (KB + 31) / 32 * 32);
+  auto launch = [&](auto* kernel, const auto* src) {
+    launch_pdl(kernel, dim3((unsigned)n_src), dim3(threads), 0, st, src, K, (int)topk, src2dst, global_scales, expert_offsets,
+               blockscale_offsets, num_experts, topk_ids, expert_map, (int)global_E, (uint8_t*)codes, (uint8_t*)sf);
+  };
   if (in_dtype == B200FP4_DTYPE_BF16)
-    launch_pdl(experts_quantize_scatter_kernel<__nv_bfloat16>, dim3((unsigned)n_src), dim3(threads), 0, st,
-               reinterpret_cast<const __nv_bfloat16*>(x), K, (int)topk, src2dst, global_scales, expert_offsets, blockscale_offsets,
-               num_experts, topk_ids, expert_map, (int)global_E, (uint8_t*)codes, (uint8_t*)sf);
+    launch(stage_sf ? experts_quantize_scatter_kernel<__nv_bfloat16, true> : experts_quantize_scatter_kernel<__nv_bfloat16, false>,
+           reinterpret_cast<const __nv_bfloat16*>(x));
   else
-    launch_pdl(experts_quantize_scatter_kernel<__half>, dim3((unsigned)n_src), dim3(threads), 0, st, reinterpret_cast<const __half*>(x), K,
-               (int)topk, src2dst, global_scales, expert_offsets, blockscale_offsets, num_experts, topk_ids, expert_map, (int)global_E,
-               (uint8_t*)codes, (uint8_t*)sf);
-  return finish_launch(zero_sf ? 2 : 1);
+    launch(stage_sf ? experts_quantize_scatter_kernel<__half, true> : experts_quantize_scatter_kernel<__half, false>,
+           reinterpret_cast<const __half*>(x));
+  return finish_launch(stage_sf ? 1 : 2);
 }
 
 }  // namespace b200fp4
@@ -489,7 +500,7 @@ extern "C" int b200fp4_experts_quantize_scatter(const void* x, int in_dtype, int
                                                 const int32_t* expert_map, int64_t global_E, void* codes, void* sf,
                                                 void* stream) {
   return experts_quantize_scatter(x, in_dtype, n_src, K, topk, src2dst, global_scales, expert_offsets, blockscale_offsets, num_experts,
-                                  sf_rows_padded, topk_ids, expert_map, global_E, codes, sf, stream, true);
+                                  sf_rows_padded, topk_ids, expert_map, global_E, codes, sf, stream, false);
 }
 
 extern "C" int b200fp4_experts_quantize_gather(const void* x, int in_dtype, int64_t M, int64_t K, const float* global_scales,

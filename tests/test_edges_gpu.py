@@ -141,3 +141,41 @@ def test_dense_gemm_tile_choice(M, N, K, dtype):
         return torch.from_numpy(oracle.dequantize(to_np(codes), lin, float(gs[0]))).cuda().double()
     ref = (deq(xc, xs, gx, M) @ deq(wc, ws, gw, N).t()).float()
     assert ((out.float() - ref).abs().max() / ref.abs().max()).item() < 5e-3
+
+
+@pytest.mark.parametrize("M,E,topk,H,I,dtype", [
+    (1, 4, 1, 64, 128, torch.bfloat16),          # one row, less than one 256-wide stage of k
+    (37, 4, 3, 320, 128, torch.float16),         # a tail stage of one k-block
+    (200, 2, 2, 704, 256, torch.bfloat16),       # tail of three k-blocks, several row tiles per expert
+    (65, 8, 5, 1024, 384, torch.bfloat16),       # a batch of four slots and one more
+    (33, 16, 16, 4160, 128, torch.float16),      # a row longer than a block of threads takes at once
+])
+def test_prefill_layer_equals_its_steps(M, E, topk, H, I, dtype):
+    from dgx_vllm_b200 import grouped_moe as gm
+    from dgx_vllm_b200.ops import scaled_fp4_quant
+    g = torch.Generator(device="cuda").manual_seed(M + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    hidden = rnd(M, H).to(dtype)
+    tw, ids = torch.softmax(rnd(M, E), -1).topk(topk, -1)
+    tw, ids = tw.contiguous(), ids.int().contiguous()
+
+    def weights(N, K):
+        gs = torch.full((1,), 6.0 * 448.0 / 0.13, device="cuda")
+        c, s = zip(*[scaled_fp4_quant((0.02 * rnd(N, K)).to(dtype), gs, True) for _ in range(E)])
+        return torch.stack(c), torch.stack([v.view(torch.uint8) for v in s]).view(E, -1), gs.expand(E).contiguous()
+
+    w13, w2 = weights(2 * I, H), weights(H, I)
+    a1, a2 = 400.0 + 50.0 * torch.arange(E, device="cuda").float(), torch.full((E,), 220.0, device="cuda")
+    al1, al2 = gm.nvfp4_moe_alphas(w13[2], w2[2], a1, a2)
+    out = gm.nvfp4_moe_prefill(hidden, tw, ids, *w13, *w2, a1, a2, alphas=(al1, al2))
+    P = M * topk
+    eo, a_map, c_map = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (E + 1, P, P))
+    bso = gm.get_cutlass_moe_mm_data(ids, eo, None, None, a_map, c_map, E, I, H, pair_indices=True)
+    xq, xsf = gm.scatter_scaled_fp4_experts_quant(hidden, c_map, topk, a1, eo, bso, ids, None)
+    hq, hsf = gm.cutlass_fp4_moe_mm_silu_and_mul_quant(xq, w13[0], xsf, w13[1], al1, eo, bso, a2, dtype)
+    c2 = torch.empty((P, H), dtype=dtype, device="cuda")
+    gm.cutlass_fp4_moe_mm(c2, hq, w2[0], hsf, w2[1], al2, None, eo, bso)
+    assert torch.equal(out, gm.moe_unpermute_reduce(c2, c_map, tw))
+    rows = c2.float()[c_map.long()].view(M, topk, H)
+    ref = (rows * tw[..., None]).sum(1)
+    assert torch.allclose(out.float(), ref, rtol=1e-2, atol=1e-3 * float(ref.abs().max()))
