@@ -231,16 +231,23 @@ struct Cfg {
   static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 };
 
-// Staging: the dense wide-tile kernel hands [32 rows x 64 columns] boxes of 8 warps to the copy engine, the grouped kernel
-// transposes [32 rows x 32 columns] of 16 warps.
+// Staging: the dense wide-tile kernel hands [32 rows x 64 columns] boxes of 8 warps to the copy engine.
 // kSplit > 1: partial sums from the other CTAs of the cluster, 128 rows x 128 / kSplit columns fp32 each.
 template <int BN, bool kGrouped, bool kSiluQuant, int kSplit = 1>
 constexpr int out_stage_bytes() {
-  return kSplit > 1 ? (kSplit - 1) * (4 / kSplit) * 16384 : (kSiluQuant ? 0 : (kGrouped ? 16 * 2048 : (BN == 256 ? 8 * 4096 : 0)));
+  return kSplit > 1 ? (kSplit - 1) * (4 / kSplit) * 16384 : (BN == 256 && !kGrouped ? 8 * 4096 : 0);
 }
 
-// kSplit > 1 (dense, 128-wide tiles, fewer tiles than SMs): the kSplit CTAs of a cluster each take a part of K of one tile; each
-// then finishes 128 / kSplit of its columns, with the other CTAs' sums of them arriving through distributed shared memory.
+// One step of a transpose across lanes: a lane with its bit clear gives b for its partner's a, one with the bit set a for b
+__device__ __forceinline__ void transpose4(uint32_t* a, uint32_t* b, bool bit, int mask) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, bit ? a[i] : b[i], mask);
+    if (bit) a[i] = got;
+    else b[i] = got;
+  }
+}
+
 // The KB scale tiles of a stage to tensor memory, `step` columns apart: all loads before the first store (one after the other
 // they were on the path of short main loops: grouped down projection of 64 x 1280 rows, K = 1024, 96 us, 85 so)
 template <int KB>
@@ -252,6 +259,8 @@ __device__ __forceinline__ void copy_sf(uint32_t tmem, uint32_t step, const unsi
   for (int kb = 0; kb < KB; ++kb) tcgen05_st_32x32_x4(tmem + kb * step, w[kb]);
 }
 
+// kSplit > 1 (dense, 128-wide tiles, fewer tiles than SMs): the kSplit CTAs of a cluster each take a part of K of one tile; each
+// then finishes 128 / kSplit of its columns, with the other CTAs' sums of them arriving through distributed shared memory.
 // kStageSf: the scales of A come as [128-row tile][256 of k][row][16 bytes]
 template <int BN, int KB, bool kGrouped, bool kSiluQuant = false, int kSplit = 1, bool kStageSf = false>
 __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
@@ -632,27 +641,24 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
       }
       if constexpr (kGrouped) if ((p.N % 8) == 0) {
         // Rows of the next expert must not be touched, so the copy engine's boxes do not fit; a lane that stored its own row
-        // directly would write 32 rows per instruction, 32 bytes each.  Instead the warp turns [32 rows x 32 columns] around
-        // in a private buffer (16-byte chunk c of row r at c ^ (r / 2) % 4: no bank conflicts either way) and stores four
-        // neighbouring lanes to a row.
-        const uint32_t stg = smem_u32(out_stage) + (uint32_t)(grp * 4 + quarter) * 2048u;
-        const int row0 = ti.a_row0 + quarter * 32;
+        // directly would write 32 rows per instruction, 32 bytes each.  Instead four neighbouring lanes turn their rows' 16-byte
+        // chunks around by shuffles, and each stores its chunk of all four.  (Turned around in shared memory, the 32 KB of
+        // buffers cost the fourth stage of the ring: 81,920 rows x 2048 x 512 138 us, 132 so; 8192 rows x 1024 x 1024, 64
+        // experts, 81 us, 73 so.  The tile in two halves of 128 columns, one drained while the other is computed: 163.)
+        const int row0 = ti.a_row0 + quarter * 32 + (lane & ~3);
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            sts128(stg + (uint32_t)lane * 64u + (uint32_t)((i ^ ((lane >> 1) & 3)) << 4), packed[c * 16 + 4 * i],
-                   packed[c * 16 + 4 * i + 1], packed[c * 16 + 4 * i + 2], packed[c * 16 + 4 * i + 3]);
-          __syncwarp();
+          uint32_t* w = packed + c * 16;
+          transpose4(w, w + 4, lane & 1, 1);
+          transpose4(w + 8, w + 12, lane & 1, 1);
+          transpose4(w, w + 8, lane & 2, 2);
+          transpose4(w + 4, w + 12, lane & 2, 2);
           const int col = ti.n0 + (c_first + c) * 32 + (lane & 3) * 8;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int r = i * 8 + (lane >> 2);
-            const uint4 v = lds128(stg + (uint32_t)r * 64u + (uint32_t)(((lane & 3) ^ ((r >> 1) & 3)) << 4));
-            if (row0 + r < ti.row_end && col < p.N)
-              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)(row0 + r) * p.N + col) = v;
-          }
+          for (int i = 0; i < 4; ++i)
+            if (row0 + i < ti.row_end && col < p.N)
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)(row0 + i) * p.N + col) =
+                  make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
         }
         continue;
       }
