@@ -186,7 +186,7 @@ B200FP4_API int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, co
  * ------------------------------------------------------------------------------------------- */
 #define B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT 1
 #define B200FP4_SPARSE_META_ORDERED 2
-#define B200FP4_MOE_SEPARATE_LAUNCHES 4   /* fused layer: one launch per projection even where one cooperative launch is possible */
+#define B200FP4_MOE_SEPARATE_LAUNCHES 4   /* fused layer: one launch per projection even where one launch for both is possible */
 #define B200FP4_MOE_HOST_DIRECT_OUT 8     /* b200fp4_fused_sparse_moe_host_async only, see there */
 
 B200FP4_API size_t b200fp4_sparse_workspace_bytes(int64_t P, int64_t K, int64_t E);
@@ -255,9 +255,9 @@ B200FP4_API int b200fp4_convert_to_sparse_2of4(const uint8_t* codes, const uint8
  *   workspace   b200fp4_fused_moe_workspace_bytes(M, topk, H, I, E) bytes
  * flags: B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT (the reference's apply_router_weight_on_input) sums the
  * expert outputs unweighted, exactly as the reference kernel does (sparse_fp4_v7.cu:592-594);
- * B200FP4_SPARSE_META_ORDERED as described above, for both weight sets.  With ordered metadata, the
- * usual shapes and up to 256 (token, expert) pairs both projections run in ONE cooperative launch
- * (blocks that finish their share of gate_up move on to the down projection of passes that are
+ * B200FP4_SPARSE_META_ORDERED as described above, for both weight sets.  With ordered metadata and the
+ * usual shapes both projections run in ONE launch
+ * (warps that finish their share of gate_up move on to the down projection of passes that are
  * already complete); B200FP4_MOE_SEPARATE_LAUNCHES keeps one launch per projection.
  *
  * Status word.  In the one-launch form a down-projection item waits (bounded, ~1 s of SM clocks by default)
