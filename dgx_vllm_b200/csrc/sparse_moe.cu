@@ -19,6 +19,7 @@
 //   * the K reduction is done in-kernel (warp shuffles, then one shared-memory pass), so there is
 //     no partial-sum tensor and no separate reduction kernel; SiLU(gate)*up is fused into the
 //     gate_up epilogue; the router-weighted sum is a small deterministic kernel (no atomics).
+#include <cmath>
 #include <type_traits>
 
 #include <mutex>
@@ -1710,8 +1711,12 @@ int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int*
 //   16 warps, one per item    35.6  49.5  67.2  102   120  134   95.1  125   133   195  306    46.7  66.3  86.1  159  247
 //   before                    43.2  65.6  68.4  97.2  125  142   95.9  119   133   189  320    54.5  66.4  95.2  144  267
 // Under three items an SM four warps share one; while single-pass items last about a round of the warps, eight warps with the
-// deepest rings stream best; in between two warps an item level the last round; sixteen warps need enough items that their
-// last round is short beside the rest, twice as many where an item is twice as long.
+// deepest rings stream best; in between two warps an item level the last round.  Sixteen warps need as many items as just fill
+// one round, 12 to 16 an SM of no more than K = 2048, or enough that the last round is short beside the rest: more than 22 an SM,
+// twice that where an item of either projection is twice as long (us with two warps per item / sixteen warps: 512 experts,
+// H=2048, I=512, M=28 62.9 / 64.8, M=32 70.5 / 68.6, M=40 80.2 / 79.3, M=48 84.1 / 93.6, M=80 112 / 112, M=96 124 / 120, M=112
+// 129 / 125; 256 experts, H=2048, I=1024, M=14 66.6 / 69.1, M=16 76.6 / 73.4, M=20 84.9 / 81.1, M=24 93.5 / 107, M=64 130 / 134,
+// M=96 141 / 145; 512 experts, H=1024, I=512, M=36 49.4 / 45.8).
 template <int kNA, int kNB>
 int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int64_t local_pairs, int64_t E, cudaStream_t st) {
   const int64_t passes = (local_pairs < E ? local_pairs : E) * ((local_pairs + 8 * E - 1) / (8 * E));
@@ -1735,7 +1740,11 @@ int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* d
     if (gb.K % 256 == 0) return launch_fused_ws_t<kNA, kNB, 8, 8, 1>(ga, gb, counter, done, need + more, st);
     if (kAny) return launch_fused_ws_t<0, 0, 8, 8, 1, 4>(ga, gb, counter, done, need + more, st);
   }
-  if (items * 2048 <= 24 * sms * (ga.K > 2048 ? ga.K : 2048)) {
+  // items if the pairs fall on the experts at random
+  const double hit = (double)E * (1.0 - std::exp(-(double)local_pairs / (double)E)) * (double)(ga.n_slabs * ((local_pairs + 8 * E - 1) / (8 * E)));
+  const bool one_round = ga.K <= 2048 && local_pairs <= 4 * E && hit > 12.0 * sms && hit <= 16.0 * sms;
+  const double longer = (ga.K > 2048 ? ga.K / 2048.0 : 1.0) * (gb.K > 512 ? 2.0 : 1.0);
+  if (!one_round && hit <= 22.0 * longer * sms) {
     const int t = turns(2), n = 2 * need + more;
     if (t == 4) return launch_fused_ws_t<kNA, kNB, 4, 12, 2>(ga, gb, counter, done, n, st);
     if (kAny && t == 3) return launch_fused_ws_t<0, 0, 4, 12, 2, 3>(ga, gb, counter, done, n, st);

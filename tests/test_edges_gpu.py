@@ -85,6 +85,7 @@ def test_quantizer_tile_edges(M, K, swizzled, offset):
     (16, 256, 256, 33, 8),        # 264 pairs
     (128, 1024, 768, 25, 10),     # eight warps, one per item
     (512, 512, 512, 64, 8),       # 12 warps, two per item
+    (256, 256, 512, 60, 10),      # 16 warps, items of about one round
     (8, 512, 384, 3, 4),          # four warps per item, down slices of three steps
     (8, 1024, 256, 3, 4),         # ... of two
     (128, 512, 384, 40, 4),       # eight warps, down turns of four
