@@ -45,7 +45,7 @@ SIGNATURES = {
     "b200fp4_moe_unpermute_reduce": (_i32, [_vp, _i32, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
     "b200fp4_moe_prefill_workspace_bytes": (_sz, [_i64] * 5),
     "b200fp4_moe_prefill": (_i32, [_vp, _i32, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
-                                   _i64, _i64, _i64, _i64, _i64, _vp, _sz, _vp]),
+                                   _i64, _i64, _i64, _i64, _i64, _vp, _sz, _vp, _vp]),
     "b200fp4_sparse_workspace_bytes": (_sz, [_i64, _i64, _i64]),
     "b200fp4_sparse_gemv": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp]),
     "b200fp4_sparse_gemv_static": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i64, _i64, _i64, _i64, _i64, _vp]),

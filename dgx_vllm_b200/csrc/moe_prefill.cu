@@ -431,7 +431,7 @@ extern "C" int b200fp4_moe_prefill(const void* hidden, int dtype, const float* t
                                    const int32_t* expert_map, int64_t global_E, const void* w13_codes, const void* w13_sf,
                                    const float* alpha1, const void* w2_codes, const void* w2_sf, const float* alpha2,
                                    const float* a1_gs, const float* a2_gs, void* out, int64_t M, int64_t topk, int64_t H, int64_t I,
-                                   int64_t E, void* workspace, size_t workspace_bytes, void* stream) {
+                                   int64_t E, void* workspace, size_t workspace_bytes, void* gemm_workspace, void* stream) {
   if (M < 0 || topk <= 0 || topk > 32 || H <= 0 || H % 64 != 0 || I <= 0 || I % 128 != 0 || E <= 0) return B200FP4_STATUS_INVALID_VALUE;
   if (M == 0) return B200FP4_STATUS_SUCCESS;
   const PrefillLayout l = prefill_layout(M, topk, H, I, E);
@@ -442,12 +442,14 @@ extern "C" int b200fp4_moe_prefill(const void* hidden, int dtype, const float* t
   int32_t* dst2src = reinterpret_cast<int32_t*>(ws + l.dst2src);
   int32_t* src2dst = reinterpret_cast<int32_t*>(ws + l.src2dst);
   const size_t gemm_bytes = b200fp4_grouped_gemm_workspace_bytes(l.P, E);
+  unsigned char* gemm_ws = gemm_workspace ? static_cast<unsigned char*>(gemm_workspace) : ws + l.gemm;
+  if (!aligned(gemm_ws, 16)) return B200FP4_STATUS_ALLOC_FAILED;
   cudaStream_t st = (cudaStream_t)stream;
   int rc = B200FP4_STATUS_SUCCESS;
   const bool one_launch = l.P <= kRouteMaxPairs && E <= kGroupMaxExperts;        // metadata and tile list together
   if (one_launch) {
     if (!topk_ids || (expert_map && global_E <= 0)) return B200FP4_STATUS_INVALID_VALUE;
-    launch_moe_route(topk_ids, (int)l.P, expert_map, (int)global_E, (int)E, eo, bso, nullptr, src2dst, ws + l.gemm, st);
+    launch_moe_route(topk_ids, (int)l.P, expert_map, (int)global_E, (int)E, eo, bso, nullptr, src2dst, gemm_ws, st);
     rc = finish_launch(1);
   } else {
     rc = b200fp4_moe_permute(topk_ids, expert_map, global_E, M, topk, E, eo, bso, dst2src, src2dst, stream);
@@ -456,10 +458,10 @@ extern "C" int b200fp4_moe_prefill(const void* hidden, int dtype, const float* t
     rc = experts_quantize_scatter(hidden, dtype, M, H, topk, src2dst, a1_gs, eo, bso, (int32_t)E, l.sf_rows, topk_ids, expert_map, global_E,
                                   ws + l.xq, ws + l.xsf, stream, true);
   if (rc == B200FP4_STATUS_SUCCESS)
-    rc = grouped_gemm(ws + l.xq, w13_codes, ws + l.xsf, w13_sf, alpha1, eo, bso, ws + l.hq, dtype, l.P, 2 * I, H, E, 0, ws + l.gemm,
+    rc = grouped_gemm(ws + l.xq, w13_codes, ws + l.xsf, w13_sf, alpha1, eo, bso, ws + l.hq, dtype, l.P, 2 * I, H, E, 0, gemm_ws,
                       gemm_bytes, stream, ws + l.hsf, a2_gs, one_launch, true);
   if (rc == B200FP4_STATUS_SUCCESS)
-    rc = grouped_gemm(ws + l.hq, w2_codes, ws + l.hsf, w2_sf, alpha2, eo, bso, ws + l.c2, dtype, l.P, H, I, E, 0, ws + l.gemm, gemm_bytes,
+    rc = grouped_gemm(ws + l.hq, w2_codes, ws + l.hsf, w2_sf, alpha2, eo, bso, ws + l.c2, dtype, l.P, H, I, E, 0, gemm_ws, gemm_bytes,
                       stream, nullptr, nullptr, true, false);
   if (rc == B200FP4_STATUS_SUCCESS)
     rc = b200fp4_moe_unpermute_reduce(ws + l.c2, dtype, src2dst, topk_weights, M, topk, H, out, stream);

@@ -405,10 +405,12 @@ B200_FN(py_moe_prefill) {
     at::Tensor out = empty({M, H}, x.scalar_type(), dev);
     cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
     const at::Tensor scratch = empty({(int64_t)b200fp4_moe_prefill_workspace_bytes(M, topk, H, I, E)}, at::kByte, dev);
+    // the GEMMs' tile list and status word lie in the stream's workspace, where the status is read
+    const at::Tensor& gemm_ws = workspace(dev, st, b200fp4_grouped_gemm_workspace_bytes(P, E));
     check(b200fp4_moe_prefill(ptr(x), dtype_code(x.scalar_type()), ptr<float>(tw), ptr<int32_t>(ids),
                               emap.defined() ? ptr<int32_t>(emap) : nullptr, emap.defined() ? emap.numel() : 0, ptr(w13), ptr(w13_sf),
                               ptr<float>(al1), ptr(w2), ptr(w2_sf), ptr<float>(al2), ptr<float>(a1), ptr<float>(a2), ptr(out), M, topk, H,
-                              I, E, ptr(scratch), scratch.nbytes(), st),
+                              I, E, ptr(scratch), scratch.nbytes(), ptr(gemm_ws), st),
           "nvfp4_moe_prefill");
     return wrap(std::move(out));
   });

@@ -392,14 +392,16 @@ B200FP4_API int b200fp4_moe_unpermute_reduce(const void* expert_out, int dtype, 
  * grouped GEMMs and moe_unpermute_reduce above, same results (vllm/model_executor/layers/fused_moe/experts/cutlass_moe.py:567-663).
  *   hidden, out [M, H] of `dtype` (BF16 or F16); w13_codes [E, 2I, H/2] gate rows first, w2_codes [E, H, I/2], w*_sf their
  *   swizzled scales per expert; alpha1 / alpha2 [E] = 1 / (activation scale * weight scale) of the two GEMMs;
- *   a1_gs / a2_gs [E] activation global scales.  H a multiple of 64, I of 128, topk <= 32. */
+ *   a1_gs / a2_gs [E] activation global scales.  H a multiple of 64, I of 128, topk <= 32.
+ *   gemm_workspace  b200fp4_grouped_gemm_workspace_bytes(M * topk, E) bytes whose first int is the GEMMs' status word, or NULL
+ *                   to keep that part inside `workspace` */
 B200FP4_API size_t b200fp4_moe_prefill_workspace_bytes(int64_t M, int64_t topk, int64_t H, int64_t I, int64_t E);
 B200FP4_API int b200fp4_moe_prefill(const void* hidden, int dtype, const float* topk_weights, const int32_t* topk_ids,
                                     const int32_t* expert_map, int64_t global_E, const void* w13_codes,
                                     const void* w13_sf, const float* alpha1, const void* w2_codes, const void* w2_sf,
                                     const float* alpha2, const float* a1_gs, const float* a2_gs, void* out, int64_t M,
                                     int64_t topk, int64_t H, int64_t I, int64_t E, void* workspace,
-                                    size_t workspace_bytes, void* stream);
+                                    size_t workspace_bytes, void* gemm_workspace, void* stream);
 
 /* MoE router for decode: gate projection, softmax over the experts, top-k, renormalisation -- the step in front of
  * the fused layer.  The reference leaves it to vLLM's torch code (its benches restate it:

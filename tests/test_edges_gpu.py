@@ -153,7 +153,7 @@ def test_dense_gemm_tile_choice(M, N, K, dtype):
 ])
 def test_prefill_layer_equals_its_steps(M, E, topk, H, I, dtype):
     from dgx_vllm_b200 import grouped_moe as gm
-    from dgx_vllm_b200.ops import scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status, scaled_fp4_quant
     g = torch.Generator(device="cuda").manual_seed(M + H)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
     hidden = rnd(M, H).to(dtype)
@@ -169,6 +169,7 @@ def test_prefill_layer_equals_its_steps(M, E, topk, H, I, dtype):
     a1, a2 = 400.0 + 50.0 * torch.arange(E, device="cuda").float(), torch.full((E,), 220.0, device="cuda")
     al1, al2 = gm.nvfp4_moe_alphas(w13[2], w2[2], a1, a2)
     out = gm.nvfp4_moe_prefill(hidden, tw, ids, *w13, *w2, a1, a2, alphas=(al1, al2))
+    assert last_gemm_status() == 0
     P = M * topk
     eo, a_map, c_map = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (E + 1, P, P))
     bso = gm.get_cutlass_moe_mm_data(ids, eo, None, None, a_map, c_map, E, I, H, pair_indices=True)
