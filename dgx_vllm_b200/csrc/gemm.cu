@@ -1064,10 +1064,10 @@ extern "C" size_t b200fp4_grouped_gemm_workspace_bytes(int64_t rows_capacity, in
 
 namespace b200fp4 {
 
-int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
-                 const int32_t* expert_offsets, const int32_t* sf_offsets, void* out, int out_dtype, int64_t rows_capacity, int64_t N,
-                 int64_t K, int64_t E, int tile_n, void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs,
-                 bool tiles_ready, bool stage_sf) {
+int grouped_gemm_check(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
+                       const int32_t* expert_offsets, const int32_t* sf_offsets, const void* out, int out_dtype, int64_t rows_capacity,
+                       int64_t N, int64_t K, int64_t E, int tile_n, const void* workspace, size_t workspace_bytes, const void* q_sf,
+                       const float* q_gs, bool stage_sf) {
   const bool fused = q_sf != nullptr;
   if (stage_sf && !fused) return B200FP4_STATUS_INVALID_VALUE;
   if (fused && (!q_gs || (N % 256) != 0 || !aligned(out, 32) || !aligned(q_sf, 4))) return B200FP4_STATUS_INVALID_VALUE;
@@ -1086,7 +1086,18 @@ int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, con
   if (fused && tile_n == 128) return B200FP4_STATUS_INVALID_VALUE;
   if (!workspace || !aligned(workspace, 16) || workspace_bytes < b200fp4_grouped_gemm_workspace_bytes(rows_capacity, E))
     return B200FP4_STATUS_ALLOC_FAILED;
+  return B200FP4_STATUS_SUCCESS;
+}
+
+int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
+                 const int32_t* expert_offsets, const int32_t* sf_offsets, void* out, int out_dtype, int64_t rows_capacity, int64_t N,
+                 int64_t K, int64_t E, int tile_n, void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs,
+                 bool tiles_ready, bool stage_sf) {
+  const int refused = grouped_gemm_check(a_codes, b_codes, a_sf, b_sf, alphas, expert_offsets, sf_offsets, out, out_dtype, rows_capacity,
+                                         N, K, E, tile_n, workspace, workspace_bytes, q_sf, q_gs, stage_sf);
+  if (refused != B200FP4_STATUS_SUCCESS || rows_capacity == 0) return refused;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
+  const bool fused = q_sf != nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   const int max_tiles = grouped_max_tiles(rows_capacity, E);
   GemmParams p;

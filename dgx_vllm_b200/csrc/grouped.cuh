@@ -29,6 +29,11 @@ int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t
                              const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
                              int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
                              int64_t global_E, void* codes, void* sf, void* stream, bool stage_sf);
+// What it refuses, without queueing anything.
+int experts_quantize_scatter_check(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
+                                   const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                                   int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
+                                   int64_t global_E, const void* codes, const void* sf, bool stage_sf);
 
 // The grouped GEMM; q_sf / q_gs non-null: the gate_up projection with SiLU(gate)*up and the NVFP4 quantization of the result
 // in the epilogue (out = packed codes [rows_capacity, N/4]).  tiles_ready: the workspace already holds the tile list.  stage_sf:
@@ -37,5 +42,10 @@ int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, con
                  const int32_t* expert_offsets, const int32_t* sf_offsets, void* out, int out_dtype, int64_t rows_capacity, int64_t N,
                  int64_t K, int64_t E, int tile_n, void* workspace, size_t workspace_bytes, void* stream, void* q_sf, const float* q_gs,
                  bool tiles_ready, bool stage_sf);
+// What it refuses of its arguments, without queueing anything (the device is not looked at).
+int grouped_gemm_check(const void* a_codes, const void* b_codes, const void* a_sf, const void* b_sf, const float* alphas,
+                       const int32_t* expert_offsets, const int32_t* sf_offsets, const void* out, int out_dtype, int64_t rows_capacity,
+                       int64_t N, int64_t K, int64_t E, int tile_n, const void* workspace, size_t workspace_bytes, const void* q_sf,
+                       const float* q_gs, bool stage_sf);
 
 }  // namespace b200fp4

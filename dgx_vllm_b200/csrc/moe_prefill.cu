@@ -354,6 +354,23 @@ PrefillLayout prefill_layout(int64_t M, int64_t topk, int64_t H, int64_t I, int6
   return l;
 }
 
+int permute_check(const int32_t* topk_ids, const int32_t* expert_map, int64_t global_E, int64_t M, int64_t topk, int64_t E,
+                  const int32_t* expert_offsets, const int32_t* blockscale_offsets, const int32_t* dst2src, const int32_t* src2dst) {
+  if (M < 0 || topk <= 0 || E <= 0 || E > kGroupMaxExperts || M * topk > (1 << 24)) return B200FP4_STATUS_INVALID_VALUE;
+  if (!expert_offsets || !blockscale_offsets) return B200FP4_STATUS_INVALID_VALUE;
+  if (M > 0 && (!topk_ids || !dst2src || !src2dst)) return B200FP4_STATUS_INVALID_VALUE;
+  if (expert_map && global_E <= 0) return B200FP4_STATUS_INVALID_VALUE;
+  return B200FP4_STATUS_SUCCESS;
+}
+
+int unpermute_check(const void* expert_out, int dtype, const int32_t* src2dst, const float* topk_weights, int64_t M, int64_t topk,
+                    int64_t H, const void* out) {
+  if (M < 0 || topk <= 0 || H <= 0 || (H % 2) != 0 || M > 65535) return B200FP4_STATUS_INVALID_VALUE;
+  if (dtype != B200FP4_DTYPE_BF16 && dtype != B200FP4_DTYPE_F16) return B200FP4_STATUS_NOT_SUPPORTED;
+  if (M > 0 && (!expert_out || !src2dst || !topk_weights || !out)) return B200FP4_STATUS_INVALID_VALUE;
+  return B200FP4_STATUS_SUCCESS;
+}
+
 }  // namespace
 
 void launch_moe_route(const int32_t* topk_ids, int P, const int32_t* expert_map, int global_E, int E, int32_t* expert_offsets,
@@ -370,10 +387,8 @@ using namespace b200fp4;
 extern "C" int b200fp4_moe_permute(const int32_t* topk_ids, const int32_t* expert_map, int64_t global_E, int64_t M,
                                    int64_t topk, int64_t E, int32_t* expert_offsets, int32_t* blockscale_offsets,
                                    int32_t* dst2src, int32_t* src2dst, void* stream) {
-  if (M < 0 || topk <= 0 || E <= 0 || E > kGroupMaxExperts || M * topk > (1 << 24)) return B200FP4_STATUS_INVALID_VALUE;
-  if (!expert_offsets || !blockscale_offsets) return B200FP4_STATUS_INVALID_VALUE;
-  if (M > 0 && (!topk_ids || !dst2src || !src2dst)) return B200FP4_STATUS_INVALID_VALUE;
-  if (expert_map && global_E <= 0) return B200FP4_STATUS_INVALID_VALUE;
+  const int refused = permute_check(topk_ids, expert_map, global_E, M, topk, E, expert_offsets, blockscale_offsets, dst2src, src2dst);
+  if (refused != B200FP4_STATUS_SUCCESS) return refused;
   const int P = (int)(M * topk);
   cudaStream_t st = (cudaStream_t)stream;
   if (P <= kRouteMaxPairs) {
@@ -394,10 +409,8 @@ extern "C" int b200fp4_moe_permute(const int32_t* topk_ids, const int32_t* exper
 extern "C" int b200fp4_moe_unpermute_reduce(const void* expert_out, int dtype, const int32_t* src2dst,
                                             const float* topk_weights, int64_t M, int64_t topk, int64_t H, void* out,
                                             void* stream) {
-  if (M < 0 || topk <= 0 || H <= 0 || (H % 2) != 0 || M > 65535) return B200FP4_STATUS_INVALID_VALUE;
-  if (dtype != B200FP4_DTYPE_BF16 && dtype != B200FP4_DTYPE_F16) return B200FP4_STATUS_NOT_SUPPORTED;
-  if (M == 0) return B200FP4_STATUS_SUCCESS;
-  if (!expert_out || !src2dst || !topk_weights || !out) return B200FP4_STATUS_INVALID_VALUE;
+  const int refused = unpermute_check(expert_out, dtype, src2dst, topk_weights, M, topk, H, out);
+  if (refused != B200FP4_STATUS_SUCCESS || M == 0) return refused;
   if ((H % 8) == 0 && aligned(expert_out, 16) && aligned(out, 16)) {
     const dim3 grid8((unsigned)((H / 8 + kUnpermuteThreads - 1) / kUnpermuteThreads), (unsigned)M);
     if (dtype == B200FP4_DTYPE_BF16)
@@ -444,11 +457,23 @@ extern "C" int b200fp4_moe_prefill(const void* hidden, int dtype, const float* t
   const size_t gemm_bytes = b200fp4_grouped_gemm_workspace_bytes(l.P, E);
   unsigned char* gemm_ws = gemm_workspace ? static_cast<unsigned char*>(gemm_workspace) : ws + l.gemm;
   if (!aligned(gemm_ws, 16)) return B200FP4_STATUS_ALLOC_FAILED;
+  // what any of the five steps would refuse, before the first of them is queued
+  int rc = permute_check(topk_ids, expert_map, global_E, M, topk, E, eo, bso, dst2src, src2dst);
+  if (rc == B200FP4_STATUS_SUCCESS)
+    rc = experts_quantize_scatter_check(hidden, dtype, M, H, topk, src2dst, a1_gs, eo, bso, (int32_t)E, l.sf_rows, topk_ids, expert_map,
+                                        global_E, ws + l.xq, ws + l.xsf, true);
+  if (rc == B200FP4_STATUS_SUCCESS)
+    rc = grouped_gemm_check(ws + l.xq, w13_codes, ws + l.xsf, w13_sf, alpha1, eo, bso, ws + l.hq, dtype, l.P, 2 * I, H, E, 0, gemm_ws,
+                            gemm_bytes, ws + l.hsf, a2_gs, true);
+  if (rc == B200FP4_STATUS_SUCCESS)
+    rc = grouped_gemm_check(ws + l.hq, w2_codes, ws + l.hsf, w2_sf, alpha2, eo, bso, ws + l.c2, dtype, l.P, H, I, E, 0, gemm_ws, gemm_bytes,
+                            nullptr, nullptr, false);
+  if (rc == B200FP4_STATUS_SUCCESS) rc = unpermute_check(ws + l.c2, dtype, src2dst, topk_weights, M, topk, H, out);
+  if (rc != B200FP4_STATUS_SUCCESS) return rc;
+  if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = B200FP4_STATUS_SUCCESS;
-  const bool one_launch = l.P <= kRouteMaxPairs && E <= kGroupMaxExperts;        // metadata and tile list together
+  const bool one_launch = l.P <= kRouteMaxPairs;                   // metadata and tile list together
   if (one_launch) {
-    if (!topk_ids || (expert_map && global_E <= 0)) return B200FP4_STATUS_INVALID_VALUE;
     launch_moe_route(topk_ids, (int)l.P, expert_map, (int)global_E, (int)E, eo, bso, nullptr, src2dst, gemm_ws, st);
     rc = finish_launch(1);
   } else {

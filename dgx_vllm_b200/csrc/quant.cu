@@ -456,10 +456,10 @@ extern "C" int b200fp4_experts_quantize(const void* x, int in_dtype, int64_t M, 
 
 namespace b200fp4 {
 
-int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
-                             const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
-                             int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
-                             int64_t global_E, void* codes, void* sf, void* stream, bool stage_sf) {
+int experts_quantize_scatter_check(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
+                                   const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                                   int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
+                                   int64_t global_E, const void* codes, const void* sf, bool stage_sf) {
   if (expert_map && (!topk_ids || global_E <= 0)) return B200FP4_STATUS_INVALID_VALUE;
   if (n_src < 0 || K <= 0 || (K % 16) != 0 || topk <= 0 || num_experts <= 0 || sf_rows_padded < 0 ||
       (sf_rows_padded % 128) != 0)
@@ -469,9 +469,20 @@ int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t
   if (!global_scales || !expert_offsets || !blockscale_offsets || !sf) return B200FP4_STATUS_INVALID_VALUE;
   if (n_src > 0 && (!x || !codes || !src2dst || !aligned(x, 16) || !aligned(codes, 8) || !aligned(sf, 4)))
     return B200FP4_STATUS_INVALID_VALUE;
+  if (stage_sf && ((K % 64) != 0 || !aligned(sf, 16))) return B200FP4_STATUS_INVALID_VALUE;
+  return B200FP4_STATUS_SUCCESS;
+}
+
+int experts_quantize_scatter(const void* x, int in_dtype, int64_t n_src, int64_t K, int64_t topk, const int32_t* src2dst,
+                             const float* global_scales, const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                             int32_t num_experts, int64_t sf_rows_padded, const int32_t* topk_ids, const int32_t* expert_map,
+                             int64_t global_E, void* codes, void* sf, void* stream, bool stage_sf) {
+  const int refused = experts_quantize_scatter_check(x, in_dtype, n_src, K, topk, src2dst, global_scales, expert_offsets,
+                                                     blockscale_offsets, num_experts, sf_rows_padded, topk_ids, expert_map, global_E,
+                                                     codes, sf, stage_sf);
+  if (refused != B200FP4_STATUS_SUCCESS) return refused;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t KB = K / 16;
-  if (stage_sf && ((K % 64) != 0 || !aligned(sf, 16))) return B200FP4_STATUS_INVALID_VALUE;
   if (!stage_sf && cudaMemsetAsync(sf, 0, (size_t)(sf_rows_padded * (((KB + 3) / 4) * 4)), st) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;

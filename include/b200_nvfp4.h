@@ -10,7 +10,8 @@
  *   - Scalars that the caller keeps on the device (global scales, alpha) are passed as device
  *     pointers so a call sequence can be captured into a CUDA graph.
  *   - Work is enqueued on `stream`; a non-zero status means nothing was enqueued, except
- *     B200FP4_STATUS_EXECUTION_FAILED which reports a launch error from the CUDA runtime.
+ *     B200FP4_STATUS_EXECUTION_FAILED and B200FP4_STATUS_INTERNAL_ERROR, which report an error of the
+ *     CUDA runtime or driver (a launch, a tensor map) that may come after earlier steps of the call.
  *   - Packed E2M1 codes: element 2i in the low nibble, 2i+1 in the high nibble of byte i
  *     (patch_nvfp4_utils_sw_e2m1.py:48-63).  Block scales are E4M3 bytes, one per 16 elements
  *     along K.

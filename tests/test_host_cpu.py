@@ -41,6 +41,31 @@ def test_no_cpu_fallback():
                                         torch.ones(1), torch.zeros(1, dtype=torch.int32))
 
 
+def _refused_unqueued(call):
+    """The status of a call that has to be refused before anything of it is queued."""
+    from dgx_vllm_b200 import _lib
+    L = _lib.lib()
+    n0 = L.b200fp4_launch_count()
+    rc = call(L)
+    assert L.b200fp4_launch_count() == n0, "part of a refused call was queued"
+    return rc
+
+
+INVALID, NOT_SUPPORTED = 7, 15
+
+
+@pytest.mark.parametrize("bad", [
+    dict(M=65536), dict(out=0), dict(topk_weights=0), dict(w13_codes=0), dict(w2_codes=0), dict(alpha2=0), dict(a1_gs=0), dict(a2_gs=0),
+    dict(dtype=2), dict(hidden=0x1008), dict(w2_sf=0x1008), dict(E=4097), dict(I=1 << 20), dict(expert_map=0x1000, global_E=0),
+])
+def test_refused_prefill_layer_queues_nothing(bad):
+    p = 0x100000                                                  # an address no step ever reads
+    a = dict(hidden=p, dtype=1, topk_weights=p, topk_ids=p, expert_map=0, global_E=0, w13_codes=p, w13_sf=p, alpha1=p, w2_codes=p,
+             w2_sf=p, alpha2=p, a1_gs=p, a2_gs=p, out=p, M=2, topk=1, H=64, I=128, E=2)
+    a.update(bad)
+    assert _refused_unqueued(lambda L: L.b200fp4_moe_prefill(*a.values(), p, 1 << 62, 0, 0)) in (INVALID, NOT_SUPPORTED)
+
+
 def test_product_does_not_import_oracle():
     pkg = os.path.join(ROOT, "dgx_vllm_b200")
     for dirpath, _, files in os.walk(pkg):
