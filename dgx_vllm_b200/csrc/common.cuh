@@ -81,6 +81,13 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// What b200fp4_quantize (quant.cu) and b200fp4_gemm_nvfp4 (gemm.cu) refuse of their arguments, without queueing anything (the
+// device is not looked at): calls of several steps check all of them before the first.
+int quantize_check(const void* x, int in_dtype, int64_t M, int64_t K, int64_t ldx, const float* global_scale, const void* codes,
+                   const void* sf);
+int dense_gemm_check(const void* a_codes, const void* b_codes, const void* sfa, const void* sfb, const float* alpha, const void* out,
+                     int out_dtype, int64_t M, int64_t N, int64_t K, int tile_n, const void* workspace, size_t workspace_bytes);
+
 // ------------------------------------------------------------------------------------------ device
 
 // 16-byte read-only global load that does not allocate in L1 (streamed weights are read once).

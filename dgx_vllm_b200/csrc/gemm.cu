@@ -958,10 +958,9 @@ extern "C" size_t b200fp4_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) 
   return 256;
 }
 
-// early_b: see GemmParams
-static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa, const void* sfb, const float* alpha, void* out,
-                      int out_dtype, int64_t M, int64_t N, int64_t K, int tile_n, void* workspace, size_t workspace_bytes, void* stream,
-                      bool early_b) {
+int b200fp4::dense_gemm_check(const void* a_codes, const void* b_codes, const void* sfa, const void* sfb, const float* alpha,
+                              const void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int tile_n, const void* workspace,
+                              size_t workspace_bytes) {
   if (M < 0 || N <= 0 || K <= 0 || (K % 64) != 0) return B200FP4_STATUS_INVALID_VALUE;
   if (out_dtype != B200FP4_DTYPE_BF16 && out_dtype != B200FP4_DTYPE_F16 && out_dtype != B200FP4_DTYPE_F32)
     return B200FP4_STATUS_NOT_SUPPORTED;
@@ -974,6 +973,15 @@ static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa,
   if (tile_n != 0 && tile_n != 128 && tile_n != 256 && tile_n != 512) return B200FP4_STATUS_INVALID_VALUE;
   if (tile_n == 512 && out_dtype == B200FP4_DTYPE_F32) return B200FP4_STATUS_NOT_SUPPORTED;
   if (M > (1 << 24) || N > (1 << 24) || K > (1 << 24)) return B200FP4_STATUS_NOT_SUPPORTED;
+  return B200FP4_STATUS_SUCCESS;
+}
+
+// early_b: see GemmParams
+static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa, const void* sfb, const float* alpha, void* out,
+                      int out_dtype, int64_t M, int64_t N, int64_t K, int tile_n, void* workspace, size_t workspace_bytes, void* stream,
+                      bool early_b) {
+  const int refused = dense_gemm_check(a_codes, b_codes, sfa, sfb, alpha, out, out_dtype, M, N, K, tile_n, workspace, workspace_bytes);
+  if (refused != B200FP4_STATUS_SUCCESS || M == 0) return refused;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
   cudaStream_t st = (cudaStream_t)stream;
   GemmParams p;
@@ -1048,11 +1056,17 @@ extern "C" int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, con
   unsigned char* codes = static_cast<unsigned char*>(workspace);
   unsigned char* sf = codes + linear_part((size_t)M * (size_t)K / 2);
   unsigned char* gemm_ws = sf + linear_part(b200fp4_sf_swizzled_bytes(M, K / 16));
-  int rc = b200fp4_quantize(x, x_dtype, M, K, ldx, x_global_scale, codes, sf, 1, stream);
+  // what either step would refuse, before the first is queued
+  const size_t gemm_bytes = b200fp4_gemm_workspace_bytes(M, N, K);
+  int rc = quantize_check(x, x_dtype, M, K, ldx, x_global_scale, codes, sf);
+  if (rc == B200FP4_STATUS_SUCCESS)
+    rc = dense_gemm_check(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, gemm_bytes);
+  if (rc != B200FP4_STATUS_SUCCESS) return rc;
+  if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
+  rc = b200fp4_quantize(x, x_dtype, M, K, ldx, x_global_scale, codes, sf, 1, stream);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   // The quantizer lets the GEMM start only after it has waited for everything before it: whatever wrote the weights is done.
-  return gemm_nvfp4(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, b200fp4_gemm_workspace_bytes(M, N, K),
-                    stream, true);
+  return gemm_nvfp4(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, gemm_bytes, stream, true);
 }
 
 // ---------------------------------------------------------------------------------------- grouped entry points

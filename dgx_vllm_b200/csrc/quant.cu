@@ -400,16 +400,22 @@ extern "C" size_t b200fp4_sf_swizzled_bytes(int64_t rows, int64_t k_blocks) {
   return (size_t)(((rows + 127) / 128) * 128 * (((k_blocks + 3) / 4) * 4));
 }
 
-extern "C" int b200fp4_quantize(const void* x, int in_dtype, int64_t M, int64_t K, int64_t ldx,
-                                const float* global_scale, void* codes, void* sf, int sf_swizzled, void* stream) {
+int b200fp4::quantize_check(const void* x, int in_dtype, int64_t M, int64_t K, int64_t ldx, const float* global_scale, const void* codes,
+                            const void* sf) {
   if (M < 0 || K <= 0 || (K % 16) != 0 || ldx < K || (ldx % 8) != 0) return B200FP4_STATUS_INVALID_VALUE;
   if (in_dtype != B200FP4_DTYPE_F16 && in_dtype != B200FP4_DTYPE_BF16) return B200FP4_STATUS_NOT_SUPPORTED;
   if (M == 0) return B200FP4_STATUS_SUCCESS;
   if (!x || !global_scale || !codes || !sf) return B200FP4_STATUS_INVALID_VALUE;
   if (!aligned(x, 16) || !aligned(codes, 4)) return B200FP4_STATUS_INVALID_VALUE;
-  if (M > (int64_t)65535 * kTY * kRows) return B200FP4_STATUS_NOT_SUPPORTED;
+  if (M > (int64_t)65535 * kTY * kRows || K > ((int64_t)1 << 30)) return B200FP4_STATUS_NOT_SUPPORTED;
+  return B200FP4_STATUS_SUCCESS;
+}
+
+extern "C" int b200fp4_quantize(const void* x, int in_dtype, int64_t M, int64_t K, int64_t ldx,
+                                const float* global_scale, void* codes, void* sf, int sf_swizzled, void* stream) {
+  const int refused = quantize_check(x, in_dtype, M, K, ldx, global_scale, codes, sf);
+  if (refused != B200FP4_STATUS_SUCCESS || M == 0) return refused;
   cudaStream_t st = (cudaStream_t)stream;
-  if (K > ((int64_t)1 << 30)) return B200FP4_STATUS_NOT_SUPPORTED;
   if (in_dtype == B200FP4_DTYPE_BF16)
     launch_rows<__nv_bfloat16>(x, M, K / 16, ldx, global_scale, codes, sf, sf_swizzled != 0, st);
   else

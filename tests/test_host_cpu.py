@@ -66,6 +66,17 @@ def test_refused_prefill_layer_queues_nothing(bad):
     assert _refused_unqueued(lambda L: L.b200fp4_moe_prefill(*a.values(), p, 1 << 62, 0, 0)) in (INVALID, NOT_SUPPORTED)
 
 
+@pytest.mark.parametrize("bad", [
+    dict(tile_n=7), dict(w_codes=0x1008), dict(w_sf=0), dict(alpha=0), dict(out=0x1008), dict(out_dtype=3), dict(N=1 << 25),
+    dict(tile_n=512, out_dtype=2), dict(ldx=60), dict(x=0),
+])
+def test_refused_linear_queues_nothing(bad):
+    p = 0x100000
+    a = dict(x=p, x_dtype=1, ldx=64, x_global_scale=p, w_codes=p, w_sf=p, alpha=p, out=p, out_dtype=1, M=2, N=128, K=64, tile_n=0)
+    a.update(bad)
+    assert _refused_unqueued(lambda L: L.b200fp4_linear_nvfp4(*a.values(), p, 1 << 62, 0)) in (INVALID, NOT_SUPPORTED)
+
+
 def test_product_does_not_import_oracle():
     pkg = os.path.join(ROOT, "dgx_vllm_b200")
     for dirpath, _, files in os.walk(pkg):
