@@ -2057,14 +2057,24 @@ extern "C" size_t b200fp4_fused_moe_workspace_bytes(int64_t M, int64_t topk, int
          align_up((size_t)max_passes(P, E) * sizeof(int), 256);
 }
 
-// ld_h / ld_w / ld_ids: row strides (in elements) of hidden, topk_weights and topk_ids.
-static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const float* topk_weights, int64_t ld_w,
-                          const int32_t* topk_ids, int64_t ld_ids, const int32_t* expert_map, int64_t global_E,
-                          const uint8_t* w13_comp, const uint8_t* w13_meta, const uint8_t* w13_scale, const float* w13_g,
-                          int64_t G13, const uint8_t* w2_comp, const uint8_t* w2_meta, const uint8_t* w2_scale,
-                          const float* w2_g, int64_t G2, void* out, int out_dtype, int64_t M, int64_t topk, int64_t H,
-                          int64_t I, int64_t E, int flags, void* workspace, size_t workspace_bytes, void* stream,
-                          OutScatter sc = OutScatter{nullptr, 1, 0}) {
+// The two projections' weights as the kernels address them.
+static void fused_moe_weights(const uint8_t* w13_comp, const uint8_t* w13_meta, const uint8_t* w13_scale, const float* w13_g, int64_t G13,
+                              const uint8_t* w2_comp, const uint8_t* w2_meta, const uint8_t* w2_scale, const float* w2_g, int64_t G2,
+                              int64_t H, int64_t I, SparseWeights& w13, SparseWeights& w2) {
+  w13.comp = w13_comp; w13.meta = w13_meta; w13.scale = w13_scale; w13.g = w13_g;
+  w13.comp_e = (H / 4) * 2 * I; w13.comp_pair = 4 * I; w13.comp_odd = 2 * I;
+  w13.meta_e = (H / 8) * 2 * I; w13.meta_row = 2 * I; w13.scale_e = G13 * 2 * I; w13.scale_row = 2 * I;
+  w2.comp = w2_comp; w2.meta = w2_meta; w2.scale = w2_scale; w2.g = w2_g;
+  w2.comp_e = (I / 4) * H; w2.comp_pair = 2 * H; w2.comp_odd = H;
+  w2.meta_e = (I / 8) * H; w2.meta_row = H; w2.scale_e = G2 * H; w2.scale_row = H;
+}
+
+// What the fused layer refuses, without queueing anything.
+static int fused_moe_check(const void* hidden, int64_t ld_h, int h_dtype, const float* topk_weights, int64_t ld_w,
+                           const int32_t* topk_ids, int64_t ld_ids, const int32_t* expert_map, int64_t global_E,
+                           const SparseWeights& w13, int64_t G13, const SparseWeights& w2, int64_t G2, const void* out, int out_dtype,
+                           int64_t M, int64_t topk, int64_t H, int64_t I, int64_t E, const void* workspace, size_t workspace_bytes,
+                           const OutScatter& sc) {
   if (M < 0 || topk <= 0 || H <= 0 || I <= 0 || E <= 0) return B200FP4_STATUS_INVALID_VALUE;
   if (ld_h < H || ld_w < topk || ld_ids < topk || (ld_h % 8) != 0) return B200FP4_STATUS_INVALID_VALUE;
   if (sc.ptrs != nullptr && (sc.rows_per_dest <= 0 || sc.dest_row0 < 0)) return B200FP4_STATUS_INVALID_VALUE;
@@ -2075,23 +2085,33 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   rc = check_common(hidden, h_dtype, out, out_dtype, P, H, I, G2, E);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   if (M == 0) return B200FP4_STATUS_SUCCESS;
-  if (!topk_weights || !topk_ids || !w13_comp || !w13_meta || !w13_scale || !w13_g || !w2_comp || !w2_meta ||
-      !w2_scale || !w2_g)
+  if (!topk_weights || !topk_ids || !w13.comp || !w13.meta || !w13.scale || !w13.g || !w2.comp || !w2.meta || !w2.scale || !w2.g)
     return B200FP4_STATUS_INVALID_VALUE;
   if (expert_map && global_E <= 0) return B200FP4_STATUS_INVALID_VALUE;
   if (E > kPlanMaxExperts) return B200FP4_STATUS_NOT_SUPPORTED;
-  SparseWeights w13, w2;
-  w13.comp = w13_comp; w13.meta = w13_meta; w13.scale = w13_scale; w13.g = w13_g;
-  w13.comp_e = (H / 4) * 2 * I; w13.comp_pair = 4 * I; w13.comp_odd = 2 * I;
-  w13.meta_e = (H / 8) * 2 * I; w13.meta_row = 2 * I; w13.scale_e = G13 * 2 * I; w13.scale_row = 2 * I;
-  w2.comp = w2_comp; w2.meta = w2_meta; w2.scale = w2_scale; w2.g = w2_g;
-  w2.comp_e = (I / 4) * H; w2.comp_pair = 2 * H; w2.comp_odd = H;
-  w2.meta_e = (I / 8) * H; w2.meta_row = H; w2.scale_e = G2 * H; w2.scale_row = H;
   // the fused layer only exists in vectorised form
   if (I % 16 != 0 || !vector_ok(2 * I, H, G13, w13, hidden, ld_h) || !vector_ok(H, I, G2, w2, hidden, I))
     return B200FP4_STATUS_NOT_SUPPORTED;
   if (!workspace || !aligned(workspace, 256) || workspace_bytes < b200fp4_fused_moe_workspace_bytes(M, topk, H, I, E))
     return B200FP4_STATUS_ALLOC_FAILED;
+  return B200FP4_STATUS_SUCCESS;
+}
+
+// ld_h / ld_w / ld_ids: row strides (in elements) of hidden, topk_weights and topk_ids.
+static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const float* topk_weights, int64_t ld_w,
+                          const int32_t* topk_ids, int64_t ld_ids, const int32_t* expert_map, int64_t global_E,
+                          const uint8_t* w13_comp, const uint8_t* w13_meta, const uint8_t* w13_scale, const float* w13_g,
+                          int64_t G13, const uint8_t* w2_comp, const uint8_t* w2_meta, const uint8_t* w2_scale,
+                          const float* w2_g, int64_t G2, void* out, int out_dtype, int64_t M, int64_t topk, int64_t H,
+                          int64_t I, int64_t E, int flags, void* workspace, size_t workspace_bytes, void* stream,
+                          OutScatter sc = OutScatter{nullptr, 1, 0}) {
+  SparseWeights w13, w2;
+  fused_moe_weights(w13_comp, w13_meta, w13_scale, w13_g, G13, w2_comp, w2_meta, w2_scale, w2_g, G2, H, I, w13, w2);
+  int rc = fused_moe_check(hidden, ld_h, h_dtype, topk_weights, ld_w, topk_ids, ld_ids, expert_map, global_E, w13, G13, w2, G2, out,
+                           out_dtype, M, topk, H, I, E, workspace, workspace_bytes, sc);
+  if (rc != B200FP4_STATUS_SUCCESS || M == 0) return rc;
+  if (sc.ptrs != nullptr && !out) out = workspace;      // not written
+  const int64_t P = M * topk;
   cudaStream_t st = (cudaStream_t)stream;
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
   Plan plan = carve_plan(ws, P, E);
@@ -2244,6 +2264,16 @@ extern "C" int b200fp4_fused_sparse_moe_host_async(const void* hidden_host, int 
   char* d_out = d_hidden + align_up(nh, 256);
   char* d_w = d_out + align_up(nh, 256);
   char* d_ids = d_w + align_up(nr, 256);
+  {
+    // what the layer would refuse, before the copies are queued
+    SparseWeights w13, w2;
+    fused_moe_weights(w13_comp, w13_meta, w13_scale, w13_g, G13, w2_comp, w2_meta, w2_scale, w2_g, G2, H, I, w13, w2);
+    const int refused = fused_moe_check(d_hidden, H, h_dtype, reinterpret_cast<const float*>(d_w), topk,
+                                        reinterpret_cast<const int32_t*>(d_ids), topk, expert_map, global_E, w13, G13, w2, G2, d_out,
+                                        out_dtype, M, topk, H, I, E, static_cast<char*>(workspace) + stage, workspace_bytes - stage,
+                                        OutScatter{nullptr, 1, 0});
+    if (refused != B200FP4_STATUS_SUCCESS) return refused;
+  }
   cudaStream_t st = (cudaStream_t)stream;
   cudaStream_t cs = copy_stream ? (cudaStream_t)copy_stream : st;
   HostSlotEvents* ev = nullptr;

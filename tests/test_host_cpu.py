@@ -77,6 +77,18 @@ def test_refused_linear_queues_nothing(bad):
     assert _refused_unqueued(lambda L: L.b200fp4_linear_nvfp4(*a.values(), p, 1 << 62, 0)) in (INVALID, NOT_SUPPORTED)
 
 
+@pytest.mark.parametrize("bad", [
+    dict(w2_meta=0), dict(w13_comp=0x100008), dict(I=24), dict(h_dtype=2), dict(global_E=0, expert_map=0x100000), dict(G13=3),
+])
+def test_refused_layer_on_host_buffers_queues_nothing(bad):
+    # (a copy that was queued all the same would fail here for want of a device: status 13)
+    p = 0x100000
+    a = dict(hidden=p, h_dtype=1, topk_weights=p, topk_ids=p, expert_map=0, global_E=0, w13_comp=p, w13_meta=p, w13_scale=p, w13_g=p,
+             G13=16, w2_comp=p, w2_meta=p, w2_scale=p, w2_g=p, G2=16, out=p, out_dtype=1, status=0, M=2, topk=1, H=256, I=256, E=2, flags=2)
+    a.update(bad)
+    assert _refused_unqueued(lambda L: L.b200fp4_fused_sparse_moe_host_async(*a.values(), p, 1 << 40, 0, 0)) in (INVALID, NOT_SUPPORTED)
+
+
 def test_product_does_not_import_oracle():
     pkg = os.path.join(ROOT, "dgx_vllm_b200")
     for dirpath, _, files in os.walk(pkg):
