@@ -221,12 +221,11 @@ extern "C" int b200fp4_convert_to_sparse_2of4(const uint8_t* codes, const uint8_
   if (E <= 0 || N <= 0 || K <= 0 || (K % 8) != 0 || G <= 0) return B200FP4_STATUS_INVALID_VALUE;
   if (!codes || !comp_T || !meta_T || !aligned(codes, 4)) return B200FP4_STATUS_INVALID_VALUE;
   if ((scales == nullptr) != (scale_T == nullptr)) return B200FP4_STATUS_INVALID_VALUE;
-  if (E > 65535 || K / 8 > 65535 || N > (1 << 24)) return B200FP4_STATUS_NOT_SUPPORTED;
+  if (E > 65535 || K / 8 > 65535 || N > (1 << 24) || (scales && (G + 31) / 32 > 65535)) return B200FP4_STATUS_NOT_SUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   launch_convert<false>(codes, E, N, K / 2, comp_T, meta_T, st);
   int launches = 1;
   if (scales) {
-    if ((G + 31) / 32 > 65535) return B200FP4_STATUS_NOT_SUPPORTED;
     launch_convert<true>(scales, E, N, G, scale_T, nullptr, st);
     ++launches;
   }

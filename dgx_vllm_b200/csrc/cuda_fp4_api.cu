@@ -157,6 +157,8 @@ int gemm_common(Handle* h, int M, int N, int K, const void* A, const uint8_t* A_
   float* d_alpha = reinterpret_cast<float*>(h->scratch + 256);
   uint8_t* sfa = h->scratch + 512;
   uint8_t* sfb = sfa + round256(b200fp4_sf_swizzled_bytes(M, KB));
+  const int refused = dense_gemm_check(A, B, sfa, sfb, d_alpha, C, B200FP4_DTYPE_F32, M, N, K, 0, h->scratch, 256);
+  if (refused != B200FP4_STATUS_SUCCESS) return refused;
   cudaStream_t st = h->stream;
   if (A_scales) sf_swizzle_kernel<<<blocks_for(mp * KT * 4, 256), 256, 0, st>>>(A_scales, M, KB, mp, KT, sfa);
   else fill_bytes_kernel<<<blocks_for(mp * KT * 4, 256), 256, 0, st>>>(sfa, mp * KT * 4, 0x38);   // E4M3 1.0

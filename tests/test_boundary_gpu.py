@@ -194,6 +194,28 @@ def test_reference_c_api_through_ctypes(golden_dir):
     assert L.cudaFP4Destroy(h) == 0
 
 
+def test_refused_calls_of_several_steps_leave_the_outputs_alone():
+    from dgx_vllm_b200 import _lib
+    L = _lib.lib()
+    # the converter: too many scale groups, which only its second launch would use
+    G = 65535 * 32 + 1
+    codes, comp, meta = (torch.full((8,), 7, dtype=torch.uint8, device="cuda") for _ in range(3))
+    scales = torch.zeros(2 * G, dtype=torch.uint8, device="cuda")
+    assert L.b200fp4_convert_to_sparse_2of4(codes.data_ptr(), scales.data_ptr(), 1, 1, 8, G, comp.data_ptr(), meta.data_ptr(),
+                                            scales.data_ptr() + G, 0) == 15
+    torch.cuda.synchronize()
+    assert bool((comp == 7).all()) and bool((meta == 7).all())
+    # the reference's GEMM: a result pointer that only the GEMM behind the scale kernels refuses
+    h = ctypes.c_void_p()
+    assert L.cudaFP4Create(ctypes.byref(h)) == 0
+    a = torch.zeros(128, 32, dtype=torch.uint8, device="cuda")
+    C = torch.empty(128 * 128 + 1, dtype=torch.float32, device="cuda")
+    n0 = L.b200fp4_launch_count()
+    assert L.cudaFP4Gemm(h, 128, 128, 64, ctypes.c_float(1.0), a.data_ptr(), a.data_ptr(), C.data_ptr() + 4) == 7
+    assert L.b200fp4_launch_count() == n0
+    assert L.cudaFP4Destroy(h) == 0
+
+
 def test_vllm_adapter_hook_and_closure_on_the_gpu():
     # the weight-loading hook on a fake layer that lives on the GPU, with the CUDA converter, then the closure it installs
     # called the way vLLM calls MarlinExperts.apply; the yardstick is the oracle over the oracle's own 2:4 conversion
