@@ -5,7 +5,8 @@
 // waited for.  Here it is plain C++ on the tensors' own objects behind METH_FASTCALL functions: 3 to 6 us, launches
 // included.  The Python mirrors keep their signatures and hand their arguments straight over.
 //
-// The functions hold the GIL throughout (nothing in them blocks), which also serialises the workspace table.
+// Arguments are read with the GIL held; allocation and launches run without it (an allocation can reach cudaMalloc, a launch
+// blocks while the stream's queue is full), under a lock per stream that keeps a call's steps and their scratch together.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -17,6 +18,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
@@ -121,28 +123,53 @@ T* ptr(const at::Tensor& t) {
   return static_cast<T*>(t.data_ptr());
 }
 
-// Grow-only scratch per (device, stream, slot): calls issued on one stream serialise on the GPU, so consecutive ops share a
-// slot; the address is stable once large enough, which CUDA-graph capture relies on.  Slot 0 is what the status readers look
-// at, slot 1 the quantized activations of the one-call linear.
-struct WorkspaceKey {
-  int dev, slot;
-  cudaStream_t stream;
-  bool operator==(const WorkspaceKey& o) const { return dev == o.dev && slot == o.slot && stream == o.stream; }
-};
-struct WorkspaceHash {
-  size_t operator()(const WorkspaceKey& k) const {
-    return reinterpret_cast<size_t>(k.stream) * 0x9E3779B97F4A7C15ull + (size_t)(k.dev * 2 + k.slot);
-  }
+// Other Python threads run while one of these is alive: nothing under it touches a Python object.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  WithoutGil() = default;
+  WithoutGil(const WithoutGil&) = delete;
+  ~WithoutGil() { PyEval_RestoreThread(state); }
 };
 
-at::Tensor& workspace(int dev, cudaStream_t stream, size_t bytes, int slot = 0) {
-  // never destroyed: at interpreter exit the allocator may be gone before this table would be
-  static auto* table = new std::unordered_map<WorkspaceKey, at::Tensor, WorkspaceHash>();
-  at::Tensor& t = (*table)[WorkspaceKey{dev, slot, stream}];
-  if (!t.defined() || (size_t)t.numel() < bytes)
-    t = empty({(int64_t)std::max(bytes, (size_t)1 << 20)}, at::kByte, dev);
-  return t;
-}
+// Grow-only scratch per (device, stream): calls issued on one stream serialise on the GPU, so consecutive ops share it; its
+// address is stable once large enough, which CUDA-graph capture relies on.  Slot 0 is what the status readers look at, slot 1
+// the quantized activations of the one-call linear.  The lock is held from the look-up to the last launch of a call: another
+// thread on the same stream neither replaces the scratch under it nor puts a launch between its steps.  It is never waited
+// for with the GIL held.
+struct StreamScratch {
+  std::mutex mu;
+  at::Tensor slots[2];
+};
+struct StreamKey {
+  int dev;
+  cudaStream_t stream;
+  bool operator==(const StreamKey& o) const { return dev == o.dev && stream == o.stream; }
+};
+struct StreamHash {
+  size_t operator()(const StreamKey& k) const { return reinterpret_cast<size_t>(k.stream) * 0x9E3779B97F4A7C15ull + (size_t)k.dev; }
+};
+
+class Workspace {
+ public:
+  Workspace(int dev, cudaStream_t stream, size_t bytes, int slot = 0) : scratch_(of(dev, stream)), lock_(scratch_.mu), t_(scratch_.slots[slot]) {
+    if (!t_.defined() || (size_t)t_.numel() < bytes) t_ = empty({(int64_t)std::max(bytes, (size_t)1 << 20)}, at::kByte, dev);
+  }
+  const at::Tensor& tensor() const { return t_; }
+  void* data() const { return t_.data_ptr(); }
+  size_t bytes() const { return t_.nbytes(); }
+
+ private:
+  static StreamScratch& of(int dev, cudaStream_t stream) {
+    // never destroyed: at interpreter exit the allocator may be gone before this table would be
+    static auto* table = new std::unordered_map<StreamKey, StreamScratch, StreamHash>();
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    return (*table)[StreamKey{dev, stream}];
+  }
+  StreamScratch& scratch_;
+  std::lock_guard<std::mutex> lock_;
+  at::Tensor& t_;
+};
 
 PyObject* wrap(at::Tensor t) {
   PyObject* o = THPVariable_Wrap(std::move(t));
@@ -170,8 +197,14 @@ B200_FN(py_workspace) {
   return guarded([&] {
     want_args(n_args, 2);
     const int dev = (int)integer(args[0]);
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-    return wrap(workspace(dev, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(), (size_t)integer(args[1])));
+    const size_t bytes = (size_t)integer(args[1]);
+    at::Tensor t;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+      t = Workspace(dev, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(), bytes).tensor();
+    }
+    return wrap(std::move(t));
   });
 }
 
@@ -188,13 +221,16 @@ B200_FN(py_quant) {
     require(is_f32_scalar(gs), "global scale must be one f32");
     const int64_t M = x.size(0), K = x.size(1), KB = K / 16;
     require(K % 16 == 0, "K must be a multiple of 16");
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-    at::Tensor codes = empty({M, K / 2}, at::kByte, dev);
-    at::Tensor sf = swizzled ? empty({round_up(M, 128), round_up(KB, 4)}, at::kFloat8_e4m3fn, dev)
-                             : empty({M, KB}, at::kFloat8_e4m3fn, dev);
-    check(b200fp4_quantize(ptr(x), dtype_code(x.scalar_type()), M, K, M > 1 ? x.stride(0) : K, ptr<float>(gs), ptr(codes), ptr(sf),
-                           swizzled ? 1 : 0, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream()),
-          "scaled_fp4_quant");
+    at::Tensor codes, sf;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+      codes = empty({M, K / 2}, at::kByte, dev);
+      sf = swizzled ? empty({round_up(M, 128), round_up(KB, 4)}, at::kFloat8_e4m3fn, dev) : empty({M, KB}, at::kFloat8_e4m3fn, dev);
+      check(b200fp4_quantize(ptr(x), dtype_code(x.scalar_type()), M, K, M > 1 ? x.stride(0) : K, ptr<float>(gs), ptr(codes), ptr(sf),
+                             swizzled ? 1 : 0, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream()),
+            "scaled_fp4_quant");
+    }
     return wrap2(std::move(codes), std::move(sf));
   });
 }
@@ -221,17 +257,22 @@ B200_FN(py_mm) {
     require(THPDtype_Check(args[5]), "out_dtype must be bfloat16 or float16");
     const at::ScalarType dt = reinterpret_cast<THPDtype*>(args[5])->scalar_type;
     require(dt == at::kBFloat16 || dt == at::kHalf, "out_dtype must be bfloat16 or float16");
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
     const at::Tensor* given = maybe_tensor(args[6]);
     if (given)
       require(given->is_cuda() && given->scalar_type() == dt && is_2d(*given, M, N) && given->is_contiguous(),
               "out must be a contiguous [M,N] CUDA tensor of out_dtype");
-    at::Tensor out = given ? *given : empty({M, N}, dt, dev);
-    cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    const at::Tensor& ws = workspace(dev, st, b200fp4_gemm_workspace_bytes(M, N, K));
-    check(b200fp4_gemm_nvfp4(ptr(a), ptr(b), ptr(sa), ptr(sb), ptr<float>(alpha), ptr(out), dtype_code(dt), M, N, K,
-                             (int)integer(args[7]), ptr(ws), ws.nbytes(), st),
-          "cutlass_scaled_fp4_mm");
+    const int tile_n = (int)integer(args[7]);
+    at::Tensor out;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+      out = given ? *given : empty({M, N}, dt, dev);
+      cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+      const Workspace ws(dev, st, b200fp4_gemm_workspace_bytes(M, N, K));
+      check(b200fp4_gemm_nvfp4(ptr(a), ptr(b), ptr(sa), ptr(sb), ptr<float>(alpha), ptr(out), dtype_code(dt), M, N, K, tile_n, ws.data(),
+                               ws.bytes(), st),
+            "cutlass_scaled_fp4_mm");
+    }
     if (given) {
       Py_INCREF(args[6]);
       return args[6];
@@ -254,19 +295,23 @@ B200_FN(py_linear) {
     require(wsf.is_contiguous() && wsf.nbytes() >= b200fp4_sf_swizzled_bytes(N, K / 16),
             "w_block_scale must be the swizzled scale tensor of the weight");
     require(is_f32_scalar(alpha) && is_f32_scalar(gs), "alpha and x_global_scale must be one f32 each");
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
     const at::Tensor* given = maybe_tensor(args[5]);
     if (given)
       require(given->is_cuda() && is_16bit(*given) && is_2d(*given, M, N) && given->is_contiguous(),
               "out must be a contiguous [M,N] 16-bit CUDA tensor");
-    at::Tensor out = given ? *given : empty({M, N}, x.scalar_type(), dev);
-    if (M > 0) {
-      cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-      const at::Tensor& ws = workspace(dev, st, b200fp4_linear_workspace_bytes(M, N, K), 1);
-      check(b200fp4_linear_nvfp4(ptr(x), dtype_code(x.scalar_type()), M > 1 ? x.stride(0) : K, ptr<float>(gs), ptr(w), ptr(wsf),
-                                 ptr<float>(alpha), ptr(out), dtype_code(out.scalar_type()), M, N, K, (int)integer(args[6]), ptr(ws),
-                                 ws.nbytes(), st),
-            "nvfp4_linear");
+    const int tile_n = (int)integer(args[6]);
+    at::Tensor out;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+      out = given ? *given : empty({M, N}, x.scalar_type(), dev);
+      if (M > 0) {
+        cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+        const Workspace ws(dev, st, b200fp4_linear_workspace_bytes(M, N, K), 1);
+        check(b200fp4_linear_nvfp4(ptr(x), dtype_code(x.scalar_type()), M > 1 ? x.stride(0) : K, ptr<float>(gs), ptr(w), ptr(wsf),
+                                   ptr<float>(alpha), ptr(out), dtype_code(out.scalar_type()), M, N, K, tile_n, ws.data(), ws.bytes(), st),
+              "nvfp4_linear");
+      }
     }
     if (given) {
       Py_INCREF(args[5]);
@@ -290,13 +335,19 @@ B200_FN(py_router) {
             "hidden_states and gate_weight must both be bfloat16 or both float16");
     require(x.stride(1) == 1 && w.is_contiguous(), "rows must be contiguous");
     const int64_t M = x.size(0), H = x.size(1), E = w.size(0);
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-    at::Tensor tw = empty({M, topk}, at::kFloat, dev), ids = empty({M, topk}, at::kInt, dev);
-    cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    const at::Tensor& ws = workspace(dev, st, b200fp4_moe_router_workspace_bytes(M, E));
-    check(b200fp4_moe_router(ptr(x), M > 1 ? x.stride(0) : H, dtype_code(x.scalar_type()), ptr(w), M, H, E, topk, truth(args[3]) ? 1 : 0,
-                             ptr<float>(tw), ptr<int32_t>(ids), ptr(ws), ws.nbytes(), st),
-          "moe_router");
+    const int renormalize = truth(args[3]) ? 1 : 0;
+    at::Tensor tw, ids;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+      tw = empty({M, topk}, at::kFloat, dev);
+      ids = empty({M, topk}, at::kInt, dev);
+      cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+      const Workspace ws(dev, st, b200fp4_moe_router_workspace_bytes(M, E));
+      check(b200fp4_moe_router(ptr(x), M > 1 ? x.stride(0) : H, dtype_code(x.scalar_type()), ptr(w), M, H, E, topk, renormalize,
+                               ptr<float>(tw), ptr<int32_t>(ids), ws.data(), ws.bytes(), st),
+            "moe_router");
+    }
     return wrap2(std::move(tw), std::move(ids));
   });
 }
@@ -345,22 +396,27 @@ B200_FN(py_moe_call) {
             "hidden_states must be a contiguous [M,H] 16-bit CUDA tensor");
     require(tw.is_cuda() && ids.is_cuda() && ids.dim() == 2, "topk_weights / topk_ids must be contiguous [M, topk]");
     const int64_t M = x.size(0), topk = ids.size(1);
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)b->dev);
-    if (tw.scalar_type() != at::kFloat) tw = tw.to(at::kFloat);
-    if (ids.scalar_type() != at::kInt) ids = ids.to(at::kInt);
-    require(tw.is_contiguous() && ids.is_contiguous() && is_2d(tw, M, topk) && ids.size(0) == M,
-            "topk_weights / topk_ids must be contiguous [M, topk]");
+    const int flags = b->flags | (truth(args[4]) ? B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT : 0);
     const at::Tensor* given = maybe_tensor(args[5]);
-    at::Tensor out = given ? *given : empty({M, b->H}, x.scalar_type(), b->dev);
-    cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)b->dev).stream();
-    const at::Tensor& ws = workspace(b->dev, st, b200fp4_fused_moe_workspace_bytes(M, topk, b->H, b->I, b->E));
-    check(b200fp4_fused_sparse_moe(
-              ptr(x), dtype_code(x.scalar_type()), ptr<float>(tw), ptr<int32_t>(ids), b->emap.defined() ? ptr<int32_t>(b->emap) : nullptr,
-              b->emap.defined() ? b->emap.numel() : 0, ptr<uint8_t>(b->w13_comp), ptr<uint8_t>(b->w13_meta), ptr<uint8_t>(b->w13_scale),
-              ptr<float>(b->w13_g), b->w13_scale.size(1), ptr<uint8_t>(b->w2_comp), ptr<uint8_t>(b->w2_meta), ptr<uint8_t>(b->w2_scale),
-              ptr<float>(b->w2_g), b->w2_scale.size(1), ptr(out), dtype_code(out.scalar_type()), M, topk, b->H, b->I, b->E,
-              b->flags | (truth(args[4]) ? B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT : 0), ptr(ws), ws.nbytes(), st),
-          "fused_sparse_moe_v7");
+    at::Tensor out;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)b->dev);
+      if (tw.scalar_type() != at::kFloat) tw = tw.to(at::kFloat);
+      if (ids.scalar_type() != at::kInt) ids = ids.to(at::kInt);
+      require(tw.is_contiguous() && ids.is_contiguous() && is_2d(tw, M, topk) && ids.size(0) == M,
+              "topk_weights / topk_ids must be contiguous [M, topk]");
+      out = given ? *given : empty({M, b->H}, x.scalar_type(), b->dev);
+      cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)b->dev).stream();
+      const Workspace ws(b->dev, st, b200fp4_fused_moe_workspace_bytes(M, topk, b->H, b->I, b->E));
+      check(b200fp4_fused_sparse_moe(
+                ptr(x), dtype_code(x.scalar_type()), ptr<float>(tw), ptr<int32_t>(ids), b->emap.defined() ? ptr<int32_t>(b->emap) : nullptr,
+                b->emap.defined() ? b->emap.numel() : 0, ptr<uint8_t>(b->w13_comp), ptr<uint8_t>(b->w13_meta), ptr<uint8_t>(b->w13_scale),
+                ptr<float>(b->w13_g), b->w13_scale.size(1), ptr<uint8_t>(b->w2_comp), ptr<uint8_t>(b->w2_meta), ptr<uint8_t>(b->w2_scale),
+                ptr<float>(b->w2_g), b->w2_scale.size(1), ptr(out), dtype_code(out.scalar_type()), M, topk, b->H, b->I, b->E, flags,
+                ws.data(), ws.bytes(), st),
+            "fused_sparse_moe_v7");
+    }
     if (given) {
       Py_INCREF(args[5]);
       return args[5];
@@ -398,20 +454,24 @@ B200_FN(py_moe_prefill) {
     require(w13_sf.nbytes() >= (size_t)E * b200fp4_sf_swizzled_bytes(N1, H / 16) &&
                 w2_sf.nbytes() >= (size_t)E * b200fp4_sf_swizzled_bytes(H, I / 16),
             "b_scales must hold one swizzled scale tensor per expert");
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-    const at::Tensor ids = as_i32(ids_in), tw = (tw_in.scalar_type() == at::kFloat ? tw_in : tw_in.to(at::kFloat)).contiguous();
-    at::Tensor emap;
-    if (emap_in) emap = as_i32(*emap_in);
-    at::Tensor out = empty({M, H}, x.scalar_type(), dev);
-    cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    const at::Tensor scratch = empty({(int64_t)b200fp4_moe_prefill_workspace_bytes(M, topk, H, I, E)}, at::kByte, dev);
-    // the GEMMs' tile list and status word lie in the stream's workspace, where the status is read
-    const at::Tensor& gemm_ws = workspace(dev, st, b200fp4_grouped_gemm_workspace_bytes(P, E));
-    check(b200fp4_moe_prefill(ptr(x), dtype_code(x.scalar_type()), ptr<float>(tw), ptr<int32_t>(ids),
-                              emap.defined() ? ptr<int32_t>(emap) : nullptr, emap.defined() ? emap.numel() : 0, ptr(w13), ptr(w13_sf),
-                              ptr<float>(al1), ptr(w2), ptr(w2_sf), ptr<float>(al2), ptr<float>(a1), ptr<float>(a2), ptr(out), M, topk, H,
-                              I, E, ptr(scratch), scratch.nbytes(), ptr(gemm_ws), st),
-          "nvfp4_moe_prefill");
+    at::Tensor out;
+    {
+      WithoutGil nogil;
+      c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+      const at::Tensor ids = as_i32(ids_in), tw = (tw_in.scalar_type() == at::kFloat ? tw_in : tw_in.to(at::kFloat)).contiguous();
+      at::Tensor emap;
+      if (emap_in) emap = as_i32(*emap_in);
+      out = empty({M, H}, x.scalar_type(), dev);
+      cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+      const at::Tensor scratch = empty({(int64_t)b200fp4_moe_prefill_workspace_bytes(M, topk, H, I, E)}, at::kByte, dev);
+      // the GEMMs' tile list and status word lie in the stream's workspace, where the status is read
+      const Workspace gemm_ws(dev, st, b200fp4_grouped_gemm_workspace_bytes(P, E));
+      check(b200fp4_moe_prefill(ptr(x), dtype_code(x.scalar_type()), ptr<float>(tw), ptr<int32_t>(ids),
+                                emap.defined() ? ptr<int32_t>(emap) : nullptr, emap.defined() ? emap.numel() : 0, ptr(w13), ptr(w13_sf),
+                                ptr<float>(al1), ptr(w2), ptr(w2_sf), ptr<float>(al2), ptr<float>(a1), ptr<float>(a2), ptr(out), M, topk,
+                                H, I, E, ptr(scratch), scratch.nbytes(), gemm_ws.data(), st),
+            "nvfp4_moe_prefill");
+    }
     return wrap(std::move(out));
   });
 }
