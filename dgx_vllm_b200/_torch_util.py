@@ -37,11 +37,21 @@ def stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Grow-only scratch buffer per (device, current stream), shared with the native host path.  Calls issued on one
+WS_SHARED, WS_LINEAR, WS_ROUTER = 0, 1, 2       # slots of a stream's scratch (csrc/torch_host.cpp)
+
+
+def workspace(device: torch.device, nbytes: int, slot: int = WS_SHARED) -> torch.Tensor:
+    """Grow-only scratch buffer per (device, current stream, slot), shared with the native host path.  Calls issued on one
     stream serialise on the GPU, so sharing it between consecutive ops is safe; its address is stable once large enough,
     which CUDA-graph capture relies on."""
-    return _lib.host().workspace(torch.cuda.current_device() if device.index is None else device.index, nbytes)
+    return _lib.host().workspace(torch.cuda.current_device() if device.index is None else device.index, nbytes, slot)
+
+
+def status_word(device, slot: int) -> int:
+    """The first int of a slot's scratch, where the ops that use it leave their status word.  Synchronises the device."""
+    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    torch.cuda.synchronize(dev)
+    return int(workspace(dev, 256, slot)[:4].view(torch.int32).item())
 
 
 def ptr(t) -> int:

@@ -132,13 +132,14 @@ struct WithoutGil {
 };
 
 // Grow-only scratch per (device, stream): calls issued on one stream serialise on the GPU, so consecutive ops share it; its
-// address is stable once large enough, which CUDA-graph capture relies on.  Slot 0 is what the status readers look at, slot 1
-// the quantized activations of the one-call linear.  The lock is held from the look-up to the last launch of a call: another
+// address is stable once large enough, which CUDA-graph capture relies on.  One slot for each family of ops with a status word of
+// its own (or whose words another's would land on).  The lock is held from the look-up to the last launch of a call: another
 // thread on the same stream neither replaces the scratch under it nor puts a launch between its steps.  It is never waited
 // for with the GIL held.
+enum Slot { kSlotShared = 0, kSlotLinear = 1, kSlotRouter = 2, kSlots = 3 };        // Python names them in _torch_util.py
 struct StreamScratch {
   std::mutex mu;
-  at::Tensor slots[2];
+  at::Tensor slots[kSlots];
 };
 struct StreamKey {
   int dev;
@@ -151,7 +152,7 @@ struct StreamHash {
 
 class Workspace {
  public:
-  Workspace(int dev, cudaStream_t stream, size_t bytes, int slot = 0) : scratch_(of(dev, stream)), lock_(scratch_.mu), t_(scratch_.slots[slot]) {
+  Workspace(int dev, cudaStream_t stream, size_t bytes, int slot = kSlotShared) : scratch_(of(dev, stream)), lock_(scratch_.mu), t_(scratch_.slots[slot]) {
     if (!t_.defined() || (size_t)t_.numel() < bytes) t_ = empty({(int64_t)std::max(bytes, (size_t)1 << 20)}, at::kByte, dev);
   }
   const at::Tensor& tensor() const { return t_; }
@@ -192,17 +193,18 @@ int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
 // ------------------------------------------------------------------------------------------ dense ops
 
-// workspace(device index, bytes) -> the scratch tensor of the current stream
+// workspace(device index, bytes, slot) -> a scratch tensor of the current stream
 B200_FN(py_workspace) {
   return guarded([&] {
-    want_args(n_args, 2);
-    const int dev = (int)integer(args[0]);
+    want_args(n_args, 3);
+    const int dev = (int)integer(args[0]), slot = (int)integer(args[2]);
     const size_t bytes = (size_t)integer(args[1]);
+    require(slot >= 0 && slot < kSlots, "no such workspace slot");
     at::Tensor t;
     {
       WithoutGil nogil;
       c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
-      t = Workspace(dev, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(), bytes).tensor();
+      t = Workspace(dev, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(), bytes, slot).tensor();
     }
     return wrap(std::move(t));
   });
@@ -307,7 +309,7 @@ B200_FN(py_linear) {
       out = given ? *given : empty({M, N}, x.scalar_type(), dev);
       if (M > 0) {
         cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-        const Workspace ws(dev, st, b200fp4_linear_workspace_bytes(M, N, K), 1);
+        const Workspace ws(dev, st, b200fp4_linear_workspace_bytes(M, N, K), kSlotLinear);
         check(b200fp4_linear_nvfp4(ptr(x), dtype_code(x.scalar_type()), M > 1 ? x.stride(0) : K, ptr<float>(gs), ptr(w), ptr(wsf),
                                    ptr<float>(alpha), ptr(out), dtype_code(out.scalar_type()), M, N, K, tile_n, ws.data(), ws.bytes(), st),
               "nvfp4_linear");
@@ -343,7 +345,7 @@ B200_FN(py_router) {
       tw = empty({M, topk}, at::kFloat, dev);
       ids = empty({M, topk}, at::kInt, dev);
       cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-      const Workspace ws(dev, st, b200fp4_moe_router_workspace_bytes(M, E));
+      const Workspace ws(dev, st, b200fp4_moe_router_workspace_bytes(M, E), kSlotRouter);
       check(b200fp4_moe_router(ptr(x), M > 1 ? x.stride(0) : H, dtype_code(x.scalar_type()), ptr(w), M, H, E, topk, renormalize,
                                ptr<float>(tw), ptr<int32_t>(ids), ws.data(), ws.bytes(), st),
             "moe_router");

@@ -6,9 +6,16 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from ._torch_util import WS_ROUTER, status_word
 
 
 def moe_router(hidden_states: torch.Tensor, gate_weight: torch.Tensor, topk: int, renormalize: bool = True):
     """hidden_states [M,H], gate_weight [E,H] (both bf16 or both f16) -> (topk_weights [M,topk] f32, topk_ids [M,topk] i32).
     Weights are softmax probabilities of the selected experts, divided by their sum when renormalize is set."""
     return _lib.host().moe_router(hidden_states, gate_weight, topk, renormalize)
+
+
+def last_router_status(device=None) -> int:
+    """Status word of the most recent moe_router on the current stream of `device`: 0, or the code of a bounded wait that ran
+    out in the projection of more than 64 tokens (that call's weights and ids are then not valid).  Synchronises."""
+    return status_word(device, WS_ROUTER)

@@ -411,7 +411,11 @@ B200FP4_API int b200fp4_moe_prefill(const void* hidden, int dtype, const float* 
  *   hidden [M, H] and gate_w [E, H] of `dtype` (BF16 or F16), hidden rows ld_h elements apart; logits accumulate in f32
  *   topk_weights [M, topk] f32 = exp(l - max) / sum over the selected experts (renormalize != 0) or over all experts
  *   topk_ids [M, topk] i32 in decreasing order of logit; equal logits go to the lower expert id
- *   workspace b200fp4_moe_router_workspace_bytes(M, E) bytes (the f32 logits, in slices over H).  topk <= 32, E <= 1024. */
+ *   workspace b200fp4_moe_router_workspace_bytes(M, E) bytes: 256 whose first int is a status word, then the f32 logits in slices
+ *             over H.  The word is 0 unless one of the bounded waits of the projection of more than 64 tokens ran out (31: a
+ *             stage was not freed, 32: its operands did not land, 33: the accumulator was not finished); weights and ids are
+ *             then made from whatever logits there are -- ids still in [0, E) -- and not to be trusted: read it after
+ *             synchronising when diagnosing (router.last_router_status).  topk <= 32, E <= 1024. */
 B200FP4_API size_t b200fp4_moe_router_workspace_bytes(int64_t M, int64_t E);
 B200FP4_API int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, const void* gate_w, int64_t M, int64_t H,
                                    int64_t E, int64_t topk, int renormalize, float* topk_weights, int32_t* topk_ids,

@@ -194,6 +194,27 @@ def test_reference_c_api_through_ctypes(golden_dir):
     assert L.cudaFP4Destroy(h) == 0
 
 
+def _set_word(slot, value):
+    from dgx_vllm_b200._torch_util import workspace
+    workspace(torch.device("cuda", 0), 256, *slot)[:4].view(torch.int32).fill_(value)
+
+
+@pytest.mark.parametrize("M", [32, 65])                            # either projection kernel
+def test_router_status_word_has_its_own_place(M):
+    from dgx_vllm_b200 import router
+    from dgx_vllm_b200.ops import last_gemm_status
+    x, gate = (torch.randn(n, 256, device="cuda", dtype=torch.bfloat16) for n in (M, 16))
+    router.moe_router(x, gate, 4)
+    _set_word((), 5)                                               # a wait of a GEMM that ran out
+    router.moe_router(x, gate, 4)
+    assert last_gemm_status() == 5 and router.last_router_status() == 0
+    _set_word((2,), 33)                                            # one of the router's
+    assert last_gemm_status() == 5 and router.last_router_status() == 33
+    router.moe_router(x, gate, 4)
+    assert router.last_router_status() == 0
+    _set_word((), 0)
+
+
 def test_refused_calls_of_several_steps_leave_the_outputs_alone():
     from dgx_vllm_b200 import _lib
     L = _lib.lib()
