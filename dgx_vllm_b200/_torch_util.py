@@ -37,7 +37,7 @@ def stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-WS_SHARED, WS_LINEAR, WS_ROUTER = 0, 1, 2       # slots of a stream's scratch (csrc/torch_host.cpp)
+WS_SHARED, WS_LINEAR, WS_ROUTER, WS_GEMM = 0, 1, 2, 3       # slots of a stream's scratch (csrc/torch_host.cpp)
 
 
 def workspace(device: torch.device, nbytes: int, slot: int = WS_SHARED) -> torch.Tensor:

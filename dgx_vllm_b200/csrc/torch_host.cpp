@@ -136,7 +136,7 @@ struct WithoutGil {
 // its own (or whose words another's would land on).  The lock is held from the look-up to the last launch of a call: another
 // thread on the same stream neither replaces the scratch under it nor puts a launch between its steps.  It is never waited
 // for with the GIL held.
-enum Slot { kSlotShared = 0, kSlotLinear = 1, kSlotRouter = 2, kSlots = 3 };        // Python names them in _torch_util.py
+enum Slot { kSlotShared = 0, kSlotLinear = 1, kSlotRouter = 2, kSlotGemm = 3, kSlots = 4 };        // Python names them in _torch_util.py
 struct StreamScratch {
   std::mutex mu;
   at::Tensor slots[kSlots];
@@ -270,7 +270,7 @@ B200_FN(py_mm) {
       c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
       out = given ? *given : empty({M, N}, dt, dev);
       cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-      const Workspace ws(dev, st, b200fp4_gemm_workspace_bytes(M, N, K));
+      const Workspace ws(dev, st, b200fp4_gemm_workspace_bytes(M, N, K), kSlotGemm);
       check(b200fp4_gemm_nvfp4(ptr(a), ptr(b), ptr(sa), ptr(sb), ptr<float>(alpha), ptr(out), dtype_code(dt), M, N, K, tile_n, ws.data(),
                                ws.bytes(), st),
             "cutlass_scaled_fp4_mm");
@@ -466,8 +466,8 @@ B200_FN(py_moe_prefill) {
       out = empty({M, H}, x.scalar_type(), dev);
       cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
       const at::Tensor scratch = empty({(int64_t)b200fp4_moe_prefill_workspace_bytes(M, topk, H, I, E)}, at::kByte, dev);
-      // the GEMMs' tile list and status word lie in the stream's workspace, where the status is read
-      const Workspace gemm_ws(dev, st, b200fp4_grouped_gemm_workspace_bytes(P, E));
+      // the GEMMs' tile list and status word lie in the stream's scratch for GEMMs, where the status is read
+      const Workspace gemm_ws(dev, st, b200fp4_grouped_gemm_workspace_bytes(P, E), kSlotGemm);
       check(b200fp4_moe_prefill(ptr(x), dtype_code(x.scalar_type()), ptr<float>(tw), ptr<int32_t>(ids),
                                 emap.defined() ? ptr<int32_t>(emap) : nullptr, emap.defined() ? emap.numel() : 0, ptr(w13), ptr(w13_sf),
                                 ptr<float>(al1), ptr(w2), ptr(w2_sf), ptr<float>(al2), ptr<float>(a1), ptr<float>(a2), ptr(out), M, topk,

@@ -9,7 +9,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._torch_util import dtype_code, ptr, require, require_cuda, stream_ptr, workspace
+from ._torch_util import WS_GEMM, dtype_code, ptr, require, require_cuda, stream_ptr, workspace
 
 
 def get_cutlass_moe_mm_data(topk_ids, expert_offsets, problem_sizes1, problem_sizes2, input_permutation,
@@ -168,7 +168,7 @@ def cutlass_fp4_moe_mm(out_tensors, a_tensors, b_tensors, a_scales, b_scales, al
     K = K2 * 2
     require(b_scales.numel() * b_scales.element_size() >= E * L.b200fp4_sf_swizzled_bytes(N, K // 16),
             "b_scales must hold one swizzled scale tensor per expert")
-    ws = workspace(dev, L.b200fp4_grouped_gemm_workspace_bytes(rows, E))
+    ws = workspace(dev, L.b200fp4_grouped_gemm_workspace_bytes(rows, E), WS_GEMM)
     with torch.cuda.device(dev):
         _lib.check(L.b200fp4_grouped_gemm_nvfp4(ptr(a_tensors), ptr(b_tensors), ptr(a_scales), ptr(b_scales), ptr(alphas),
                                                 ptr(expert_offsets), ptr(sf_offsets), ptr(out_tensors),
@@ -201,7 +201,7 @@ def cutlass_fp4_moe_mm_silu_and_mul_quant(a_tensors, b_tensors, a_scales, b_scal
     sf_rows = (rows + 127) // 128 * 128 + 128 * E
     codes = torch.empty((rows, I // 2), dtype=torch.uint8, device=dev)
     sf = torch.empty((sf_rows, (I // 16 + 3) // 4 * 4), dtype=torch.uint8, device=dev)
-    ws = workspace(dev, L.b200fp4_grouped_gemm_workspace_bytes(rows, E))
+    ws = workspace(dev, L.b200fp4_grouped_gemm_workspace_bytes(rows, E), WS_GEMM)
     with torch.cuda.device(dev):
         _lib.check(L.b200fp4_grouped_gemm_nvfp4_silu_quant(
             ptr(a_tensors), ptr(b_tensors), ptr(a_scales), ptr(b_scales), ptr(alphas), ptr(expert_offsets), ptr(sf_offsets),

@@ -205,14 +205,34 @@ def test_router_status_word_has_its_own_place(M):
     from dgx_vllm_b200.ops import last_gemm_status
     x, gate = (torch.randn(n, 256, device="cuda", dtype=torch.bfloat16) for n in (M, 16))
     router.moe_router(x, gate, 4)
-    _set_word((), 5)                                               # a wait of a GEMM that ran out
+    _set_word((3,), 5)                                             # a wait of a GEMM that ran out
     router.moe_router(x, gate, 4)
     assert last_gemm_status() == 5 and router.last_router_status() == 0
     _set_word((2,), 33)                                            # one of the router's
     assert last_gemm_status() == 5 and router.last_router_status() == 33
     router.moe_router(x, gate, 4)
     assert router.last_router_status() == 0
-    _set_word((), 0)
+    _set_word((3,), 0)
+
+
+def test_gemm_and_layer_status_words_have_their_own_places():
+    from dgx_vllm_b200 import cutlass_scaled_fp4_mm, scaled_fp4_quant, sparse_fp4_v7 as sp7
+    from dgx_vllm_b200.ops import last_gemm_status
+    import synth
+    w13, w2 = _layer(4, 256, 128, 1)
+    tw, ids = synth.make_routing(3, 4, 2, 3, "cuda")
+    x, gs = synth.make_hidden(3, 256, 4, "cuda"), torch.full((1,), 400.0, device="cuda")
+    layer = lambda: sp7.fused_sparse_moe_v7(x, tw, ids, None, *[w13[k].cuda() for k in KEYS], *[w2[k].cuda() for k in KEYS], 128, False)
+    codes, sf = scaled_fp4_quant(x, gs)
+    gemm = lambda: cutlass_scaled_fp4_mm(codes, codes, sf, sf, gs, torch.bfloat16)
+    gemm()
+    layer()
+    assert last_gemm_status() == 0                                 # not the layer's number of experts
+    _set_word((3,), 5)                                             # a wait of a GEMM that ran out stays on record
+    layer()
+    assert last_gemm_status() == 5 and sp7.last_moe_status() == 0
+    gemm()
+    assert last_gemm_status() == 0
 
 
 def test_refused_calls_of_several_steps_leave_the_outputs_alone():
