@@ -1037,7 +1037,7 @@ extern "C" int b200fp4_gemm_nvfp4(const void* a_codes, const void* b_codes, cons
 
 // y = NVFP4(x) @ W^T: the activation quantizer and the GEMM queued by one call (two launches a few microseconds apart;
 // through two Python calls the GPU idles between them for longer than either kernel runs at prefill sizes).
-// workspace: [codes M*K/2 | swizzled block scales | GEMM workspace], each part 256-byte aligned.
+// workspace: [GEMM workspace (status word first) | codes M*K/2 | swizzled block scales], each part 256-byte aligned.
 static size_t linear_part(size_t v) { return (v + 255) / 256 * 256; }
 
 extern "C" size_t b200fp4_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
@@ -1053,11 +1053,11 @@ extern "C" int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, con
   if (M == 0) return B200FP4_STATUS_SUCCESS;
   if (!workspace || !aligned(workspace, 256) || workspace_bytes < b200fp4_linear_workspace_bytes(M, N, K))
     return B200FP4_STATUS_ALLOC_FAILED;
-  unsigned char* codes = static_cast<unsigned char*>(workspace);
-  unsigned char* sf = codes + linear_part((size_t)M * (size_t)K / 2);
-  unsigned char* gemm_ws = sf + linear_part(b200fp4_sf_swizzled_bytes(M, K / 16));
-  // what either step would refuse, before the first is queued
   const size_t gemm_bytes = b200fp4_gemm_workspace_bytes(M, N, K);
+  unsigned char* gemm_ws = static_cast<unsigned char*>(workspace);
+  unsigned char* codes = gemm_ws + linear_part(gemm_bytes);
+  unsigned char* sf = codes + linear_part((size_t)M * (size_t)K / 2);
+  // what either step would refuse, before the first is queued
   int rc = quantize_check(x, x_dtype, M, K, ldx, x_global_scale, codes, sf);
   if (rc == B200FP4_STATUS_SUCCESS)
     rc = dense_gemm_check(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, gemm_bytes);

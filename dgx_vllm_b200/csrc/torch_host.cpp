@@ -153,7 +153,9 @@ struct StreamHash {
 class Workspace {
  public:
   Workspace(int dev, cudaStream_t stream, size_t bytes, int slot = kSlotShared) : scratch_(of(dev, stream)), lock_(scratch_.mu), t_(scratch_.slots[slot]) {
-    if (!t_.defined() || (size_t)t_.numel() < bytes) t_ = empty({(int64_t)std::max(bytes, (size_t)1 << 20)}, at::kByte, dev);
+    if (t_.defined() && (size_t)t_.numel() >= bytes) return;
+    t_ = empty({(int64_t)std::max(bytes, (size_t)1 << 20)}, at::kByte, dev);
+    t_.narrow(0, 0, 256).zero_();                  // a status word that no op has written yet reads 0
   }
   const at::Tensor& tensor() const { return t_; }
   void* data() const { return t_.data_ptr(); }

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._torch_util import WS_GEMM, status_word
+from ._torch_util import WS_GEMM, WS_LINEAR, status_word
 
 
 def scaled_fp4_quant(input: torch.Tensor, input_global_scale: torch.Tensor, is_sf_swizzled_layout: bool = True):
@@ -40,5 +40,6 @@ def nvfp4_linear(x: torch.Tensor, x_global_scale: torch.Tensor, w_codes: torch.T
 
 
 def last_gemm_status(device=None) -> int:
-    """Status word of the most recent GEMM on the current stream of `device` (0 = ok).  Synchronises."""
-    return status_word(device, WS_GEMM)
+    """Status word of the most recent GEMM op on the current stream of `device` (0 = ok) or, where that is 0, of the most recent
+    nvfp4_linear.  Synchronises."""
+    return status_word(device, WS_GEMM) or status_word(device, WS_LINEAR)

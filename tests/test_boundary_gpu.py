@@ -235,6 +235,20 @@ def test_gemm_and_layer_status_words_have_their_own_places():
     assert last_gemm_status() == 0
 
 
+def test_linear_status_word_is_read():
+    from dgx_vllm_b200 import scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status, nvfp4_linear
+    x, gs = torch.randn(300, 256, device="cuda", dtype=torch.bfloat16), torch.full((1,), 400.0, device="cuda")
+    codes, sf = scaled_fp4_quant(x, gs)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        nvfp4_linear(x, gs, codes, sf, gs)
+        assert last_gemm_status() == 0
+        _set_word((1,), 3)                                         # a wait that ran out
+        assert last_gemm_status() == 3
+        nvfp4_linear(x, gs, codes, sf, gs)                         # cleared by the next
+        assert last_gemm_status() == 0
+
+
 def test_refused_calls_of_several_steps_leave_the_outputs_alone():
     from dgx_vllm_b200 import _lib
     L = _lib.lib()
