@@ -144,12 +144,74 @@ def test_dense_gemm_tile_choice(M, N, K, dtype):
     assert ((out.float() - ref).abs().max() / ref.abs().max()).item() < 5e-3
 
 
+def _linear_operands(M, N, K, seed):
+    from dgx_vllm_b200 import scaled_fp4_quant
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").mul_(0.02).to(torch.bfloat16)
+    gx, gw = torch.full((1,), 2688 / 6.5, device="cuda"), torch.full((1,), 2688 / 0.13, device="cuda")
+    return x, gx, *scaled_fp4_quant(w, gw), 1.0 / (gx * gw)
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (8, 512, 2048),           # split of K over four CTAs: every CTA requests its own first stages early
+    (33, 136, 2112),          # ... ragged, nine stages on four CTAs, the last one short
+    (129, 1000, 4096),        # ... two row tiles
+    (5, 5000, 1024),          # split over two
+    (8, 264, 64),             # a single short stage
+    (128, 14336, 1024),       # narrow tiles, fewer stages than the ring holds
+    (385, 6000, 1088),        # wide tiles; the columns of the second scale tile lie past N
+])
+def test_linear_early_weights(M, N, K):
+    from dgx_vllm_b200 import cutlass_scaled_fp4_mm, scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status, nvfp4_linear
+    x, gx, wc, ws, alpha = _linear_operands(M, N, K, M + K)
+    out = nvfp4_linear(x, gx, wc, ws, alpha)
+    assert last_gemm_status() == 0
+    xc, xs = scaled_fp4_quant(x, gx)
+    assert torch.equal(out, cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, torch.bfloat16))
+
+
+@pytest.mark.parametrize("M", [8, 128, 300])
+@pytest.mark.parametrize("last", ["codes", "scales", "quantizer"])
+def test_linear_reads_weights_the_kernel_before_it_wrote(M, last):
+    # the GEMM requests weights before it waits for the quantizer; the quantizer lets it start only after whatever wrote them
+    from dgx_vllm_b200 import scaled_fp4_quant
+    from dgx_vllm_b200.ops import nvfp4_linear
+    N, K, rounds = 4096, 4096, 12
+    sets = [_linear_operands(M, N, K, s) for s in range(2)]
+    x, gx, alpha = sets[0][0], sets[0][1], sets[0][4]
+    want = [nvfp4_linear(x, gx, s[2], s[3], alpha) for s in sets]
+    assert not torch.equal(*want)
+    dense = [torch.randn(N, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(s)).mul_(0.02).bfloat16() for s in (5, 6)]
+    gw = torch.full((1,), 2688 / 0.13, device="cuda")
+    if last == "quantizer":
+        want = [nvfp4_linear(x, gx, *scaled_fp4_quant(d, gw), alpha) for d in dense]
+    codes, sf = torch.empty_like(sets[0][2]), torch.empty_like(sets[0][3])
+    torch.cuda.synchronize()
+    got = []
+    torch.cuda._sleep(4_000_000)                      # everything below is queued before the first of it runs
+    for i in range(rounds):
+        if last == "quantizer":
+            codes, sf = scaled_fp4_quant(dense[i % 2], gw)
+        else:
+            copy = [lambda: torch.bitwise_or(sets[i % 2][2], 0, out=codes),
+                    lambda: torch.bitwise_or(sets[i % 2][3].view(torch.uint8), 0, out=sf.view(torch.uint8))]
+            for c in copy if last == "scales" else copy[::-1]:
+                c()
+        got.append(nvfp4_linear(x, gx, codes, sf, alpha))
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
+
+
 @pytest.mark.parametrize("M,E,topk,H,I,dtype", [
     (1, 4, 1, 64, 128, torch.bfloat16),          # one row, less than one 256-wide stage of k
     (37, 4, 3, 320, 128, torch.float16),         # a tail stage of one k-block
     (200, 2, 2, 704, 256, torch.bfloat16),       # tail of three k-blocks, several row tiles per expert
     (65, 8, 5, 1024, 384, torch.bfloat16),       # a batch of four slots and one more
     (33, 16, 16, 4160, 128, torch.float16),      # a row longer than a block of threads takes at once
+    (16384, 8, 8, 64, 128, torch.bfloat16),      # 131,072 pairs: the most that one launch routes
+    (16385, 8, 8, 64, 128, torch.bfloat16),      # ... more: grid-wide routing steps, the tile list made by the first GEMM
 ])
 def test_prefill_layer_equals_its_steps(M, E, topk, H, I, dtype):
     from dgx_vllm_b200 import grouped_moe as gm
