@@ -1002,11 +1002,11 @@ struct WsUnit {
 struct WsClaims {
   int cur, nxt;                      // KS == 1: cur only
 };
-template <bool kSilu, int kN, int kDep, int kS = kWsStages, int KS = 1>
+template <bool kSilu, int kDep, int kS = kWsStages, int KS = 1>
 __device__ __forceinline__ void ws_phase(const GemvArgs& g, int* counter, const int base, WsClaims& claims, const WsLane& L, const WsUnit& U,
                                          int* done, const int need) {
   const int lane = L.lane, q = L.q, t = L.t;
-  const int N = kN ? kN : g.N;
+  const int N = g.N;
   const int nblk = g.K / (32 * kS * KS);     // blocks of kS 32-wide k-steps (one turn of the ring)
   const int groups = g.n_slabs;              // 128-column groups per pass
   const int n_items = g.plan.hdr[1] * groups;
@@ -1328,7 +1328,7 @@ __device__ __forceinline__ WsUnit ws_unit(const WsLane& L, WsClaims& claims) {
 template <int kS, int kW, int KS>
 constexpr size_t ws_smem_bytes() { return (size_t)kW * kS * kWsStageBytes + 128 + (KS > 1 ? (size_t)kW * 4096 + 4 * (kW / KS) : 0); }
 
-template <bool kSilu, int kN, int kS = kWsStages, int kW = kWsWarps>
+template <bool kSilu, int kS = kWsStages, int kW = kWsWarps>
 __global__ void __launch_bounds__(32 * kW, 1) sparse_gemv_ws_kernel(const GemvArgs g, int* counter) {
   extern __shared__ __align__(16) unsigned char smem[];
   pdl_wait();
@@ -1336,14 +1336,14 @@ __global__ void __launch_bounds__(32 * kW, 1) sparse_gemv_ws_kernel(const GemvAr
   const WsLane L = ws_lane<kS>(smem);
   WsClaims claims;
   const WsUnit U = ws_unit<kS, kW, 1>(L, claims);
-  ws_phase<kSilu, kN, 0, kS>(g, counter, 0, claims, L, U, nullptr, 0);
+  ws_phase<kSilu, 0, kS>(g, counter, 0, claims, L, U, nullptr, 0);
 }
 
 // Both projections of the MoE layer in one launch: the claim sequence runs through the gate_up items and on into the
 // down items, so a warp that finds no gate_up item left starts on the down projection of passes that are complete
 // instead of idling until the slowest warp of a first launch has finished and a second launch has ramped up.
 // kSB: ring slots the down projection turns through (its slice of K may be shorter than a ring).
-template <int kNA, int kNB, int kS, int kW, int KS, int kSB>
+template <int kS, int kW, int KS, int kSB>
 __global__ void __launch_bounds__(32 * kW, 1)
     fused_moe_ws_kernel(const GemvArgs ga, const GemvArgs gb, int* counter, int* done, int need) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1353,8 +1353,8 @@ __global__ void __launch_bounds__(32 * kW, 1)
   WsClaims claims;
   const WsUnit U = ws_unit<kS, kW, KS>(L, claims);
   const int n_a = ga.plan.hdr[1] * ga.n_slabs;
-  ws_phase<true, kNA, 1, kS, KS>(ga, counter, 0, claims, L, U, done, need);
-  ws_phase<false, kNB, 2, kSB, KS>(gb, counter, n_a, claims, L, U, done, need);
+  ws_phase<true, 1, kS, KS>(ga, counter, 0, claims, L, U, done, need);
+  ws_phase<false, 2, kSB, KS>(gb, counter, n_a, claims, L, U, done, need);
 }
 
 // ------------------------------------------------------------------------------------------ generic
@@ -1660,15 +1660,15 @@ int64_t ws_grid(int64_t max_items) {
   return grid < 1 ? 1 : grid;
 }
 
-template <bool kSilu, int kN, int kS = kWsStages, int kW = kWsWarps>
+template <bool kSilu, int kS = kWsStages, int kW = kWsWarps>
 int launch_ws_t(const GemvArgs& g, int* counter, int64_t max_items, cudaStream_t st) {
   static bool attr_set[64] = {false};
   constexpr size_t smem = (size_t)kW * kS * kWsStageBytes + 128;
-  if (!ws_prepare(sparse_gemv_ws_kernel<kSilu, kN, kS, kW>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
+  if (!ws_prepare(sparse_gemv_ws_kernel<kSilu, kS, kW>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
   int64_t grid = (max_items + kW - 1) / kW;
   if (grid > (int64_t)sm_count()) grid = sm_count();
   if (grid < 1) grid = 1;
-  launch_pdl(sparse_gemv_ws_kernel<kSilu, kN, kS, kW>, dim3((unsigned)grid), dim3(32 * kW), smem, st, g, counter);
+  launch_pdl(sparse_gemv_ws_kernel<kSilu, kS, kW>, dim3((unsigned)grid), dim3(32 * kW), smem, st, g, counter);
   return B200FP4_STATUS_SUCCESS;
 }
 
@@ -1682,22 +1682,18 @@ int run_projection_ws(const SparseWeights& w, const Plan& plan, const __half* A,
   GemvArgs g = make_args(w, plan, A, lda, a_div, out, out_dtype, ldo, N, K, inter_silu);
   g.n_slabs = inter_silu > 0 ? inter_silu / 64 : (int)(N / 128);
   const int64_t items = max_passes(P, E) * g.n_slabs;
-  if (K % 256 == 0) {      // 8 warps x 8-stage rings (see the fused layer for the measurements)
-    if (inter_silu > 0)
-      return N == 1024 ? launch_ws_t<true, 1024, 8, 8>(g, counter, items, st) : launch_ws_t<true, 0, 8, 8>(g, counter, items, st);
-    return N == 2048 ? launch_ws_t<false, 2048, 8, 8>(g, counter, items, st) : launch_ws_t<false, 0, 8, 8>(g, counter, items, st);
-  }
-  if (inter_silu > 0) return N == 1024 ? launch_ws_t<true, 1024>(g, counter, items, st) : launch_ws_t<true, 0>(g, counter, items, st);
-  return N == 2048 ? launch_ws_t<false, 2048>(g, counter, items, st) : launch_ws_t<false, 0>(g, counter, items, st);
+  if (K % 256 == 0)        // 8 warps x 8-stage rings (see the fused layer for the measurements)
+    return inter_silu > 0 ? launch_ws_t<true, 8, 8>(g, counter, items, st) : launch_ws_t<false, 8, 8>(g, counter, items, st);
+  return inter_silu > 0 ? launch_ws_t<true>(g, counter, items, st) : launch_ws_t<false>(g, counter, items, st);
 }
 
-template <int kNA, int kNB, int kS, int kW, int KS, int kSB = kS>
+template <int kS, int kW, int KS, int kSB = kS>
 int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int need, cudaStream_t st) {
   static bool attr_set[64] = {false};
   constexpr size_t smem = ws_smem_bytes<kS, kW, KS>();
   static_assert(smem <= 227 * 1024, "shared memory of the ring");
-  if (!ws_prepare(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS, kSB>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
-  launch_pdl(fused_moe_ws_kernel<kNA, kNB, kS, kW, KS, kSB>, dim3((unsigned)sm_count()), dim3(32 * kW), smem, st, ga, gb, counter, done, need);
+  if (!ws_prepare(fused_moe_ws_kernel<kS, kW, KS, kSB>, attr_set, smem)) return B200FP4_STATUS_EXECUTION_FAILED;
+  launch_pdl(fused_moe_ws_kernel<kS, kW, KS, kSB>, dim3((unsigned)sm_count()), dim3(32 * kW), smem, st, ga, gb, counter, done, need);
   return B200FP4_STATUS_SUCCESS;
 }
 
@@ -1717,7 +1713,6 @@ int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int*
 // H=2048, I=512, M=28 62.9 / 64.8, M=32 70.5 / 68.6, M=40 80.2 / 79.3, M=48 84.1 / 93.6, M=80 112 / 112, M=96 124 / 120, M=112
 // 129 / 125; 256 experts, H=2048, I=1024, M=14 66.6 / 69.1, M=16 76.6 / 73.4, M=20 84.9 / 81.1, M=24 93.5 / 107, M=64 130 / 134,
 // M=96 141 / 145; 512 experts, H=1024, I=512, M=36 49.4 / 45.8).
-template <int kNA, int kNB>
 int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int64_t local_pairs, int64_t E, cudaStream_t st) {
   const int64_t passes = (local_pairs < E ? local_pairs : E) * ((local_pairs + 8 * E - 1) / (8 * E));
   const int64_t items = passes * ga.n_slabs, sms = sm_count();
@@ -1729,16 +1724,15 @@ int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* d
     if (a % (4 * KS) != 0 || b % KS != 0) return 0;
     return b / KS % 4 == 0 ? 4 : (b / KS % 3 == 0 ? 3 : (b / KS % 2 == 0 ? 2 : 0));
   };
-  constexpr bool kAny = kNA == 0;              // the instantiation for one model's widths has K = 2048 and 512 only
   if (items <= 3 * sms) {
     const int t = turns(4), n = 4 * need + more;
-    if (t == 4) return launch_fused_ws_t<kNA, kNB, 4, 12, 4>(ga, gb, counter, done, n, st);
-    if (kAny && t == 3) return launch_fused_ws_t<0, 0, 4, 12, 4, 3>(ga, gb, counter, done, n, st);
-    if (kAny && t == 2) return launch_fused_ws_t<0, 0, 4, 12, 4, 2>(ga, gb, counter, done, n, st);
+    if (t == 4) return launch_fused_ws_t<4, 12, 4>(ga, gb, counter, done, n, st);
+    if (t == 3) return launch_fused_ws_t<4, 12, 4, 3>(ga, gb, counter, done, n, st);
+    if (t == 2) return launch_fused_ws_t<4, 12, 4, 2>(ga, gb, counter, done, n, st);
   }
   if (items <= 10 * sms && local_pairs <= E && ga.K % 256 == 0) {
-    if (gb.K % 256 == 0) return launch_fused_ws_t<kNA, kNB, 8, 8, 1>(ga, gb, counter, done, need + more, st);
-    if (kAny) return launch_fused_ws_t<0, 0, 8, 8, 1, 4>(ga, gb, counter, done, need + more, st);
+    if (gb.K % 256 == 0) return launch_fused_ws_t<8, 8, 1>(ga, gb, counter, done, need + more, st);
+    return launch_fused_ws_t<8, 8, 1, 4>(ga, gb, counter, done, need + more, st);
   }
   // items if the pairs fall on the experts at random
   const double hit = (double)E * (1.0 - std::exp(-(double)local_pairs / (double)E)) * (double)(ga.n_slabs * ((local_pairs + 8 * E - 1) / (8 * E)));
@@ -1746,11 +1740,11 @@ int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* d
   const double longer = (ga.K > 2048 ? ga.K / 2048.0 : 1.0) * (gb.K > 512 ? 2.0 : 1.0);
   if (!one_round && hit <= 22.0 * longer * sms) {
     const int t = turns(2), n = 2 * need + more;
-    if (t == 4) return launch_fused_ws_t<kNA, kNB, 4, 12, 2>(ga, gb, counter, done, n, st);
-    if (kAny && t == 3) return launch_fused_ws_t<0, 0, 4, 12, 2, 3>(ga, gb, counter, done, n, st);
-    if (kAny && t == 2) return launch_fused_ws_t<0, 0, 4, 12, 2, 2>(ga, gb, counter, done, n, st);
+    if (t == 4) return launch_fused_ws_t<4, 12, 2>(ga, gb, counter, done, n, st);
+    if (t == 3) return launch_fused_ws_t<4, 12, 2, 3>(ga, gb, counter, done, n, st);
+    if (t == 2) return launch_fused_ws_t<4, 12, 2, 2>(ga, gb, counter, done, n, st);
   }
-  return launch_fused_ws_t<kNA, kNB, 4, 16, 1>(ga, gb, counter, done, need + more, st);
+  return launch_fused_ws_t<4, 16, 1>(ga, gb, counter, done, need + more, st);
 }
 
 template <bool kScale8, bool kSilu>
@@ -2141,8 +2135,7 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
       GemvArgs gb = make_args(w2, plan, act, I, 1, down, B200FP4_DTYPE_F32, H, H, I, 0);
       ga.n_slabs = (int)(I / 64);
       gb.n_slabs = (int)(H / 128);
-      rc = (2 * I == 1024 && H == 2048) ? launch_fused_ws<1024, 2048>(ga, gb, plan.hdr + 2, done, local_pairs, E, st)
-                                        : launch_fused_ws<0, 0>(ga, gb, plan.hdr + 2, done, local_pairs, E, st);
+      rc = launch_fused_ws(ga, gb, plan.hdr + 2, done, local_pairs, E, st);
       if (rc != B200FP4_STATUS_SUCCESS) return rc;
       if (g_prof_events[1]) cudaEventRecord(g_prof_events[1], st);
     } else {
