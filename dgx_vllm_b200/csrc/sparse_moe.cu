@@ -1697,26 +1697,43 @@ int launch_fused_ws_t(const GemvArgs& ga, const GemvArgs& gb, int* counter, int*
   return B200FP4_STATUS_SUCCESS;
 }
 
-// Block shape of the one-launch layer by the number of gate_up items (expected passes if every expert is hit, times 64-column
-// groups).  Measured on B200, top-10, us per layer; the former K-sliced and 8 x 8 kernels in the last row:
-//   experts, H, I             512, 2048, 512                    128, 4096, 1024                16, 4096, 1024
-//   M                         8     16    32    64    128  256   8     32    64    128  256    8     32    64    128  256
-//   12 warps, four per item   34.2  50.2  75.3  109   140  159   73.4  124   140   206  348    32.1  55.3  88.1  159  300
-//    8 warps, one per item    33.0  47.0  67.9  96.6  125  142   72.9  118   130   189  312    40.5  57.7  93.2  142  262
-//   12 warps, two per item    34.6  49.8  67.9  96.1  125  141   80.2  120   128   189  312    33.8  54.7  79.5  137  255
-//   16 warps, one per item    35.6  49.5  67.2  102   120  134   95.1  125   133   195  306    46.7  66.3  86.1  159  247
-//   before                    43.2  65.6  68.4  97.2  125  142   95.9  119   133   189  320    54.5  66.4  95.2  144  267
-// Under three items an SM four warps share one; while single-pass items last about a round of the warps, eight warps with the
-// deepest rings stream best; in between two warps an item level the last round.  Sixteen warps need as many items as just fill
-// one round, 12 to 16 an SM of no more than K = 2048, or enough that the last round is short beside the rest: more than 22 an SM,
-// twice that where an item of either projection is twice as long (us with two warps per item / sixteen warps: 512 experts,
-// H=2048, I=512, M=28 62.9 / 64.8, M=32 70.5 / 68.6, M=40 80.2 / 79.3, M=48 84.1 / 93.6, M=80 112 / 112, M=96 124 / 120, M=112
-// 129 / 125; 256 experts, H=2048, I=1024, M=14 66.6 / 69.1, M=16 76.6 / 73.4, M=20 84.9 / 81.1, M=24 93.5 / 107, M=64 130 / 134,
-// M=96 141 / 145; 512 experts, H=1024, I=512, M=36 49.4 / 45.8).
+// Passes of eight tokens if the pairs fall on the experts at random (a Poisson number of pairs each): E times the sum over j of
+// P(more than 8 j pairs); with many pairs the remainders are even, which makes ceil(n / 8) n / 8 + 7 / 16 on average.
+double expected_passes(double pairs, double E) {
+  const double mean = pairs / E;
+  if (mean > 32.0) return E * (mean / 8.0 + 0.4375);
+  double p = std::exp(-mean), upto = 0.0, sum = 0.0;
+  for (int n = 0; n < 128 && upto < 1.0 - 1e-6; ++n) {
+    upto += p;
+    if (n % 8 == 0) sum += 1.0 - upto;
+    p *= mean / (n + 1);
+  }
+  return E * sum;
+}
+
+// Block shape of the one-launch layer by the items an SM is expected to get of either projection.  Four shapes, with 3, 6, 8 or
+// 16 items of an SM in work at a time; what decides is which of them has its last round of gate_up items nearly full:
+//   up to 3        12 warps, four per item (1.3 where a warp's quarter of K is under 16 steps of 32: what an item costs beside
+//                  its steps then counts for more than the shorter chain; H = 1024, I = 256, M = 8: 21.0 us against 18.4)
+//   6 to 7.75       8 warps, one per item, rings of eight stages (the count is an expectation: at 8 a second round is as likely)
+//   12 to 16       16 warps, one per item (long gate_up items, K over 2048: only beside down items of at most a sixth of their
+//                  length, whose last round is short too; 128 experts, 4096, 1024, M = 48: 133 us against 127 with two per item);
+//                  and from where the last rounds of both projections are short beside the rest
+//   otherwise      12 warps, two per item
+// Measured on B200, us per layer:
+//                    experts, H, I    512, 2048, 512                          256, 2048, 1024                 128, 4096, 1024
+//   M                                 1     8     16    32    64    128  256  4     16    32    64    256     8     24    64   256
+//   gate_up items an SM               0.5   4.0   7.4   12.9  19.8  25.4 29.4 4.0   12.9  19.8  25.4  46.9    6.4   11.7  14.7 40.7
+//   12 warps, four per item           15.9  35.5  52.2  77.6  114   143  171  34.6  77.7  105   133   236     73.9  117   152  366
+//   12 warps, two per item            19.0  35.5  51.3  70.1  99.2  125  145  35.3  77.4  97.3  122   200     81.5  112   137  310
+//    8 warps, one per item            24.8  34.7  48.5  69.9  100   126  146  37.7  76.2  99.9  124   204     72.8  118   139  320
+//   16 warps, one per item            27.0  37.4  51.2  69.4  107   123  137  40.2  75.2  115   130   184     95.3  119   139  299
+// Over 947 cases (H 1024 to 4096, I 256 to 1024, 16 to 512 experts, M 1 to 256) the shape this picks takes 0.6 % more than the best
+// of the four on average and 9 % at most; lines by counts that also grew with the widths took 1.6 and 20 %.
 int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* done, int64_t local_pairs, int64_t E, cudaStream_t st) {
-  const int64_t passes = (local_pairs < E ? local_pairs : E) * ((local_pairs + 8 * E - 1) / (8 * E));
-  const int64_t items = passes * ga.n_slabs, sms = sm_count();
   const int need = ga.n_slabs, more = g_wait_extra_need;       // per warp of an item: counts a pass's down items wait for
+  const double passes = expected_passes((double)local_pairs, (double)E) / sm_count();
+  const double up = passes * ga.n_slabs, down = passes * gb.n_slabs;
   // 32-wide steps per warp with the item shared by KS warps; whole turns of a 4-slot ring in the gate_up projection, of 4, 3 or
   // 2 slots in the down projection
   auto turns = [&](int KS) {
@@ -1724,21 +1741,18 @@ int launch_fused_ws(const GemvArgs& ga, const GemvArgs& gb, int* counter, int* d
     if (a % (4 * KS) != 0 || b % KS != 0) return 0;
     return b / KS % 4 == 0 ? 4 : (b / KS % 3 == 0 ? 3 : (b / KS % 2 == 0 ? 2 : 0));
   };
-  if (items <= 3 * sms) {
+  if (up <= (ga.K >= 4 * 16 * 32 ? 3.0 : 1.3)) {
     const int t = turns(4), n = 4 * need + more;
     if (t == 4) return launch_fused_ws_t<4, 12, 4>(ga, gb, counter, done, n, st);
     if (t == 3) return launch_fused_ws_t<4, 12, 4, 3>(ga, gb, counter, done, n, st);
     if (t == 2) return launch_fused_ws_t<4, 12, 4, 2>(ga, gb, counter, done, n, st);
   }
-  if (items <= 10 * sms && local_pairs <= E && ga.K % 256 == 0) {
+  if (up > 6.0 && up <= 7.75 && ga.K % 256 == 0) {
     if (gb.K % 256 == 0) return launch_fused_ws_t<8, 8, 1>(ga, gb, counter, done, need + more, st);
     return launch_fused_ws_t<8, 8, 1, 4>(ga, gb, counter, done, need + more, st);
   }
-  // items if the pairs fall on the experts at random
-  const double hit = (double)E * (1.0 - std::exp(-(double)local_pairs / (double)E)) * (double)(ga.n_slabs * ((local_pairs + 8 * E - 1) / (8 * E)));
-  const bool one_round = ga.K <= 2048 && local_pairs <= 4 * E && hit > 12.0 * sms && hit <= 16.0 * sms;
-  const double longer = (ga.K > 2048 ? ga.K / 2048.0 : 1.0) * (gb.K > 512 ? 2.0 : 1.0);
-  if (!one_round && hit <= 22.0 * longer * sms) {
+  const bool one_round = up > 12.0 && up <= 16.0 && (ga.K <= 2048 || 6 * gb.K <= ga.K);
+  if (!one_round && up + down / 7.0 <= 31.0) {
     const int t = turns(2), n = 2 * need + more;
     if (t == 4) return launch_fused_ws_t<4, 12, 2>(ga, gb, counter, done, n, st);
     if (t == 3) return launch_fused_ws_t<4, 12, 2, 3>(ga, gb, counter, done, n, st);

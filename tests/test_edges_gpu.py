@@ -79,18 +79,20 @@ def test_quantizer_tile_edges(M, K, swizzled, offset):
 
 
 @pytest.mark.parametrize("E,H,I,M,topk", [
-    (4, 256, 128, 1, 1),          # smallest: one item, K = 128 on the down side
+    (4, 256, 128, 1, 1),          # smallest: one item, K = 128 on the down side; two warps per item, down turns of two
     (8, 512, 512, 3, 4),          # four warps per item
     (16, 256, 256, 32, 8),        # 256 pairs: last size of the small plan; several passes per expert
     (16, 256, 256, 33, 8),        # 264 pairs
-    (128, 1024, 768, 25, 10),     # eight warps, one per item
-    (512, 512, 512, 64, 8),       # 12 warps, two per item
+    (128, 1024, 768, 25, 10),     # 12 warps, two per item, nine items an SM
+    (512, 512, 512, 64, 8),       # ... 17
     (256, 256, 512, 60, 10),      # 16 warps, items of about one round
     (8, 512, 384, 3, 4),          # four warps per item, down slices of three steps
     (8, 1024, 256, 3, 4),         # ... of two
-    (128, 512, 384, 40, 4),       # eight warps, down turns of four
-    (256, 512, 384, 64, 4),       # 12 warps, two per item, down turns of three
+    (128, 512, 384, 40, 4),       # 12 warps, two per item, down turns of three
+    (256, 512, 384, 64, 4),       # eight warps, one per item, down turns of four
+    (256, 512, 512, 25, 8),       # ... of eight
     (8, 384, 128, 200, 4),        # 16 warps, one per item: K no multiple of 256, many pairs per expert
+    (64, 512, 1024, 256, 10),     # 16 warps, many items of several passes per expert
 ])
 def test_fused_moe_block_shapes(E, H, I, M, topk):
     import synth
