@@ -914,7 +914,7 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
 // 64-wide k-blocks per shared-memory stage.  The kernel template also builds with 2 or 1 (64- and
 // 32-byte swizzled rows, 8 or 16 stages); on B200 those measured 190 and 317 us against 150 us at
 // M=4096 (TMA issues one request per box row, so narrower rows double and quadruple the requests).
-int stage_kblocks() { return 4; }
+constexpr int kStageKb = 4;
 
 // Tile of the dense GEMM: 128- or 256-wide on single CTAs (one per SM), 256 x 256 on CTA pairs, and for few tiles the split of K
 // over clusters of two or four.  Each takes whole rounds over the SMs, so the choice is the least of
@@ -941,11 +941,10 @@ void pick_dense_tile(int64_t M, int64_t N, int64_t stages, bool f32, int& bn, in
 }
 
 template <bool kGrouped>
-int dispatch_gemm(int bn, int kb, const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int max_m_tiles,
-                  cudaStream_t st, const CUtensorMap* mo = nullptr) {
-  (void)kb;
-  if (bn == 256) return launch_gemm<256, 4, kGrouped>(ma, mb, p, max_m_tiles, st, mo);
-  return launch_gemm<128, 4, kGrouped>(ma, mb, p, max_m_tiles, st);
+int dispatch_gemm(int bn, const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int max_m_tiles, cudaStream_t st,
+                  const CUtensorMap* mo = nullptr) {
+  if (bn == 256) return launch_gemm<256, kStageKb, kGrouped>(ma, mb, p, max_m_tiles, st, mo);
+  return launch_gemm<128, kStageKb, kGrouped>(ma, mb, p, max_m_tiles, st);
 }
 
 }  // namespace
@@ -997,7 +996,6 @@ static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa,
   p.early_b = early_b;
   int bn = tile_n, split = 1;
   if (bn == 0) pick_dense_tile(M, N, (K + 255) / 256, p.out_f32 != 0, bn, split);
-  const int kb = stage_kblocks();
   if (bn == 512) {
     // 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2)
     CUtensorMap pa, pb;
@@ -1009,8 +1007,8 @@ static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa,
     return finish_launch(1);
   }
   CUtensorMap ma, mb;
-  if (!make_map(&ma, a_codes, (uint64_t)M, (uint64_t)K / 2, kBM, kb * 32) ||
-      !make_map(&mb, b_codes, (uint64_t)N, (uint64_t)K / 2, (uint32_t)bn, kb * 32))
+  if (!make_map(&ma, a_codes, (uint64_t)M, (uint64_t)K / 2, kBM, kStageKb * 32) ||
+      !make_map(&mb, b_codes, (uint64_t)N, (uint64_t)K / 2, (uint32_t)bn, kStageKb * 32))
     return B200FP4_STATUS_INTERNAL_ERROR;
   p.g_hdr = nullptr;
   p.g_mtiles = nullptr;
@@ -1020,9 +1018,9 @@ static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa,
   CUtensorMap mo;
   const bool tma_out = bn == 256 && !p.out_f32 && (N % 8) == 0 && make_out_map(&mo, out, (uint64_t)M, (uint64_t)N);
   p.out_tma = tma_out ? 1 : 0;
-  int rc = split == 4   ? launch_gemm<128, 4, false, false, 4>(ma, mb, p, p.m_tiles, st)
-           : split == 2 ? launch_gemm<128, 4, false, false, 2>(ma, mb, p, p.m_tiles, st)
-                        : dispatch_gemm<false>(bn, kb, ma, mb, p, p.m_tiles, st, tma_out ? &mo : nullptr);
+  int rc = split == 4   ? launch_gemm<128, kStageKb, false, false, 4>(ma, mb, p, p.m_tiles, st)
+           : split == 2 ? launch_gemm<128, kStageKb, false, false, 2>(ma, mb, p, p.m_tiles, st)
+                        : dispatch_gemm<false>(bn, ma, mb, p, p.m_tiles, st, tma_out ? &mo : nullptr);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   return finish_launch(1);
 }
@@ -1142,17 +1140,16 @@ int grouped_gemm(const void* a_codes, const void* b_codes, const void* a_sf, con
     bn = (N % 256 == 0 && (K >= 2048 || wide_tiles >= 4LL * sm_count())) ? 256 : 128;
   }
   if (fused) bn = 256;
-  const int kb = stage_kblocks();
   CUtensorMap ma, mb;
-  if (!make_map(&ma, a_codes, (uint64_t)rows_capacity, (uint64_t)K / 2, kBM, kb * 32) ||
-      !make_map(&mb, b_codes, (uint64_t)(E * N), (uint64_t)K / 2, fused ? 128u : (uint32_t)bn, kb * 32))
+  if (!make_map(&ma, a_codes, (uint64_t)rows_capacity, (uint64_t)K / 2, kBM, kStageKb * 32) ||
+      !make_map(&mb, b_codes, (uint64_t)(E * N), (uint64_t)K / 2, fused ? 128u : (uint32_t)bn, kStageKb * 32))
     return B200FP4_STATUS_INTERNAL_ERROR;
   if (!tiles_ready)
     grouped_tiles_kernel<<<1, 1024, 0, st>>>(expert_offsets, sf_offsets, (int)E, grouped_hdr(workspace), grouped_tiles(workspace),
                                              max_tiles);
-  int rc = stage_sf ? launch_gemm<256, 4, true, true, 1, true>(ma, mb, p, max_tiles, st)
-           : fused  ? launch_gemm<256, 4, true, true>(ma, mb, p, max_tiles, st)
-                    : dispatch_gemm<true>(bn, kb, ma, mb, p, max_tiles, st);
+  int rc = stage_sf ? launch_gemm<256, kStageKb, true, true, 1, true>(ma, mb, p, max_tiles, st)
+           : fused  ? launch_gemm<256, kStageKb, true, true>(ma, mb, p, max_tiles, st)
+                    : dispatch_gemm<true>(bn, ma, mb, p, max_tiles, st);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   return finish_launch(tiles_ready ? 1 : 2);
 }

@@ -109,11 +109,6 @@ __device__ __forceinline__ void cluster_sync_any() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
 
 // 32 bytes (eight 32-bit registers) to a 32-byte aligned global address in one instruction
 __device__ __forceinline__ void st_global_v8(void* dst, const uint32_t* r) {

@@ -63,10 +63,6 @@ __device__ __forceinline__ void cp_async16_s(uint32_t smem_dst, const void* gmem
   asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(smem_dst), "l"(gmem_src) : "memory");
 }
 
-__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 template <int SEL>
 __device__ __forceinline__ void mma_sp_m16n8k32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                 const uint32_t (&b)[4], uint32_t e) {
@@ -98,10 +94,7 @@ __device__ __forceinline__ __half2 e4m3x2_to_h2(uint32_t w) {
 
 constexpr int kWsStages = 4;
 constexpr int kWsWarps = 16;
-constexpr int kWsThreads = 32 * kWsWarps;
 constexpr int kWsStageBytes = 14 * 128 + 512;     // 8 compressed + 4 metadata + 2 scale rows of 128 bytes, B fragments of 8 tokens
-constexpr size_t kWsSmemBytes = (size_t)kWsWarps * kWsStages * kWsStageBytes + 128;
-// (warps per block = 64 / stages, so both shapes use the same shared memory)
 
 // Lane-constant shared-memory offsets of the warp-scheduled kernel.
 // Stage layout: compressed rows 0..7 | metadata rows 0..3 | scale rows 0..1 (128 bytes each) | B fragments.  The 16-byte

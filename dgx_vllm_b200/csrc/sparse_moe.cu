@@ -1640,7 +1640,7 @@ bool ws_ok(int64_t N, int64_t K, int64_t G, int64_t inter_silu, const SparseWeig
 // Opt a kernel in to the large dynamic shared memory, once per device; `attr_set` belongs to the caller, one array per
 // kernel instantiation (instantiations share their function type, so a static in here would be shared between them).
 template <typename Kernel>
-bool ws_prepare(Kernel kernel, bool* attr_set, size_t smem_bytes = kWsSmemBytes) {
+bool ws_prepare(Kernel kernel, bool* attr_set, size_t smem_bytes) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return false;
@@ -1652,12 +1652,6 @@ bool ws_prepare(Kernel kernel, bool* attr_set, size_t smem_bytes = kWsSmemBytes)
     attr_set[dev] = true;
   }
   return true;
-}
-
-int64_t ws_grid(int64_t max_items) {
-  int64_t grid = (max_items + kWsWarps - 1) / kWsWarps;
-  if (grid > (int64_t)sm_count()) grid = sm_count();
-  return grid < 1 ? 1 : grid;
 }
 
 template <bool kSilu, int kS = kWsStages, int kW = kWsWarps>
