@@ -37,9 +37,9 @@ E_TOTAL, HIDDEN, INTER, TOPK = 512, 2048, 512, 10
 BYTES_PER_EXPERT_GATE_UP = 2 * INTER * HIDDEN * 7 // 16          # comp 1/4 + meta 1/8 + scale 1/16 B per weight
 BYTES_PER_EXPERT_DOWN = HIDDEN * INTER * 7 // 16
 N_ROUTINGS = 8
-# dram__bytes_read.sum + dram__bytes_write.sum of the gate_up and down GEMV launches of one layer, per routed expert,
-# from the ncu capture whose summary is committed with the profiles (244 routed experts: 233.61 MB + 118.83 MB)
-NCU_TRAFFIC_BYTES_PER_EXPERT = (323.90e6 + 4.31e6) / 244.0
+# dram__bytes_read.sum + dram__bytes_write.sum of the layer's one GEMV launch (gate_up and down), per routed expert, from the
+# ncu capture whose summary is committed with the profiles (244 routed experts: 323.66 MB read, 4.01 MB written)
+NCU_TRAFFIC_BYTES_PER_EXPERT = (323.66e6 + 4.01e6) / 244.0
 NCU_TRAFFIC_SOURCE = "ncu capture of the one-launch GEMV kernel (batch 32, 244 routed experts), scaled by routed experts"
 
 
@@ -452,7 +452,7 @@ def bench_moe_prefill(dev, flush, hbm_peak, steps: int = 5):
     wbytes = E * (2 * I * H + H * I) * 0.5625
     return {"tokens_per_s": T / t, "ms": t * 1e3, "tflops": flops / t / 1e12, "weight_GBps": wbytes / t / 1e9,
             "frac_of_measured_hbm_weights_only": wbytes / t / 1e9 / hbm_peak, "gemm_status": status,
-            "config": "8192 tokens, 512 experts, Zipf(1.1) top-10, dense NVFP4 experts, grouped path, 10 kernel launches"}
+            "config": "8192 tokens, 512 experts, Zipf(1.1) top-10, dense NVFP4 experts, grouped path, 5 kernel launches"}
 
 
 def bench_decode_stack(dev, batches=(1, 32, 128), layers: int = 48, distinct_layers: int = 4, reps: int = 5):
@@ -944,8 +944,7 @@ def main():
         layer.phase_events = None
         L.b200fp4_fused_moe_profile_events(0, 0, 0)
     torch.cuda.synchronize()
-    # events 0 -> 2 bracket the two projections of the layer's default path (two launches at this batch
-    # size; one cooperative launch up to 256 pairs)
+    # events 0 -> 2 bracket the two projections of the layer's default path (one launch)
     t_both = [evs[i][0].elapsed_time(evs[i][2]) * 1e-3 for i in range(args.steps)]
     # per-projection times: the same layer with one launch per projection (a few steps, cold L2)
     k4 = ("comp_T", "meta_T", "scale_T", "g_scales")

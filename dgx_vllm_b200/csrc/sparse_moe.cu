@@ -962,27 +962,28 @@ __global__ void __launch_bounds__(kMmaThreads, 1) sparse_gemv_mma_kernel(const G
 // The same arithmetic as gemv_mma_phase (mma.sp m16n8k32, hardware E2M1 / E4M3 decode), organised so that a warp
 // never has to meet another warp:
 //   * a work item is (pass of up to eight tokens, group of 128 output columns) over the WHOLE K, owned by one warp:
-//     no K-slices, so no partial sums in shared memory, no block-wide barrier and no block-wide epilogue;
+//     no K-slices, so no partial sums in shared memory, no block-wide barrier and no block-wide epilogue (in the layer's
+//     one launch two or four warps share an item where items are few, see KS below);
 //   * warps take items from a global counter (atomicAdd by lane 0), always holding the next item while they
 //     compute the current one, so the tail of the launch is at most one item long whatever the routing;
 //   * the activations are not staged per block: the plan kernel (or the gate_up epilogue) leaves them in
 //     "fragment order" (see kConv*), and each lane copies the 16 bytes that are its own B-operand registers for a
 //     k-step asynchronously into its ring stage, next to the weights of that step;
 //   * a ring stage is one 32-wide k-step: 8 compressed rows, 4 metadata rows and 2 scale rows of 128 columns
-//     (1792 bytes) + 512 bytes of B fragments.  Four stages per warp; the copy for step j+4 is issued into the slot
-//     of step j as soon as step j's shared-memory reads are done, so that four steps are in flight per warp and the
-//     slot of every step is a compile-time constant in the loop unrolled by four (K is a multiple of 128).  The
+//     (1792 bytes) + 512 bytes of B fragments.  kS stages per warp (four or eight); the copy for step j+kS is issued into
+//     the slot of step j as soon as step j's shared-memory reads are done, so that kS steps are in flight per warp and the
+//     slot of every step is a compile-time constant in the loop unrolled by kS (a warp's share of K is whole turns).  The
 //     stream runs across item boundaries.
 //   * 16-byte chunks are XOR-swizzled inside the compressed and metadata rows so that the fragment loads
 //     (rows t and t+4 for lane t of a quad; metadata rows 2(t%2), 2(t%2)+1) touch every bank once.
 // Epilogue from registers: the lane that holds 16 consecutive columns of a token writes them with 16-byte stores;
 // with SiLU the warp's 128 columns are 64 gate + the matching 64 up columns, the two halves of the warp swap one
 // token's values through shuffles, and SiLU(gate)*up leaves in fragment order for the down projection.
-// Two shapes of the same ring budget: 8 warps x 8 stages per block (the default where K is a multiple of 256: two warps
-// per scheduler, each with twice the bytes in flight, measured faster at every batch size tried), or 16 warps x 4 stages.
+// Which blocks and rings: see launch_fused_ws for the layer; a stand-alone projection takes 8 warps x 8 stages where K is a
+// multiple of 256, else 16 warps x 4 stages.
 // One projection for this warp: the items [base, base + passes * groups) of the claim sequence that `counter` hands out.
-// `first` is an index this warp has already claimed; the return value is the first index it claimed that lies past
-// this projection (the caller passes it on to the next one).
+// `claims` holds the index this warp (or its unit) has already claimed and, with KS > 1, the one after it; on return the first
+// ones it claimed that lie past this projection, which the caller passes on to the next one.
 // kDep links the two projections of the MoE layer when they run in one launch: 1 = producer (done[pass] counts the
 // finished items of a pass, fenced), 2 = consumer (the B fragments of an item -- the activations the producer wrote
 // for that pass -- are fetched only once done[pass] has reached `need`), 0 = stand-alone.
