@@ -2,9 +2,9 @@
 //
 // Why pairs: a single CTA's MMA (128 x 256 x 64) reads 4 KiB of A and 8 KiB of B from shared memory and issues at about
 // 206 cycles per MMA.  In a pair each CTA holds its own 128 rows of A and HALF of the B tile (128 of the 256 rows): 8 KiB
-// per CTA per MMA for the same work per SM, and a third fewer operand bytes from L2.  Measured: a 256 x 256 x 64 MMA of
-// the pair issues every 176 cycles; M=4096, N=14336, K=4096 takes about 200 k cycles against 223 k for the single-CTA
-// kernel (123 us against 129 us: the SM clock settles near 1.6-1.7 GHz under either).
+// per CTA per MMA for the same work per SM, and a third fewer operand bytes from L2.  Measured with the same stage loop in
+// both: M=4096, N=14336, K=4096 takes about 200 k cycles against 223 k for the single-CTA kernel (123 us against 129 us: the SM
+// clock settles near 1.6-1.7 GHz under either); with the shorter loop below 189 k cycles, 113 us.
 //
 // Roles per CTA (23 warps): warp 0 loads operands, warp 1 issues the MMAs (leader CTA only) and owns tensor memory,
 // warps 2-5, 10-13 and 15-22 drain and store the CTA's 128 accumulator rows (four warps per tensor-memory lane quarter, 64
