@@ -685,8 +685,8 @@ def verify_layer_step(layer, batch0, w13, w2, world, rank, dev, n_tok: int = 4):
 def bench_ep_local_call(dev, flush, hbm_peak, ranks: int = 8, batch: int = 32, steps: int = 20):
     """What ONE rank of an expert-parallel group of `ranks` GPUs runs per step, on this GPU alone: the fused layer over
     the ranks*batch tokens of all ranks with only E_TOTAL/ranks experts resident (`expert_map` masks the others).  No
-    exchange: this isolates the local layer, whose GEMV launch has few items per SM and takes the 8-warp x 8-stage
-    shape of the warp-scheduled kernel.  Cold L2, CUDA events from the library's benchmark hook."""
+    exchange: this isolates the local layer, whose GEMV launch has few items per SM (two warps share each).  Cold L2, CUDA
+    events from the library's benchmark hook."""
     import torch
     import synth
     from dgx_vllm_b200 import _lib, scaled_fp4_quant, sparse_fp4_v7 as sp7

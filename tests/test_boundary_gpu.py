@@ -113,7 +113,7 @@ def test_reference_patch_module_runs_on_this_library():
 
 
 def test_fused_layer_wait_that_runs_out_sets_the_status_word_and_returns():
-    # one-launch layer (<= 256 pairs): with one more finished gate_up item asked for than a pass ever has, and a
+    # one-launch layer: with one more finished gate_up item asked for than a pass ever has, and a
     # budget of ~50 us, the first wait gives up, records the status and every later wait is skipped; the kernel
     # returns and the context stays usable.  Nothing is in flight when a wait gives up (a plain counter poll).
     import synth

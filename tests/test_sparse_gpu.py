@@ -249,10 +249,10 @@ def test_metadata_ordered_check():
 
 
 @pytest.mark.parametrize("E,N,K,P,dtype", [
-    (4, 512, 128, 9, torch.float16),          # plain slab of 4 column groups, two steps per K-slice
-    (3, 1024, 2048, 17, torch.bfloat16),      # several slabs, experts with more than four tokens (two passes)
-    (5, 256, 512, 6, torch.bfloat16),         # N only allows two column groups
-    (2, 128, 1024, 5, torch.float16),         # N only allows one column group
+    (4, 512, 128, 9, torch.float16),          # 16 warps with rings of four, one turn of the ring per item
+    (3, 1024, 2048, 17, torch.bfloat16),      # eight warps with rings of eight, experts with several tokens
+    (5, 256, 512, 6, torch.bfloat16),         # two column groups
+    (2, 128, 1024, 5, torch.float16),         # one column group
     (70, 512, 256, 300, torch.bfloat16),      # more items than SMs: every block walks several items
 ])
 def test_batched_sparse_v7_tensor_core_path(E, N, K, P, dtype):
@@ -362,7 +362,14 @@ def test_bound_layer_queued_host_steps_match_device_call(overlap, direct):
 @pytest.mark.parametrize("M,topk,E,H,I,separate", [
     (64, 8, 16, 2048, 512, False),      # 32 tokens per expert on average: eight-token passes, one launch
     (64, 8, 16, 2048, 512, True),       # ... and one launch per projection
-    (48, 6, 8, 1024, 256, False),       # shapes that take other slab widths
+    (48, 6, 8, 1024, 256, False),       # other widths
+    # one launch per projection up to 256 pairs: the K-sliced kernel, its column groups by the widths and the number of passes
+    (5, 4, 16, 512, 256, True),         # four-token passes; two column groups, and four for the down projection
+    (1, 2, 8, 2048, 512, True),         # ... one column group in gate_up, few items
+    (30, 8, 64, 2048, 512, True),       # ... more items than SMs
+    (32, 8, 16, 2048, 512, True),       # eight-token passes, 256 pairs
+    (48, 4, 8, 1024, 256, True),        # ... several passes per expert
+    (21, 6, 8, 4096, 128, True),        # four-token passes; K = 128 on the down side goes to the general kernel
 ])
 def test_fused_moe_eight_token_passes(M, topk, E, H, I, separate):
     from dgx_vllm_b200 import sparse_fp4_v7 as sp7

@@ -72,7 +72,7 @@ def test_a_full_queue_does_not_stop_other_threads(name):
         t.join()
         torch.cuda.synchronize()
     assert waited > 0.4, "the queue never filled"
-    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.25
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.5 * waited        # the GIL held: as long as the wait
 
 
 def test_two_threads_on_one_stream_keep_their_calls_apart():
