@@ -23,6 +23,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "gemm_small.cuh"
 #include "grouped.cuh"
 #include "sm100_ptx.cuh"
 
@@ -983,6 +984,15 @@ static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa,
   if (refused != B200FP4_STATUS_SUCCESS || M == 0) return refused;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
   cudaStream_t st = (cudaStream_t)stream;
+  if (tile_n == 0) {
+    const SmallPlan small = small_gemm_plan(M, N, K);
+    CUtensorMap mw;
+    if (small.ok) {
+      if (!make_map(&mw, b_codes, (uint64_t)N, (uint64_t)K / 2, kBM, kStageKb * 32)) return B200FP4_STATUS_INTERNAL_ERROR;
+      return launch_gemm_small(small, mw, a_codes, 0, K, nullptr, reinterpret_cast<const uint8_t*>(sfa), reinterpret_cast<const uint8_t*>(sfb),
+                               alpha, out, out_dtype, (int)M, (int)N, (int)K, reinterpret_cast<int*>(workspace), st);
+    }
+  }
   GemmParams p;
   p.sfa = reinterpret_cast<const uint8_t*>(sfa);
   p.sfb = reinterpret_cast<const uint8_t*>(sfb);
@@ -1061,6 +1071,14 @@ extern "C" int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, con
     rc = dense_gemm_check(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, gemm_bytes);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
+  const SmallPlan small = small_gemm_plan(M, N, K);
+  if (tile_n == 0 && small.ok) {
+    // few tokens: quantized inside the GEMM
+    CUtensorMap mw;
+    if (!make_map(&mw, w_codes, (uint64_t)N, (uint64_t)K / 2, kBM, kStageKb * 32)) return B200FP4_STATUS_INTERNAL_ERROR;
+    return launch_gemm_small(small, mw, x, x_dtype, ldx, x_global_scale, nullptr, reinterpret_cast<const uint8_t*>(w_sf), alpha, out, out_dtype,
+                             (int)M, (int)N, (int)K, reinterpret_cast<int*>(gemm_ws), (cudaStream_t)stream);
+  }
   rc = b200fp4_quantize(x, x_dtype, M, K, ldx, x_global_scale, codes, sf, 1, stream);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   // The quantizer lets the GEMM start only after it has waited for everything before it: whatever wrote the weights is done.

@@ -10,6 +10,7 @@
 // cvt.rn.satfinite.e2m1x2.f32 that replaces the reference's software routine
 // (patch_nvfp4_utils_sw_e2m1.py:31-63).
 #include "grouped.cuh"
+#include "quant.cuh"
 
 namespace b200fp4 {
 
@@ -20,64 +21,6 @@ namespace {
 constexpr int kTX = 64;    // threads along K (each 8 elements): 512 elements per block row
 constexpr int kTY = 4;     // rows per block per pass
 constexpr int kRows = 4;   // passes (rows) per thread, loads issued together
-
-// Packed helpers on two 16-bit floats in one register.
-template <typename T>
-struct Pk;
-template <>
-struct Pk<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
-    const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
-  static __device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
-  static __device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-};
-template <>
-struct Pk<__half> {
-  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
-    const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
-  static __device__ __forceinline__ float lo(uint32_t w) { return __low2float(*reinterpret_cast<const __half2*>(&w)); }
-  static __device__ __forceinline__ float hi(uint32_t w) { return __high2float(*reinterpret_cast<const __half2*>(&w)); }
-};
-
-template <typename T>
-__device__ __forceinline__ void unpack8(const uint4& raw, float* v) {
-  v[0] = Pk<T>::lo(raw.x); v[1] = Pk<T>::hi(raw.x); v[2] = Pk<T>::lo(raw.y); v[3] = Pk<T>::hi(raw.y);
-  v[4] = Pk<T>::lo(raw.z); v[5] = Pk<T>::hi(raw.z); v[6] = Pk<T>::lo(raw.w); v[7] = Pk<T>::hi(raw.w);
-}
-
-// max |x| over the 8 packed values (exact: the maximum of 16-bit floats is one of them)
-template <typename T>
-__device__ __forceinline__ float amax8(const uint4& raw) {
-  const uint32_t m = 0x7FFF7FFFu;
-  const uint32_t w = Pk<T>::max2(Pk<T>::max2(raw.x & m, raw.y & m), Pk<T>::max2(raw.z & m, raw.w & m));
-  return fmaxf(Pk<T>::lo(w), Pk<T>::hi(w));
-}
-
-// 32 bytes in one load
-__device__ __forceinline__ void ldg_stream_v8(const void* p, uint4& a, uint4& b) {
-  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-               : "l"(p));
-}
-
-// Quantizes one block of 16 with the scale byte's exact arithmetic: codes and scale byte.
-template <typename T>
-__device__ __forceinline__ uint2 quantize_block16(const uint4& r0, const uint4& r1, float gs, float rcp_gs, uint32_t& sfb) {
-  const float amax = fmaxf(amax8<T>(r0), amax8<T>(r1));
-  sfb = f32_to_e4m3(fminf(__fmul_rn(gs, __fmul_rn(amax, 0.16666667163372039794921875f)), 448.f));    // fl32(1/6)
-  const float os = out_scale_of((uint8_t)sfb, rcp_gs);
-  float v[16];
-  unpack8<T>(r0, v);
-  unpack8<T>(r1, v + 8);
-  return make_uint2(f32x8_to_e2m1(__fmul_rn(v[0], os), __fmul_rn(v[1], os), __fmul_rn(v[2], os), __fmul_rn(v[3], os),
-                                  __fmul_rn(v[4], os), __fmul_rn(v[5], os), __fmul_rn(v[6], os), __fmul_rn(v[7], os)),
-                    f32x8_to_e2m1(__fmul_rn(v[8], os), __fmul_rn(v[9], os), __fmul_rn(v[10], os), __fmul_rn(v[11], os),
-                                  __fmul_rn(v[12], os), __fmul_rn(v[13], os), __fmul_rn(v[14], os), __fmul_rn(v[15], os)));
-}
 
 // One global scale for the tensor.  Bound by HBM (2.5625 bytes per element); what it takes to get near that:
 //   * a thread owns whole blocks of 16 (32-byte loads, no shuffle for the maximum, the scale arithmetic once per block and no
@@ -124,7 +67,7 @@ __global__ void __launch_bounds__(kQrThreads, 4)
     const int64_t m = m0 + 32 * i;
     const bool ok = col_ok && m < M;
     uint32_t sfb;
-    const uint2 c = quantize_block16<T>(r0[i], r1[i], gs, rcp_gs, sfb);
+    const uint2 c = quantize_block16<T>(r0[i], r1[i], gs, [&](uint32_t b) { return out_scale_of((uint8_t)b, rcp_gs); }, sfb);
     if (!ok) sfb = 0;
     if (ok) {
       uint8_t* dst = codes + (m * KB + kb) * 8;

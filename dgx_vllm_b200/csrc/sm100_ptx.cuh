@@ -66,6 +66,35 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
   return true;
 }
 
+// The same by a whole warp, which stays together: true for all lanes or for none.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) {
+      atomicCAS(status, 0, code);
+      return false;
+    }
+  }
+  return true;
+}
+
+// One lane of a warp that is together: the copies, MMAs and commits of a loop are issued under this predicate, the loop and its
+// waits run by all lanes.  A loop entered by one lane only (if (lane == 0)) costs the issuing warp twice the time: the operands of these
+// instructions are uniform registers, which the compiler fills by a vote over the active lanes wherever it does not know that
+// the warp is together (a stage of wait, fence, four MMAs and a commit: 460 cycles so, 250-270 with the warp together; B200).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(e));
+  return e != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),

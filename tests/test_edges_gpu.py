@@ -245,3 +245,42 @@ def test_prefill_layer_equals_its_steps(M, E, topk, H, I, dtype):
     rows = c2.float()[c_map.long()].view(M, topk, H)
     ref = (rows * tw[..., None]).sum(1)
     assert torch.allclose(out.float(), ref, rtol=1e-2, atol=1e-3 * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 128, 64),              # one tile, one short stage, one column of the narrowest MMA
+    (8, 512, 2048),            # a stage to each of the eight CTAs of a cluster
+    (9, 130, 2112),            # N past the tile, nine stages on eight CTAs, the last one short
+    (16, 14336, 4096),         # K not split, more stages than the ring holds; the most blocks a CTA quantizes
+    (17, 1000, 1280),          # five stages on five CTAs
+    (31, 2056, 1536),          # clusters of six
+    (33, 6400, 768),           # a second word of activation scales
+    (39, 392, 5120),           # two or three stages to a CTA, tokens not a multiple of the cluster
+    (64, 1024, 4096),          # the most tokens
+    (1, 18937, 576),           # as many tiles as SMs
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_few_token_linear(M, N, K, dtype):
+    # the kernel that quantizes its own operand: the same bytes as on codes made before, and the exact product of those codes within
+    # one rounding to 16 bits (7 or 10 stored bits: half a unit in the last place is 2^-8 or 2^-11 of the value) and the f32 sum over K
+    from dgx_vllm_b200 import _lib, cutlass_scaled_fp4_mm, scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status, nvfp4_linear
+    x, gx, wc, ws, alpha = _linear_operands(M, N, K, M + N)
+    x = x.to(dtype)
+    n0 = _lib.lib().b200fp4_launch_count()
+    out = nvfp4_linear(x, gx, wc, ws, alpha)
+    assert _lib.lib().b200fp4_launch_count() == n0 + 1 and last_gemm_status() == 0
+    wide = torch.zeros(M, K + 8, dtype=dtype, device="cuda")          # rows that are 16-byte, not 32-byte aligned
+    wide[:, :K] = x
+    assert torch.equal(nvfp4_linear(wide[:, :K], gx, wc, ws, alpha), out)
+    xc, xs = scaled_fp4_quant(x, gx)
+    assert torch.equal(cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype), out)
+
+    def deq(codes, sf, rows):
+        lin = oracle.sf_swizzled_to_linear(to_np(sf.view(torch.uint8)).reshape(-1), rows, K // 16)
+        return torch.from_numpy(oracle.dequantize(to_np(codes), lin, 1.0)).cuda().double()
+
+    a, b = deq(xc, xs, M), deq(wc, ws, N)
+    ref, size = (a @ b.t()) * alpha.double(), (a.abs() @ b.abs().t()) * alpha.double()
+    half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert bool(((out.double() - ref).abs() <= half_ulp * ref.abs() + 2.0 ** -20 * size + 2.0 ** -24).all())
