@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   // The weights of a linear layer do not depend on the quantizer that runs just before: the first ring of B and its scales is
   // requested while that kernel still runs (N=14336, K=4096: M=1 14.4 -> 13.2 us, M=32 13.4 -> 12.1, M=128 13.4 -> 12.7).
   int early = 0;
-  if (!kGrouped && p.early_b && lane == 0 && (warp == 0 || warp == kWarpSf) && first_tile < p.m_tiles * p.n_tiles) {
+  if (!kGrouped && p.early_b && (warp == 0 || warp == kWarpSf) && first_tile < p.m_tiles * p.n_tiles) {
+    const bool elected = elect_one();
     const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, first_tile, p.m_tiles);
     const uint8_t* sfb0 = p.sfb + (size_t)ti.sfb_tile0 * KT * 512;
     const uint8_t* sfb1 = p.sfb + (size_t)ti.sfb_tile1 * KT * 512;
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     for (int s = 0; s < early; ++s) {
       const int ks = ks_begin + s;
       const uint32_t st = smem_u32(smem) + s * C::kStageBytes, sbar = smem_u32(&sf_full[s]), bar = smem_u32(&full_bar[s]);
+      if (!elected) continue;
       if (warp == 0) {
         mbar_expect_tx(bar, (uint32_t)(C::kStageA + C::kStageB));
         tma_load_2d(st + C::kStageA, &map_b, ks * C::kRowBytes, ti.b_row0, bar);
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         if (sf_tiles > 1) bulk_load_1d(dst + C::kStageSFA + KB * 512, sfb1 + off, bytes, sbar);
       }
     }
+    __syncwarp();
   }
   pdl_wait();                 // everything above overlaps the end of the kernel before this one
   pdl_launch_dependents();
@@ -347,21 +350,23 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
 
   if (warp == 0 || warp == kWarpSf) {
     // ------------------------------------------------------------------ copies into shared memory: operands, scale factors
-    if (lane == 0) {
-      uint32_t s = 0, ph = 0;
-      bool ok = true;
-      for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride) {
-        const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, tile, m_tiles);
-        const uint8_t* sfa = p.sfa + (size_t)ti.sfa_tile * (kStageSf ? p.k_stages * KB : KT) * 512;
-        const uint8_t* sfb = p.sfb + (kGrouped ? (size_t)ti.expert * (size_t)p.g_sfb_expert_bytes : (size_t)0);
-        const uint8_t* sfb0 = sfb + (size_t)ti.sfb_tile0 * KT * 512;
-        const uint8_t* sfb1 = sfb + (size_t)ti.sfb_tile1 * KT * 512;
-        const int sf_tiles = C::kSfTiles == 1 || ti.sfb_tile1 * 128 >= p.N ? 1 : 2;      // the second 128 columns may lie past N
-        for (int ks = ks_begin; ks < ks_end; ++ks) {
-          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, p.status, 1)) { ok = false; break; }
+    const bool elected = elect_one();
+    uint32_t s = 0, ph = 0;
+    bool ok = true;
+    for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride) {
+      const TileInfo ti = tile_info<BN, kGrouped, kSiluQuant>(p, tile, m_tiles);
+      const uint8_t* sfa = p.sfa + (size_t)ti.sfa_tile * (kStageSf ? p.k_stages * KB : KT) * 512;
+      const uint8_t* sfb = p.sfb + (kGrouped ? (size_t)ti.expert * (size_t)p.g_sfb_expert_bytes : (size_t)0);
+      const uint8_t* sfb0 = sfb + (size_t)ti.sfb_tile0 * KT * 512;
+      const uint8_t* sfb1 = sfb + (size_t)ti.sfb_tile1 * KT * 512;
+      const int sf_tiles = C::kSfTiles == 1 || ti.sfb_tile1 * 128 >= p.N ? 1 : 2;      // the second 128 columns may lie past N
+      for (int ks = ks_begin; ks < ks_end; ++ks) {
+        ok = mbar_wait_warp(smem_u32(&empty_bar[s]), ph ^ 1, p.status, 1);
+        if (!ok) break;
+        const bool b_requested = !kGrouped && early > 0;
+        if (!kGrouped) --early;
+        if (elected) {
           const uint32_t st = smem_u32(smem) + s * C::kStageBytes, bar = smem_u32(&full_bar[s]);
-          const bool b_requested = !kGrouped && early > 0;
-          if (!kGrouped) --early;
           if (warp == 0) {
             if (!b_requested) mbar_expect_tx(bar, (uint32_t)(C::kStageA + C::kStageB));
             tma_load_2d(st, &map_a, ks * C::kRowBytes, ti.a_row0, bar);
@@ -381,55 +386,51 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
               if (sf_tiles > 1) bulk_load_1d(dst + C::kStageSFA + KB * 512, sfb1 + off, bytes, sbar);
             }
           }
-          if (++s == C::kStages) {
-            s = 0;
-            ph ^= 1;
-          }
+        }
+        __syncwarp();
+        if (++s == C::kStages) {
+          s = 0;
+          ph ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // The thread can run only one or two MMAs ahead of the tensor core, so whatever it does between stages leaves the tensor
-    // core idle: with two barriers per stage, descriptors built per MMA and the wait after the fourth MMA it spent 280 cycles
-    // per stage on that (a stage of four 128 x 256 x 64 MMAs is 512 cycles).  Hence one barrier per stage (operands landed and
-    // scales in tensor memory), descriptors by addition, and a look at the next stage's barrier before the last MMA.
-    if (lane == 0) {
-      const uint64_t a_desc0 = desc_kmajor<C::kRowBytes>(smem_u32(smem)), b_desc0 = desc_kmajor<C::kRowBytes>(smem_u32(smem) + C::kStageA);
-      const uint32_t full0 = smem_u32(full_bar);
-      uint32_t s = 0, ph = 0, tcount = 0;
-      bool ok = true, ready = false;
-      for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride, ++tcount) {
-        const uint32_t acc = tcount % C::kAcc, aph = (tcount / C::kAcc) & 1;
-        if (!mbar_wait(smem_u32(&acc_empty[acc]), aph ^ 1, p.status, 2)) { ok = false; break; }
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int ks = ks_begin; ks < ks_end; ++ks) {
-          if (!ready && !mbar_wait(full0 + s * 8, ph, p.status, 3)) { ok = false; break; }
-          tcgen05_fence_after();
+    // The warp can run only one or two MMAs ahead of the tensor core, so whatever it does between stages leaves the tensor
+    // core idle: one barrier per stage (operands landed and scales in tensor memory), descriptors by addition, and the whole warp in
+    // the loop (elect_one).
+    const bool elected = elect_one();
+    const uint64_t a_desc0 = desc_kmajor<C::kRowBytes>(smem_u32(smem)), b_desc0 = desc_kmajor<C::kRowBytes>(smem_u32(smem) + C::kStageA);
+    const uint32_t full0 = smem_u32(full_bar);
+    uint32_t s = 0, ph = 0, tcount = 0;
+    bool ok = true;
+    for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_stride, ++tcount) {
+      const uint32_t acc = tcount % C::kAcc, aph = (tcount / C::kAcc) & 1;
+      ok = mbar_wait_warp(smem_u32(&acc_empty[acc]), aph ^ 1, p.status, 2);
+      if (!ok) break;
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int ks = ks_begin; ks < ks_end; ++ks) {
+        ok = mbar_wait_warp(full0 + s * 8, ph, p.status, 3);
+        if (!ok) break;
+        tcgen05_fence_after();
+        if (elected) {
           // each 64-wide k-block is 32 bytes further along the swizzled 128-byte rows (descriptors count 16 bytes)
           const uint64_t a_desc = a_desc0 + s * (C::kStageBytes >> 4), b_desc = b_desc0 + s * (C::kStageBytes >> 4);
           const uint32_t sfa_tmem = tmem_base + C::kSfBase + s * C::kSfCols, sfb_tmem = sfa_tmem + 4 * KB;
-          const uint32_t empty = smem_u32(&empty_bar[s]);
-          const uint32_t s_next = s + 1 == C::kStages ? 0 : s + 1, ph_next = s + 1 == C::kStages ? ph ^ 1 : ph;
-          const int kblocks = min(KB, KT - ks * KB);
-          if (kblocks == KB) {
+          const int kblocks = KT - ks * KB;
 #pragma unroll
-            for (int kb = 0; kb < KB; ++kb) {
-              if (kb == KB - 1) ready = mbar_test_wait(full0 + s_next * 8, ph_next);
+          for (int kb = 0; kb < KB; ++kb)
+            if (kb < kblocks)
               tcgen05_mma_nvf4(d_tmem, a_desc + kb * 2, b_desc + kb * 2, C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles),
                                (ks > ks_begin || kb > 0) ? 1u : 0u);
-            }
-          } else {
-            ready = false;
-            for (int kb = 0; kb < kblocks; ++kb)
-              tcgen05_mma_nvf4(d_tmem, a_desc + kb * 2, b_desc + kb * 2, C::kIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * (4 * C::kSfTiles),
-                               (ks > ks_begin || kb > 0) ? 1u : 0u);
-          }
-          tcgen05_commit(empty);    // frees the stage when these MMAs have read it
-          s = s_next;
-          ph = ph_next;
+          tcgen05_commit(smem_u32(&empty_bar[s]));    // frees the stage when these MMAs have read it
+          if (ks == ks_end - 1) tcgen05_commit(smem_u32(&acc_full[acc]));
         }
-        if (ok) tcgen05_commit(smem_u32(&acc_full[acc]));
+        __syncwarp();
+        if (++s == C::kStages) {
+          s = 0;
+          ph ^= 1;
+        }
       }
     }
   } else if (warp >= 6 && warp < 10) {

@@ -156,38 +156,43 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ operand loads (both CTAs)
-    if (lane == 0) {
-      const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[0]), 0);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs) {
-        const int mp = tile % p.m_pairs, nt = tile / p.m_pairs;
-        const int a_row0 = mp * 256 + (int)rank * 128, b_row0 = nt * 256 + (int)rank * 128;
-        for (int ks = 0; ks < p.k_stages; ++ks, ++it) {
-          const uint32_t s = it % kPStages, ph = (it / kPStages) & 1;
-          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, p.status, 21)) { ok = false; break; }
+    const bool elected = elect_one();
+    const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[0]), 0);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs) {
+      const int mp = tile % p.m_pairs, nt = tile / p.m_pairs;
+      const int a_row0 = mp * 256 + (int)rank * 128, b_row0 = nt * 256 + (int)rank * 128;
+      for (int ks = 0; ks < p.k_stages; ++ks, ++it) {
+        const uint32_t s = it % kPStages, ph = (it / kPStages) & 1;
+        ok = mbar_wait_warp(smem_u32(&empty_bar[s]), ph ^ 1, p.status, 21);
+        if (!ok) break;
+        if (elected) {
           unsigned char* st = smem + (size_t)s * kPStageOp;
           // the leader announces the bytes of both CTAs; the peer's copies may complete before or after that
           if (leader) mbar_expect_tx(smem_u32(&full_bar[s]), 2u * kPStageOp);
           tma_load_2d_pair(smem_u32(st), &map_a, ks * 128, a_row0, full_leader + s * 8);
           tma_load_2d_pair(smem_u32(st + kPStageA), &map_b, ks * 128, b_row0, full_leader + s * 8);
         }
+        __syncwarp();
       }
     }
   } else if (warp == 14) {
     // ------------------------------------------------------------------ scale-factor loads (both CTAs)
-    if (lane == 0) {
-      uint32_t jt = 0;
-      bool ok = true;
-      for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs) {
-        const int mp = tile % p.m_pairs, nt = tile / p.m_pairs;
-        const int sfa_tile = mp * 2 + (int)rank;
-        const bool sfa_ok = sfa_tile * 128 < p.M;        // the peer's A rows may lie entirely past M
-        int sf_tiles = 0;
-        for (int j = 0; j < 2; ++j) sf_tiles += ((nt * 2 + j) * 128 < p.N) ? 1 : 0;
-        for (int ks = 0; ks < p.k_stages; ++ks, ++jt) {
-          const uint32_t j = jt % kPSfStages, ph = (jt / kPSfStages) & 1;
-          if (!mbar_wait(smem_u32(&sf_free[j]), ph ^ 1, p.status, 22)) { ok = false; break; }
+    const bool elected = elect_one();
+    uint32_t jt = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs) {
+      const int mp = tile % p.m_pairs, nt = tile / p.m_pairs;
+      const int sfa_tile = mp * 2 + (int)rank;
+      const bool sfa_ok = sfa_tile * 128 < p.M;        // the peer's A rows may lie entirely past M
+      int sf_tiles = 0;
+      for (int j = 0; j < 2; ++j) sf_tiles += ((nt * 2 + j) * 128 < p.N) ? 1 : 0;
+      for (int ks = 0; ks < p.k_stages; ++ks, ++jt) {
+        const uint32_t j = jt % kPSfStages, ph = (jt / kPSfStages) & 1;
+        ok = mbar_wait_warp(smem_u32(&sf_free[j]), ph ^ 1, p.status, 22);
+        if (!ok) break;
+        if (elected) {
           unsigned char* sf = sf_ring + (size_t)j * kPSfStage;
           const int kblocks = min(4, KT - ks * 4);
           const uint32_t bar = smem_u32(&sf_full[j]);
@@ -198,46 +203,44 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             bulk_load_1d(smem_u32(sf + kPSfA + t * 2048), p.sfb + ((size_t)(nt * 2 + t) * KT + (size_t)ks * 4) * 512,
                          (uint32_t)kblocks * 512, bar);
         }
+        __syncwarp();
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    // The thread runs only one or two MMAs ahead of the tensor cores, so what it does between stages leaves them idle: one
-    // barrier per stage, descriptors by addition, and a look at the next stage's barrier before the last MMA of a stage.
-    if (leader && lane == 0) {
+    // The warp runs only one or two MMAs ahead of the tensor cores, so what it does between stages leaves them idle: one
+    // barrier per stage, descriptors by addition, the whole warp in the loop (elect_one).
+    if (leader) {
+      const bool elected = elect_one();
       const uint64_t a_desc0 = desc_kmajor<128>(smem_u32(smem)), b_desc0 = desc_kmajor<128>(smem_u32(smem) + kPStageA);
       const uint32_t full0 = smem_u32(full_bar);
       uint32_t s = 0, ph = 0, tcount = 0;
-      bool ok = true, ready = false;
+      bool ok = true;
       for (int tile = pair; ok && tile < n_tiles_total; tile += n_pairs, ++tcount) {
-        if (!mbar_wait(smem_u32(acc_empty), (tcount & 1) ^ 1, p.status, 23)) { ok = false; break; }
+        ok = mbar_wait_warp(smem_u32(acc_empty), (tcount & 1) ^ 1, p.status, 23);
+        if (!ok) break;
         for (int ks = 0; ks < p.k_stages; ++ks) {
-          if (!ready && !mbar_wait(full0 + s * 8, ph, p.status, 25)) { ok = false; break; }
+          ok = mbar_wait_warp(full0 + s * 8, ph, p.status, 25);
+          if (!ok) break;
           tcgen05_fence_after();
-          const uint64_t a_desc = a_desc0 + s * (kPStageOp >> 4), b_desc = b_desc0 + s * (kPStageOp >> 4);
-          const uint32_t sfa_tmem = tmem_base + kPSfBase + s * kPSfCols, sfb_tmem = sfa_tmem + 16;
-          const uint32_t empty = smem_u32(&empty_bar[s]);
-          const bool wrap = s + 1 == kPStages;
-          const uint32_t s_next = wrap ? 0 : s + 1, ph_next = wrap ? ph ^ 1 : ph;
-          const int kblocks = min(4, KT - ks * 4);
-          if (kblocks == 4) {
+          if (elected) {
+            const uint64_t a_desc = a_desc0 + s * (kPStageOp >> 4), b_desc = b_desc0 + s * (kPStageOp >> 4);
+            const uint32_t sfa_tmem = tmem_base + kPSfBase + s * kPSfCols, sfb_tmem = sfa_tmem + 16;
+            const int kblocks = KT - ks * 4;
 #pragma unroll
-            for (int kb = 0; kb < 4; ++kb) {
-              if (kb == 3) ready = mbar_test_wait(full0 + s_next * 8, ph_next);
-              tcgen05_mma_nvf4_pair(tmem_base, a_desc + kb * 2, b_desc + kb * 2, kPIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * 8,
-                                    (ks > 0 || kb > 0) ? 1u : 0u);
-            }
-          } else {
-            ready = false;
-            for (int kb = 0; kb < kblocks; ++kb)
-              tcgen05_mma_nvf4_pair(tmem_base, a_desc + kb * 2, b_desc + kb * 2, kPIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * 8,
-                                    (ks > 0 || kb > 0) ? 1u : 0u);
+            for (int kb = 0; kb < 4; ++kb)
+              if (kb < kblocks)
+                tcgen05_mma_nvf4_pair(tmem_base, a_desc + kb * 2, b_desc + kb * 2, kPIdesc, sfa_tmem + kb * 4, sfb_tmem + kb * 8,
+                                      (ks > 0 || kb > 0) ? 1u : 0u);
+            tcgen05_commit_pair(smem_u32(&empty_bar[s]), 3);                          // both CTAs may refill this stage and its scale slot
+            if (ks == p.k_stages - 1) tcgen05_commit_pair(smem_u32(acc_full), 3);     // both epilogues may start
           }
-          tcgen05_commit_pair(empty, 3);                          // both CTAs may refill this stage and its scale slot
-          s = s_next;
-          ph = ph_next;
+          __syncwarp();
+          if (++s == kPStages) {
+            s = 0;
+            ph ^= 1;
+          }
         }
-        if (ok) tcgen05_commit_pair(smem_u32(acc_full), 3);     // both epilogues may start
       }
     }
   } else if (warp >= 6 && warp < 10) {
