@@ -1,28 +1,28 @@
 // MoE router for decode: gate projection (16-bit weights), softmax over the experts, top-k, renormalisation.
 //
 // The reference leaves routing to vLLM (its benches build it in torch: softmax of the gate logits, topk, weights
-// divided by their sum -- sparse_fp4_kernel/bench_moe_layer_e2e.py:230-236); here it is two small kernels whose
+// divided by their sum -- sparse_fp4_kernel/bench_moe_layer_e2e.py:230-236); here it is one or two small kernels whose
 // outputs (topk_weights f32, topk_ids i32) are exactly the device tensors the fused MoE layer and the expert-parallel
 // dispatch take, so no host round trip sits between the router and the experts.
-//   router_mma_kernel      small batches: 16 experts x up to 64 tokens per block, mma.sync, operands straight from global
-//                          memory into fragments; bound by latency, so K is split over warps and blocks until every
-//                          warp has about one round of loads (M=32, H=2048, E=512: 31 us with one dot product per warp and
-//                          weight row on 32 blocks)
+//   router_cluster_kernel  up to 64 tokens: projection (mma.sync, operands straight from global memory into fragments), exchange of
+//                          the logits through distributed shared memory and selection in one launch
 //   router_gemm_kernel     larger batches: 128 tokens x 128 or 256 experts per CTA on tcgen05 (kind::f16, fp32 accumulators
 //                          in tensor memory), operands by TMA; bound by L2 -> shared-memory bandwidth
 //   router_topk_kernel     one warp per token: adds the K-slices of its logits in a fixed order, then k rounds of warp-wide
 //                          arg-max (ties -> lower expert id), weights exp(l - max) normalised over the selected experts
 //                          (or over all of them)
+#include <mutex>
+
 #include "sm100_ptx.cuh"
 
 namespace b200fp4 {
 namespace {
 
-// ------------------------------------------------------------------------------------------ projection, small batches
+// ------------------------------------------------------------------------------------------ small batches, one kernel
 
-constexpr int kRtThreads = 256;
-constexpr int kRtWarps = kRtThreads / 32;
-constexpr int kRtMaxTokens = 64;       // per block
+constexpr int kRcWarps = 16;
+constexpr int kRcThreads = 32 * kRcWarps;
+constexpr int kRtPerLane = 32;         // experts per lane of a warp that selects: 1024
 
 template <typename T>
 __device__ __forceinline__ void mma_m16n8k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -40,66 +40,6 @@ __device__ __forceinline__ void mma_m16n8k16<__half>(float (&c)[4], uint32_t a0,
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// parts[z][m][e] = sum over the k of slice z of hidden[m][k] * gate_w[e][k].
-// Block = experts [16 x, +16) x tokens [8 NT y, +8 NT), slice z of K; its warps take 64-wide pieces of K in turn.  In a 32-wide
-// step lane (g, t) = (lane / 4, lane % 4) loads the 8 elements at k = 8t of rows g and g + 8 (experts) and g (tokens): the
-// order of k inside a product sum is free, so elements 0-3 of the 8 serve as the lane's k of one mma and 4-7 as those of
-// another, on both sides alike.
-template <typename T, int NT>
-__global__ void __launch_bounds__(kRtThreads)
-    router_mma_kernel(const T* __restrict__ hidden, int64_t ld_h, const T* __restrict__ gate_w, int M, int H, int E,
-                      int* __restrict__ status, float* __restrict__ parts) {
-  __shared__ float s_part[kRtWarps][16][8 * NT + 1];
-  pdl_wait();
-  pdl_launch_dependents();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int e0 = blockIdx.x * 16, m0 = blockIdx.y * 8 * NT;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *status = 0;
-  float acc[NT][4];
-#pragma unroll
-  for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-  const T* wa = gate_w + (int64_t)min(e0 + g, E - 1) * H;            // rows past the end repeat the last: never stored
-  const T* wb = gate_w + (int64_t)min(e0 + g + 8, E - 1) * H;
-  const T* x[NT];
-#pragma unroll
-  for (int n = 0; n < NT; ++n) x[n] = hidden + (int64_t)min(m0 + 8 * n + g, M - 1) * ld_h;
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  for (int k0 = 64 * (blockIdx.z * kRtWarps + warp); k0 < H; k0 += 64 * kRtWarps * gridDim.z) {
-    uint4 a[2][2], b[2][NT];
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int k = k0 + 32 * s + 8 * t;
-      const bool in = k < H;
-      a[s][0] = in ? ldg_stream_u4(wa + k) : zero;
-      a[s][1] = in ? ldg_stream_u4(wb + k) : zero;
-#pragma unroll
-      for (int n = 0; n < NT; ++n) b[s][n] = in ? *reinterpret_cast<const uint4*>(x[n] + k) : zero;
-    }
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        mma_m16n8k16<T>(acc[n], a[s][0].x, a[s][1].x, a[s][0].y, a[s][1].y, b[s][n].x, b[s][n].y);
-        mma_m16n8k16<T>(acc[n], a[s][0].z, a[s][1].z, a[s][0].w, a[s][1].w, b[s][n].z, b[s][n].w);
-      }
-  }
-#pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    s_part[warp][g][8 * n + 2 * t] = acc[n][0];
-    s_part[warp][g][8 * n + 2 * t + 1] = acc[n][1];
-    s_part[warp][g + 8][8 * n + 2 * t] = acc[n][2];
-    s_part[warp][g + 8][8 * n + 2 * t + 1] = acc[n][3];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 16 * 8 * NT; i += kRtThreads) {
-    const int r = i & 15, c = i >> 4;
-    float v = 0.f;
-#pragma unroll
-    for (int w = 0; w < kRtWarps; ++w) v += s_part[w][r][c];
-    if (e0 + r < E && m0 + c < M) parts[((int64_t)blockIdx.z * M + m0 + c) * E + e0 + r] = v;
-  }
 }
 
 // ------------------------------------------------------------------------------------------ projection, larger batches
@@ -163,32 +103,34 @@ __global__ void __launch_bounds__(kRgThreads, 1)
   pdl_launch_dependents();
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *status = 0;    // a wait writes it only after ~1 s
   if (warp == 0) {
-    if (lane == 0) {
-      for (int i = 0; i < n_steps; ++i) {
-        const uint32_t s = i % kRgStages, ph = (i / kRgStages) & 1;
-        if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, status, 31)) break;
+    const bool elected = elect_one();
+    for (int i = 0; i < n_steps; ++i) {
+      const uint32_t s = i % kRgStages, ph = (i / kRgStages) & 1;
+      if (!mbar_wait_warp(smem_u32(&empty_bar[s]), ph ^ 1, status, 31)) break;
+      if (elected) {
         unsigned char* st = smem + s * C::kStage;
         const uint32_t bar = smem_u32(&full_bar[s]);
         mbar_expect_tx(bar, C::kStage);
         tma_load_2d(smem_u32(st), &map_x, (first + i) * 128, m0, bar);
         tma_load_2d(smem_u32(st + C::kStageA), &map_w, (first + i) * 128, e0, bar);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int i = 0; i < n_steps; ++i) {
-        const uint32_t s = i % kRgStages, ph = (i / kRgStages) & 1;
-        ok = mbar_wait(smem_u32(&full_bar[s]), ph, status, 32);
-        if (!ok) break;
-        tcgen05_fence_after();
+    const bool elected = elect_one();
+    for (int i = 0; i < n_steps; ++i) {
+      const uint32_t s = i % kRgStages, ph = (i / kRgStages) & 1;
+      if (!mbar_wait_warp(smem_u32(&full_bar[s]), ph, status, 32)) break;
+      tcgen05_fence_after();
+      if (elected) {
         const uint32_t a = smem_u32(smem + s * C::kStage), b = a + C::kStageA;
 #pragma unroll
         for (int k = 0; k < kRgK / 16; ++k)       // 16 elements are 32 bytes further along the swizzled rows
           tcgen05_mma_f16(tmem, desc_kmajor<128>(a + 32 * k), desc_kmajor<128>(b + 32 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
         tcgen05_commit(smem_u32(&empty_bar[s]));
+        if (i == n_steps - 1) tcgen05_commit(smem_u32(acc_full));
       }
-      if (ok) tcgen05_commit(smem_u32(acc_full));
+      __syncwarp();
     }
   } else {
     bool ok = mbar_wait(smem_u32(acc_full), 0, status, 33);
@@ -235,33 +177,11 @@ __device__ __forceinline__ uint32_t float_key(float v) {
 }
 __device__ __forceinline__ float key_float(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
 
-// One warp per token; E <= 32 * PER.  The warp-wide arg-max of a round is two warp reductions (largest key, then the lowest
-// expert id that holds it); shuffle trees of (value, id) pairs over 32 slots per lane took 5.8 us at M=32.
-constexpr int kRtPerLane = 32;
-
+// The k largest of the 32 * PER keys of a warp (lane-interleaved: expert e in lane e % 32, slot e / 32) for one token, and their weights.
+// The arg-max of a round is two warp reductions (largest key, then the lowest expert id that holds it); shuffle trees of
+// (value, id) pairs over 32 slots per lane took 5.8 us at M=32.
 template <int PER>
-__global__ void __launch_bounds__(128)
-    router_topk_kernel(const float* __restrict__ parts, int splits, int M, int E, int topk, int renormalize,
-                       float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int lane = threadIdx.x & 31;
-  const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (m >= M) return;
-  uint32_t key[PER];
-  {
-    float v[PER];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) v[i] = 0.f;
-    for (int z = 0; z < splits; ++z) {
-      const float* src = parts + ((int64_t)z * M + m) * E + lane;
-#pragma unroll
-      for (int i = 0; i < PER; ++i)                // lane-interleaved: expert e lives in lane e % 32, slot e / 32
-        if (i * 32 + lane < E) v[i] += src[i * 32];
-    }
-#pragma unroll
-    for (int i = 0; i < PER; ++i) key[i] = i * 32 + lane < E ? float_key(v[i]) : 0u;
-  }
+__device__ __forceinline__ void select_topk(uint32_t (&key)[PER], int lane, int topk, int renormalize, float* topk_w, int32_t* topk_ids) {
   float mx = 0.f, total = 0.f, sel_sum = 0.f, my_w = 0.f;
   int my_id = 0;
   for (int r = 0; r < topk; ++r) {
@@ -297,54 +217,187 @@ __global__ void __launch_bounds__(128)
   }
   const float denom = renormalize ? sel_sum : total;
   if (lane < topk) {
-    topk_w[(int64_t)m * topk + lane] = my_w / denom;
-    topk_ids[(int64_t)m * topk + lane] = my_id;
+    topk_w[lane] = my_w / denom;
+    topk_ids[lane] = my_id;
+  }
+}
+
+// One warp per token; E <= 32 * PER.
+template <int PER>
+__global__ void __launch_bounds__(128)
+    router_topk_kernel(const float* __restrict__ parts, int splits, int M, int E, int topk, int renormalize,
+                       float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31;
+  const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (m >= M) return;
+  uint32_t key[PER];
+  {
+    float v[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) v[i] = 0.f;
+    for (int z = 0; z < splits; ++z) {
+      const float* src = parts + ((int64_t)z * M + m) * E + lane;
+#pragma unroll
+      for (int i = 0; i < PER; ++i)                // lane-interleaved: expert e lives in lane e % 32, slot e / 32
+        if (i * 32 + lane < E) v[i] += src[i * 32];
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) key[i] = i * 32 + lane < E ? float_key(v[i]) : 0u;
+  }
+  select_topk<PER>(key, lane, topk, renormalize, topk_w + (int64_t)m * topk, topk_ids + (int64_t)m * topk);
+}
+
+// Projection, exchange and selection in one launch.  A cluster of CL blocks takes eight tokens: block r the experts
+// [16 r tiles, +16 tiles), its warps the 16-expert tiles times slices of K.  In a 32-wide step lane (g, t) = (lane / 4, lane % 4) loads the
+// 8 elements at k = 8t of rows g and g + 8 (experts) and g (tokens): the order of k inside a product sum is free, so elements 0-3 of the 8
+// serve as the lane's k of one mma and 4-7 as those of another, on both sides alike.  The slices of a logit are added in a fixed order; logits
+// go through distributed shared memory to the block that selects for their token: nothing is written to memory but the result.
+// Bound by latency (launch, rounds of loads, exchange, selection) and by what one SM reads of the gate through L2.
+template <typename T, int CL, int PER>
+__global__ void __launch_bounds__(kRcThreads, 1)
+    router_cluster_kernel(const T* __restrict__ hidden, int64_t ld_h, const T* __restrict__ gate_w, int M, int H, int E, int tiles, int topk,
+                          int renormalize, int* __restrict__ status, float* __restrict__ topk_w, int32_t* __restrict__ topk_ids) {
+  __shared__ float s_part[kRcWarps][16][9];       // [slice of K and tile][expert][token]
+  __shared__ float s_logit[32 * PER];                      // this block's token, all experts
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int rank = (int)(blockIdx.x % CL), m0 = (int)(blockIdx.x / CL) * 8;
+  const int slices = kRcWarps / tiles, tile = warp % tiles, slice = warp / tiles, e_block = rank * tiles * 16, e0 = e_block + tile * 16;
+  cluster_sync_any();                                      // the other blocks run before anything is sent to them
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  if (slice < slices) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const T* wa = gate_w + (int64_t)min(e0 + g, E - 1) * H;            // rows past the end repeat the last: never used
+    const T* wb = gate_w + (int64_t)min(e0 + g + 8, E - 1) * H;
+    const T* x = hidden + (int64_t)min(m0 + g, M - 1) * ld_h;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    constexpr int U = 4;                                   // 32-wide steps in flight
+    for (int k0 = 32 * slice; k0 < H; k0 += 32 * U * slices) {
+      uint4 a[U][2], b[U];
+#pragma unroll
+      for (int s = 0; s < U; ++s) {
+        const int k = k0 + 32 * slices * s + 8 * t;
+        const bool in = k < H;
+        a[s][0] = in ? ldg_stream_u4(wa + k) : zero;
+        a[s][1] = in ? ldg_stream_u4(wb + k) : zero;
+        b[s] = in ? *reinterpret_cast<const uint4*>(x + k) : zero;
+      }
+#pragma unroll
+      for (int s = 0; s < U; ++s) {
+        mma_m16n8k16<T>(acc, a[s][0].x, a[s][1].x, a[s][0].y, a[s][1].y, b[s].x, b[s].y);
+        mma_m16n8k16<T>(acc, a[s][0].z, a[s][1].z, a[s][0].w, a[s][1].w, b[s].z, b[s].w);
+      }
+    }
+    s_part[warp][g][2 * t] = acc[0];
+    s_part[warp][g][2 * t + 1] = acc[1];
+    s_part[warp][g + 8][2 * t] = acc[2];
+    s_part[warp][g + 8][2 * t + 1] = acc[3];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < tiles * 16 * 8; i += kRcThreads) {
+    const int e = i % (tiles * 16), tok = i / (tiles * 16);
+    float v = 0.f;
+    for (int z = 0; z < slices; ++z) v += s_part[z * tiles + (e >> 4)][e & 15][tok];
+    if (e_block + e < E) {
+      const uint32_t to = map_to_cta(smem_u32(&s_logit[e_block + e]), (uint32_t)tok);
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(v) : "memory");
+    }
+  }
+  cluster_sync_any();
+  const int m = m0 + rank;
+  if (warp == 0 && rank < 8 && m < M) {
+    uint32_t key[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) key[i] = i * 32 + lane < E ? float_key(s_logit[i * 32 + lane]) : 0u;
+    select_topk<PER>(key, lane, topk, renormalize, topk_w + (int64_t)m * topk, topk_ids + (int64_t)m * topk);
   }
 }
 
 // ------------------------------------------------------------------------------------------ host
 
-// K-slices of the projection: enough blocks to cover the SMs, at most eight (the top-k kernel reads them all).
-// Up to one block of tokens (64) the mma.sync kernel is the faster one (M=32: 3.4 us); it reads every weight row once per block
-// of tokens through L2, so from there on the tcgen05 tiles win (M=200: 12.7 us against about 6; M=1000: 7.9 us, M=8192: 22 us
-// where one dot product per warp and weight row took 832 us).
-constexpr int kRtMmaMaxTokens = kRtMaxTokens;
+// Up to 64 tokens and 512 experts (16 tokens above, as far as 1/16 of the gate is not more than one SM reads in about 4 us) everything is
+// one launch of clusters; else the tcgen05 tiles and the separate selection: every cluster of eight tokens reads all weight rows, 1/8 or 1/16
+// of them through one SM (1000 experts, H=4096, M=64 22.7 us as clusters, 15.2 as tiles; 1024 experts, M=4 10.7 / 13.0).
+constexpr int kRtClusterMaxTokens = 64;
 constexpr int kRtMaxSplits = 8;
 
+// K-slices of the projection of many tokens: enough blocks to cover the SMs, at most eight (the top-k kernel reads them all)
 struct RouterShape {
   bool small;
-  int tokens, bn, splits;      // small: tokens per block; else the expert tile
+  int bn, splits;
 };
 
-RouterShape router_shape(int64_t M, int64_t E) {
+RouterShape router_shape(int64_t M, int64_t H, int64_t E) {
   RouterShape s = {};
-  s.small = M <= kRtMmaMaxTokens;
-  int64_t blocks;
-  if (s.small) {
-    s.tokens = M <= 8 ? 8 : (M <= 16 ? 16 : (M <= 32 ? 32 : kRtMaxTokens));
-    blocks = ((E + 15) / 16) * ((M + s.tokens - 1) / s.tokens);
-  } else {
-    const int64_t mt = (M + 127) / 128;
-    s.bn = mt * ((E + 127) / 128) <= sm_count() ? 128 : 256;
-    blocks = mt * ((E + s.bn - 1) / s.bn);
-  }
-  const int64_t z = sm_count() / (blocks > 0 ? blocks : 1);
+  s.small = E <= 512 ? M <= kRtClusterMaxTokens : M <= 16 && E * H <= (int64_t)1024 * 4096;
+  if (s.small) return s;
+  const int64_t mt = (M + 127) / 128;
+  s.bn = mt * ((E + 127) / 128) <= sm_count() ? 128 : 256;
+  const int64_t blocks = mt * ((E + s.bn - 1) / s.bn), z = sm_count() / (blocks > 0 ? blocks : 1);
   s.splits = (int)(z < 1 ? 1 : (z > kRtMaxSplits ? kRtMaxSplits : z));
   return s;
 }
 
-template <typename T>
-void launch_router_mma(const RouterShape& s, int splits, const void* hidden, int64_t ld_h, const void* gate_w, int M, int H, int E,
-                       int* status, float* parts, cudaStream_t st) {
-  const dim3 grid((unsigned)((E + 15) / 16), (unsigned)((M + s.tokens - 1) / s.tokens), (unsigned)splits);
-  auto go = [&](auto kernel) {
-    launch_pdl(kernel, grid, dim3(kRtThreads), 0, st, static_cast<const T*>(hidden), ld_h, static_cast<const T*>(gate_w), M, H, E,
-               status, parts);
+// Clusters of CL blocks that are resident at once (0: none)
+template <typename T, int CL, int PER>
+int resident_router_clusters() {
+  struct PerDevice {
+    std::once_flag once;
+    int n = 0;
   };
-  if (s.tokens == 8) go(router_mma_kernel<T, 1>);
-  else if (s.tokens == 16) go(router_mma_kernel<T, 2>);
-  else if (s.tokens == 32) go(router_mma_kernel<T, 4>);
-  else go(router_mma_kernel<T, 8>);
+  static PerDevice devices[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  PerDevice& d = devices[dev];
+  std::call_once(d.once, [&] {
+    auto* kernel = router_cluster_kernel<T, CL, PER>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CL);
+    cfg.blockDim = dim3(kRcThreads);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = CL;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if ((CL > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+        cudaOccupancyMaxActiveClusters(&d.n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      d.n = 0;
+    }
+  });
+  return d.n;
+}
+
+template <typename T, int CL, int PER>
+cudaError_t launch_router_cluster_t(const void* hidden, int64_t ld_h, const void* gate_w, int M, int H, int E, int topk, int renormalize,
+                                    int* status, float* topk_w, int32_t* topk_ids, cudaStream_t st) {
+  const int tiles = (E + 16 * CL - 1) / (16 * CL);
+  return launch_pdl_cluster(CL, router_cluster_kernel<T, CL, PER>, dim3((unsigned)(CL * ((M + 7) / 8))), dim3(kRcThreads), 0, st,
+                            static_cast<const T*>(hidden), ld_h, static_cast<const T*>(gate_w), M, H, E, tiles, topk, renormalize, status,
+                            topk_w, topk_ids);
+}
+
+// Sixteen blocks to a cluster where there are experts for them and all clusters run at once (512 experts, H=2048, us with 8 / 16: M=1 6.5 / 4.8,
+// M=32 7.6 / 5.6, M=64 7.4 / 10.5 with an eighth cluster that waits; 256 experts, M=32 4.8 / 4.0), else eight.
+template <typename T>
+int launch_router_cluster(const void* hidden, int64_t ld_h, const void* gate_w, int M, int H, int E, int topk, int renormalize, int* status,
+                          float* topk_w, int32_t* topk_ids, cudaStream_t st) {
+  auto go = [&](auto* launch) { return launch(hidden, ld_h, gate_w, M, H, E, topk, renormalize, status, topk_w, topk_ids, st); };
+  const int clusters = (M + 7) / 8;
+  cudaError_t rc;
+  if (E <= 128) rc = go(launch_router_cluster_t<T, 8, 4>);
+  else if (E <= 256) rc = clusters <= resident_router_clusters<T, 16, 8>() ? go(launch_router_cluster_t<T, 16, 8>) : go(launch_router_cluster_t<T, 8, 8>);
+  else if (E > 512) rc = resident_router_clusters<T, 16, kRtPerLane>() > 0 ? go(launch_router_cluster_t<T, 16, kRtPerLane>) : go(launch_router_cluster_t<T, 8, kRtPerLane>);
+  else rc = clusters <= resident_router_clusters<T, 16, 16>() ? go(launch_router_cluster_t<T, 16, 16>) : go(launch_router_cluster_t<T, 8, 16>);
+  if (rc != cudaSuccess) {
+    cudaGetLastError();
+    return B200FP4_STATUS_EXECUTION_FAILED;
+  }
+  return finish_launch(1);
 }
 
 template <int BN>
@@ -376,7 +429,8 @@ using namespace b200fp4;
 // workspace: 256 bytes (first int: status word of the tcgen05 kernel's bounded waits), then the K-slices of the logits
 extern "C" size_t b200fp4_moe_router_workspace_bytes(int64_t M, int64_t E) {
   if (M <= 0 || E <= 0) return 0;
-  return 256 + (size_t)router_shape(M, E).splits * (size_t)M * (size_t)E * sizeof(float);
+  const RouterShape s = router_shape(M, (int64_t)1 << 20, E);        // as for a gate of many columns: whichever path H leads to fits
+  return 256 + (size_t)s.splits * (size_t)M * (size_t)E * sizeof(float);
 }
 
 extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, const void* gate_w, int64_t M, int64_t H,
@@ -394,15 +448,12 @@ extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, c
   cudaStream_t st = (cudaStream_t)stream;
   int* status = static_cast<int*>(workspace);
   float* parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
-  const RouterShape sh = router_shape(M, E);
+  const RouterShape sh = router_shape(M, H, E);
   const bool bf = dtype == B200FP4_DTYPE_BF16;
   int splits = sh.splits;
   if (sh.small) {
-    // no more slices than there are rounds of 64 per warp
-    const int most = (int)((H + 64 * kRtWarps - 1) / (64 * kRtWarps));
-    if (splits > most) splits = most;
-    if (bf) launch_router_mma<__nv_bfloat16>(sh, splits, hidden, ld_h, gate_w, (int)M, (int)H, (int)E, status, parts, st);
-    else launch_router_mma<__half>(sh, splits, hidden, ld_h, gate_w, (int)M, (int)H, (int)E, status, parts, st);
+    auto* go = bf ? launch_router_cluster<__nv_bfloat16> : launch_router_cluster<__half>;
+    return go(hidden, ld_h, gate_w, (int)M, (int)H, (int)E, (int)topk, renormalize, status, topk_weights, topk_ids, st);
   } else {
     if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
     const int most = (int)((H + 4 * kRgK - 1) / (4 * kRgK));       // at least about four stages per slice

@@ -1,4 +1,4 @@
-"""MoE router on the GPU: gate projection + softmax + top-k + renormalisation in two small kernels, producing the
+"""MoE router on the GPU: gate projection + softmax + top-k + renormalisation in one or two small kernels, producing the
 (topk_weights f32, topk_ids i32) pair the fused MoE ops take.  The reference leaves this step to vLLM; its benches
 restate it in torch (sparse_fp4_kernel/bench_moe_layer_e2e.py:230-236), which is what the parity test compares with."""
 from __future__ import annotations

@@ -39,6 +39,12 @@ def test_convert_2of4_tile_edges(E, N, K, G):
     (1024, 2048, 512, 10, torch.bfloat16, True),      # several K-slices
     (4864, 1024, 512, 10, torch.bfloat16, False),     # 256-wide expert tiles
     (4865, 256, 290, 4, torch.float16, True),         # ... past their end, E no multiple of four
+    (17, 4096, 128, 8, torch.bfloat16, False),        # clusters of eight: one tile of experts to a block, sixteen slices of K
+    (31, 72, 129, 4, torch.float16, True),            # clusters of sixteen, most blocks without experts, less K than slices
+    (56, 2048, 512, 10, torch.bfloat16, False),       # ... as many as run at once
+    (64, 1024, 500, 10, torch.float16, False),        # ... one more: clusters of eight again, four tiles to a block
+    (16, 1000, 1023, 32, torch.bfloat16, True),       # more than 512 experts
+    (3, 12800, 600, 4, torch.bfloat16, True),         # ... with a gate for the tile kernel
 ])
 def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
     from dgx_vllm_b200.router import moe_router
