@@ -24,6 +24,7 @@
 
 #include <mutex>
 
+#include "moe_small.cuh"
 #include "sparse_mma.cuh"
 
 extern "C" size_t b200fp4_sparse_workspace_bytes(int64_t P, int64_t K, int64_t E);
@@ -2146,6 +2147,20 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   // from the gate_up epilogue).  Both projections share one launch and one claim sequence unless
   // B200FP4_MOE_SEPARATE_LAUNCHES asks for one launch each (which takes other kernels up to 256 pairs).
   if (ordered && (P > 256 || !(flags & B200FP4_MOE_SEPARATE_LAUNCHES)) && ws_ok(2 * I, H, G13, I, w13) && ws_ok(H, I, G2, 0, w2)) {
+    // few pairs, which rarely share an expert: a cluster of blocks for each
+    const int cluster = (flags & B200FP4_MOE_SEPARATE_LAUNCHES) || 2 * local_pairs > E ? 0 : moe_small_cluster(P, H, I);
+    if (cluster > 0) {
+      const MoeSmallArgs a = {w13, w2, hidden, ld_h, topk_ids, ld_ids, expert_map, (int)global_E, (int)E, (int)topk, (int)H, (int)I,
+                              plan.mapped, plan.hdr + 3, down};
+      if (g_prof_events[0]) cudaEventRecord(g_prof_events[0], st);
+      rc = launch_moe_small(cluster, bf, a, P, st);
+      if (rc != B200FP4_STATUS_SUCCESS) return rc;
+      if (g_prof_events[1]) cudaEventRecord(g_prof_events[1], st);
+      if (g_prof_events[2]) cudaEventRecord(g_prof_events[2], st);
+      launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, topk_weights, (const int*)plan.mapped,
+                 out, out_dtype, (int)M, (int)topk, (int)H, (flags & B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT) ? 1 : 0, ld_w, sc);
+      return finish_launch(2);
+    }
     launch_plan(topk_ids, P, topk, ld_ids, expert_map, global_E, E, plan, hidden, h16, M, H, ld_h, st, done, (int)n_done, 8,
                 bf ? kConvBf16Frag : kConvF16Frag);
     if (g_prof_events[0]) cudaEventRecord(g_prof_events[0], st);

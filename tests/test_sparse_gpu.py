@@ -381,3 +381,28 @@ def test_fused_moe_eight_token_passes(M, topk, E, H, I, separate):
     assert rel_err(to_np(out), ref) < TOL
     general = sp7.fused_sparse_moe_v7(hidden.cuda(), tw.cuda(), ids.cuda(), None, *c(w13), *c(w2), I, False, meta_ordered=False)
     assert rel_err(to_np(general), ref) < TOL
+
+
+@pytest.mark.parametrize("M,topk,E,H,I,dtype", [
+    (1, 10, 20, 2048, 512, torch.bfloat16),      # eight blocks to a pair, one gate_up group and two down groups each
+    (1, 3, 8, 128, 128, torch.float16),          # one down group, fewer steps than warps
+    (1, 2, 4, 3072, 256, torch.bfloat16),        # three down groups to a block, one warp without a share
+    (5, 4, 40, 512, 384, torch.float16),         # six gate_up groups
+    (10, 3, 64, 384, 640, torch.bfloat16),       # groups that do not divide by the blocks
+    (23, 2, 92, 256, 128, torch.float16),        # two blocks to a pair
+    (20, 4, 160, 256, 128, torch.bfloat16),      # one
+])
+def test_fused_moe_few_pairs(M, topk, E, H, I, dtype):
+    from dgx_vllm_b200 import _lib, sparse_fp4_v7 as sp7
+    w13, w2, tw, ids, hidden = _moe_case(E, H, I, M, topk, seed=M + E + H, dtype=dtype)
+    emap = np.arange(E, dtype=np.int32)
+    if M > 1:
+        emap[::5] = -1                            # experts of another rank
+        ids[0, 0], ids[M - 1, topk - 1] = -1, E + 3
+    n0 = _lib.lib().b200fp4_launch_count()
+    out = _run_fused(w13, w2, tw, ids, hidden, I, emap)
+    assert _lib.lib().b200fp4_launch_count() == n0 + 2 and sp7.last_moe_status() == 0
+    foreign = (ids < 0) | (ids >= E)
+    ref = _ref_fused(w13, w2, torch.where(foreign, torch.zeros_like(tw), tw), ids.clamp(0, E - 1), hidden, I, emap)
+    assert rel_err(to_np(out), ref) < TOL
+    assert torch.equal(out, _run_fused(w13, w2, tw, ids, hidden, I, emap))
