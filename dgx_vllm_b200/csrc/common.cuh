@@ -32,6 +32,11 @@ inline int finish_launch(int n_kernels) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+inline bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
 // cluster: blocks per cluster along x (1: plain blocks)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl_cluster(int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
@@ -52,8 +57,7 @@ inline cudaError_t launch_pdl_cluster(int cluster, void (*kernel)(KArgs...), dim
   }
   // not while a CUDA graph is being captured: replayed graphs have no launch gap to hide, and the 48-layer decode stack
   // measured 3-4 % slower with programmatic edges than with plain ones
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+  if (!stream_capturing(st)) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;

@@ -393,8 +393,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const uint8_t
   cfg.gridDim = dim3((unsigned)(2 * pairs));
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // as in launch_pdl
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cfg.numAttrs = (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ? 2 : 1;
+  cfg.numAttrs = stream_capturing(st) ? 1 : 2;
   if (cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel, ma, mb, p) != cudaSuccess) {
     cudaGetLastError();
     return B200FP4_STATUS_EXECUTION_FAILED;

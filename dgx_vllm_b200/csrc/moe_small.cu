@@ -82,10 +82,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
   int e = a.ids[(int64_t)m * a.ids_ld + (pair - m * a.topk)];
   if (a.expert_map != nullptr) e = (e >= 0 && e < a.global_E) ? a.expert_map[e] : -1;
   if (e < 0 || e >= a.E) e = -1;
-  if (rank == 0 && threadIdx.x == 0) {
-    a.mapped[pair] = e;
-    if (pair == 0) *a.status = 0;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0;
   if (e < 0) {                                     // the same for all blocks of the cluster
     cluster_wait();
     return;

@@ -13,9 +13,8 @@ struct MoeSmallArgs {
   int64_t ids_ld;
   const int32_t* expert_map;
   int global_E, E, topk, H, I;
-  int* mapped;                      // [P]: written, the expert of each pair or -1
   int* status;                      // status word of the layer: cleared
-  float* down;                      // [P, H]: written
+  float* down;                      // [P, H]: written, but for the rows of experts that are not local
 };
 
 // Blocks per pair, or 0 where the general path is to be taken.  Both projections in the layout of the warp-scheduled kernels, ordered metadata.

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kPlanThreads)
     moe_plan_kernel(const int32_t* __restrict__ ids, int P, const int32_t* __restrict__ expert_map, int global_E, int E,
                     Plan plan, const void* __restrict__ conv_src_v, __half* __restrict__ conv_dst,
                     int64_t conv_chunks, int ids_topk, int64_t ids_ld, int64_t conv_row_chunks, int64_t conv_ld_chunks,
-                    int* zero_buf, int zero_count, int max_tok, int conv_mode) {
+                    int* zero_buf, int zero_count, int max_tok, int conv_mode, int conv_block) {
   pdl_wait();                 // the kernel before this one may still be reading the workspace this one rewrites
   pdl_launch_dependents();
   if (blockIdx.x > 0) {
@@ -182,22 +182,25 @@ __global__ void __launch_bounds__(kPlanThreads)
             make_uint4(bf16x2_to_f16x2(raw.x), bf16x2_to_f16x2(raw.y), bf16x2_to_f16x2(raw.z), bf16x2_to_f16x2(raw.w));
       }
     } else {
-      // one thread per group of 32 elements: four 16-byte loads, a 4 x 4 word transpose, four 16-byte stores
-      const int64_t groups = conv_chunks >> 2, row_groups = conv_row_chunks >> 2;
-      for (int64_t i = (int64_t)(blockIdx.x - 1) * kPlanThreads + threadIdx.x; i < groups; i += stride) {
-        const int64_t row = i / row_groups, col = i - row * row_groups;
-        uint4 r[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          r[k] = conv_src[row * conv_ld_chunks + col * 4 + k];
-          if (conv_mode == kConvBf16Frag)
-            r[k] = make_uint4(bf16x2_to_f16x2(r[k].x), bf16x2_to_f16x2(r[k].y), bf16x2_to_f16x2(r[k].z), bf16x2_to_f16x2(r[k].w));
+      // A quad of lanes per group of 32 elements: a 16-byte load each, the 4 x 4 word transpose by shuffles, a 16-byte store each.
+      // (A thread per group, 64 bytes in and out, left the copy of 32 tokens to two SMs.)
+      const int lane = threadIdx.x & 31;
+      for (int64_t i0 = (int64_t)(blockIdx.x - 1) * conv_block; i0 < conv_chunks; i0 += (int64_t)(gridDim.x - 1) * conv_block) {
+        for (int j = threadIdx.x; j < conv_block; j += kPlanThreads) {       // whole warps: conv_block is a multiple of 32
+          const int64_t i = i0 + j, row = i / conv_row_chunks, col = i - row * conv_row_chunks;
+          uint4 v = make_uint4(0, 0, 0, 0);
+          if (i < conv_chunks) {
+            v = conv_src[row * conv_ld_chunks + col];
+            if (conv_mode == kConvBf16Frag) v = make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
+          }
+          const bool odd = lane & 1, high = lane & 2;
+          uint32_t got0 = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1), got1 = __shfl_xor_sync(0xffffffffu, odd ? v.z : v.w, 1);
+          v = odd ? make_uint4(got0, v.y, got1, v.w) : make_uint4(v.x, got0, v.z, got1);
+          got0 = __shfl_xor_sync(0xffffffffu, high ? v.x : v.z, 2);
+          got1 = __shfl_xor_sync(0xffffffffu, high ? v.y : v.w, 2);
+          v = high ? make_uint4(got0, got1, v.z, v.w) : make_uint4(v.x, v.y, got0, got1);
+          if (i < conv_chunks) reinterpret_cast<uint4*>(conv_dst)[i] = v;
         }
-        uint4* dst = reinterpret_cast<uint4*>(conv_dst) + i * 4;
-        dst[0] = make_uint4(r[0].x, r[1].x, r[2].x, r[3].x);
-        dst[1] = make_uint4(r[0].y, r[1].y, r[2].y, r[3].y);
-        dst[2] = make_uint4(r[0].z, r[1].z, r[2].z, r[3].z);
-        dst[3] = make_uint4(r[0].w, r[1].w, r[2].w, r[3].w);
       }
     }
     return;
@@ -1431,37 +1434,53 @@ struct OutScatter {
 };
 
 // out[m, h] = sum_t weight(m,t) * down[m*topk + t, h] over pairs whose expert is local.
-// One thread = four columns of one token; the rows of eight slots are requested before the first is used (the kernel is
-// pure latency: 2.6 MB at batch 32), the sum runs in slot order.  H % 4 == 0.
+// One thread = four columns of one token; the rows of sixteen slots are requested before the first is used (the kernel is
+// pure latency: 2.6 MB at batch 32), the sum runs in slot order.  H % 4 == 0.  Which slots count and with what weight is read while the
+// kernel before still runs: ids and weights are arguments of the layer, written before its first kernel.
 constexpr int kRedThreads = 128;
+constexpr int kRedSlots = 16;
+struct RedRouting {
+  const float* topk_w;
+  const int32_t* ids;
+  const int32_t* expert_map;
+  int64_t ld_w, ld_ids;
+  int topk, global_E, E, unweighted;
+};
+__device__ __forceinline__ float slot_weight(const RedRouting& r, int m, int t, bool& on) {
+  on = false;
+  if (t >= r.topk) return 0.f;
+  int e = __ldcg(r.ids + (int64_t)m * r.ld_ids + t);
+  if (r.expert_map != nullptr) e = (e >= 0 && e < r.global_E) ? __ldcg(r.expert_map + e) : -1;
+  on = e >= 0 && e < r.E;
+  return r.unweighted ? 1.0f : __ldcg(r.topk_w + (int64_t)m * r.ld_w + t);
+}
 __global__ void __launch_bounds__(kRedThreads)
-    weighted_reduce_kernel(const float* __restrict__ down, const float* __restrict__ topk_w, const int* __restrict__ mapped,
-                           void* out, int out_dtype, int M, int topk, int H, int unweighted, int64_t ld_w, OutScatter sc) {
+    weighted_reduce_kernel(const float* __restrict__ down, const RedRouting r, void* out, int out_dtype, int M, int H, OutScatter sc) {
+  const int h = (blockIdx.x * kRedThreads + threadIdx.x) * 4, m_src = blockIdx.y, topk = r.topk;
+  float w[kRedSlots];
+  bool on[kRedSlots];
+#pragma unroll
+  for (int i = 0; i < kRedSlots; ++i) w[i] = slot_weight(r, m_src, i, on[i]);
   pdl_wait();
   pdl_launch_dependents();
-  const int h = (blockIdx.x * kRedThreads + threadIdx.x) * 4;
-  int m = blockIdx.y;
+  int m = m_src;
   if (sc.status_out != nullptr && h == 0 && m == 0) *sc.status_out = *sc.status_src;
-  if (h >= H || m >= M) return;
-  const int m_src = m;
+  if (h >= H) return;
   if (sc.ptrs != nullptr) {
     out = sc.ptrs[m / sc.rows_per_dest];
     m = sc.dest_row0 + m % sc.rows_per_dest;
   }
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int t0 = 0; t0 < topk; t0 += 8) {
-    float4 v[8];
-    float w[8];
+  for (int t0 = 0; t0 < topk; t0 += kRedSlots) {
+    float4 v[kRedSlots];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int t = t0 + i;
-      const int p = m_src * topk + t;
-      const bool on = t < topk && mapped[p] >= 0;
-      v[i] = on ? *reinterpret_cast<const float4*>(down + (int64_t)p * H + h) : make_float4(0.f, 0.f, 0.f, 0.f);
-      w[i] = on ? (unweighted ? 1.0f : topk_w[(int64_t)m_src * ld_w + t]) : 0.f;
+    for (int i = 0; i < kRedSlots; ++i) {
+      if (t0 > 0) w[i] = slot_weight(r, m_src, t0 + i, on[i]);
+      v[i] = on[i] ? *reinterpret_cast<const float4*>(down + ((int64_t)m_src * topk + t0 + i) * H + h) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kRedSlots; ++i) {
+      if (!on[i]) continue;
       a.x += v[i].x * w[i];
       a.y += v[i].y * w[i];
       a.z += v[i].z * w[i];
@@ -1810,16 +1829,19 @@ void launch_plan(const int32_t* ids, int64_t P, int64_t ids_topk, int64_t ids_ld
                  int max_tok = kMaxTok, int conv_mode = kConvBf16) {
   int64_t chunks = 0;
   unsigned blocks = 1;
+  int conv_block = kPlanThreads;      // 16-byte chunks a block copies at a time
   if (a_src == nullptr) conv_mode = kConvNone;
   if (conv_mode != kConvNone) {
     chunks = a_rows * a_cols / 8;
-    int64_t nb = (chunks + kPlanThreads - 1) / kPlanThreads;
+    // in fragment order few chunks are spread over the SMs
+    if (conv_mode != kConvBf16 && chunks <= 64 * 256) conv_block = 256;
+    int64_t nb = (chunks + conv_block - 1) / conv_block;
     if (nb > 2 * (int64_t)sm_count()) nb = 2 * (int64_t)sm_count();
     blocks += (unsigned)(nb < 1 ? 1 : nb);
   }
   launch_pdl(moe_plan_kernel, dim3(blocks), dim3(kPlanThreads), 0, st, ids, (int)P, expert_map, (int)global_E, (int)E, plan,
              a_src, a_f16, chunks, (int)ids_topk, ids_ld, a_cols / 8 > 0 ? a_cols / 8 : (int64_t)1, a_ld / 8, zero_buf, zero_count,
-             max_tok, conv_mode);
+             max_tok, conv_mode, conv_block);
 }
 
 // Runs one projection for P pairs with a plan already in `plan`.  A is fp16.
@@ -2141,6 +2163,7 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   off += align_up((size_t)P * H * sizeof(float), 256);
   int* done = reinterpret_cast<int*>(ws + off);
   const int64_t n_done = max_passes(P, E);
+  const RedRouting routing = {topk_weights, topk_ids, expert_map, ld_w, ld_ids, (int)topk, (int)global_E, (int)E, (flags & B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT) ? 1 : 0};
   const int64_t local_pairs = (expert_map && global_E > 0) ? P * E / global_E : P;      // expected
 
   // The warp-scheduled tensor-core kernel (passes of eight tokens, activations in fragment order from the plan kernel and
@@ -2151,14 +2174,13 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
     const int cluster = (flags & B200FP4_MOE_SEPARATE_LAUNCHES) || 2 * local_pairs > E ? 0 : moe_small_cluster(P, H, I);
     if (cluster > 0) {
       const MoeSmallArgs a = {w13, w2, hidden, ld_h, topk_ids, ld_ids, expert_map, (int)global_E, (int)E, (int)topk, (int)H, (int)I,
-                              plan.mapped, plan.hdr + 3, down};
+                              plan.hdr + 3, down};
       if (g_prof_events[0]) cudaEventRecord(g_prof_events[0], st);
       rc = launch_moe_small(cluster, bf, a, P, st);
       if (rc != B200FP4_STATUS_SUCCESS) return rc;
       if (g_prof_events[1]) cudaEventRecord(g_prof_events[1], st);
       if (g_prof_events[2]) cudaEventRecord(g_prof_events[2], st);
-      launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, topk_weights, (const int*)plan.mapped,
-                 out, out_dtype, (int)M, (int)topk, (int)H, (flags & B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT) ? 1 : 0, ld_w, sc);
+      launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, routing, out, out_dtype, (int)M, (int)H, sc);
       return finish_launch(2);
     }
     launch_plan(topk_ids, P, topk, ld_ids, expert_map, global_E, E, plan, hidden, h16, M, H, ld_h, st, done, (int)n_done, 8,
@@ -2180,8 +2202,7 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
       if (rc != B200FP4_STATUS_SUCCESS) return rc;
     }
     if (g_prof_events[2]) cudaEventRecord(g_prof_events[2], st);
-    launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, topk_weights, (const int*)plan.mapped,
-               out, out_dtype, (int)M, (int)topk, (int)H, (flags & B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT) ? 1 : 0, ld_w, sc);
+    launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, routing, out, out_dtype, (int)M, (int)H, sc);
     return finish_launch((flags & B200FP4_MOE_SEPARATE_LAUNCHES) ? 4 : 3);
   }
 
@@ -2204,8 +2225,7 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   rc = run_projection(w2, plan, act, I, 1, down, B200FP4_DTYPE_F32, H, P, H, I, G2, E, 0, ordered, st, tm);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   if (g_prof_events[2]) cudaEventRecord(g_prof_events[2], st);
-  launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, topk_weights, (const int*)plan.mapped, out,
-             out_dtype, (int)M, (int)topk, (int)H, (flags & B200FP4_MOE_ROUTER_WEIGHT_ON_INPUT) ? 1 : 0, ld_w, sc);
+  launch_pdl(weighted_reduce_kernel, reduce_grid(H, M), dim3(kRedThreads), 0, st, (const float*)down, routing, out, out_dtype, (int)M, (int)H, sc);
   return finish_launch(4);
 }
 
