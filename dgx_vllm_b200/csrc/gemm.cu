@@ -548,7 +548,8 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
       }
       if constexpr (kSplit > 1) {
         // 32-column chunk c of the tile belongs to CTA c * kSplit / 4: kept if that is this one, sent there otherwise as
-        // [sender][chunk][quarter][column][row] so that a warp's store of one column is 128 contiguous bytes
+        // [sender][chunk][quarter][four columns][row]: a warp's store of four columns is 512 contiguous bytes (a column at a time, 128 bytes,
+        // the exchange took four times as many stores to another SM)
         constexpr int kOwn = 4 / kSplit;
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
@@ -561,10 +562,13 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
             for (int i = 0; i < 32; ++i) keep[(kOwn == 1 ? 0 : c * 32) + i] = __uint_as_float(r[i]);
           } else if (row < ti.row_end) {
             const int slot = rank < owner ? rank : rank - 1;
-            const uint32_t dst = map_to_cta(smem_u32(out_stage) + (uint32_t)((slot * kOwn + chunk % kOwn) * 4 + quarter) * 4096u + lane * 4u,
+            const uint32_t dst = map_to_cta(smem_u32(out_stage) + (uint32_t)((slot * kOwn + chunk % kOwn) * 4 + quarter) * 4096u + lane * 16u,
                                             (uint32_t)owner);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + i * 128u), "r"(r[i]) : "memory");
+            for (int i = 0; i < 8; ++i)
+              asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + i * 512u), "r"(r[4 * i]), "r"(r[4 * i + 1]),
+                           "r"(r[4 * i + 2]), "r"(r[4 * i + 3])
+                           : "memory");
           }
         }
         continue;
@@ -708,17 +712,27 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         for (int c = 0; c < kOwn; ++c) {
           float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float sum = 0.f;
+          for (int i = 0; i < 32; ++i) v[i] = 0.f;
 #pragma unroll
-            for (int src = 0; src < kSplit; ++src) {         // in the order of K
+          for (int src = 0; src < kSplit; ++src) {           // in the order of K
+            if (src == rank) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] += keep[c * 32 + i];
+            } else {
               const int slot = src < rank ? src : src - 1;
-              sum += src == rank ? keep[c * 32 + i]
-                                 : __uint_as_float(lds32(smem_u32(out_stage) + (uint32_t)((slot * kOwn + c) * 4 + quarter) * 4096u +
-                                                         (uint32_t)i * 128u + lane * 4u));
+              const uint32_t at = smem_u32(out_stage) + (uint32_t)((slot * kOwn + c) * 4 + quarter) * 4096u + lane * 16u;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint4 x = lds128(at + i * 512u);
+                v[4 * i] += __uint_as_float(x.x);
+                v[4 * i + 1] += __uint_as_float(x.y);
+                v[4 * i + 2] += __uint_as_float(x.z);
+                v[4 * i + 3] += __uint_as_float(x.w);
+              }
             }
-            v[i] = sum * alpha;
           }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] *= alpha;
           store_row32(p, row, ti.n0 + (rank * kOwn + c) * 32, v);
         }
       }
@@ -935,10 +949,16 @@ void pick_dense_tile(int64_t M, int64_t N, int64_t stages, bool f32, int& bn, in
   const double pair = 3.8 + rounds(m256 * n256, sms / 2) * (0.46 * S + 1.6 + (N % 16 != 0 ? 1.5 : 0.0));
   bn = wide < narrow ? 256 : 128;
   if (!f32 && pair < (wide < narrow ? wide : narrow)) bn = 512;
+  // Splitting K costs 1 to 2 us (the exchange, and clusters to place) and saves time by stage: over four CTAs it pays from eight stages on, as
+  // far as the clusters run at once, over two from sixteen, or from 22 where there are tiles for more than a third of the SMs.  us with one / two /
+  // four CTAs: 471x1672x1216 (56 tiles, 5 stages) 8.2 / 9.2 / -; 512x2048x2048 (64, 8) 8.9 / 10.6 / -; 93x1960x2560 (16, 10) 9.0 / 8.8 / 8.4;
+  // 323x1536x7616 (36, 30; 36 clusters of four are more than run at once) 15.6 / 13.3 / 18.2; 152x2456x7168 (40, 28) 16.7 / 14.0 / -;
+  // 320x2192x5760 (54, 23) 14.2 / 14.0 / -; 300x1024x8192 (24, 32) 15.9 / 12.5 / 12.3.
   split = 1;
-  if (bn == 128 && stages >= 4) {
-    if (m128 * n128 * 4 <= sms && stages >= 8) split = 4;
-    else if (m128 * n128 * 2 <= sms) split = 2;
+  if (bn == 128 && stages >= 8) {
+    const int64_t tiles = m128 * n128;
+    if (tiles <= resident_clusters(4)) split = 4;
+    else if (tiles * 2 <= sms && stages >= (tiles * 3 <= sms ? 16 : 22)) split = 2;
   }
 }
 

@@ -79,12 +79,6 @@ __device__ __forceinline__ void tcgen05_ld_32x8(uint32_t taddr, uint32_t (&r)[8]
                : "memory");
 }
 
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ void store_one(const SmallParams& p, int m, int n, float v) {
   const size_t at = (size_t)m * p.N + n;
   if (p.out_dtype == B200FP4_DTYPE_BF16) static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(v);
@@ -376,7 +370,28 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Clusters of k CTAs that are resident at once, one CTA per SM
+template <typename T, bool kCodes>
+int launch_small_t(const CUtensorMap& mw, const SmallParams& p, unsigned grid, size_t smem, cudaStream_t st) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return B200FP4_STATUS_NOT_SUPPORTED;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(nvfp4_small_kernel<T, kCodes>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost) != cudaSuccess) {
+      cudaGetLastError();
+      return B200FP4_STATUS_EXECUTION_FAILED;
+    }
+    attr_set[dev] = true;
+  }
+  if (launch_pdl_cluster(p.split, nvfp4_small_kernel<T, kCodes>, dim3(grid), dim3(kThreads), smem, st, mw, p) != cudaSuccess) {
+    cudaGetLastError();
+    return B200FP4_STATUS_EXECUTION_FAILED;
+  }
+  return finish_launch(1);
+}
+
+}  // namespace
+
 int resident_clusters(int k) {
   struct PerDevice {
     std::once_flag once;
@@ -408,28 +423,6 @@ int resident_clusters(int k) {
   });
   return d.n[k];
 }
-
-template <typename T, bool kCodes>
-int launch_small_t(const CUtensorMap& mw, const SmallParams& p, unsigned grid, size_t smem, cudaStream_t st) {
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return B200FP4_STATUS_NOT_SUPPORTED;
-  if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(nvfp4_small_kernel<T, kCodes>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost) != cudaSuccess) {
-      cudaGetLastError();
-      return B200FP4_STATUS_EXECUTION_FAILED;
-    }
-    attr_set[dev] = true;
-  }
-  if (launch_pdl_cluster(p.split, nvfp4_small_kernel<T, kCodes>, dim3(grid), dim3(kThreads), smem, st, mw, p) != cudaSuccess) {
-    cudaGetLastError();
-    return B200FP4_STATUS_EXECUTION_FAILED;
-  }
-  return finish_launch(1);
-}
-
-}  // namespace
 
 SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K) {
   SmallPlan s = {};

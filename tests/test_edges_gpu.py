@@ -169,6 +169,9 @@ def _linear_operands(M, N, K, seed):
     (8, 264, 64),             # a single short stage
     (128, 14336, 1024),       # narrow tiles, fewer stages than the ring holds
     (385, 6000, 1088),        # wide tiles; the columns of the second scale tile lie past N
+    (70, 136, 2112),          # more tokens than the few-token kernel takes: split over four, nine stages, the last one short
+    (130, 2304, 4160),        # ... over two, 36 tiles of 17 stages
+    (72, 264, 64),            # ... a single short stage
 ])
 def test_linear_early_weights(M, N, K):
     from dgx_vllm_b200 import cutlass_scaled_fp4_mm, scaled_fp4_quant
