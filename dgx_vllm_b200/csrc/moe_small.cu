@@ -87,29 +87,48 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
     cluster_wait();
     return;
   }
-  const uint8_t* c13 = a.w13.comp + (int64_t)e * a.w13.comp_e + (int64_t)fr * N13 + col_a;
-  const uint8_t* m13 = a.w13.meta + (int64_t)e * a.w13.meta_e + (int64_t)fr * N13 + col_a;
-  const uint8_t* s13 = a.w13.scale + (int64_t)e * a.w13.scale_e + (int64_t)fr * N13 + col_a;
-  const uint8_t* c2 = a.w2.comp + (int64_t)e * a.w2.comp_e + (int64_t)fr * H + col_b;
-  const uint8_t* m2 = a.w2.meta + (int64_t)e * a.w2.meta_e + (int64_t)fr * H + col_b;
-  const uint8_t* s2 = a.w2.scale + (int64_t)e * a.w2.scale_e + (int64_t)fr * H + col_b;
-  // steps 0 .. n_a - 1 are the gate_up projection's, the rest the down projection's; always one commit group, so that the wait counts
-  // stay fixed
-  auto fetch = [&](int j) {
-    if (j < n_a + n_b) {
-      const bool first = j < n_a;
-      const int step = first ? a_slice + j * sh.wa : b_slice + (j - n_a) * sh.wb, N = first ? N13 : H;
-      const uint32_t dst = ring + (uint32_t)(j % kSlots) * kStage;
-      const uint8_t* c = (first ? c13 : c2) + (int64_t)step * 8 * N;
-      cp_async16_s(dst + d_comp, c);
-      cp_async16_s(dst + 512u + d_comp, c + (int64_t)4 * N);
-      cp_async16_s(dst + d_meta, (first ? m13 : m2) + (int64_t)step * 4 * N);
-      if (lane < 16) cp_async16_s(dst + d_scale, (first ? s13 : s2) + (int64_t)step * 2 * N);
+  // The stream of this warp's steps: those of the gate_up projection, then those of the down projection.  Where its next copies come from and
+  // go to, and how far apart the steps of the projection lie; always one commit group a step, so that the wait counts stay fixed.
+  struct Stream {
+    const uint8_t *comp, *meta, *scale;
+    int64_t comp_step, half;          // bytes between steps and between compressed rows 0 and 4 of one; metadata 1/2, scales 1/4 of that
+    int left, then;                   // steps of this projection, of the next
+    uint32_t slot;
+  } f;
+  auto start = [&](const SparseWeights& w, int N, int col, int first, int stride) {
+    const int64_t lane_off = (int64_t)fr * N + col;
+    f.comp = w.comp + (int64_t)e * w.comp_e + (int64_t)first * 8 * N + lane_off;
+    f.meta = w.meta + (int64_t)e * w.meta_e + (int64_t)first * 4 * N + lane_off;
+    f.scale = w.scale + (int64_t)e * w.scale_e + (int64_t)first * 2 * N + lane_off;
+    f.comp_step = (int64_t)stride * 8 * N;
+    f.half = (int64_t)4 * N;
+  };
+  start(a.w13, N13, col_a, a_slice, sh.wa);
+  f.left = n_a;
+  f.then = n_b;
+  f.slot = ring;
+  const uint32_t ring_end = ring + kSlots * kStage;
+  auto fetch = [&]() {
+    if (f.left == 0 && f.then > 0) {
+      start(a.w2, H, col_b, b_slice, sh.wb);
+      f.left = f.then;
+      f.then = 0;
     }
+    if (f.left > 0) {
+      cp_async16_s(f.slot + d_comp, f.comp);
+      cp_async16_s(f.slot + 512u + d_comp, f.comp + f.half);
+      cp_async16_s(f.slot + d_meta, f.meta);
+      if (lane < 16) cp_async16_s(f.slot + d_scale, f.scale);
+      f.comp += f.comp_step;
+      f.meta += f.comp_step >> 1;
+      f.scale += f.comp_step >> 2;
+      --f.left;
+    }
+    f.slot = f.slot + kStage == ring_end ? ring : f.slot + kStage;
     cp_async_commit();
   };
 #pragma unroll 1
-  for (int j = 0; j < kSlots; ++j) fetch(j);
+  for (int j = 0; j < kSlots; ++j) fetch();
   const float g13 = a.w13.g[e], g2 = a.w2.g[e];
   // the token's activations as f16 in fragment order
 #pragma unroll
@@ -131,15 +150,14 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
   const uint32_t off_meta = 1024u + (uint32_t)(2 * (t & 1)) * 128u + (uint32_t)((q ^ (4 * (t & 1))) << 4) + (uint32_t)(t >> 1) * 8u;
   const uint32_t off_scale = 1536u + (uint32_t)q * 16u;
   float acc[8][4];
-  int j = 0;
-  auto project = [&](uint32_t x, int first_step, int stride, int n) {
+  uint32_t st = ring;
+  auto project = [&](uint32_t x, int stride, int n) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 #pragma unroll 1
-    for (int s = 0; s < n; ++s, ++j) {
+    for (int s = 0; s < n; ++s, x += (uint32_t)stride * 64u) {
       cp_async_wait<kSlots - 1>();
       __syncwarp();
-      const uint32_t st = ring + (uint32_t)(j % kSlots) * kStage;
       WsStep w;
       w.v0 = lds128_at(st + off_comp);
       w.v1 = lds128_at(st + off_comp + 512u);
@@ -147,9 +165,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
       w.m1 = lds64_at(st + off_meta + 128u);
       w.s0 = lds128_at(st + off_scale);
       w.s1 = lds128_at(st + off_scale + 128u);
-      w.b = lds128_at(x + (uint32_t)(first_step + s * stride) * 64u + (uint32_t)t * 16u);
+      w.b = lds128_at(x);
       __syncwarp();                                // all lanes have read the slot
-      fetch(j + kSlots);
+      fetch();
+      st = st + kStage == ring_end ? ring : st + kStage;
       ws_mma_step(acc, w);
     }
     // The sums of this warp's slice, 128 columns: column 2h + r of a quad's 16 is element 2r of mma kJ[h] in the quad's first lane.
@@ -171,7 +190,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
     return v;
   };
 
-  project(xs, a_slice, sh.wa, n_a);
+  project(xs + (uint32_t)a_slice * 64u + (uint32_t)t * 16u, sh.wa, n_a);
   cluster_wait();
   {
     // a warp finishes four columns at a time: quads 0-3 sum the gate, 4-7 the up half
@@ -194,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
   __syncwarp();
   cluster_arrive();
   cluster_wait();                                  // all of the token's activations are here, and the partial sums have been read
-  project(acts, b_slice, sh.wb, n_b);
+  project(acts + (uint32_t)b_slice * 64u + (uint32_t)t * 16u, sh.wb, n_b);
   {
     const int used = min(sh.wb, I / 32);
     for (int i = warp; i < gb_here * 16; i += kWarps) {
@@ -260,9 +279,9 @@ int resident_clusters(int c) {
 
 // The cluster size with the fewest steps per warp of those whose clusters all run at once, if the layer is then expected to take less time
 // than on the general path.  Times fitted to B200, us per layer (pairs, H, I: general / here, blocks per pair):
-//   10, 2048, 512: 15.6 / 11.0, 8     20: 20.0 / 15.4, 6     40: 27.0 / 20.8, 3     60: 31.0 / 24.7, 2     112: 39.0 / 40.0, 1     140: 44.8 / 39.4, 1
-//   30, 4096, 1024: 44.3 / 38.6, 4    50, 4096, 768: 50.4 / 55.6, 2    80, 1024, 256: 18.5 / 14.4, 1    100, 2048, 1024: 56.4 / 66.7, 1
-// A block's time here is its warps' steps (16 of them take 0.64 us: instruction issue) and 8.5 us; the general path spreads all steps evenly over
+//   10, 2048, 512: 15.7 / 10.5, 8     20: 20.0 / 14.2, 6     40: 27.0 / 19.4, 3     60: 31.0 / 23.5, 2     120: 40.5 / 37.6, 1     140: 44.8 / 39.3, 1
+//   30, 4096, 1024: 44.3 / 35.3, 4    50, 4096, 768: 50.4 / 55.6, 2    80, 1024, 256: 18.5 / 14.4, 1    100, 2048, 1024: 56.4 / 66.7, 1
+// A block's time here is its warps' steps (one of all 16 warps takes 0.58 us: instruction issue) and 8.5 us; the general path spreads all steps evenly over
 // the SMs, at four warps a scheduler, and takes 20 us beside (less for a few pairs).
 int moe_small_cluster(int64_t P, int64_t H, int64_t I) {
   if (P < 1 || H > kMaxWidth || I > kMaxWidth) return 0;
@@ -278,7 +297,7 @@ int moe_small_cluster(int64_t P, int64_t H, int64_t I) {
     }
   }
   const double all = (double)P * (double)(H / 32) * (double)(I / 32) * 0.75;              // steps of both projections: H/32 I/64 + I/32 H/128
-  const double here = 0.64 * (double)best_steps + 8.5, general = 0.000215 * all + (P < 20 ? 13.0 + 0.35 * (double)P : 20.0);
+  const double here = 0.58 * (double)best_steps + 8.5, general = 0.000215 * all + (P < 20 ? 13.0 + 0.35 * (double)P : 20.0);
   return best > 0 && here < general ? best : 0;
 }
 

@@ -80,9 +80,8 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
 }
 
 // One lane of a warp that is together: the copies, MMAs and commits of a loop are issued under this predicate, the loop and its
-// waits run by all lanes.  A loop entered by one lane only (if (lane == 0)) costs the issuing warp twice the time: the operands of these
-// instructions are uniform registers, which the compiler fills by a vote over the active lanes wherever it does not know that
-// the warp is together (a stage of wait, fence, four MMAs and a commit: 460 cycles so, 250-270 with the warp together; B200).
+// waits run by all lanes.  A loop entered by one lane only (if (lane == 0)) costs the issuing warp nearly twice the time: a stage of wait,
+// fence, four MMAs and a commit 460 cycles, 250-270 with the warp together (B200; N = 8, operands in place).
 __device__ __forceinline__ bool elect_one() {
   uint32_t e;
   asm volatile(
