@@ -957,7 +957,7 @@ void pick_dense_tile(int64_t M, int64_t N, int64_t stages, bool f32, int& bn, in
   split = 1;
   if (bn == 128 && stages >= 8) {
     const int64_t tiles = m128 * n128;
-    if (tiles <= resident_clusters(4)) split = 4;
+    if (tiles * 4 <= sms && tiles <= resident_clusters(4)) split = 4;
     else if (tiles * 2 <= sms && stages >= (tiles * 3 <= sms ? 16 : 22)) split = 2;
   }
 }

@@ -393,35 +393,33 @@ int launch_small_t(const CUtensorMap& mw, const SmallParams& p, unsigned grid, s
 }  // namespace
 
 int resident_clusters(int k) {
-  struct PerDevice {
+  struct Count {
     std::once_flag once;
-    int n[kMaxSplit + 1] = {0};
+    int n = 0;
   };
-  static PerDevice devices[64];
+  static Count counts[64][kMaxSplit + 1];      // asked for when first needed: a query takes some microseconds
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  PerDevice& d = devices[dev];
-  std::call_once(d.once, [&] {
+  if (k < 2 || k > kMaxSplit || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  Count& c = counts[dev][k];
+  std::call_once(c.once, [&] {
     auto* kernel = nvfp4_small_kernel<__nv_bfloat16, false>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost);
-    for (int c = 2; c <= kMaxSplit; ++c) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)c);
-      cfg.blockDim = dim3(kThreads);
-      cfg.dynamicSmemBytes = kSmemMost;
-      cudaLaunchAttribute attr;
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = (unsigned)c;
-      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&d.n[c], kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        d.n[c] = 0;
-      }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)k);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemMost;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)k;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&c.n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      c.n = 0;
     }
   });
-  return d.n[k];
+  return c.n;
 }
 
 SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K) {
@@ -432,7 +430,7 @@ SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K) {
   // eight; a 16th waits for the others: M=33, N=K=2048 11.8 us, 7.2 so).  Fewer than four stages are not split.
   int split = 1;
   for (int k = 2; k <= kMaxSplit && stages >= 4 && k <= stages; ++k)
-    if (tiles <= resident_clusters(k)) split = k;
+    if (tiles * k <= sms && tiles <= resident_clusters(k)) split = k;
   const int own = (int)((stages + split - 1) / split), m_pad = (int)(M + 7) / 8 * 8;
   if (own > kMaxStages) return s;
   // Every CTA quantizes its part of K for all tokens (a block of 16 takes an SM 1.4 cycles), where the general path does that once:

@@ -248,31 +248,33 @@ bool prepare() {
   return ok[dev];
 }
 
-// Clusters of c blocks that are resident at once
+// Clusters of c blocks that are resident at once; asked for when first needed
 int resident_clusters(int c) {
-  static std::once_flag once[64];
-  static int n[64][kMaxCluster + 1] = {};
+  struct Count {
+    std::once_flag once;
+    int n = 0;
+  };
+  static Count counts[64][kMaxCluster + 1];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !prepare<true>()) return 0;
-  std::call_once(once[dev], [&] {
-    for (int k = 1; k <= kMaxCluster; ++k) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)k);
-      cfg.blockDim = dim3(kThreads);
-      cfg.dynamicSmemBytes = small_smem(kMaxWidth, kMaxWidth);
-      cudaLaunchAttribute attr;
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = (unsigned)k;
-      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&n[dev][k], moe_small_kernel<true>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n[dev][k] = 0;
-      }
+  Count& count = counts[dev][c];
+  std::call_once(count.once, [&] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = small_smem(kMaxWidth, kMaxWidth);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)c;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&count.n, moe_small_kernel<true>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      count.n = 0;
     }
   });
-  return n[dev][c];
+  return count.n;
 }
 
 }  // namespace
@@ -289,7 +291,7 @@ int moe_small_cluster(int64_t P, int64_t H, int64_t I) {
   int64_t best_steps = 0;
   for (int c = 1; c <= kMaxCluster; ++c) {
     const SmallShape s = shape_for(c, H, I);
-    if (s.ga > kWarps || s.gb > kWarps || P > resident_clusters(c)) continue;
+    if (s.ga > kWarps || s.gb > kWarps || P * c > sm_count() || P > resident_clusters(c)) continue;
     const int64_t steps = (H / 32 + s.wa - 1) / s.wa + (I / 32 + s.wb - 1) / s.wb;       // of a warp
     if (best == 0 || steps < best_steps) {
       best = c;

@@ -120,11 +120,13 @@ def test_fused_moe_block_shapes(E, H, I, M, topk):
 
 
 @pytest.mark.parametrize("M,N,K", [
-    (1, 8, 2048),             # split of K over four CTAs, one row and less than a 32-column piece
+    (1, 8, 2048),             # few tokens: K over eight CTAs, one row and less than a 32-column piece
     (33, 136, 2112),          # ... ragged everywhere, last k-stage short
-    (129, 1000, 4096),        # ... two row tiles
-    (5, 5000, 1024),          # split over two
-    (200, 4096, 1088),        # ... two row tiles
+    (129, 1000, 4096),        # split of K over four CTAs, two row tiles
+    (5, 5000, 1024),          # few tokens, over three
+    (200, 4096, 1088),        # five stages: no split
+    (70, 136, 2112),          # split over four, ragged everywhere, last k-stage short
+    (130, 2304, 4160),        # ... over two
     (8, 264, 768),            # three stages: no split
     (385, 6000, 1024),        # wide tiles, ragged
     (520, 7000, 2048),        # pairs of CTAs, ragged
@@ -162,11 +164,11 @@ def _linear_operands(M, N, K, seed):
 
 
 @pytest.mark.parametrize("M,N,K", [
-    (8, 512, 2048),           # split of K over four CTAs: every CTA requests its own first stages early
-    (33, 136, 2112),          # ... ragged, nine stages on four CTAs, the last one short
-    (129, 1000, 4096),        # ... two row tiles
-    (5, 5000, 1024),          # split over two
-    (8, 264, 64),             # a single short stage
+    (8, 512, 2048),           # few tokens: one kernel, K over eight CTAs
+    (33, 136, 2112),          # ... ragged, nine stages on eight CTAs, the last one short
+    (129, 1000, 4096),        # quantizer and GEMM, K split over four CTAs: every CTA requests its own first stages early
+    (5, 5000, 1024),          # few tokens, over three
+    (8, 264, 64),             # ... a single short stage
     (128, 14336, 1024),       # narrow tiles, fewer stages than the ring holds
     (385, 6000, 1088),        # wide tiles; the columns of the second scale tile lie past N
     (70, 136, 2112),          # more tokens than the few-token kernel takes: split over four, nine stages, the last one short
