@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
         ok = mbar_wait(smem_u32(&sf_full[s]), ph, p.status, 6);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
+        tcgen05_fence_after();                     // the copy waited for the commit of the MMAs that read this slot's columns, and so has this
         const unsigned char* sf = smem + (size_t)s * C::kStageBytes + C::kStageA + C::kStageB;
         const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + C::kSfBase + s * C::kSfCols;
         const int kblocks = min(KB, KT - ks * KB);

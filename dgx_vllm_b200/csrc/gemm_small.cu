@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int kb = 0; kb < 4; ++kb)
             w[kb] = make_uint4(lane < M ? lds32(src + kb * words * 128) : 0u, lane + 32 < M ? lds32(src + (kb * words + 1) * 128) : 0u, 0u, 0u);
         }
+        tcgen05_fence_after();                     // the slot's columns were read by MMAs whose commit these waits follow
         const uint32_t t0 = tmem_sf + lanes + t * 32 + (warp < 6 ? 0 : 16);
 #pragma unroll
         for (int kb = 0; kb < 4; ++kb) tcgen05_st_32x32_x4(t0 + kb * 4, w[kb]);

@@ -299,3 +299,23 @@ def test_torch_custom_ops_registered_with_fake_impls():
     assert tuple(codes.shape) == (200, 2048) and tuple(sf.shape) == (256, 256) and sf.dtype == torch.float8_e4m3fn
     with pytest.raises((RuntimeError, NotImplementedError)):
         ns.scaled_fp4_quant(torch.zeros(4, 16, dtype=torch.bfloat16), torch.ones(1), True)     # no CPU kernel
+
+
+def test_tensor_memory_accesses_follow_a_fence_after_their_wait():
+    """tcgen05 loads, stores and MMAs that an mbarrier wait orders after another thread's tcgen05 work need a
+    tcgen05.fence::after_thread_sync between the two: read off the kernels' source, since no run shows its absence."""
+    token = re.compile(r"\b(?:(?P<wait>mbar_wait(?:_warp)?)|(?P<fence>tcgen05_fence_after)|(?P<use>tcgen05_(?:st|ld|mma)_\w+|copy_sf<KB>))\(")
+    csrc, seen = os.path.join(ROOT, "dgx_vllm_b200", "csrc"), 0
+    for name in sorted(f for f in os.listdir(csrc) if f.endswith(".cu")):
+        waited = 0                                            # line of a wait with no fence behind it yet
+        for n, line in enumerate(open(os.path.join(csrc, name)), 1):
+            if "__device__" in line:                          # another function
+                waited = 0
+                continue
+            for m in token.finditer(line.split("//")[0]):
+                if m["use"]:
+                    seen += 1
+                    assert not waited, f"{name}:{n} after the wait in line {waited}"
+                else:
+                    waited = n if m["wait"] else 0
+    assert seen >= 20
