@@ -295,3 +295,17 @@ def test_few_token_linear(M, N, K, dtype):
     ref, size = (a @ b.t()) * alpha.double(), (a.abs() @ b.abs().t()) * alpha.double()
     half_ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
     assert bool(((out.double() - ref).abs() <= half_ulp * ref.abs() + 2.0 ** -20 * size + 2.0 ** -24).all())
+
+
+@pytest.mark.parametrize("gs", [-2688 / 6.5, 0.0])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_few_token_linear_any_global_scale(gs, dtype):
+    # scale bytes with the sign bit set, and the guard for zero: still the stand-alone quantizer's bytes
+    from dgx_vllm_b200 import cutlass_scaled_fp4_mm, scaled_fp4_quant
+    from dgx_vllm_b200.ops import nvfp4_linear
+    x, _, wc, ws, alpha = _linear_operands(9, 512, 2048, 5)
+    x, gx = x.to(dtype), torch.full((1,), gs, device="cuda")
+    x[0, :16] = 0.0
+    xc, xs = scaled_fp4_quant(x, gx)
+    out, want = nvfp4_linear(x, gx, wc, ws, alpha), cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype)
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
