@@ -309,3 +309,60 @@ def test_few_token_linear_any_global_scale(gs, dtype):
     xc, xs = scaled_fp4_quant(x, gx)
     out, want = nvfp4_linear(x, gx, wc, ws, alpha), cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype)
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("M,E,ranks,topk,launches", [
+    (1, 128, 1, 10, 2),           # few pairs: ids and map read by the sum
+    (2, 256, 8, 10, 2),           # ... on one of eight expert-parallel ranks, most pairs not local
+    (32, 64, 1, 10, 3),           # plan, one launch, sum
+    (256, 128, 8, 10, 3),         # ... one local slot of ten on average
+    (3, 64, 1, 32, 3),            # every lane of a warp holds a slot
+    (3, 64, 4, 40, 3),            # more slots than lanes
+])
+@pytest.mark.parametrize("written_by", ["router", "copies"])
+def test_layer_reads_the_routing_the_kernel_before_it_wrote(M, E, ranks, topk, launches, written_by):
+    # the sum looks at its routing before the kernel in front of it ends: ids and weights new for every call, eager and from a graph
+    import synth
+    from dgx_vllm_b200 import _lib, sparse_fp4_v7 as sp7
+    from dgx_vllm_b200.moe_ep import expert_map_for_rank
+    from dgx_vllm_b200.router import moe_router
+    from util import expert_fetch, gpu_quantize_fn, rel_err
+    if written_by == "router" and topk > 32:
+        pytest.skip("the router selects up to 32")
+    keys, H, I, here = ("comp_T", "meta_T", "scale_T", "g_scales"), 512, 256, E // ranks
+    w13 = synth.make_sparse_experts(here, 2 * I, H, 1, "cuda", gpu_quantize_fn)
+    w2 = synth.make_sparse_experts(here, H, I, 2, "cuda", gpu_quantize_fn)
+    emap = expert_map_for_rank(E, ranks, ranks - 1, "cuda") if ranks > 1 else None
+    layer = sp7.FusedSparseMoE(*[w13[k] for k in keys], *[w2[k] for k in keys], I, expert_map=emap)
+    gate = torch.randn(E, H, device="cuda", generator=torch.Generator(device="cuda").manual_seed(7)).mul_(H ** -0.5).bfloat16()
+    xs = [synth.make_hidden(M, H, 4 + s, "cuda") for s in range(2)]
+    routes = [moe_router(x, gate, topk) if topk <= 32 else synth.make_routing(M, E, topk, 8 + s, "cuda") for s, x in enumerate(xs)]
+    torch.cuda.synchronize()
+    n0 = _lib.lib().b200fp4_launch_count()
+    want = [layer(x, *r) for x, r in zip(xs, routes)]
+    assert _lib.lib().b200fp4_launch_count() == n0 + 2 * launches
+    for x, (tw, ids), got in zip(xs, routes, want):
+        local = ids if emap is None else emap[ids.long()]
+        ref = oracle.fused_sparse_moe_by_expert(x.float().cpu().numpy(), tw.cpu().numpy(), local.cpu().numpy(), expert_fetch(w13, w2), I)
+        assert rel_err(to_np(got), ref) < 1e-2
+    tw, ids = torch.zeros_like(routes[0][0]), torch.zeros_like(routes[0][1])
+
+    def step(i):
+        if written_by == "router":
+            return layer(xs[i % 2], *moe_router(xs[i % 2], gate, topk))
+        tw.copy_(routes[i % 2][0])
+        ids.copy_(routes[i % 2][1])
+        return layer(xs[i % 2], tw, ids)
+
+    torch.cuda.synchronize()
+    torch.cuda._sleep(4_000_000)                      # everything below is queued before the first of it runs
+    got = [step(i) for i in range(12)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [step(i) for i in range(4)]
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
