@@ -67,7 +67,7 @@ __host__ __device__ __forceinline__ Layout small_layout(int ring, int own_stages
   l.xsf = l.xq + (uint32_t)own_stages * m_pad * 128;
   l.part = l.xsf + (uint32_t)own_stages * 4 * ((m_pad + 31) / 32) * 128;
   l.table = l.part + (split > 1 ? (uint32_t)split * ((M + split - 1) / split) * 512 : 0);
-  l.bars = l.table + 256 * 4;
+  l.bars = l.table + 128 * 4;
   l.bytes = l.bars + (3 * kRingMost + kMaxStages + 2) * 8;
   return l;
 }
@@ -275,7 +275,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int first = (xw - group * wps) * 32 + lane, step = wps * 32;
     const int units = M * 16, KB = p.K >> 4;
     const float* table = reinterpret_cast<const float*>(smem + L.table);
-    const float gs = kCodes ? 0.f : p.gs[0];
+    // A negative global scale gives every scale byte its sign and the codes of its magnitude: 1 / (decoded scale / global scale) is the same.
+    const float given_gs = kCodes ? 0.f : p.gs[0], gs = fabsf(given_gs);
+    const uint32_t sf_sign = (__float_as_uint(given_gs) >> 31) << 7;
     bool table_made = false;
     // The multiplier of every scale byte, made while the first loads are on their way: with it a block's chain of dependent
     // operations is two reciprocals shorter.
@@ -283,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (kCodes || table_made) return;
       table_made = true;
       const int t = threadIdx.x - 32 * kFirstXWarp;
-      if (t < 256) {                               // bytes with the sign bit: a negative global scale
+      if (t < 128) {
         const float rcp_gs = __frcp_rn(gs + (gs == 0.f ? 1.0e8f : 0.f));
         reinterpret_cast<float*>(smem + L.table)[t] = out_scale_of((uint8_t)t, rcp_gs);
       }
@@ -326,10 +328,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (u < units) {
               uint32_t sfb = r0[j].z;
               uint2 c = make_uint2(r0[j].x, r0[j].y);
-              if constexpr (!kCodes) c = quantize_block16<T>(r0[j], r1[j], gs, [&](uint32_t b) { return table[b]; }, sfb);
+              if constexpr (!kCodes) c = quantize_block16<T>(r0[j], r1[j], gs, [&](uint32_t b) { return table[b & 127]; }, sfb);
               // rows of 128 bytes in atoms of eight, 16-byte chunk k of row r at k ^ (r % 8)
               *reinterpret_cast<uint2*>(xq + (m >> 3) * 1024 + (m & 7) * 128 + (((kb >> 1) ^ (m & 7)) << 4) + (kb & 1) * 8) = c;
-              xsf[((kb >> 2) * words + (m >> 5)) * 128 + (m & 31) * 4 + (kb & 3)] = (uint8_t)sfb;
+              xsf[((kb >> 2) * words + (m >> 5)) * 128 + (m & 31) * 4 + (kb & 3)] = (uint8_t)(sfb | sf_sign);
             }
           }
         }

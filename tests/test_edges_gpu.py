@@ -297,7 +297,7 @@ def test_few_token_linear(M, N, K, dtype):
     assert bool(((out.double() - ref).abs() <= half_ulp * ref.abs() + 2.0 ** -20 * size + 2.0 ** -24).all())
 
 
-@pytest.mark.parametrize("gs", [-2688 / 6.5, 0.0])
+@pytest.mark.parametrize("gs", [-2688 / 6.5, 0.0, -0.0])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_few_token_linear_any_global_scale(gs, dtype):
     # scale bytes with the sign bit set, and the guard for zero: still the stand-alone quantizer's bytes
@@ -306,6 +306,7 @@ def test_few_token_linear_any_global_scale(gs, dtype):
     x, _, wc, ws, alpha = _linear_operands(9, 512, 2048, 5)
     x, gx = x.to(dtype), torch.full((1,), gs, device="cuda")
     x[0, :16] = 0.0
+    x[1, :16] *= 1e-6                                 # a scale that rounds to zero
     xc, xs = scaled_fp4_quant(x, gx)
     out, want = nvfp4_linear(x, gx, wc, ws, alpha), cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype)
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
