@@ -13,6 +13,8 @@
 // projections, f32 rows out.  The token's value stands in all eight columns of an mma; one is read.
 #include "moe_small.cuh"
 
+#include <math.h>
+
 #include <mutex>
 
 namespace b200fp4 {
@@ -279,27 +281,35 @@ int resident_clusters(int c) {
 
 }  // namespace
 
-// The cluster size with the fewest steps per warp of those whose clusters all run at once, if the layer is then expected to take less time
-// than on the general path.  Times fitted to B200, us per layer (pairs, H, I: general / here, blocks per pair):
-//   10, 2048, 512: 15.7 / 10.5, 8     20: 20.0 / 14.2, 6     40: 27.0 / 19.4, 3     60: 31.0 / 23.5, 2     120: 40.5 / 37.6, 1     140: 44.8 / 39.3, 1
-//   30, 4096, 1024: 44.3 / 35.3, 4    50, 4096, 768: 50.4 / 55.6, 2    80, 1024, 256: 18.5 / 14.4, 1    100, 2048, 1024: 56.4 / 66.7, 1
-// A block's time here is its warps' steps (one of all 16 warps takes 0.58 us: instruction issue) and 8.5 us; the general path spreads all steps evenly over
-// the SMs, at four warps a scheduler, and takes 20 us beside (less for a few pairs).
-int moe_small_cluster(int64_t P, int64_t H, int64_t I) {
-  if (P < 1 || H > kMaxWidth || I > kMaxWidth) return 0;
+// The cluster size that is expected to take the least time, if that is less than on the general path.  `local` of the P pairs are expected to
+// have an expert here (fewer than P on an expert-parallel rank); the clusters of the others leave when they have seen their id.  Those that
+// stay, twice the standard deviation above the expected number, run at once; where all P do not, each further round of them is 2.37 us.
+// Times fitted to B200, us per layer (pairs, H, I: general / here, blocks per pair):
+//   10, 2048, 512: 15.1 / 10.4, 8     20: 19.3 / 14.1, 6     40: 25.9 / 18.8, 3     60: 30.5 / 22.2, 2     140: 42.8 / 38.9, 1
+//   24, 4096, 1024: 36.9 / 34.2, 4    64, 4096, 1024: 61.3 / 61.6, 2
+// and of 512 experts on 8 ranks, 2048, 512: 10: 10.4 / 7.7, 8     40: 12.7 / 12.6, 8     100: 15.5 / 18.2, 4     140: 18.1 / 21.4, 4
+// A block's time here is its warps' steps (one of all 16 warps takes 0.566 us: instruction issue) and 5.7 us.  The general path spreads all steps
+// evenly over the SMs; a few pairs take their time in its chain of launches and loads.  Over 220 sizes, 1 to 8 ranks, the choice takes 1.2 % more
+// than the best of all, 15 % at most, and 8 % at most more than the general path.
+// Only the number of pairs is known here.  Tokens that route alike stream an expert once each, where the general path reads it once for
+// eight: 12 tokens on the same ten of 512 experts 36.4 us here, 21.3 there, two by two alike 36.8 and 33.1, all different 37.6 and 40.9.
+int moe_small_cluster(int64_t P, double local, int64_t H, int64_t I) {
+  if (P < 1 || local <= 0 || H > kMaxWidth || I > kMaxWidth) return 0;
+  const double most = local + 2.0 * sqrt(local * (1.0 - local / (double)P));
   int best = 0;
-  int64_t best_steps = 0;
+  double here = 0;
   for (int c = 1; c <= kMaxCluster; ++c) {
     const SmallShape s = shape_for(c, H, I);
-    if (s.ga > kWarps || s.gb > kWarps || P * c > sm_count() || P > resident_clusters(c)) continue;
+    if (s.ga > kWarps || s.gb > kWarps || most * c > sm_count() || most > resident_clusters(c)) continue;
     const int64_t steps = (H / 32 + s.wa - 1) / s.wa + (I / 32 + s.wb - 1) / s.wb;       // of a warp
-    if (best == 0 || steps < best_steps) {
+    const double rounds = (double)P / resident_clusters(c) - 1.0, t = 5.66 + 0.566 * (double)steps + (rounds > 0 ? 2.37 * rounds : 0.0);
+    if (best == 0 || t < here) {
       best = c;
-      best_steps = steps;
+      here = t;
     }
   }
-  const double all = (double)P * (double)(H / 32) * (double)(I / 32) * 0.75;              // steps of both projections: H/32 I/64 + I/32 H/128
-  const double here = 0.58 * (double)best_steps + 8.5, general = 0.000215 * all + (P < 20 ? 13.0 + 0.35 * (double)P : 20.0);
+  const double all = local * (double)(H / 32) * (double)(I / 32) * 0.75;                  // steps of both projections: H/32 I/64 + I/32 H/128
+  const double width = (double)((H + I) / 32), general = 9.5 + 0.00025 * all + (0.0143 + 0.0033 * (local < 20 ? local : 20.0)) * width;
   return best > 0 && here < general ? best : 0;
 }
 

@@ -17,8 +17,9 @@ struct MoeSmallArgs {
   float* down;                      // [P, H]: written, but for the rows of experts that are not local
 };
 
-// Blocks per pair, or 0 where the general path is to be taken.  Both projections in the layout of the warp-scheduled kernels, ordered metadata.
-int moe_small_cluster(int64_t P, int64_t H, int64_t I);
+// Blocks per pair, or 0 where the general path is to be taken.  Both projections in the layout of the warp-scheduled kernels, ordered metadata;
+// local: how many of the P pairs are expected to have their expert here.
+int moe_small_cluster(int64_t P, double local, int64_t H, int64_t I);
 int launch_moe_small(int cluster, bool bf16, const MoeSmallArgs& a, int64_t P, cudaStream_t st);
 
 }  // namespace b200fp4

@@ -2196,7 +2196,8 @@ static int fused_moe_impl(const void* hidden, int64_t ld_h, int h_dtype, const f
   // B200FP4_MOE_SEPARATE_LAUNCHES asks for one launch each (which takes other kernels up to 256 pairs).
   if (ordered && (P > 256 || !(flags & B200FP4_MOE_SEPARATE_LAUNCHES)) && ws_ok(2 * I, H, G13, I, w13) && ws_ok(H, I, G2, 0, w2)) {
     // few pairs, which rarely share an expert: a cluster of blocks for each
-    const int cluster = (flags & B200FP4_MOE_SEPARATE_LAUNCHES) || 2 * local_pairs > E ? 0 : moe_small_cluster(P, H, I);
+    const double local = (double)P * (expert_map && global_E > E ? (double)E / (double)global_E : 1.0);
+    const int cluster = (flags & B200FP4_MOE_SEPARATE_LAUNCHES) || 2 * local_pairs > E ? 0 : moe_small_cluster(P, local, H, I);
     if (cluster > 0) {
       const MoeSmallArgs a = {w13, w2, hidden, ld_h, topk_ids, ld_ids, expert_map, (int)global_E, (int)E, (int)topk, (int)H, (int)I,
                               plan.hdr + 3, down};

@@ -367,3 +367,32 @@ def test_layer_reads_the_routing_the_kernel_before_it_wrote(M, E, ranks, topk, l
         graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(g, want[i % 2]) for i, g in enumerate(got))
+
+
+@pytest.mark.parametrize("M,ranks,launches", [
+    (1, 1, 2), (14, 1, 2),        # few pairs, a cluster for each (and the sum)
+    (1, 2, 2), (4, 2, 2),         # half of them here
+    (14, 2, 3),                   # clusters narrow enough for all that may stay take longer than plan, layer and sum
+    (2, 4, 2), (14, 4, 2), (30, 4, 3),
+    (1, 8, 2), (6, 8, 3), (14, 8, 3),
+])
+def test_fused_moe_few_pairs_of_one_rank(M, ranks, launches):
+    # which path an expert-parallel rank takes goes by the pairs that are expected to be its own, not by all of them
+    import synth
+    from dgx_vllm_b200 import _lib, sparse_fp4_v7 as sp7
+    from dgx_vllm_b200.moe_ep import expert_map_for_rank
+    from util import expert_fetch, gpu_quantize_fn, rel_err
+    keys, E, H, I = ("comp_T", "meta_T", "scale_T", "g_scales"), 512, 2048, 512
+    w13 = synth.make_sparse_experts(64, 2 * I, H, 1, "cuda", gpu_quantize_fn)
+    w2 = synth.make_sparse_experts(64, H, I, 2, "cuda", gpu_quantize_fn)
+    w13, w2 = ({k: w[k].repeat(E // ranks // 64, *[1] * (w[k].dim() - 1)) for k in keys} for w in (w13, w2))      # the same 64 again
+    tw, ids = synth.make_routing(M, E, 10, 3 + M, "cuda")
+    emap = expert_map_for_rank(E, ranks, ranks - 1, "cuda") if ranks > 1 else None
+    hidden = synth.make_hidden(M, H, 4, "cuda")
+    layer = sp7.FusedSparseMoE(*[w13[k] for k in keys], *[w2[k] for k in keys], I, expert_map=emap)
+    n0 = _lib.lib().b200fp4_launch_count()
+    out = layer(hidden, tw, ids)
+    assert _lib.lib().b200fp4_launch_count() == n0 + launches and sp7.last_moe_status() == 0
+    local = ids if emap is None else emap[ids.long()]
+    ref = oracle.fused_sparse_moe_by_expert(hidden.float().cpu().numpy(), tw.cpu().numpy(), local.cpu().numpy(), expert_fetch(w13, w2), I)
+    assert np.abs(to_np(out) - ref).max() <= 1e-2 * max(np.abs(ref).max(), 1e-6)
