@@ -6,6 +6,7 @@
 // dispatch take, so no host round trip sits between the router and the experts.
 //   router_cluster_kernel  up to 64 tokens: projection (mma.sync, operands straight from global memory into fragments), exchange of
 //                          the logits through distributed shared memory and selection in one launch
+//   router_slices_kernel   up to 32 tokens and a gate of many bytes: the same products with K split over blocks of 16 experts each
 //   router_gemm_kernel     larger batches: 128 tokens x 128 or 256 experts per CTA on tcgen05 (kind::f16, fp32 accumulators
 //                          in tensor memory), operands by TMA; bound by L2 -> shared-memory bandwidth
 //   router_topk_kernel     one warp per token: adds the K-slices of its logits in a fixed order, then k rounds of warp-wide
@@ -40,6 +41,71 @@ __device__ __forceinline__ void mma_m16n8k16<__half>(float (&c)[4], uint32_t a0,
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// ------------------------------------------------------------------------------------------ few tokens, large gates
+
+constexpr int kRsWarps = 8;
+constexpr int kRsThreads = 32 * kRsWarps;
+
+// parts[z][m][e] = sum over the k of slice z of hidden[m][k] * gate_w[e][k].
+// Block = experts [16 x, +16) x tokens [8 NT y, +8 NT), slice z of K; its warps take 64-wide pieces of K in turn.  In a 32-wide
+// step lane (g, t) = (lane / 4, lane % 4) loads the 8 elements at k = 8t of rows g and g + 8 (experts) and g (tokens): the
+// order of k inside a product sum is free, so elements 0-3 of the 8 serve as the lane's k of one mma and 4-7 as those of
+// another, on both sides alike.  Every SM reads its share of the gate once, whatever the number of experts; a second launch selects.
+template <typename T, int NT>
+__global__ void __launch_bounds__(kRsThreads)
+    router_slices_kernel(const T* __restrict__ hidden, int64_t ld_h, const T* __restrict__ gate_w, int M, int H, int E,
+                         int* __restrict__ status, float* __restrict__ parts) {
+  __shared__ float s_part[kRsWarps][16][8 * NT + 1];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int e0 = blockIdx.x * 16, m0 = blockIdx.y * 8 * NT;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *status = 0;
+  float acc[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  const T* wa = gate_w + (int64_t)min(e0 + g, E - 1) * H;            // rows past the end repeat the last: never stored
+  const T* wb = gate_w + (int64_t)min(e0 + g + 8, E - 1) * H;
+  const T* x[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) x[n] = hidden + (int64_t)min(m0 + 8 * n + g, M - 1) * ld_h;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int k0 = 64 * (blockIdx.z * kRsWarps + warp); k0 < H; k0 += 64 * kRsWarps * gridDim.z) {
+    uint4 a[2][2], b[2][NT];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int k = k0 + 32 * s + 8 * t;
+      const bool in = k < H;
+      a[s][0] = in ? ldg_stream_u4(wa + k) : zero;
+      a[s][1] = in ? ldg_stream_u4(wb + k) : zero;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) b[s][n] = in ? *reinterpret_cast<const uint4*>(x[n] + k) : zero;
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        mma_m16n8k16<T>(acc[n], a[s][0].x, a[s][1].x, a[s][0].y, a[s][1].y, b[s][n].x, b[s][n].y);
+        mma_m16n8k16<T>(acc[n], a[s][0].z, a[s][1].z, a[s][0].w, a[s][1].w, b[s][n].z, b[s][n].w);
+      }
+  }
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    s_part[warp][g][8 * n + 2 * t] = acc[n][0];
+    s_part[warp][g][8 * n + 2 * t + 1] = acc[n][1];
+    s_part[warp][g + 8][8 * n + 2 * t] = acc[n][2];
+    s_part[warp][g + 8][8 * n + 2 * t + 1] = acc[n][3];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * 8 * NT; i += kRsThreads) {
+    const int r = i & 15, c = i >> 4;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kRsWarps; ++w) v += s_part[w][r][c];
+    if (e0 + r < E && m0 + c < M) parts[((int64_t)blockIdx.z * M + m0 + c) * E + e0 + r] = v;
+  }
 }
 
 // ------------------------------------------------------------------------------------------ projection, larger batches
@@ -318,27 +384,58 @@ __global__ void __launch_bounds__(kRcThreads, 1)
 
 // ------------------------------------------------------------------------------------------ host
 
-// Up to 64 tokens and 512 experts (16 tokens above, as far as 1/16 of the gate is not more than one SM reads in about 4 us) everything is
-// one launch of clusters; else the tcgen05 tiles and the separate selection: every cluster of eight tokens reads all weight rows, 1/8 or 1/16
-// of them through one SM (1000 experts, H=4096, M=64 22.7 us as clusters, 15.2 as tiles; 1024 experts, M=4 10.7 / 13.0).
+// Which way a call goes.  One launch of clusters saves a launch, but only 8 or 16 SMs read the gate for eight tokens, and those without experts
+// none of it (us, slices and selection in two launches / clusters, back to back and from a graph):
+//   M=8: 32 experts H=2048 3.2 / 3.7, 3.4 / 4.0, H=12800 5.8 / 8.4, 5.2 / 8.9   64, 4096 4.4 / 4.6, 3.9 / 4.9   128, 6144 5.8 / 5.5, 5.5 / 5.8
+//   128, 9216 6.2 / 6.9, 6.0 / 7.3   512, 6144 8.6 / 8.8, 8.8 / 9.2   512, 9216 9.7 / 11.4, 9.8 / 11.8   1000, 4096 10.0 / 11.9, 9.9 / 12.5
+//   M=16: 128, 12800 7.3 / 8.8, 7.2 / 9.0   512, 6144 9.4 / 8.7, 9.7 / 9.5   512, 9216 10.8 / 11.4, 10.8 / 12.0
+// From 17 tokens on clusters are the faster ones up to 512 experts; the tiles read the whole gate once for 128 tokens, the slices once for 8 to 32
+// (slices / tiles; M=17: 1000 experts H=2048 10.9 / 13.1, H=4096 13.3 / 14.1, H=7168 18.5 / 15.8; M=64, H=4096 19.4 / 15.2; M=8, H=12800 20.8 / 19.4).
 constexpr int kRtClusterMaxTokens = 64;
+constexpr int kRtSlicesMaxTokens = 32;
 constexpr int kRtMaxSplits = 8;
 
-// K-slices of the projection of many tokens: enough blocks to cover the SMs, at most eight (the top-k kernel reads them all)
-struct RouterShape {
-  bool small;
+enum class RouterPath { kClusters, kSlices, kTiles };
+
+RouterPath router_path(int64_t M, int64_t H, int64_t E) {
+  const int64_t gate = E * H;
+  if (M <= 16) {
+    if (E <= 128) return H > (E <= 32 ? 1536 : (E <= 64 ? 2560 : 6144)) ? RouterPath::kSlices : RouterPath::kClusters;
+    if (gate <= (M <= 8 ? 3200000 : 3900000)) return RouterPath::kClusters;
+    return E <= 512 || gate <= (M <= 8 ? 9300000 : 7500000) ? RouterPath::kSlices : RouterPath::kTiles;
+  }
+  if (E <= 512) return M <= kRtClusterMaxTokens ? RouterPath::kClusters : RouterPath::kTiles;
+  return M <= kRtSlicesMaxTokens && H <= (E > 896 ? 4608 : 3072) ? RouterPath::kSlices : RouterPath::kTiles;
+}
+
+// K-slices of the projection: enough blocks to cover the SMs, at most eight (the top-k kernel reads them all)
+int router_splits(int64_t blocks) {
+  const int64_t z = sm_count() / (blocks > 0 ? blocks : 1);
+  return (int)(z < 1 ? 1 : (z > kRtMaxSplits ? kRtMaxSplits : z));
+}
+int slices_splits(int64_t E) { return router_splits((E + 15) / 16); }       // one block of tokens
+
+struct TileShape {
   int bn, splits;
 };
-
-RouterShape router_shape(int64_t M, int64_t H, int64_t E) {
-  RouterShape s = {};
-  s.small = E <= 512 ? M <= kRtClusterMaxTokens : M <= 16 && E * H <= (int64_t)1024 * 4096;
-  if (s.small) return s;
+TileShape tile_shape(int64_t M, int64_t E) {
+  TileShape s;
   const int64_t mt = (M + 127) / 128;
   s.bn = mt * ((E + 127) / 128) <= sm_count() ? 128 : 256;
-  const int64_t blocks = mt * ((E + s.bn - 1) / s.bn), z = sm_count() / (blocks > 0 ? blocks : 1);
-  s.splits = (int)(z < 1 ? 1 : (z > kRtMaxSplits ? kRtMaxSplits : z));
+  s.splits = router_splits(mt * ((E + s.bn - 1) / s.bn));
   return s;
+}
+
+template <typename T>
+void launch_router_slices(int splits, const void* hidden, int64_t ld_h, const void* gate_w, int M, int H, int E, int* status, float* parts,
+                          cudaStream_t st) {
+  auto go = [&](auto kernel) {
+    launch_pdl(kernel, dim3((unsigned)((E + 15) / 16), 1, (unsigned)splits), dim3(kRsThreads), 0, st, static_cast<const T*>(hidden), ld_h,
+               static_cast<const T*>(gate_w), M, H, E, status, parts);
+  };
+  if (M <= 8) go(router_slices_kernel<T, 1>);
+  else if (M <= 16) go(router_slices_kernel<T, 2>);
+  else go(router_slices_kernel<T, 4>);
 }
 
 // Clusters of CL blocks that are resident at once (0: none)
@@ -429,8 +526,9 @@ using namespace b200fp4;
 // workspace: 256 bytes (first int: status word of the tcgen05 kernel's bounded waits), then the K-slices of the logits
 extern "C" size_t b200fp4_moe_router_workspace_bytes(int64_t M, int64_t E) {
   if (M <= 0 || E <= 0) return 0;
-  const RouterShape s = router_shape(M, (int64_t)1 << 20, E);        // as for a gate of many columns: whichever path H leads to fits
-  return 256 + (size_t)s.splits * (size_t)M * (size_t)E * sizeof(float);
+  int splits = M > kRtClusterMaxTokens || E > 512 ? tile_shape(M, E).splits : 0;      // whichever path the width of the gate leads to fits
+  if (M <= kRtSlicesMaxTokens && slices_splits(E) > splits) splits = slices_splits(E);
+  return 256 + (size_t)splits * (size_t)M * (size_t)E * sizeof(float);
 }
 
 extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, const void* gate_w, int64_t M, int64_t H,
@@ -448,13 +546,21 @@ extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, c
   cudaStream_t st = (cudaStream_t)stream;
   int* status = static_cast<int*>(workspace);
   float* parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
-  const RouterShape sh = router_shape(M, H, E);
+  const RouterPath path = router_path(M, H, E);
   const bool bf = dtype == B200FP4_DTYPE_BF16;
-  int splits = sh.splits;
-  if (sh.small) {
+  int splits;
+  if (path == RouterPath::kClusters) {
     auto* go = bf ? launch_router_cluster<__nv_bfloat16> : launch_router_cluster<__half>;
     return go(hidden, ld_h, gate_w, (int)M, (int)H, (int)E, (int)topk, renormalize, status, topk_weights, topk_ids, st);
+  } else if (path == RouterPath::kSlices) {
+    splits = slices_splits(E);
+    const int most = (int)((H + 64 * kRsWarps - 1) / (64 * kRsWarps));       // no more slices than there are rounds of 64 per warp
+    if (splits > most) splits = most;
+    auto* go = bf ? launch_router_slices<__nv_bfloat16> : launch_router_slices<__half>;
+    go(splits, hidden, ld_h, gate_w, (int)M, (int)H, (int)E, status, parts, st);
   } else {
+    const TileShape sh = tile_shape(M, E);
+    splits = sh.splits;
     if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
     const int most = (int)((H + 4 * kRgK - 1) / (4 * kRgK));       // at least about four stages per slice
     if (splits > most) splits = most;

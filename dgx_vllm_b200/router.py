@@ -17,5 +17,5 @@ def moe_router(hidden_states: torch.Tensor, gate_weight: torch.Tensor, topk: int
 
 def last_router_status(device=None) -> int:
     """Status word of the most recent moe_router on the current stream of `device`: 0, or the code of a bounded wait that ran
-    out in the projection of more than 64 tokens (that call's weights and ids are then not valid).  Synchronises."""
+    out in the projection of many tokens (that call's weights and ids are then not valid).  Synchronises."""
     return status_word(device, WS_ROUTER)

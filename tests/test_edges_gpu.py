@@ -44,7 +44,15 @@ def test_convert_2of4_tile_edges(E, N, K, G):
     (56, 2048, 512, 10, torch.bfloat16, False),       # ... as many as run at once
     (64, 1024, 500, 10, torch.float16, False),        # ... one more: clusters of eight again, four tiles to a block
     (16, 1000, 1023, 32, torch.bfloat16, True),       # more than 512 experts
-    (3, 12800, 600, 4, torch.bfloat16, True),         # ... with a gate for the tile kernel
+    (3, 12800, 600, 4, torch.bfloat16, True),         # ... with a gate for K-slices: eight tokens a block
+    (3, 12800, 1000, 4, torch.bfloat16, True),        # ... and for the tile kernel
+    (8, 1544, 1, 1, torch.float16, True),             # K-slices: one expert, the last of four slices with little to do
+    (7, 3080, 33, 5, torch.bfloat16, False),          # ... experts past a block
+    (16, 2568, 64, 8, torch.float16, True),           # ... sixteen tokens a block
+    (9, 12800, 511, 10, torch.bfloat16, True),        # ... fewer tokens than that
+    (17, 1032, 640, 10, torch.bfloat16, True),        # ... thirty-two
+    (32, 4608, 1024, 32, torch.float16, False),       # ... the largest
+    (33, 1024, 640, 10, torch.bfloat16, True),        # one more: tiles
 ])
 def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
     from dgx_vllm_b200.router import moe_router
@@ -62,6 +70,21 @@ def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
     assert clear.float().mean() > 0.8
     assert torch.equal(ids[clear].long(), ref_ids[clear])
     assert ((tw[clear].double() - w[clear]).abs() / w[clear]).max() < 1e-4
+
+
+@pytest.mark.parametrize("M,H,E,launches", [
+    (8, 1536, 32, 1), (8, 2048, 32, 2), (16, 2560, 64, 1), (16, 4096, 64, 2), (8, 6144, 128, 1), (8, 7168, 128, 2), (17, 12800, 128, 1),
+    (8, 6144, 512, 1), (8, 9216, 512, 2), (16, 7168, 512, 1), (32, 9216, 512, 1), (4, 3072, 1000, 1), (4, 4096, 1000, 2), (17, 2048, 1000, 2),
+])
+def test_router_path(M, H, E, launches):
+    # clusters in one launch, or two launches that have every SM read its share of a large gate
+    from dgx_vllm_b200 import _lib
+    from dgx_vllm_b200.router import moe_router
+    x, gate = torch.zeros(M, H, device="cuda", dtype=torch.bfloat16), torch.zeros(E, H, device="cuda", dtype=torch.bfloat16)
+    n0 = _lib.lib().b200fp4_launch_count()
+    tw, ids = moe_router(x, gate, 8)
+    assert _lib.lib().b200fp4_launch_count() == n0 + launches
+    assert torch.equal(ids, torch.arange(8, device="cuda", dtype=torch.int32).expand(M, 8)) and bool((tw == 0.125).all())
 
 
 @pytest.mark.parametrize("M,K", [(1, 16), (31, 48), (33, 512), (97, 528), (129, 80), (200, 2064)])
