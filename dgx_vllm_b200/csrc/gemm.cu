@@ -1006,8 +1006,8 @@ static int gemm_nvfp4(const void* a_codes, const void* b_codes, const void* sfa,
   if (refused != B200FP4_STATUS_SUCCESS || M == 0) return refused;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
   cudaStream_t st = (cudaStream_t)stream;
-  if (tile_n == 0) {
-    const SmallPlan small = small_gemm_plan(M, N, K);
+  if (tile_n == 0 && M <= kSmallMaxM) {
+    const SmallPlan small = small_gemm_plan(M, N, K, stream_capturing(st) ? SmallUse::kCodesInGraph : SmallUse::kCodes);
     CUtensorMap mw;
     if (small.ok) {
       if (!make_map(&mw, b_codes, (uint64_t)N, (uint64_t)K / 2, kBM, kStageKb * 32)) return B200FP4_STATUS_INTERNAL_ERROR;
@@ -1093,7 +1093,7 @@ extern "C" int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, con
     rc = dense_gemm_check(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, gemm_bytes);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
-  const SmallPlan small = small_gemm_plan(M, N, K);
+  const SmallPlan small = small_gemm_plan(M, N, K, SmallUse::kLinear);
   if (tile_n == 0 && small.ok) {
     // few tokens: quantized inside the GEMM
     CUtensorMap mw;

@@ -9,8 +9,8 @@
 //     through memory.  The arithmetic is the quantizer's (quant.cuh), the bytes are the same;
 //   * K is split over clusters of up to eight CTAs, whatever number fits the SMs; the partial sums of a token meet in one CTA of the
 //     cluster through distributed shared memory and are added in the order of K.
-// The GEMM on codes that are already there (cutlass_scaled_fp4_mm) takes the same kernel, with the quantization replaced by a
-// copy: the two give the same bytes.
+// The GEMM on codes that are already there (cutlass_scaled_fp4_mm) takes the same kernel where that is the faster one, with the quantization
+// replaced by a copy.
 // What bounds it: the chain of copy, quantization, scales, MMA, exchange and store where the weight is small, HBM where it is large.
 // Measured back to back (us; quantizer and general kernel / so): M=8 N=512 K=2048 7.1 / 4.1, M=1 N=K=4096 8.9 / 6.1, M=1 N=14336
 // K=4096 14.0 / 8.9 (3.8 TB/s), M=16 of that 13.5 / 12.0, M=24 N=1536 K=3008 7.8 / 6.4.  Weight scales take about as long to reach tensor memory as a
@@ -425,7 +425,7 @@ int resident_clusters(int k) {
   return c.n;
 }
 
-SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K) {
+SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use) {
   SmallPlan s = {};
   const int64_t sms = sm_count(), tiles = (N + 127) / 128, stages = (K + 255) / 256;
   if (M < 1 || M > kSmallMaxM || tiles > sms) return s;
@@ -436,9 +436,23 @@ SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K) {
     if (tiles * k <= sms && tiles <= resident_clusters(k)) split = k;
   const int own = (int)((stages + split - 1) / split), m_pad = (int)(M + 7) / 8 * 8;
   if (own > kMaxStages) return s;
-  // Every CTA quantizes its part of K for all tokens (a block of 16 takes an SM 1.4 cycles), where the general path does that once:
-  // from about 2048 blocks per CTA on it is the faster one, for up to 16 tokens from 4096.
-  if (M * own > (M <= 16 ? 256 : 128)) return s;
+  // Every CTA brings in its part of K for all tokens and sends its 128 columns out token by token, some 70 cycles a token, where the general path
+  // quantizes once and stores tiles; and clusters that nearly fill the chip leave the next launch no room to start in.  So the number of tokens
+  // up to which this kernel is the faster one falls with the stages a CTA owns and with the CTAs.  Linear, us (quantizer and general kernel / so):
+  // N=4096 K=512 M=32 5.8 / 5.3, M=48 6.0 / 6.2; N=1024 K=2048 M=32 6.6 / 5.4, M=64 7.0 / 7.1; N=4096 K=2048 M=24 6.8 / 6.6, M=32 6.9 / 7.5;
+  // N=9600 K=1024 M=24 6.4 / 6.4, M=32 6.4 / 6.9.
+  const int64_t ctas = tiles * split;
+  if (M <= 16 ? M * own > 256 : ctas <= 64 ? M * own > 128 || (stages <= 4 && M > 44) : M * own > 96 || M > (ctas > 110 ? 24 : 32)) return s;
+  // On codes that are there already no launch is saved.  In a graph the longer way to the first MMA is not hidden behind the kernel before, so
+  // that only long K pays.  GEMM, us eager and from a graph (general kernel / so): M=8 N=512 K=1024 4.1 / 3.6, 4.6 / 5.2; M=24 N=512 K=1536
+  // 4.7 / 4.2, 5.2 / 5.8; M=8 N=4096 K=1024 4.1 / 4.8, 4.7 / 5.4; M=32 N=2048 K=512 3.5 / 4.4, 4.1 / 5.7; M=8 N=14336 K=4096 12.2 / 9.5, 12.0 / 10.6.
+  const bool pays = use == SmallUse::kLinear         ? true
+                    : use == SmallUse::kCodesInGraph ? M <= 8 && stages >= 8 && own >= 3
+                    : stages < 4                     ? M <= 4
+                    : split == 1                     ? M <= 8 || own >= 16
+                    : ctas <= 64                     ? M <= (stages < 6 ? 16 : 24)
+                                                     : M <= 8 && own >= 3;
+  if (!pays) return s;
   int ring = own < kRingMost ? own : kRingMost;
   while (ring > 0 && small_layout(ring, own, m_pad, (int)M, split).bytes + 1024 > kSmemMost) --ring;
   if (ring < (own < 4 ? own : 4)) return s;

@@ -17,7 +17,8 @@ struct SmallPlan {
   int split, ring, stages, m_pad;
   size_t smem;
 };
-SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K);
+enum class SmallUse { kLinear, kCodes, kCodesInGraph };      // quantizes its operand; given codes, launched or captured
+SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use);
 
 // gs given: x is [M, K] bf16 / f16 (rows ldx elements apart), quantized in the kernel; gs null: x are packed codes [M, K/2] and x_sf
 // their swizzled scales.  mw: the weight [N, K/2] in boxes of 128 rows x 128 bytes.

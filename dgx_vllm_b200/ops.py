@@ -33,9 +33,9 @@ def nvfp4_linear(x: torch.Tensor, x_global_scale: torch.Tensor, w_codes: torch.T
                  alpha: torch.Tensor, *, out: torch.Tensor | None = None, tile_n: int = 0) -> torch.Tensor:
     """y[M,N] = alpha * NVFP4(x) @ W^T: scaled_fp4_quant followed by cutlass_scaled_fp4_mm in ONE library call
     (b200fp4_linear_nvfp4), which is what a quantized linear layer does on every forward (the pair of ops in vLLM's
-    NVFP4 linear apply, nvfp4_utils.py; emulated by the reference at fix_nvfp4_emulation_backend.py:60-102).  Same bytes
-    as calling the two ops; the launches are a few microseconds apart instead of a Python call apart, and for few tokens it is one
-    kernel that quantizes its own operand.
+    NVFP4 linear apply, nvfp4_utils.py; emulated by the reference at fix_nvfp4_emulation_backend.py:60-102).  Same codes
+    and products as calling the two ops (for few tokens the f32 sums over K may be grouped otherwise); the launches are a few
+    microseconds apart instead of a Python call apart, and for few tokens it is one kernel that quantizes its own operand.
     x [M,K] bf16/f16 (rows may be strided), w_codes [N,K/2] u8, w_block_scale swizzled, alpha / x_global_scale one f32."""
     return _lib.host().nvfp4_linear(x, x_global_scale, w_codes, w_block_scale, alpha, out, tile_n)
 

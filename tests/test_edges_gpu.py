@@ -419,3 +419,52 @@ def test_fused_moe_few_pairs_of_one_rank(M, ranks, launches):
     local = ids if emap is None else emap[ids.long()]
     ref = oracle.fused_sparse_moe_by_expert(hidden.float().cpu().numpy(), tw.cpu().numpy(), local.cpu().numpy(), expert_fetch(w13, w2), I)
     assert np.abs(to_np(out) - ref).max() <= 1e-2 * max(np.abs(ref).max(), 1e-6)
+
+
+@pytest.mark.parametrize("M,N,K,launches", [
+    (32, 512, 512, 1), (45, 512, 512, 2), (64, 1024, 4096, 1), (24, 4096, 2048, 1), (25, 4096, 2048, 2), (32, 2048, 1536, 1), (33, 2048, 1536, 2),
+    (24, 9600, 1024, 1), (25, 9600, 1024, 2), (16, 14336, 4096, 1), (17, 14336, 4096, 2),
+])
+def test_linear_path(M, N, K, launches):
+    # one kernel for few tokens, quantizer and GEMM where those are the faster ones
+    from dgx_vllm_b200 import _lib, cutlass_scaled_fp4_mm, scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status, nvfp4_linear
+    x, gx, wc, ws, alpha = _linear_operands(M, N, K, M + N)
+    n0 = _lib.lib().b200fp4_launch_count()
+    out = nvfp4_linear(x, gx, wc, ws, alpha)
+    assert _lib.lib().b200fp4_launch_count() == n0 + launches and last_gemm_status() == 0
+    xc, xs = scaled_fp4_quant(x, gx)
+    assert torch.equal(out, cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, torch.bfloat16))
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (1, 128, 64), (4, 512, 512), (5, 512, 512),               # short K: the few-token kernel for up to four tokens, never in a graph
+    (16, 520, 1088), (17, 520, 1088), (24, 512, 1536),        # few CTAs: up to 16 or 24
+    (8, 4096, 4096), (9, 4096, 4096), (8, 4096, 2048),        # clusters that nearly fill the chip; the first in a graph too
+    (8, 9600, 2112), (16, 14336, 4096),                       # K not split
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_of_few_tokens_eager_and_captured(M, N, K, dtype):
+    # the two may be different kernels: both within one rounding to 16 bits and the f32 sum over K of the exact product of the codes
+    from dgx_vllm_b200 import cutlass_scaled_fp4_mm, scaled_fp4_quant
+    from dgx_vllm_b200.ops import last_gemm_status
+    x, gx, wc, ws, alpha = _linear_operands(M, N, K, M + K)
+    xc, xs = scaled_fp4_quant(x, gx)
+    outs = [cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype, tile_n=t) for t in (0, 128)]
+    assert last_gemm_status() == 0
+    graph, out = torch.cuda.CUDAGraph(), torch.full((M, N), 7.0, dtype=dtype, device="cuda")
+    with torch.cuda.graph(graph):
+        cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, dtype, out=out)
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+
+    def deq(codes, sf, rows):
+        lin = oracle.sf_swizzled_to_linear(to_np(sf.view(torch.uint8)).reshape(-1), rows, K // 16)
+        return torch.from_numpy(oracle.dequantize(to_np(codes), lin, 1.0)).cuda().double()
+
+    a, b = deq(xc, xs, M), deq(wc, ws, N)
+    ref, size = (a @ b.t()) * alpha.double(), (a.abs() @ b.abs().t()) * alpha.double()
+    bound = 2.0 ** (-8 if dtype == torch.bfloat16 else -11) * ref.abs() + 2.0 ** -20 * size + 2.0 ** -24
+    for o in outs + [out]:
+        assert bool(((o.double() - ref).abs() <= bound).all())
