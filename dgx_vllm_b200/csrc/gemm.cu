@@ -699,6 +699,8 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   }
   if constexpr (kSplit > 1) {
     // every CTA's sums have arrived (also after a timed-out wait: the status word then says that the result is not valid)
+    // Over two CTAs the sums and the two kept chunks take 128 registers and spill 40 bytes.  Four values at a time onto what is kept, 122 registers
+    // and no spills, took 1 to 2 % longer (28 sizes: 256x4096x4096 7.77 / 7.95 us, 323x1536x7616 9.69 / 9.86).
     __syncwarp();
     cluster_sync_any();
     constexpr int kOwn = 4 / kSplit;
