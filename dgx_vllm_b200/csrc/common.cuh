@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/b200_nvfp4.h"
 
@@ -85,6 +86,38 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// Clusters of `cluster` blocks of a kernel that run at once on the current device (a cluster lies within a GPC); 0: none, or the query failed.
+// Asked for when first needed and kept per device by the caller: a query takes some microseconds.
+struct ResidentClusters {
+  std::once_flag once;
+  int n = 0;
+};
+template <typename... KArgs>
+inline int resident_clusters_of(ResidentClusters (&per_device)[64], void (*kernel)(KArgs...), int cluster, int threads, size_t smem) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  ResidentClusters& r = per_device[dev];
+  std::call_once(r.once, [&] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cluster);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if ((cluster > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+        (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+        cudaOccupancyMaxActiveClusters(&r.n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      r.n = 0;
+    }
+  });
+  return r.n;
+}
+
 // What b200fp4_quantize (quant.cu) and b200fp4_gemm_nvfp4 (gemm.cu) refuse of their arguments, without queueing anything (the
 // device is not looked at): calls of several steps check all of them before the first.
 int quantize_check(const void* x, int in_dtype, int64_t M, int64_t K, int64_t ldx, const float* global_scale, const void* codes,
@@ -93,6 +126,20 @@ int dense_gemm_check(const void* a_codes, const void* b_codes, const void* sfa, 
                      int out_dtype, int64_t M, int64_t N, int64_t K, int tile_n, const void* workspace, size_t workspace_bytes);
 
 // ------------------------------------------------------------------------------------------ device
+
+// shared::cluster address of the same shared-memory offset in block `rank` of this cluster
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+// all threads of the cluster, converged or not
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync_any() {
+  cluster_arrive();
+  cluster_wait();
+}
 
 // 16-byte read-only global load that does not allocate in L1 (streamed weights are read once).
 __device__ __forceinline__ uint4 ldg_stream_u4(const void* p) {

@@ -17,7 +17,6 @@
 // stage takes to arrive, which is why two stages share a wait there.
 // One tile per CTA.  Warps: 0 copies of the weight and its scales, 1 MMA, 2-5 the weight's and 6-9 the activations' scale factors into
 // tensor memory, all eight the epilogue, 10-25 activations.  Every mbarrier wait is bounded (status word), tensor memory is always freed.
-#include <mutex>
 #include <type_traits>
 
 #include "gemm_small.cuh"
@@ -396,33 +395,9 @@ int launch_small_t(const CUtensorMap& mw, const SmallParams& p, unsigned grid, s
 }  // namespace
 
 int resident_clusters(int k) {
-  struct Count {
-    std::once_flag once;
-    int n = 0;
-  };
-  static Count counts[64][kMaxSplit + 1];      // asked for when first needed: a query takes some microseconds
-  int dev = 0;
-  if (k < 2 || k > kMaxSplit || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  Count& c = counts[dev][k];
-  std::call_once(c.once, [&] {
-    auto* kernel = nvfp4_small_kernel<__nv_bfloat16, false>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)k);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemMost;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)k;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&c.n, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      c.n = 0;
-    }
-  });
-  return c.n;
+  static ResidentClusters counts[kMaxSplit + 1][64];
+  if (k < 2 || k > kMaxSplit) return 0;
+  return resident_clusters_of(counts[k], nvfp4_small_kernel<__nv_bfloat16, false>, k, kThreads, kSmemMost);
 }
 
 SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use) {

@@ -37,14 +37,6 @@ __host__ __device__ __forceinline__ size_t small_smem(int H, int I) {
   return 128 + (size_t)kWarps * kSlots * kStage + (size_t)kWarps * 512 + (size_t)(H + I) * 2;
 }
 
-__device__ __forceinline__ uint32_t map_to(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-
 // where the 16 bits of element k stand in the fragment order of its group of 32 (word 4i + t at 4t + i)
 __device__ __forceinline__ uint32_t frag_byte(int k) {
   const int w = (k & 31) >> 1;
@@ -208,7 +200,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_small_kernel(const MoeSmallAr
       if (lane < 16 && (q & 1) == 0) {
         const uint32_t at = acts + frag_byte((ga_first + group) * 64 + col);
         for (int r = t; r < sh.cluster; r += 4)
-          asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(map_to(at, (uint32_t)r)), "r"(*reinterpret_cast<const uint32_t*>(&h)) : "memory");
+          asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(map_to_cta(at, (uint32_t)r)), "r"(*reinterpret_cast<const uint32_t*>(&h)) : "memory");
       }
     }
   }
@@ -250,33 +242,10 @@ bool prepare() {
   return ok[dev];
 }
 
-// Clusters of c blocks that are resident at once; asked for when first needed
-int resident_clusters(int c) {
-  struct Count {
-    std::once_flag once;
-    int n = 0;
-  };
-  static Count counts[64][kMaxCluster + 1];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !prepare<true>()) return 0;
-  Count& count = counts[dev][c];
-  std::call_once(count.once, [&] {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)c);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = small_smem(kMaxWidth, kMaxWidth);
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)c;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&count.n, moe_small_kernel<true>, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      count.n = 0;
-    }
-  });
-  return count.n;
+// Clusters of c blocks that run at once
+int resident_pairs(int c) {
+  static ResidentClusters counts[kMaxCluster + 1][64];
+  return resident_clusters_of(counts[c], moe_small_kernel<true>, c, kThreads, small_smem(kMaxWidth, kMaxWidth));
 }
 
 }  // namespace
@@ -300,9 +269,9 @@ int moe_small_cluster(int64_t P, double local, int64_t H, int64_t I) {
   double here = 0;
   for (int c = 1; c <= kMaxCluster; ++c) {
     const SmallShape s = shape_for(c, H, I);
-    if (s.ga > kWarps || s.gb > kWarps || most * c > sm_count() || most > resident_clusters(c)) continue;
+    if (s.ga > kWarps || s.gb > kWarps || most * c > sm_count() || most > resident_pairs(c)) continue;
     const int64_t steps = (H / 32 + s.wa - 1) / s.wa + (I / 32 + s.wb - 1) / s.wb;       // of a warp
-    const double rounds = (double)P / resident_clusters(c) - 1.0, t = 5.66 + 0.566 * (double)steps + (rounds > 0 ? 2.37 * rounds : 0.0);
+    const double rounds = (double)P / resident_pairs(c) - 1.0, t = 5.66 + 0.566 * (double)steps + (rounds > 0 ? 2.37 * rounds : 0.0);
     if (best == 0 || t < here) {
       best = c;
       here = t;

@@ -12,8 +12,6 @@
 //   router_topk_kernel     one warp per token: adds the K-slices of its logits in a fixed order, then k rounds of warp-wide
 //                          arg-max (ties -> lower expert id), weights exp(l - max) normalised over the selected experts
 //                          (or over all of them)
-#include <mutex>
-
 #include "sm100_ptx.cuh"
 
 namespace b200fp4 {
@@ -438,35 +436,10 @@ void launch_router_slices(int splits, const void* hidden, int64_t ld_h, const vo
   else go(router_slices_kernel<T, 4>);
 }
 
-// Clusters of CL blocks that are resident at once (0: none)
 template <typename T, int CL, int PER>
 int resident_router_clusters() {
-  struct PerDevice {
-    std::once_flag once;
-    int n = 0;
-  };
-  static PerDevice devices[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  PerDevice& d = devices[dev];
-  std::call_once(d.once, [&] {
-    auto* kernel = router_cluster_kernel<T, CL, PER>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CL);
-    cfg.blockDim = dim3(kRcThreads);
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = CL;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if ((CL > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-        cudaOccupancyMaxActiveClusters(&d.n, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      d.n = 0;
-    }
-  });
-  return d.n;
+  static ResidentClusters counts[64];
+  return resident_clusters_of(counts, router_cluster_kernel<T, CL, PER>, CL, kRcThreads, 0);
 }
 
 template <typename T, int CL, int PER>

@@ -435,6 +435,13 @@ def test_linear_path(M, N, K, launches):
     assert _lib.lib().b200fp4_launch_count() == n0 + launches and last_gemm_status() == 0
     xc, xs = scaled_fp4_quant(x, gx)
     assert torch.equal(out, cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, torch.bfloat16))
+    graph, captured = torch.cuda.CUDAGraph(), torch.zeros_like(out)
+    with torch.cuda.graph(graph):
+        nvfp4_linear(x, gx, wc, ws, alpha, out=captured)
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, out)
 
 
 @pytest.mark.parametrize("M,N,K", [
