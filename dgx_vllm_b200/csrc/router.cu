@@ -129,8 +129,8 @@ __device__ __forceinline__ void tcgen05_mma_f16(uint32_t d_tmem, uint64_t a_desc
       : "memory");
 }
 
-// parts[z][m][e] as above, for the tile of 128 tokens (blockIdx.y) x BN experts (blockIdx.x) and K-slice z.  Rows and columns
-// past the tensors are filled with zeros by the copies and not stored.
+// parts[z][m][e] = the sum over the k of K-slice z of hidden[m][k] * gate_w[e][k], for the tile of 128 tokens (blockIdx.y)
+// x BN experts (blockIdx.x).  Rows and columns past the tensors are filled with zeros by the copies and not stored.
 template <int BN>
 __global__ void __launch_bounds__(kRgThreads, 1)
     router_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int M, int H, int E,
@@ -496,12 +496,13 @@ int launch_router_gemm(const CUtensorMap& mx, const CUtensorMap& mw, int splits,
 
 using namespace b200fp4;
 
-// workspace: 256 bytes (first int: status word of the tcgen05 kernel's bounded waits), then the K-slices of the logits
+// workspace: 256 bytes (first int: status word of the tcgen05 kernel's bounded waits), then the K-slices of the logits.  Enough for whichever
+// path the width of the gate leads to, and up to 128 tokens for every smaller batch too.
 extern "C" size_t b200fp4_moe_router_workspace_bytes(int64_t M, int64_t E) {
   if (M <= 0 || E <= 0) return 0;
-  int splits = M > kRtClusterMaxTokens || E > 512 ? tile_shape(M, E).splits : 0;      // whichever path the width of the gate leads to fits
-  if (M <= kRtSlicesMaxTokens && slices_splits(E) > splits) splits = slices_splits(E);
-  return 256 + (size_t)splits * (size_t)M * (size_t)E * sizeof(float);
+  const int64_t tiles = M > kRtClusterMaxTokens || E > 512 ? tile_shape(M, E).splits * M : 0;
+  const int64_t slices = slices_splits(E) * (M < kRtSlicesMaxTokens ? M : (int64_t)kRtSlicesMaxTokens);
+  return 256 + (size_t)(tiles > slices ? tiles : slices) * (size_t)E * sizeof(float);
 }
 
 extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, const void* gate_w, int64_t M, int64_t H,
@@ -513,13 +514,13 @@ extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, c
   if (M == 0) return B200FP4_STATUS_SUCCESS;
   if (!hidden || !gate_w || !topk_weights || !topk_ids || !aligned(hidden, 16) || !aligned(gate_w, 16))
     return B200FP4_STATUS_INVALID_VALUE;
-  if (!workspace || workspace_bytes < b200fp4_moe_router_workspace_bytes(M, E) || !aligned(workspace, 4))
-    return B200FP4_STATUS_ALLOC_FAILED;
+  const RouterPath path = router_path(M, H, E);
+  const size_t need = path == RouterPath::kClusters ? 256 : b200fp4_moe_router_workspace_bytes(M, E);      // clusters keep their logits on chip
+  if (!workspace || workspace_bytes < need || !aligned(workspace, 4)) return B200FP4_STATUS_ALLOC_FAILED;
   if (M > (int64_t)65535 * 128) return B200FP4_STATUS_NOT_SUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   int* status = static_cast<int*>(workspace);
   float* parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
-  const RouterPath path = router_path(M, H, E);
   const bool bf = dtype == B200FP4_DTYPE_BF16;
   int splits;
   if (path == RouterPath::kClusters) {

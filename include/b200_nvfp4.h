@@ -413,8 +413,8 @@ B200FP4_API int b200fp4_moe_prefill(const void* hidden, int dtype, const float* 
  *   hidden [M, H] and gate_w [E, H] of `dtype` (BF16 or F16), hidden rows ld_h elements apart; logits accumulate in f32
  *   topk_weights [M, topk] f32 = exp(l - max) / sum over the selected experts (renormalize != 0) or over all experts
  *   topk_ids [M, topk] i32 in decreasing order of logit; equal logits go to the lower expert id
- *   workspace b200fp4_moe_router_workspace_bytes(M, E) bytes: 256 whose first int is a status word, then the f32 logits in slices
- *             over H.  The word is 0 unless one of the bounded waits of the projection of more than 64 tokens ran out (31: a
+ *   workspace b200fp4_moe_router_workspace_bytes(M, E) bytes (up to 128 tokens also enough for fewer): 256 whose first int is a status
+ *             word, then the f32 logits in slices over H.  The word is 0 unless a bounded wait of the projection in tiles ran out (31: a
  *             stage was not freed, 32: its operands did not land, 33: the accumulator was not finished); weights and ids are
  *             then made from whatever logits there are -- ids still in [0, E) -- and not to be trusted: read it after
  *             synchronising when diagnosing (router.last_router_status).  topk <= 32, E <= 1024. */

@@ -87,6 +87,27 @@ def test_router_path(M, H, E, launches):
     assert torch.equal(ids, torch.arange(8, device="cuda", dtype=torch.int32).expand(M, 8)) and bool((tw == 0.125).all())
 
 
+@pytest.mark.parametrize("E", [1, 32, 128, 512, 513, 1000])
+def test_router_workspace_of_a_larger_batch(E):
+    # a program that sizes its workspace for its largest decode batch may call with fewer tokens, whichever path these take
+    from dgx_vllm_b200 import _lib
+    from dgx_vllm_b200.router import moe_router
+    L, most, topk = _lib.lib(), 64, min(E, 8)
+    sizes = [L.b200fp4_moe_router_workspace_bytes(m, E) for m in range(1, 129)]
+    assert sizes == sorted(sizes)
+    nbytes, st = sizes[most - 1], torch.cuda.current_stream().cuda_stream
+    for M, H in [(8, 1536), (8, 12800), (16, 12800), (32, 4096), (64, 2048)]:
+        g = torch.Generator(device="cuda").manual_seed(M + H)
+        x, gate = (torch.randn(n, H, generator=g, device="cuda").mul_(H ** -0.25).bfloat16() for n in (M, E))
+        ws = torch.full((nbytes + 256,), 77, dtype=torch.uint8, device="cuda")
+        tw, ids = torch.empty(M, topk, device="cuda"), torch.empty(M, topk, dtype=torch.int32, device="cuda")
+        _lib.check(L.b200fp4_moe_router(x.data_ptr(), H, _lib.BF16, gate.data_ptr(), M, H, E, topk, 1, tw.data_ptr(), ids.data_ptr(),
+                                        ws.data_ptr(), nbytes, st), "router")
+        want = moe_router(x, gate, topk)
+        assert torch.equal(tw, want[0]) and torch.equal(ids, want[1])
+        assert bool((ws[nbytes:] == 77).all())
+
+
 @pytest.mark.parametrize("M,K", [(1, 16), (31, 48), (33, 512), (97, 528), (129, 80), (200, 2064)])
 @pytest.mark.parametrize("swizzled", [True, False])
 @pytest.mark.parametrize("offset", [0, 8])            # elements: rows on 32-byte and only on 16-byte boundaries
