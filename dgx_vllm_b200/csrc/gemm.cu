@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
   const int first_tile = blockIdx.x / kSplit, tile_stride = gridDim.x / kSplit;
   const int ks_begin = p.k_stages * rank / kSplit, ks_end = p.k_stages * (rank + 1) / kSplit;
   // The weights of a linear layer do not depend on the quantizer that runs just before: the first ring of B and its scales is
-  // requested while that kernel still runs (N=14336, K=4096: M=1 14.4 -> 13.2 us, M=32 13.4 -> 12.1, M=128 13.4 -> 12.7).
+  // requested while that kernel still runs (N=14336, K=4096: M=32 13.4 -> 12.1 us, M=128 13.4 -> 12.7).
   int early = 0;
   if (!kGrouped && p.early_b && (warp == 0 || warp == kWarpSf) && first_tile < p.m_tiles * p.n_tiles) {
     const bool elected = elect_one();
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(gemm_threads(kGrouped), 1)
     // With long K the epilogue hides behind the next tile either way; with short K (the grouped down
     // projection: 8 MMAs per tile) the kernel is bound by how fast a tile can be drained and stored, and with SiLU and
     // quantization by the epilogue's arithmetic: about 3000 instructions per row and 64 columns keep eight warps busy for
-    // twice the 6600 cycles of the main loop (gate_up of 81,920 rows: 182 us with eight epilogue warps).
+    // longer than the tile's stages take (gate_up of 81,920 rows: 182 us with eight epilogue warps).
     const int quarter = warp & 3;                 // tensor-memory lanes [32*quarter, +32) belong to this warp
     constexpr int CH = BN / 32 / kEpi;            // 32-column chunks per warp
     const int grp = warp < 6 ? 0 : (warp - 6) >> 2;
@@ -935,6 +935,13 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int 
 // M=4096 (TMA issues one request per box row, so narrower rows double and quadruple the requests).
 constexpr int kStageKb = 4;
 
+// Clusters of four CTAs of the kernel that splits K, which run at once
+int resident_splits_of_four() {
+  static ResidentClusters counts[64];
+  return resident_clusters_of(counts, nvfp4_gemm_kernel<128, kStageKb, false, false, 4>, 4, gemm_threads(false),
+                              (size_t)Cfg<128, kStageKb, out_stage_bytes<128, false, false, 4>()>::kSmemBytes);
+}
+
 // Tile of the dense GEMM: 128- or 256-wide on single CTAs (one per SM), 256 x 256 on CTA pairs, and for few tiles the split of K
 // over clusters of two or four.  Each takes whole rounds over the SMs, so the choice is the least of
 //   fixed + rounds x (stages x time per 256-k stage + tile)
@@ -960,7 +967,7 @@ void pick_dense_tile(int64_t M, int64_t N, int64_t stages, bool f32, int& bn, in
   split = 1;
   if (bn == 128 && stages >= 8) {
     const int64_t tiles = m128 * n128;
-    if (tiles * 4 <= sms && tiles <= resident_clusters(4)) split = 4;
+    if (tiles * 4 <= sms && tiles <= resident_splits_of_four()) split = 4;
     else if (tiles * 2 <= sms && stages >= (tiles * 3 <= sms ? 16 : 22)) split = 2;
   }
 }

@@ -1,10 +1,10 @@
 // Dense block-scaled NVFP4 GEMM on CTA pairs: tcgen05.mma.cta_group::2, one 256 (M) x 256 (N) tile per pair of SMs.
 //
-// Why pairs: a single CTA's MMA (128 x 256 x 64) reads 4 KiB of A and 8 KiB of B from shared memory and issues at about
-// 206 cycles per MMA.  In a pair each CTA holds its own 128 rows of A and HALF of the B tile (128 of the 256 rows): 8 KiB
-// per CTA per MMA for the same work per SM, and a third fewer operand bytes from L2.  Measured with the same stage loop in
-// both: M=4096, N=14336, K=4096 takes about 200 k cycles against 223 k for the single-CTA kernel (123 us against 129 us: the SM
-// clock settles near 1.6-1.7 GHz under either); with the shorter loop below 189 k cycles, 113 us.
+// Why pairs: a stage of a single CTA (256 k of a 128 x 256 tile) brings 54 KiB into its SM (A 16, B 32, scales 6), and an SM takes in
+// about 57 bytes per cycle: some 900 cycles for four MMAs that need 128 each.  In a pair each CTA holds its own 128 rows of A and HALF of
+// the B tile (128 of the 256 rows): 38 KiB a stage for the same work per SM.  Measured with the same stage loop in both: M=4096,
+// N=14336, K=4096 takes about 200 k cycles against 223 k for the single-CTA kernel (123 us against 129 us: the SM clock settles near
+// 1.6-1.7 GHz under either); with the shorter loop below 189 k cycles, 113 us.
 //
 // Roles per CTA (23 warps): warp 0 loads operands, warp 1 issues the MMAs (leader CTA only) and owns tensor memory,
 // warps 2-5, 10-13 and 15-22 drain and store the CTA's 128 accumulator rows (four warps per tensor-memory lane quarter, 64
@@ -21,8 +21,8 @@
 //     three 16-column tcgen05.st and arrive on the leader's `full` (remotely from the peer);
 //   * arrivals on a barrier of the other CTA are RELAXED at cluster scope: with release semantics each one stalled the
 //     arriving warp for about 1100 cycles and the whole kernel ran at one stage per 2000 cycles (242 us).
-// The MMA thread waits on one barrier per stage and looks at the next one before a stage's last MMA (M=4096, quantizer
-// included, under the power cap: 149 us with two barriers per stage and descriptors built per MMA, 139 us so).
+// The MMA warp waits on one barrier per stage, all lanes together, and one elected lane issues (M=4096, quantizer included, under the
+// power cap: 149 us with two barriers per stage and descriptors built per MMA, 134 to 136 us so).
 // No copy uses cluster multicast.  Every wait is bounded and reports through the status word; the pair leaves through a
 // cluster barrier so neither CTA frees tensor memory or exits while the other may still signal it.
 #include "sm100_ptx.cuh"

@@ -7,8 +7,8 @@
 //   * the activations are quantized by the kernel itself, each CTA its own part of K for all tokens, straight into the operand's
 //     shared-memory layout while the first weight tiles are on their way: one launch instead of two, no trip of codes and scales
 //     through memory.  The arithmetic is the quantizer's (quant.cuh), the bytes are the same;
-//   * K is split over clusters of up to eight CTAs, whatever number fits the SMs; the partial sums of a token meet in one CTA of the
-//     cluster through distributed shared memory and are added in the order of K.
+//   * K is split over clusters of up to eight CTAs, whatever number fits the SMs; the partial sums of a token go through distributed
+//     shared memory, each of its four 32-column pieces to another CTA of the cluster, and are added there in the order of K.
 // The GEMM on codes that are already there (cutlass_scaled_fp4_mm) takes the same kernel where that is the faster one, with the quantization
 // replaced by a copy.
 // What bounds it: the chain of copy, quantization, scales, MMA, exchange and store where the weight is small, HBM where it is large.
@@ -392,13 +392,13 @@ int launch_small_t(const CUtensorMap& mw, const SmallParams& p, unsigned grid, s
   return finish_launch(1);
 }
 
-}  // namespace
-
+// Clusters of k CTAs (2 to 8) that run at once
 int resident_clusters(int k) {
   static ResidentClusters counts[kMaxSplit + 1][64];
-  if (k < 2 || k > kMaxSplit) return 0;
   return resident_clusters_of(counts[k], nvfp4_small_kernel<__nv_bfloat16, false>, k, kThreads, kSmemMost);
 }
+
+}  // namespace
 
 SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use) {
   SmallPlan s = {};

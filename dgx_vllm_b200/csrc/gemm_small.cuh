@@ -9,9 +9,6 @@ namespace b200fp4 {
 
 constexpr int64_t kSmallMaxM = 64;
 
-// Clusters of k CTAs (2 to 8) that run at once on this device, one CTA to an SM: a cluster lies within a GPC.
-int resident_clusters(int k);
-
 struct SmallPlan {
   bool ok;                // false: the general kernel's case
   int split, ring, stages, m_pad;

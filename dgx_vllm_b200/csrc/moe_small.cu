@@ -9,8 +9,8 @@
 //     activations are even converted -- the down projection's do not depend on anything;
 //   * SiLU(gate)*up goes to the other blocks of the cluster through distributed shared memory and a cluster barrier instead of memory,
 //     fence and counter.
-// Arithmetic as in the general kernel: E2M1 x E4M3 products exact in f16, mma.sp with f32 sums (K-slices added in order), f16 between the
-// projections, f32 rows out.  The token's value stands in all eight columns of an mma; one is read.
+// Arithmetic as in the general kernel: E2M1 x E4M3 products exact in f16, mma.sp with f32 sums, f16 between the projections, f32 rows out.  The
+// K-slices of a column are added in a fixed order: every fourth by one of four lanes, then those four sums by a butterfly.  The token's value stands in all eight columns of an mma; one is read.
 #include "moe_small.cuh"
 
 #include <math.h>
