@@ -129,7 +129,8 @@ def test_quantizer_tile_edges(M, K, swizzled, offset):
 
 
 @pytest.mark.parametrize("E,H,I,M,topk", [
-    (4, 256, 128, 1, 1),          # smallest: one item, K = 128 on the down side; two warps per item, down turns of two
+    (4, 256, 128, 1, 1),          # smallest: one pair and that not local, on the path for few pairs
+    (1, 256, 128, 2, 1),          # smallest of the one-launch kernel: one item, K = 128 on the down side; two warps per item, down turns of two
     (8, 512, 512, 3, 4),          # four warps per item
     (16, 256, 256, 32, 8),        # 256 pairs: last size of the small plan; several passes per expert
     (16, 256, 256, 33, 8),        # 264 pairs
@@ -146,7 +147,7 @@ def test_quantizer_tile_edges(M, K, swizzled, offset):
 ])
 def test_fused_moe_block_shapes(E, H, I, M, topk):
     import synth
-    from dgx_vllm_b200 import sparse_fp4_v7 as sp7
+    from dgx_vllm_b200 import _lib, sparse_fp4_v7 as sp7
     from util import expert_fetch, gpu_quantize_fn, rel_err
     keys = ("comp_T", "meta_T", "scale_T", "g_scales")
     w13 = synth.make_sparse_experts(E, 2 * I, H, 1, "cuda", gpu_quantize_fn)
@@ -155,7 +156,9 @@ def test_fused_moe_block_shapes(E, H, I, M, topk):
     ids[0, 0] = -1                                    # not local
     hidden = synth.make_hidden(M, H, 4, "cuda")
     args = (hidden, tw, ids, None, *[w13[k] for k in keys], *[w2[k] for k in keys], I, False)
+    n0 = _lib.lib().b200fp4_launch_count()
     out = sp7.fused_sparse_moe_v7(*args)
+    assert _lib.lib().b200fp4_launch_count() == n0 + (3 if 2 * M * topk > E else 2)      # few pairs have no plan
     again = sp7.fused_sparse_moe_v7(*args)
     assert sp7.last_moe_status() == 0
     assert torch.equal(out, again)
@@ -440,6 +443,44 @@ def test_fused_moe_few_pairs_of_one_rank(M, ranks, launches):
     local = ids if emap is None else emap[ids.long()]
     ref = oracle.fused_sparse_moe_by_expert(hidden.float().cpu().numpy(), tw.cpu().numpy(), local.cpu().numpy(), expert_fetch(w13, w2), I)
     assert np.abs(to_np(out) - ref).max() <= 1e-2 * max(np.abs(ref).max(), 1e-6)
+
+
+@pytest.mark.parametrize("M,topk,E,ranks,H,I,dtype", [
+    (1, 4, 16, 1, 5760, 128, torch.bfloat16),      # the widest row that the layer takes: many threads bring in a second 16-byte piece of it
+    (2, 3, 32, 2, 4224, 256, torch.float16),       # a few threads have a second one
+    (3, 2, 64, 4, 256, 1024, torch.bfloat16),      # two pairs in four elsewhere, K short in gate_up and long in down
+])
+def test_fused_moe_few_pairs_in_records(M, topk, E, ranks, H, I, dtype):
+    # rows, ids and weights apart by the length of a dispatch record; the same result as from tensors of their own
+    import synth
+    from dgx_vllm_b200 import _lib, sparse_fp4_v7 as sp7
+    from dgx_vllm_b200._torch_util import workspace
+    from dgx_vllm_b200.moe_ep import expert_map_for_rank
+    from util import expert_fetch, gpu_quantize_fn, rel_err
+    L, keys, here = _lib.lib(), ("comp_T", "meta_T", "scale_T", "g_scales"), E // ranks
+    w13 = synth.make_sparse_experts(here, 2 * I, H, 1, "cuda", gpu_quantize_fn)
+    w2 = synth.make_sparse_experts(here, H, I, 2, "cuda", gpu_quantize_fn)
+    tw, ids = synth.make_routing(M, E, topk, 3, "cuda")
+    ids[0, 0] = (ranks - 1) * here                  # at least one pair is this rank's
+    hidden, emap = synth.make_hidden(M, H, 4, "cuda", dtype), expert_map_for_rank(E, ranks, ranks - 1, "cuda")
+    code, R = (_lib.BF16 if dtype == torch.bfloat16 else _lib.F16), L.b200fp4_ep_record_bytes(H, topk)
+    rec = torch.empty(M * R, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(L.b200fp4_ep_pack(hidden.data_ptr(), ids.data_ptr(), tw.data_ptr(), M, H, topk, 1, rec.data_ptr(), st), "pack")
+    out = torch.full((M, H), 7.0, dtype=dtype, device="cuda")
+    ws = workspace(torch.device("cuda", torch.cuda.current_device()), L.b200fp4_fused_moe_workspace_bytes(M, topk, H, I, here))
+    n0 = L.b200fp4_launch_count()
+    _lib.check(L.b200fp4_fused_sparse_moe_records(
+        rec.data_ptr(), R, code, emap.data_ptr(), E, *[w13[k].data_ptr() for k in keys], w13["scale_T"].shape[1],
+        *[w2[k].data_ptr() for k in keys], w2["scale_T"].shape[1], out.data_ptr(), code, M, topk, H, I, here, _lib.SPARSE_META_ORDERED,
+        ws.data_ptr(), ws.numel(), st), "records")
+    assert L.b200fp4_launch_count() == n0 + 2
+    want = sp7.fused_sparse_moe_v7(hidden, tw, ids, emap, *[w13[k] for k in keys], *[w2[k] for k in keys], I, False)
+    assert L.b200fp4_launch_count() == n0 + 4 and sp7.last_moe_status() == 0
+    assert torch.equal(out, want)
+    ref = oracle.fused_sparse_moe_by_expert(hidden.float().cpu().numpy(), tw.cpu().numpy(), emap[ids.long()].cpu().numpy(),
+                                            expert_fetch(w13, w2), I)
+    assert rel_err(to_np(out), ref) < 1e-2
 
 
 @pytest.mark.parametrize("M,N,K,launches", [
