@@ -383,10 +383,12 @@ __global__ void __launch_bounds__(kRcThreads, 1)
 // ------------------------------------------------------------------------------------------ host
 
 // Which way a call goes.  One launch of clusters saves a launch, but only 8 or 16 SMs read the gate for eight tokens, and those without experts
-// none of it (us, slices and selection in two launches / clusters, back to back and from a graph):
-//   M=8: 32 experts H=2048 3.2 / 3.7, 3.4 / 4.0, H=12800 5.8 / 8.4, 5.2 / 8.9   64, 4096 4.4 / 4.6, 3.9 / 4.9   128, 6144 5.8 / 5.5, 5.5 / 5.8
-//   128, 9216 6.2 / 6.9, 6.0 / 7.3   512, 6144 8.6 / 8.8, 8.8 / 9.2   512, 9216 9.7 / 11.4, 9.8 / 11.8   1000, 4096 10.0 / 11.9, 9.9 / 12.5
-//   M=16: 128, 12800 7.3 / 8.8, 7.2 / 9.0   512, 6144 9.4 / 8.7, 9.7 / 9.5   512, 9216 10.8 / 11.4, 10.8 / 12.0
+// none of it.  In a graph only the GPU's time counts (us, clusters / slices and selection):
+//   M=8: 32 experts H=2048 3.9 / 3.3, H=12800 8.8 / 5.0   64, 3072 4.5 / 3.8   128, 7168 6.3 / 5.3   512, 7168 9.8 / 7.4
+//   M=16: 32, 2048 3.9 / 3.6   64, 3072 4.5 / 4.2   128, 7168 6.4 / 5.7   512, 9216 11.7 / 9.0
+// Called one by one, two launches take the host about 7 us, whatever they are, one 4.4: clusters as far as they take less than that (from Python):
+//   M=8: 32, 2048 4.4 / 7.3, H=9216 6.6 / 7.2, H=10240 6.9 / 7.2, H=12800 8.2 / 7.1   128, 7168 5.8 / 7.3, H=10240 7.0 / 7.0, H=12800 8.3 / 7.0
+//   M=16: 64, 9216 6.9 / 6.8, H=10240 7.1 / 6.9, H=12800 8.4 / 6.9   512 (M=8), 7168 9.3 / 7.4, H=9216 11.1 / 8.0
 // From 17 tokens on clusters are the faster ones up to 512 experts; the tiles read the whole gate once for 128 tokens, the slices once for 8 to 32
 // (slices / tiles; M=17: 1000 experts H=2048 10.9 / 13.1, H=4096 13.3 / 14.1, H=7168 18.5 / 15.8; M=64, H=4096 19.4 / 15.2; M=8, H=12800 20.8 / 19.4).
 constexpr int kRtClusterMaxTokens = 64;
@@ -395,10 +397,11 @@ constexpr int kRtMaxSplits = 8;
 
 enum class RouterPath { kClusters, kSlices, kTiles };
 
-RouterPath router_path(int64_t M, int64_t H, int64_t E) {
+RouterPath router_path(int64_t M, int64_t H, int64_t E, cudaStream_t st) {
   const int64_t gate = E * H;
   if (M <= 16) {
-    if (E <= 128) return H > (E <= 32 ? 1536 : (E <= 64 ? 2560 : 6144)) ? RouterPath::kSlices : RouterPath::kClusters;
+    if (E <= 128)
+      return H > 10240 || (H > (E <= 32 ? 1536 : E <= 64 ? 2560 : 6144) && stream_capturing(st)) ? RouterPath::kSlices : RouterPath::kClusters;
     if (gate <= (M <= 8 ? 3200000 : 3900000)) return RouterPath::kClusters;
     return E <= 512 || gate <= (M <= 8 ? 9300000 : 7500000) ? RouterPath::kSlices : RouterPath::kTiles;
   }
@@ -514,11 +517,11 @@ extern "C" int b200fp4_moe_router(const void* hidden, int64_t ld_h, int dtype, c
   if (M == 0) return B200FP4_STATUS_SUCCESS;
   if (!hidden || !gate_w || !topk_weights || !topk_ids || !aligned(hidden, 16) || !aligned(gate_w, 16))
     return B200FP4_STATUS_INVALID_VALUE;
-  const RouterPath path = router_path(M, H, E);
+  cudaStream_t st = (cudaStream_t)stream;
+  const RouterPath path = router_path(M, H, E, st);
   const size_t need = path == RouterPath::kClusters ? 256 : b200fp4_moe_router_workspace_bytes(M, E);      // clusters keep their logits on chip
   if (!workspace || workspace_bytes < need || !aligned(workspace, 4)) return B200FP4_STATUS_ALLOC_FAILED;
   if (M > (int64_t)65535 * 128) return B200FP4_STATUS_NOT_SUPPORTED;
-  cudaStream_t st = (cudaStream_t)stream;
   int* status = static_cast<int*>(workspace);
   float* parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
   const bool bf = dtype == B200FP4_DTYPE_BF16;

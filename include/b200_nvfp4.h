@@ -411,6 +411,7 @@ B200FP4_API int b200fp4_moe_prefill(const void* hidden, int dtype, const float* 
  * sparse_fp4_kernel/bench_moe_layer_e2e.py:230-236, softmax(logits).topk(k), weights / their sum); here the outputs are
  * the device tensors b200fp4_fused_sparse_moe and b200fp4_ep_pack take, so routing never leaves the GPU.
  *   hidden [M, H] and gate_w [E, H] of `dtype` (BF16 or F16), hidden rows ld_h elements apart; logits accumulate in f32
+ *   (in an order that goes by sizes and, up to 16 tokens, by whether the call is captured)
  *   topk_weights [M, topk] f32 = exp(l - max) / sum over the selected experts (renormalize != 0) or over all experts
  *   topk_ids [M, topk] i32 in decreasing order of logit; equal logits go to the lower expert id
  *   workspace b200fp4_moe_router_workspace_bytes(M, E) bytes (up to 128 tokens also enough for fewer): 256 whose first int is a status

@@ -60,7 +60,12 @@ def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
     wide = torch.randn(M, H + 8, generator=g, device="cuda").to(dtype)
     hidden = wide[:, :H]                              # strided rows
     gate = (torch.randn(E, H, generator=g, device="cuda") / H ** 0.5).to(dtype)
-    tw, ids = moe_router(hidden, gate, topk, renormalize=renorm)
+    results = [moe_router(hidden, gate, topk, renormalize=renorm)]
+    graph = torch.cuda.CUDAGraph()                    # takes the K-slices at more sizes
+    with torch.cuda.graph(graph):
+        results.append(moe_router(hidden, gate, topk, renormalize=renorm))
+    graph.replay()
+    torch.cuda.synchronize()
     logits = hidden.double() @ gate.double().t()
     w, ref_ids = torch.softmax(logits, dim=-1).topk(topk, dim=-1)
     if renorm:
@@ -68,23 +73,32 @@ def test_router_kernel_edges(M, H, E, topk, dtype, renorm):
     srt = torch.cat((logits, torch.full((M, 1), -1e9, device="cuda", dtype=torch.double)), 1).sort(dim=-1, descending=True).values
     clear = (srt[:, :topk] - srt[:, 1:topk + 1]).min(dim=-1).values > 2e-5
     assert clear.float().mean() > 0.8
-    assert torch.equal(ids[clear].long(), ref_ids[clear])
-    assert ((tw[clear].double() - w[clear]).abs() / w[clear]).max() < 1e-4
+    for tw, ids in results:
+        assert torch.equal(ids[clear].long(), ref_ids[clear])
+        assert ((tw[clear].double() - w[clear]).abs() / w[clear]).max() < 1e-4
 
 
-@pytest.mark.parametrize("M,H,E,launches", [
-    (8, 1536, 32, 1), (8, 2048, 32, 2), (16, 2560, 64, 1), (16, 4096, 64, 2), (8, 6144, 128, 1), (8, 7168, 128, 2), (17, 12800, 128, 1),
-    (8, 6144, 512, 1), (8, 9216, 512, 2), (16, 7168, 512, 1), (32, 9216, 512, 1), (4, 3072, 1000, 1), (4, 4096, 1000, 2), (17, 2048, 1000, 2),
+@pytest.mark.parametrize("M,H,E,launches,captured", [
+    (8, 1536, 32, 1, 1), (8, 2048, 32, 1, 2), (8, 10240, 32, 1, 2), (8, 10248, 32, 2, 2), (16, 2560, 64, 1, 1), (16, 4096, 64, 1, 2),
+    (8, 6144, 128, 1, 1), (8, 7168, 128, 1, 2), (16, 12800, 128, 2, 2), (17, 12800, 128, 1, 1), (8, 6144, 512, 1, 1), (8, 9216, 512, 2, 2),
+    (16, 7168, 512, 1, 1), (32, 9216, 512, 1, 1), (4, 3072, 1000, 1, 1), (4, 4096, 1000, 2, 2), (17, 2048, 1000, 2, 2),
 ])
-def test_router_path(M, H, E, launches):
-    # clusters in one launch, or two launches that have every SM read its share of a large gate
+def test_router_path(M, H, E, launches, captured):
+    # clusters in one launch, or two launches that have every SM read its share of a large gate: the second launch costs little in a graph only
     from dgx_vllm_b200 import _lib
     from dgx_vllm_b200.router import moe_router
     x, gate = torch.zeros(M, H, device="cuda", dtype=torch.bfloat16), torch.zeros(E, H, device="cuda", dtype=torch.bfloat16)
     n0 = _lib.lib().b200fp4_launch_count()
-    tw, ids = moe_router(x, gate, 8)
+    results = [moe_router(x, gate, 8)]
     assert _lib.lib().b200fp4_launch_count() == n0 + launches
-    assert torch.equal(ids, torch.arange(8, device="cuda", dtype=torch.int32).expand(M, 8)) and bool((tw == 0.125).all())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        results.append(moe_router(x, gate, 8))
+    assert _lib.lib().b200fp4_launch_count() == n0 + launches + captured
+    graph.replay()
+    torch.cuda.synchronize()
+    for tw, ids in results:
+        assert torch.equal(ids, torch.arange(8, device="cuda", dtype=torch.int32).expand(M, 8)) and bool((tw == 0.125).all())
 
 
 @pytest.mark.parametrize("E", [1, 32, 128, 512, 513, 1000])
