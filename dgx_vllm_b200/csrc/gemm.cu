@@ -1102,7 +1102,8 @@ extern "C" int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, con
     rc = dense_gemm_check(codes, w_codes, sf, w_sf, alpha, out, out_dtype, M, N, K, tile_n, gemm_ws, gemm_bytes);
   if (rc != B200FP4_STATUS_SUCCESS) return rc;
   if (b200fp4_has_hardware_acceleration() != 1) return B200FP4_STATUS_ARCH_MISMATCH;
-  const SmallPlan small = small_gemm_plan(M, N, K, SmallUse::kLinear);
+  const bool captured = M > 16 && M <= kSmallMaxM && stream_capturing((cudaStream_t)stream);      // up to 16 tokens the plan is the same
+  const SmallPlan small = small_gemm_plan(M, N, K, captured ? SmallUse::kLinearInGraph : SmallUse::kLinear);
   if (tile_n == 0 && small.ok) {
     // few tokens: quantized inside the GEMM
     CUtensorMap mw;

@@ -413,20 +413,35 @@ SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use) {
   if (own > kMaxStages) return s;
   // Every CTA brings in its part of K for all tokens and sends its 128 columns out token by token, some 70 cycles a token, where the general path
   // quantizes once and stores tiles; and clusters that nearly fill the chip leave the next launch no room to start in.  So the number of tokens
-  // up to which this kernel is the faster one falls with the stages a CTA owns and with the CTAs.  Linear, us (quantizer and general kernel / so):
-  // N=4096 K=512 M=32 5.8 / 5.3, M=48 6.0 / 6.2; N=1024 K=2048 M=32 6.6 / 5.4, M=64 7.0 / 7.1; N=4096 K=2048 M=24 6.8 / 6.6, M=32 6.9 / 7.5;
-  // N=9600 K=1024 M=24 6.4 / 6.4, M=32 6.4 / 6.9.
+  // up to which this kernel is the faster one falls with the stages a CTA owns and with the CTAs.  Called one by one, the two launches of the
+  // general path take the host at least 6.5 us, so that it reaches further there than in a graph.  Linear, us (quantizer and general kernel /
+  // so), from Python and from a graph:
+  //   N=K=512 M=45 6.6 / 5.7, 6.5 / 7.0, M=64 6.5 / 6.4, 6.5 / 7.8           N=4096 K=512 M=48 6.7 / 6.0, 6.5 / 7.2, M=64 6.5 / 6.7, 6.7 / 8.0
+  //   N=2048 K=1536 M=33 7.1 / 6.4, 7.9 / 7.3   N=1536 K=2048 M=40 7.1 / 6.5, 7.7 / 7.4   N=K=2048 M=48 7.1 / 7.6, 7.7 / 8.5
+  //   N=1624 K=2240 M=54 8.2 / 8.0, 9.4 / 8.8   N=1664 K=3072 M=48 - / 7.6, 8.2 / 8.3   N=3200 K=1024 M=52 - / 7.2, 7.4 / 8.0
+  //   N=4096 K=2048 M=25 6.9 / 7.2, 7.9 / 7.9   N=9600 K=1024 M=32 6.6 / 6.7, 7.4 / 7.8
+  //   N=14336 K=512 M=25 6.6 / 5.5, 6.8 / 6.4, M=40 6.5 / 6.3, 6.7 / 7.1, M=64 6.5 / 7.2, 6.8 / 8.0
   const int64_t ctas = tiles * split;
-  if (M <= 16 ? M * own > 256 : ctas <= 64 ? M * own > 128 || (stages <= 4 && M > 44) : M * own > 96 || M > (ctas > 110 ? 24 : 32)) return s;
+  const bool captured = use == SmallUse::kLinearInGraph || use == SmallUse::kCodesInGraph;
+  if (M <= 16) {
+    if (M * own > 256) return s;
+  } else if (ctas <= 64) {
+    if (M * own > 128 || (stages <= 4 && M > (captured ? 44 : 60))) return s;
+  } else if (split == 1) {
+    if (M * own > (captured ? 96 : 112) || M > (captured ? 32 : 48)) return s;
+  } else if (M * own > 112 || M > (ctas > 110 ? 24 : captured && stages <= 4 ? 44 : 56)) {
+    return s;
+  }
   // On codes that are there already no launch is saved.  In a graph the longer way to the first MMA is not hidden behind the kernel before, so
   // that only long K pays.  GEMM, us eager and from a graph (general kernel / so): M=8 N=512 K=1024 4.1 / 3.6, 4.6 / 5.2; M=24 N=512 K=1536
   // 4.7 / 4.2, 5.2 / 5.8; M=8 N=4096 K=1024 4.1 / 4.8, 4.7 / 5.4; M=32 N=2048 K=512 3.5 / 4.4, 4.1 / 5.7; M=8 N=14336 K=4096 12.2 / 9.5, 12.0 / 10.6.
-  const bool pays = use == SmallUse::kLinear         ? true
-                    : use == SmallUse::kCodesInGraph ? M <= 8 && stages >= 8 && own >= 3
-                    : stages < 4                     ? M <= 4
-                    : split == 1                     ? M <= 8 || own >= 16
-                    : ctas <= 64                     ? M <= (stages < 6 ? 16 : 24)
-                                                     : M <= 8 && own >= 3;
+  const bool linear = use == SmallUse::kLinear || use == SmallUse::kLinearInGraph;
+  const bool pays = linear         ? true
+                    : captured     ? M <= 8 && stages >= 8 && own >= 3
+                    : stages < 4   ? M <= 4
+                    : split == 1   ? M <= 8 || own >= 16
+                    : ctas <= 64   ? M <= (stages < 6 ? 16 : 24)
+                                   : M <= 8 && own >= 3;
   if (!pays) return s;
   int ring = own < kRingMost ? own : kRingMost;
   while (ring > 0 && small_layout(ring, own, m_pad, (int)M, split).bytes + 1024 > kSmemMost) --ring;

@@ -14,7 +14,7 @@ struct SmallPlan {
   int split, ring, stages, m_pad;
   size_t smem;
 };
-enum class SmallUse { kLinear, kCodes, kCodesInGraph };      // quantizes its operand; given codes, launched or captured
+enum class SmallUse { kLinear, kLinearInGraph, kCodes, kCodesInGraph };      // quantizes its operand, given codes; launched, captured
 SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use);
 
 // gs given: x is [M, K] bf16 / f16 (rows ldx elements apart), quantized in the kernel; gs null: x are packed codes [M, K/2] and x_sf

@@ -154,8 +154,9 @@ B200FP4_API int b200fp4_gemm_nvfp4(const void* a_codes, const void* b_codes, con
  * cutlass_scaled_fp4_mm: vllm/model_executor/layers/quantization/utils/nvfp4_utils.py, the call pair the reference's
  * emulation replaces at fix_nvfp4_emulation_backend.py:60-102); one host call keeps the two launches a few
  * microseconds apart.  x [M, K] bf16/f16 with row stride ldx; x_global_scale, alpha device pointers as above.
- * Up to 64 tokens, as far as quantizing them in every block pays, it is one kernel; b200fp4_gemm_nvfp4 on their codes may take
- * another one, eager or captured: the products are the same, the f32 sums over K may be grouped otherwise.
+ * Up to 64 tokens, as far as quantizing them in every block pays, it is one kernel (for more tokens launched than captured);
+ * b200fp4_gemm_nvfp4 on their codes may take another one, eager or captured: the products are the same, the f32 sums over K may be
+ * grouped otherwise.
  * workspace: b200fp4_linear_workspace_bytes(M, N, K) bytes, 256-byte aligned; its first int is the GEMM's status word. */
 B200FP4_API size_t b200fp4_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 B200FP4_API int b200fp4_linear_nvfp4(const void* x, int x_dtype, int64_t ldx, const float* x_global_scale,

@@ -497,12 +497,14 @@ def test_fused_moe_few_pairs_in_records(M, topk, E, ranks, H, I, dtype):
     assert rel_err(to_np(out), ref) < 1e-2
 
 
-@pytest.mark.parametrize("M,N,K,launches", [
-    (32, 512, 512, 1), (45, 512, 512, 2), (64, 1024, 4096, 1), (24, 4096, 2048, 1), (25, 4096, 2048, 2), (32, 2048, 1536, 1), (33, 2048, 1536, 2),
-    (24, 9600, 1024, 1), (25, 9600, 1024, 2), (16, 14336, 4096, 1), (17, 14336, 4096, 2),
+@pytest.mark.parametrize("M,N,K,launches,in_graph", [
+    (44, 512, 512, 1, 1), (45, 512, 512, 1, 2), (60, 512, 512, 1, 2), (61, 512, 512, 2, 2), (64, 1024, 4096, 1, 1), (24, 4096, 2048, 1, 1),
+    (25, 4096, 2048, 2, 2), (56, 2048, 1536, 1, 1), (57, 2048, 1536, 2, 2), (44, 3200, 1024, 1, 1), (45, 3200, 1024, 1, 2), (24, 9600, 1024, 1, 1),
+    (28, 9600, 1024, 1, 2), (29, 9600, 1024, 2, 2), (32, 14336, 512, 1, 1), (33, 14336, 512, 1, 2), (48, 14336, 512, 1, 2), (49, 14336, 512, 2, 2),
+    (16, 14336, 4096, 1, 1), (17, 14336, 4096, 2, 2),
 ])
-def test_linear_path(M, N, K, launches):
-    # one kernel for few tokens, quantizer and GEMM where those are the faster ones
+def test_linear_path(M, N, K, launches, in_graph):
+    # one kernel for few tokens, quantizer and GEMM where those are the faster ones: sooner in a graph, where a launch costs the host nothing
     from dgx_vllm_b200 import _lib, cutlass_scaled_fp4_mm, scaled_fp4_quant
     from dgx_vllm_b200.ops import last_gemm_status, nvfp4_linear
     x, gx, wc, ws, alpha = _linear_operands(M, N, K, M + N)
@@ -513,7 +515,9 @@ def test_linear_path(M, N, K, launches):
     assert torch.equal(out, cutlass_scaled_fp4_mm(xc, wc, xs, ws, alpha, torch.bfloat16))
     graph, captured = torch.cuda.CUDAGraph(), torch.zeros_like(out)
     with torch.cuda.graph(graph):
+        n0 = _lib.lib().b200fp4_launch_count()
         nvfp4_linear(x, gx, wc, ws, alpha, out=captured)
+        assert _lib.lib().b200fp4_launch_count() == n0 + in_graph
     for _ in range(2):
         graph.replay()
     torch.cuda.synchronize()
