@@ -434,10 +434,11 @@ SmallPlan small_gemm_plan(int64_t M, int64_t N, int64_t K, SmallUse use) {
   }
   // On codes that are there already no launch is saved.  In a graph the longer way to the first MMA is not hidden behind the kernel before, so
   // that only long K pays.  GEMM, us eager and from a graph (general kernel / so): M=8 N=512 K=1024 4.1 / 3.6, 4.6 / 5.2; M=24 N=512 K=1536
-  // 4.7 / 4.2, 5.2 / 5.8; M=8 N=4096 K=1024 4.1 / 4.8, 4.7 / 5.4; M=32 N=2048 K=512 3.5 / 4.4, 4.1 / 5.7; M=8 N=14336 K=4096 12.2 / 9.5, 12.0 / 10.6.
+  // 4.7 / 4.2, 5.2 / 5.8; M=8 N=4096 K=1024 4.1 / 4.8, 4.7 / 5.4; M=32 N=2048 K=512 3.5 / 4.4, 4.1 / 5.7; M=8 N=14336 K=4096 12.2 / 9.5, 12.0 / 10.6;
+  // M=16 of that 12.0 / 10.0, 12.3 / 11.2.
   const bool linear = use == SmallUse::kLinear || use == SmallUse::kLinearInGraph;
   const bool pays = linear         ? true
-                    : captured     ? M <= 8 && stages >= 8 && own >= 3
+                    : captured     ? M <= (own >= 16 ? 16 : 8) && stages >= 8 && own >= 3
                     : stages < 4   ? M <= 4
                     : split == 1   ? M <= 8 || own >= 16
                     : ctas <= 64   ? M <= (stages < 6 ? 16 : 24)
