@@ -259,7 +259,7 @@ int resident_pairs(int c) {
 // and of 512 experts on 8 ranks, 2048, 512: 10: 10.4 / 7.7, 8     40: 12.7 / 12.6, 8     100: 15.5 / 18.2, 4     140: 18.1 / 21.4, 4
 // A block's time here is its warps' steps (one of all 16 warps takes 0.566 us: instruction issue) and 5.7 us.  The general path spreads all steps
 // evenly over the SMs; a few pairs take their time in its chain of launches and loads.  Over 220 sizes, 1 to 8 ranks, the choice takes 1.2 % more
-// than the best of all, 15 % at most, and 8 % at most more than the general path.
+// than the best of all, 15 % at most, and 9 % at most more than the general path.
 // Only the number of pairs is known here.  Tokens that route alike stream an expert once each, where the general path reads it once for
 // eight: 12 tokens on the same ten of 512 experts 36.4 us here, 21.3 there, two by two alike 36.8 and 33.1, all different 37.6 and 40.9.
 int moe_small_cluster(int64_t P, double local, int64_t H, int64_t I) {
